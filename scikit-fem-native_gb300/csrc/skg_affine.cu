@@ -17,14 +17,17 @@
 //
 // Passes.
 //  1. element pass (thread per element): G (4x4) from coordinates and the
-//     coefficient, written to a scratch array.
-//  2. row pass (thread per CSR row, warp per group of up to 32 rows): the
-//     thread walks its row's incidence records (element, local row, column
-//     offsets) in ascending element order, evaluates row a of K_e on the fly
-//     and adds it into shared-memory accumulators of the row's slots; the
-//     warp then writes the group's slot range with coalesced stores.  Every
-//     slot is summed by one thread in a fixed order: results are bitwise
-//     reproducible, with no atomics.
+//     coefficient, then the packed upper triangle of the element matrix (10
+//     entries for P1, 55 for P2), staged in shared memory and stored as one
+//     bulk copy per tile.  Tiles with a nonsymmetric
+//     coefficient also leave the lower triangles.
+//  2. pair sums (skg_pairs.cuh): one thread per pair of DOFs sums its
+//     contributions in ascending element order and writes the values of
+//     (r, c) and (c, r).  Every value is written by one thread from sums in a
+//     fixed order: results are bitwise reproducible, with no atomics.
+// FP32-pair modes with a rule not exact on quadratics, FP32-pair P1, and
+// patterns without a pair plan keep G per element and evaluate the rows of
+// K_e in a row pass (k_rows_group; k_rows_global without row groups).
 //
 // Precision modes.
 //  SKG_FP64           FP64 end to end (FP64 pipe).
@@ -48,6 +51,7 @@
 
 #include "skg_common.cuh"
 #include "skg_df64.cuh"
+#include "skg_pairs.cuh"
 #include "skg_rows.cuh"
 
 namespace skg {
@@ -231,83 +235,7 @@ __global__ void __launch_bounds__(kElemBlock) k_elem_fp64(int64_t ne, const doub
     flush_stage(stage, G, e0, ne);
 }
 
-// P2 element matrices in FP64 (the FP64 mode on row-grouped patterns): the
-// element pass evaluates K_ab = sum G T over the supports once per entry,
-// the 55 entries of the upper triangle only when the element's coefficient
-// is symmetric to rounding (then K is), and writes the full 10 x 10 matrix; the row
-// pass only adds rows.  This halves the FP64 multiply-adds of the
-// row-by-row evaluation, whose rows a and b each recompute K_ab.
-constexpr int kKeBlock = 128;
-constexpr int kKeChunk = 25;  // entries staged per round; 4 rounds cover the 100
-
-__host__ __device__ constexpr int tri10(int a, int b) {  // packed upper triangle, a <= b
-    return a * 10 - a * (a - 1) / 2 + (b - a);
-}
-
-__global__ void __launch_bounds__(kKeBlock) k_elem_ke_fp64(int64_t ne, int64_t e_begin, int64_t e_end,
-                                                           const double *__restrict__ p, int64_t npts,
-                                                           const int32_t *__restrict__ t, int coef_kind,
-                                                           const double *__restrict__ coef,
-                                                           const double *__restrict__ Tg, double *__restrict__ Ke) {
-    __shared__ double Ts[10 * 10 * 4];
-    __shared__ double stage[kKeBlock * kKeChunk];
-    for (int i = threadIdx.x; i < 400; i += blockDim.x) Ts[i] = Tg[i];
-    __syncthreads();
-    const int64_t e0 = e_begin + (int64_t)blockIdx.x * kKeBlock;
-    const int64_t e = e0 + threadIdx.x;
-    const bool valid = e < e_end;
-    double g[16];
-    bool sym = true;
-    if (valid) {
-        sym = elem_g_fp64(ne, p, npts, t, coef_kind, coef, e, g);
-    } else {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) g[k] = 0.0;
-    }
-    auto entry = [&](int a, int bb) -> double {
-        const int ka0 = sup_lo(a), ka1 = sup_hi(a), kb0 = sup_lo(bb), kb1 = sup_hi(bb);
-        const double *T = Ts + (a * 10 + bb) * 4;
-        double v = g[ka0 * 4 + kb0] * T[0];
-        if (kb1 != kb0) v += g[ka0 * 4 + kb1] * T[1];
-        if (ka1 != ka0) {
-            v += g[ka1 * 4 + kb0] * T[2];
-            if (kb1 != kb0) v += g[ka1 * 4 + kb1] * T[3];
-        }
-        return v;
-    };
-    double U[55];
-    if (sym) {
-#pragma unroll
-        for (int a = 0; a < 10; ++a)
-#pragma unroll
-            for (int bb = a; bb < 10; ++bb) U[tri10(a, bb)] = entry(a, bb);
-    }
-    const int nvalid = (int)(e_end - e0 < kKeBlock ? e_end - e0 : kKeBlock);
-    double *st = stage + threadIdx.x * kKeChunk;
-#pragma unroll
-    for (int r = 0; r < 100 / kKeChunk; ++r) {
-        if (sym) {
-#pragma unroll
-            for (int q = 0; q < kKeChunk; ++q) {
-                const int k = r * kKeChunk + q, a = k / 10, bb = k % 10;
-                st[q] = U[a <= bb ? tri10(a, bb) : tri10(bb, a)];
-            }
-        } else {
-#pragma unroll
-            for (int q = 0; q < kKeChunk; ++q) {
-                const int k = r * kKeChunk + q;
-                st[q] = entry(k / 10, k % 10);
-            }
-        }
-        __syncthreads();
-        // coalesced copy-out: element rows are 100 doubles apart
-        for (int i = threadIdx.x; i < nvalid * kKeChunk; i += kKeBlock) {
-            const int el = i / kKeChunk, q = i - el * kKeChunk;
-            Ke[(e0 + el) * 100 + r * kKeChunk + q] = stage[el * kKeChunk + q];
-        }
-        __syncthreads();
-    }
-}
+__host__ __device__ constexpr int tri10(int a, int b) { return tri_index(10, a, b); }  // a <= b
 
 // Scale exponent s: vertex coordinates times 2^-s are at most 1 in magnitude.
 // The largest |x| is found on the bit patterns (for non-negative doubles the
@@ -908,7 +836,7 @@ __device__ __forceinline__ double shared_entry(const double g[16], const double 
     }
 }
 
-__device__ __forceinline__ void shared_entries(const double g[16], double U[55]) {
+__device__ __forceinline__ void shared_entries(const double g[16], double *U) {
     double S[4][6];  // S_v(b) for vertex v off edge b only (the others are not used)
     static_for<0, 24>([&](auto kk) {
         constexpr int k = decltype(kk)::value, v = k / 6, e = k % 6;
@@ -921,456 +849,195 @@ __device__ __forceinline__ void shared_entries(const double g[16], double U[55])
     });
 }
 
-// k_elem_ke_fp64 for a rule exact on quadratics (the 4-point and the 11-point
-// Keast rule): the entries from the integer table with compile-time factors
-// (about 30 FP64 instructions per element fewer than the table read from
-// shared memory); same staging and coalesced stores.
-__global__ void __launch_bounds__(kKeBlock) k_elem_ke_fp64_exact(int64_t ne, int64_t e_begin, int64_t e_end,
-                                                                 const double *__restrict__ p, int64_t npts,
-                                                                 const int32_t *__restrict__ t, int coef_kind,
-                                                                 const double *__restrict__ coef,
-                                                                 double *__restrict__ Ke) {
-    __shared__ double stage[kKeBlock * kKeChunk];
-    const int64_t e0 = e_begin + (int64_t)blockIdx.x * kKeBlock;
-    const int64_t e = e0 + threadIdx.x;
-    double g[16];
-    bool sym = true;
-    if (e < e_end) {
-        sym = elem_g_fp64(ne, p, npts, t, coef_kind, coef, e, g, 1.0 / 30.0);
-    } else {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) g[k] = 0.0;
+// Where the element pass leaves the packed matrices of a tile, and the lower
+// triangles of the tiles that hold a nonsymmetric coefficient.
+template <class E>
+struct PackedOut {
+    E *upper, *lower;
+    uint8_t *tiles;  // per tile: the lower triangles are there too
+    int *any;        // set when a tile is flagged
+};
+
+// Writes the block's stage (`n` packed matrices of NP entries) to `upper`, and
+// for a tile with a nonsymmetric element the lower triangles (`entry_ba` of
+// the nonsymmetric elements; a symmetric one's stage already holds them) to
+// `lower`.
+template <int NP, class E, class F>
+__device__ __forceinline__ void store_packed(E *stage, int64_t tile, int n, bool sym, const PackedOut<E> &out,
+                                             F &&lower_entries) {
+    const int64_t at = tile * kTile * NP;
+    store_tile(stage, out.upper + at, n * NP * (int)sizeof(E));
+    const bool all = __syncthreads_and(sym);
+    if (out.tiles && threadIdx.x == 0) out.tiles[tile] = all ? 0 : 1;
+    if (all) return;
+    if (threadIdx.x == 0) *out.any = 1;
+    if (!sym) lower_entries();
+    store_tile(stage, out.lower + at, n * NP * (int)sizeof(E));
+}
+
+// FP64 element pass, thread per element: the packed upper triangle of K_e.
+// P1: the 10 entries wsum G (RULE unused).  P2: the 55 entries from G, for a
+// rule exact on quadratics (EXACT; the 4-point and the 11-point Keast rule)
+// from the integer table with compile-time factors and shared sums
+// (shared_entry), else from the rule's table in shared memory.  Each entry
+// goes to the shared-memory stage as it is computed (an odd or 10-double
+// stride per thread: at most two-way bank conflicts), so no entry array is
+// held in registers.  Bound by the FP64 pipe: about 105 instructions for G
+// and 58 for the P2 entries.
+//
+// With `redo`, the pass runs only when the FP32-pair pass before it left its
+// range (its blocks then walk the tiles: the launch that finds nothing to do
+// is small).
+template <int NN, bool EXACT>
+__global__ void __launch_bounds__(kTile) k_elem_packed(int64_t ne, int64_t e_begin, int64_t e_end,
+                                                          const double *__restrict__ p, int64_t npts,
+                                                          const int32_t *__restrict__ t, int coef_kind,
+                                                          const double *__restrict__ coef, double gscale,
+                                                          const double *__restrict__ Tg, PackedOut<double> out,
+                                                          const int *__restrict__ redo) {
+    constexpr int NP = NN * (NN + 1) / 2;
+    extern __shared__ __align__(16) unsigned char smem[];
+    double *stage = reinterpret_cast<double *>(smem);  // kTile x NP, then the table
+    double *Ts = stage + kTile * NP;
+    if (redo && !out_of_range(redo)) return;
+    if constexpr (NN == 10 && !EXACT) {
+        for (int i = threadIdx.x; i < 400; i += kTile) Ts[i] = Tg[i];
+        __syncthreads();
     }
-    double U[55];
-    if (sym) {
-        if (shared_entries_ok(g)) {
-            shared_entries(g, U);
+    const int64_t last = (e_end + kTile - 1) / kTile;
+    for (int64_t tile = e_begin / kTile + blockIdx.x; tile < last; tile += gridDim.x) {
+        const int64_t e0 = tile * kTile, e = e0 + threadIdx.x;
+        double *st = stage + threadIdx.x * NP;
+        double g[16];
+        bool sym = true;
+        if (e < e_end) sym = elem_g_fp64(ne, p, npts, t, coef_kind, coef, e, g, gscale);
+        auto table_entry = [&](int a, int bb) -> double {
+            const int ka0 = sup_lo(a), ka1 = sup_hi(a), kb0 = sup_lo(bb), kb1 = sup_hi(bb);
+            const double *T = Ts + (a * 10 + bb) * 4;
+            double v = g[ka0 * 4 + kb0] * T[0];
+            if (kb1 != kb0) v += g[ka0 * 4 + kb1] * T[1];
+            if (ka1 != ka0) {
+                v += g[ka1 * 4 + kb0] * T[2];
+                if (kb1 != kb0) v += g[ka1 * 4 + kb1] * T[3];
+            }
+            return v;
+        };
+        if (e < e_end) {
+            if constexpr (NN == 4) {
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = a; b < 4; ++b) st[tri_index(4, a, b)] = g[a * 4 + b];
+            } else if constexpr (EXACT) {
+                if (sym && shared_entries_ok(g)) {
+                    shared_entries(g, st);
+                } else {
+                    static_for<0, 100>([&](auto kk) {
+                        constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
+                        if constexpr (A <= BB) st[tri10(A, BB)] = exact_entry_fp64<A, BB>(g);
+                    });
+                }
+            } else {
+#pragma unroll
+                for (int a = 0; a < 10; ++a)
+#pragma unroll
+                    for (int b = a; b < 10; ++b) st[tri10(a, b)] = table_entry(a, b);
+            }
+        }
+        const int n = (int)(e_end - e0 < kTile ? e_end - e0 : kTile);
+        store_packed<NP>(stage, tile, n, sym, out, [&] {
+            if constexpr (NN == 4) {
+#pragma unroll
+                for (int a = 0; a < 4; ++a)
+#pragma unroll
+                    for (int b = a; b < 4; ++b) st[tri_index(4, a, b)] = g[b * 4 + a];
+            } else if constexpr (EXACT) {
+                static_for<0, 100>([&](auto kk) {
+                    constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
+                    if constexpr (A <= BB) st[tri10(A, BB)] = exact_entry_fp64<BB, A>(g);
+                });
+            } else {
+#pragma unroll
+                for (int a = 0; a < 10; ++a)
+#pragma unroll
+                    for (int b = a; b < 10; ++b) st[tri10(a, b)] = table_entry(b, a);
+            }
+        });
+    }
+}
+
+// Element pass of the FP32-pair modes (P2, rule exact on quadratics): G / 30
+// in double-float, the entries from the integer table (exact_entry_sym for a
+// symmetric coefficient) summed error-free in double-float (MODE_DF64, stored
+// as (hi, lo) pairs) or in FP32 with split products (MODE_SPLIT, rounded to
+// FP32), each stored to the stage as it is computed.
+template <int MODE>
+__global__ void __launch_bounds__(kTile) k_elem_packed_df(
+    int64_t ne, int64_t e_begin, int64_t e_end, const double *__restrict__ p, int64_t npts, const int32_t *__restrict__ t, int coef_kind,
+    const double *__restrict__ coef, int *__restrict__ misc,
+    PackedOut<typename std::conditional<MODE == MODE_DF64, float2, float>::type> out) {
+    using E = typename std::conditional<MODE == MODE_DF64, float2, float>::type;
+    extern __shared__ __align__(16) unsigned char smem[];
+    E *stage = reinterpret_cast<E *>(smem);  // kTile x 55
+    const int64_t tile = e_begin / kTile + blockIdx.x, e0 = tile * kTile, e = e0 + threadIdx.x;
+    E *st = stage + threadIdx.x * 55;
+    auto store = [&](int k, df64 v) {
+        if constexpr (MODE == MODE_DF64) st[k] = make_float2(v.hi, v.lo);
+        else st[k] = v.hi + v.lo;
+    };
+    df64 g[16];
+    bool ok = true, sym = true;
+    if (e < e_end) {
+        sym = elem_g_df64(ne, p, npts, t, coef_kind, coef, misc[0], true, e, g, ok);
+        if (!ok) misc[1] = 1;
+        if (sym) {
+            static_for<0, 100>([&](auto kk) {
+                constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
+                if constexpr (A <= BB) store(tri10(A, BB), exact_entry_sym<A, BB, MODE>(g));
+            });
         } else {
             static_for<0, 100>([&](auto kk) {
                 constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
-                if constexpr (A <= BB) U[tri10(A, BB)] = exact_entry_fp64<A, BB>(g);
+                if constexpr (A <= BB) store(tri10(A, BB), exact_entry<A, BB, MODE>(g));
             });
         }
     }
-    const int nvalid = (int)(e_end - e0 < kKeBlock ? e_end - e0 : kKeBlock);
-    double *st = stage + threadIdx.x * kKeChunk;
-    static_for<0, 100 / kKeChunk>([&](auto rr) {
-        constexpr int r = decltype(rr)::value;
-        if (sym) {
-            static_for<0, kKeChunk>([&](auto qq) {
-                constexpr int q = decltype(qq)::value, k = r * kKeChunk + q, A = k / 10, BB = k % 10;
-                st[q] = U[A <= BB ? tri10(A, BB) : tri10(BB, A)];
-            });
-        } else {
-            static_for<0, kKeChunk>([&](auto qq) {
-                constexpr int q = decltype(qq)::value, k = r * kKeChunk + q, A = k / 10, BB = k % 10;
-                st[q] = exact_entry_fp64<A, BB>(g);
-            });
-        }
-        __syncthreads();
-        // coalesced copy-out: element rows are 100 doubles apart
-        for (int i = threadIdx.x; i < nvalid * kKeChunk; i += kKeBlock) {
-            const int el = i / kKeChunk, q = i - el * kKeChunk;
-            Ke[(e0 + el) * 100 + r * kKeChunk + q] = stage[el * kKeChunk + q];
-        }
-        __syncthreads();
-    });
-}
-
-// Tile `tile` (kKeBlock elements) of k_elem_ke_df64; `stage` kKeBlock *
-// kKeChunk pairs of shared memory.
-template <int MODE>
-__device__ __forceinline__ void elem_ke_df64_tile(int64_t tile, int64_t ne, const double *__restrict__ p,
-                                                  int64_t npts, const int32_t *__restrict__ t, int coef_kind,
-                                                  const double *__restrict__ coef, const int *__restrict__ s_ptr,
-                                                  float2 *__restrict__ Ke, int *__restrict__ range_flag,
-                                                  float2 *stage) {
-    const int64_t e0 = tile * kKeBlock;
-    const int64_t e = e0 + threadIdx.x;
-    const bool valid = e < ne;
-    df64 g[16];
-    bool ok = true, sym = true;
-    if (valid) {
-        sym = elem_g_df64(ne, p, npts, t, coef_kind, coef, *s_ptr, true, e, g, ok);
-        if (!ok) atomicExch(range_flag, 1);
-    } else {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) g[k] = df64{0.f, 0.f};
-    }
-    df64 U[55];
-    if (sym) {  // the same entries as k_elem_ke_df64_packed gives a symmetric element
+    store_packed<55>(stage, tile, (int)(e_end - e0 < kTile ? e_end - e0 : kTile), sym, out, [&] {
         static_for<0, 100>([&](auto kk) {
             constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
-            if constexpr (A <= BB) U[tri10(A, BB)] = exact_entry_sym<A, BB, MODE>(g);
+            if constexpr (A <= BB) store(tri10(A, BB), exact_entry<BB, A, MODE>(g));
         });
-    }
-    const int nvalid = (int)(ne - e0 < kKeBlock ? ne - e0 : kKeBlock);
-    float2 *st = stage + threadIdx.x * kKeChunk;
-    static_for<0, 100 / kKeChunk>([&](auto rr) {
-        constexpr int r = decltype(rr)::value;
-        if (sym) {
-            static_for<0, kKeChunk>([&](auto qq) {
-                constexpr int q = decltype(qq)::value, k = r * kKeChunk + q, A = k / 10, BB = k % 10;
-                const df64 v = U[A <= BB ? tri10(A, BB) : tri10(BB, A)];
-                st[q] = make_float2(v.hi, v.lo);
-            });
-        } else {
-            static_for<0, kKeChunk>([&](auto qq) {
-                constexpr int q = decltype(qq)::value, k = r * kKeChunk + q;
-                const df64 v = exact_entry<k / 10, k % 10, MODE>(g);
-                st[q] = make_float2(v.hi, v.lo);
-            });
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < nvalid * kKeChunk; i += kKeBlock) {
-            const int el = i / kKeChunk, q = i - el * kKeChunk;
-            Ke[(e0 + el) * 100 + r * kKeChunk + q] = stage[el * kKeChunk + q];
-        }
-        __syncthreads();
     });
 }
 
-// The blocks walk the tiles (grid-stride); with `only` non-NULL they
-// assemble only the tiles with only[tile] set.
-template <int MODE>
-__global__ void __launch_bounds__(kKeBlock, 3) k_elem_ke_df64(int64_t ne, const double *__restrict__ p, int64_t npts,
-                                                           const int32_t *__restrict__ t, int coef_kind,
-                                                           const double *__restrict__ coef,
-                                                           const int *__restrict__ s_ptr, float2 *__restrict__ Ke,
-                                                           int *__restrict__ range_flag,
-                                                           const uint8_t *__restrict__ only = nullptr) {
-    __shared__ float2 stage[kKeBlock * kKeChunk];
-    __shared__ uint8_t flag[kKeBlock];
-    const int64_t n_tiles = (ne + kKeBlock - 1) / kKeBlock;
-    if (!only) {
-        for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x)
-            elem_ke_df64_tile<MODE>(tile, ne, p, npts, t, coef_kind, coef, s_ptr, Ke, range_flag, stage);
-        return;
-    }
-    // kKeBlock flags per round, read by the block at once
-    for (int64_t base = (int64_t)blockIdx.x * kKeBlock; base < n_tiles; base += (int64_t)gridDim.x * kKeBlock) {
-        flag[threadIdx.x] = base + threadIdx.x < n_tiles ? only[base + threadIdx.x] : 0;
-        if (!__syncthreads_or(flag[threadIdx.x])) continue;
-        for (int j = 0; j < kKeBlock; ++j)
-            if (flag[j])
-                elem_ke_df64_tile<MODE>(base + j, ne, p, npts, t, coef_kind, coef, s_ptr, Ke, range_flag, stage);
-        __syncthreads();  // flags of the next round
-    }
+// Packed matrices of one assembly: scratch, launches and the sums.
+template <class E>
+PairLower<E> lower_of(const PackedOut<E> &o) {
+    return o.lower ? PairLower<E>{o.lower, o.any, o.tiles} : PairLower<E>{};
 }
 
-// Element matrices of SKG_SPLIT_FP32 (P2, exact rule): G in double-float, each
-// entry's integer-factor terms summed in FP32 with split products
-// (exact_entry<MODE_SPLIT>), the entry rounded to FP32.  Each entry goes to
-// shared memory as it is computed (the packed upper triangle of a symmetric
-// matrix, mirrored by the copy-out; every entry, in two rounds of five rows,
-// when a tile holds a nonsymmetric coefficient), so no entry array is held
-// in registers: enough warps to hide the coordinate and coefficient loads.
-__global__ void __launch_bounds__(kKeBlock) k_elem_ke_split(int64_t ne, const double *__restrict__ p, int64_t npts,
-                                                            const int32_t *__restrict__ t, int coef_kind,
-                                                            const double *__restrict__ coef,
-                                                            const int *__restrict__ s_ptr, float *__restrict__ Ke,
-                                                            int *__restrict__ range_flag) {
-    constexpr int kPacked = 55, kHalf = 51;  // odd strides: conflict-free per-thread stores
-    __shared__ float stage[kKeBlock * kPacked];
-    const int64_t e0 = (int64_t)blockIdx.x * kKeBlock;
-    const int64_t e = e0 + threadIdx.x;
-    df64 g[16];
-    bool ok = true, sym = true;
-    if (e < ne) {
-        sym = elem_g_df64(ne, p, npts, t, coef_kind, coef, *s_ptr, true, e, g, ok);
-        if (!ok) atomicExch(range_flag, 1);
-    } else {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) g[k] = df64{0.f, 0.f};
-    }
-    const int nvalid = (int)(ne - e0 < kKeBlock ? ne - e0 : kKeBlock);
-    if (__syncthreads_and(sym)) {
-        float *st = stage + threadIdx.x * kPacked;
-        static_for<0, 100>([&](auto kk) {
-            constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
-            if constexpr (A <= BB) {
-                const df64 v = exact_entry_sym<A, BB, MODE_SPLIT>(g);
-                st[tri10(A, BB)] = v.hi + v.lo;
-            }
-        });
-        __syncthreads();
-        for (int i = threadIdx.x; i < nvalid * 100; i += kKeBlock) {
-            const int el = i / 100, k = i - el * 100, a = k / 10, b = k - a * 10;
-            Ke[(e0 + el) * 100 + k] = stage[el * kPacked + (a <= b ? tri10(a, b) : tri10(b, a))];
-        }
-    } else {
-        float *st = stage + threadIdx.x * kHalf;
-        static_for<0, 2>([&](auto rr) {
-            constexpr int r = decltype(rr)::value;
-            static_for<0, 50>([&](auto qq) {
-                constexpr int q = decltype(qq)::value, k = r * 50 + q;
-                const df64 v = exact_entry<k / 10, k % 10, MODE_SPLIT>(g);
-                st[q] = v.hi + v.lo;
-            });
-            __syncthreads();
-            for (int i = threadIdx.x; i < nvalid * 50; i += kKeBlock) {
-                const int el = i / 50, q = i - el * 50;
-                Ke[(e0 + el) * 100 + r * 50 + q] = stage[el * kHalf + q];
-            }
-            __syncthreads();
-        });
-    }
-}
-
-// SKG_FP64_EMULATED element matrices with a symmetric coefficient: each of
-// the 55 distinct entries is stored to shared memory as it is computed
-// (packed upper triangle, mirrored by the copy-out) instead of being held in
-// registers until its row is staged as in k_elem_ke_df64: 64 registers
-// against 168, so more warps per SM (0.53 -> 0.41 ms at 64^3).  A tile with a
-// nonsymmetric coefficient is flagged in `redo` and left to k_elem_ke_df64.
-template <typename T>
-__device__ __forceinline__ void copy_packed(const T *stage, int nvalid, int64_t e0, T *__restrict__ Ke) {
-    for (int i = threadIdx.x; i < nvalid * 100; i += kKeBlock) {
-        const int el = i / 100, k = i - el * 100, a = k / 10, b = k - a * 10;
-        Ke[(e0 + el) * 100 + k] = stage[el * 55 + (a <= b ? tri10(a, b) : tri10(b, a))];
-    }
-}
-
-__global__ void __launch_bounds__(kKeBlock) k_elem_ke_df64_packed(int64_t ne, const double *__restrict__ p,
-                                                                  int64_t npts, const int32_t *__restrict__ t,
-                                                                  int coef_kind, const double *__restrict__ coef,
-                                                                  const int *__restrict__ s_ptr,
-                                                                  float2 *__restrict__ Ke,
-                                                                  int *__restrict__ range_flag,
-                                                                  uint8_t *__restrict__ redo) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    float2 *stage = reinterpret_cast<float2 *>(smem);  // kKeBlock x 55
-    const int64_t e0 = (int64_t)blockIdx.x * kKeBlock;
-    const int64_t e = e0 + threadIdx.x;
-    df64 g[16];
-    bool ok = true, sym = true;
-    if (e < ne) {
-        sym = elem_g_df64(ne, p, npts, t, coef_kind, coef, *s_ptr, true, e, g, ok);
-        if (!ok) atomicExch(range_flag, 1);
-    } else {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) g[k] = df64{0.f, 0.f};
-    }
-    if (!__syncthreads_and(sym)) {  // a nonsymmetric coefficient: k_elem_ke_df64 redoes this tile
-        if (threadIdx.x == 0) redo[blockIdx.x] = 1;
-        return;
-    }
-    float2 *st = stage + threadIdx.x * 55;
-    static_for<0, 100>([&](auto kk) {
-        constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
-        if constexpr (A <= BB) {
-            const df64 v = exact_entry_sym<A, BB, MODE_DF64>(g);
-            st[tri10(A, BB)] = make_float2(v.hi, v.lo);
-        }
-    });
-    __syncthreads();
-    copy_packed(stage, (int)(ne - e0 < kKeBlock ? ne - e0 : kKeBlock), e0, Ke);
-}
-
-constexpr int kPackedSmem = kKeBlock * 55 * 8;  // 56,320 bytes
-
-
-// Row pass over double-float element matrices: rows of 10 (hi, lo) pairs added
-// into double-float slots, converted to FP64 at write-out.
-template <int SLOTS, int P>
-__global__ void __launch_bounds__(kRowWarps * 32) k_rows_ke_df(int n_groups, const int2 *__restrict__ groups,
-                                                              const int32_t *__restrict__ indptr,
-                                                              const int32_t *__restrict__ inc_ptr,
-                                                              const int4 *__restrict__ rec,
-                                                              const float2 *__restrict__ Ke,
-                                                              const int *__restrict__ s_ptr,
-                                                              double *__restrict__ values) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gi = blockIdx.x * kRowWarps + warp;
-    if (gi >= n_groups) return;
-    df64 *acc = reinterpret_cast<df64 *>(smem + (size_t)warp * SLOTS * 8);
-    const int2 grp = groups[gi];
-    const int32_t s0 = indptr[grp.x];
-    const int nslots = indptr[grp.y] - s0;
-    for (int j = lane; j < P * nslots; j += 32) acc[j] = df64{0.f, 0.f};
-    __syncwarp();
-    const int ridx = lane / P, part = lane - (lane / P) * P;
-    const int32_t r = grp.x + ridx;
-    if (ridx < 32 / P && r < grp.y) {
-        const int base = indptr[r] - s0 + part * nslots;
-        const int32_t it1 = inc_ptr[r + 1];
-        int32_t it = inc_ptr[r] + part;
-        if (it < it1) {
-            // records two incidences ahead of the rows they address, rows one
-            int4 rc = rec[it];
-            int4 rcn = it + P < it1 ? rec[it + P] : make_int4(0, 0, 0, 0);
-            float4 cur[5];
-            {
-                const float4 *src = reinterpret_cast<const float4 *>(Ke + (int64_t)rc.x * 10);
-#pragma unroll
-                for (int q = 0; q < 5; ++q) cur[q] = __ldg(src + q);
-            }
-            bool first = true;
-            for (; it < it1; it += P) {
-                const bool has_next = it + P < it1;
-                float4 nxt[5];
-                if (has_next) {
-                    const float4 *src = reinterpret_cast<const float4 *>(Ke + (int64_t)rcn.x * 10);
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) nxt[q] = __ldg(src + q);
-                }
-                const int4 rcnn = it + 2 * P < it1 ? rec[it + 2 * P] : make_int4(0, 0, 0, 0);
-                const unsigned ow[3] = {(unsigned)rc.y, (unsigned)rc.z, (unsigned)rc.w};
-                int off[10];
-#pragma unroll
-                for (int bb = 0; bb < 10; ++bb) off[bb] = base + (int)((ow[bb >> 2] >> (8 * (bb & 3))) & 0xffu);
-                if (first) {  // the part's first incidence: its row initialises the slots
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) {
-                        acc[off[2 * q]] = df64{cur[q].x, cur[q].y};
-                        acc[off[2 * q + 1]] = df64{cur[q].z, cur[q].w};
-                    }
-                    first = false;
-                } else {
-                    df64 a[10];
-#pragma unroll
-                    for (int bb = 0; bb < 10; ++bb) a[bb] = acc[off[bb]];
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) {
-                        df_acc(a[2 * q], df64{cur[q].x, cur[q].y});
-                        df_acc(a[2 * q + 1], df64{cur[q].z, cur[q].w});
-                    }
-#pragma unroll
-                    for (int bb = 0; bb < 10; ++bb) acc[off[bb]] = a[bb];
-                }
-                if (has_next) {
-                    rc = rcn;
-                    rcn = rcnn;
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) cur[q] = nxt[q];
-                }
-            }
-        }
-    }
-    __syncwarp();
-    const int sc = *s_ptr;
-    for (int j = lane; j < nslots; j += 32) {
-        df64 v = fast_two_sum(acc[j].hi, acc[j].lo);
-#pragma unroll
-        for (int c = 1; c < P; ++c) v = df_add(v, fast_two_sum(acc[c * nslots + j].hi, acc[c * nslots + j].lo));
-        values[s0 + j] = df_to_double(v, sc);
-    }
-}
-
-template <int SLOTS, int P>
-void launch_ke_df_class(int n_groups, const int2 *groups, const skg_pattern *pat, const float2 *Ke, const int *s_ptr,
-                        double *values, cudaStream_t s) {
-    if (n_groups == 0) return;
-    const size_t smem = (size_t)kRowWarps * SLOTS * 8;
+template <int NN, bool EXACT>
+void launch_elem_packed(int64_t ne, int64_t e0, int64_t e1, const double *p, int64_t npts, const int32_t *t, int kind,
+                        const double *coef, double gscale, const double *Tg, const PackedOut<double> &out,
+                        const int *redo, cudaStream_t s) {
+    constexpr int smem = kTile * NN * (NN + 1) / 2 * 8 + (NN == 10 && !EXACT ? 400 * 8 : 0);
     if (smem > 48 * 1024)
-        SKG_CUDA(cudaFuncSetAttribute(k_rows_ke_df<SLOTS, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned grid = (unsigned)((n_groups + kRowWarps - 1) / kRowWarps);
-    k_rows_ke_df<SLOTS, P><<<grid, kRowWarps * 32, smem, s>>>(n_groups, groups, pat->indptr.get(), pat->inc_ptr.get(),
-                                                              pat->rec.get(), Ke, s_ptr, values);
-    SKG_LAUNCH_CHECK("rows_ke_df");
+        SKG_CUDA(cudaFuncSetAttribute(k_elem_packed<NN, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    unsigned grid = grid_for(e1 - e0, kTile);
+    if (redo) grid = std::min(grid, 2u * kSmCount);
+    k_elem_packed<NN, EXACT><<<grid, kTile, smem, s>>>(ne, e0, e1, p, npts, t, kind, coef, gscale, Tg, out, redo);
+    SKG_LAUNCH_CHECK("elem_packed");
 }
 
-// Row pass over FP32 element matrices (SKG_SPLIT_FP32): rows of 10 floats
-// added into double-float slots, converted to FP64 at write-out; otherwise as
-// k_rows_ke_df (40-byte rows: half the element-matrix bytes).
-template <int SLOTS, int P>
-__global__ void __launch_bounds__(kRowWarps * 32) k_rows_ke_f32(int n_groups, const int2 *__restrict__ groups,
-                                                               const int32_t *__restrict__ indptr,
-                                                               const int32_t *__restrict__ inc_ptr,
-                                                               const int4 *__restrict__ rec,
-                                                               const float *__restrict__ Ke,
-                                                               const int *__restrict__ s_ptr,
-                                                               double *__restrict__ values) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gi = blockIdx.x * kRowWarps + warp;
-    if (gi >= n_groups) return;
-    df64 *acc = reinterpret_cast<df64 *>(smem + (size_t)warp * SLOTS * 8);
-    const int2 grp = groups[gi];
-    const int32_t s0 = indptr[grp.x];
-    const int nslots = indptr[grp.y] - s0;
-    for (int j = lane; j < P * nslots; j += 32) acc[j] = df64{0.f, 0.f};
-    __syncwarp();
-    const int ridx = lane / P, part = lane - (lane / P) * P;
-    const int32_t r = grp.x + ridx;
-    if (ridx < 32 / P && r < grp.y) {
-        const int base = indptr[r] - s0 + part * nslots;
-        const int32_t it1 = inc_ptr[r + 1];
-        int32_t it = inc_ptr[r] + part;
-        if (it < it1) {
-            // records two incidences ahead of the rows they address, rows one
-            int4 rc = rec[it];
-            int4 rcn = it + P < it1 ? rec[it + P] : make_int4(0, 0, 0, 0);
-            float2 cur[5];
-            {
-                const float2 *src = reinterpret_cast<const float2 *>(Ke + (int64_t)rc.x * 10);
-#pragma unroll
-                for (int q = 0; q < 5; ++q) cur[q] = __ldg(src + q);
-            }
-            bool first = true;
-            for (; it < it1; it += P) {
-                const bool has_next = it + P < it1;
-                float2 nxt[5];
-                if (has_next) {
-                    const float2 *src = reinterpret_cast<const float2 *>(Ke + (int64_t)rcn.x * 10);
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) nxt[q] = __ldg(src + q);
-                }
-                const int4 rcnn = it + 2 * P < it1 ? rec[it + 2 * P] : make_int4(0, 0, 0, 0);
-                const unsigned ow[3] = {(unsigned)rc.y, (unsigned)rc.z, (unsigned)rc.w};
-                int off[10];
-#pragma unroll
-                for (int bb = 0; bb < 10; ++bb) off[bb] = base + (int)((ow[bb >> 2] >> (8 * (bb & 3))) & 0xffu);
-                if (first) {  // the part's first incidence: its row initialises the slots
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) {
-                        acc[off[2 * q]] = df64{cur[q].x, 0.f};
-                        acc[off[2 * q + 1]] = df64{cur[q].y, 0.f};
-                    }
-                    first = false;
-                } else {
-                    df64 a[10];
-#pragma unroll
-                    for (int bb = 0; bb < 10; ++bb) a[bb] = acc[off[bb]];
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) {
-                        df_acc(a[2 * q], df64{cur[q].x, 0.f});
-                        df_acc(a[2 * q + 1], df64{cur[q].y, 0.f});
-                    }
-#pragma unroll
-                    for (int bb = 0; bb < 10; ++bb) acc[off[bb]] = a[bb];
-                }
-                if (has_next) {
-                    rc = rcn;
-                    rcn = rcnn;
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) cur[q] = nxt[q];
-                }
-            }
-        }
-    }
-    __syncwarp();
-    const int sc = *s_ptr;
-    for (int j = lane; j < nslots; j += 32) {
-        df64 v = fast_two_sum(acc[j].hi, acc[j].lo);
-#pragma unroll
-        for (int c = 1; c < P; ++c) v = df_add(v, fast_two_sum(acc[c * nslots + j].hi, acc[c * nslots + j].lo));
-        values[s0 + j] = df_to_double(v, sc);
-    }
-}
-
-template <int SLOTS, int P>
-void launch_ke_f32_class(int n_groups, const int2 *groups, const skg_pattern *pat, const float *Ke, const int *s_ptr,
-                         double *values, cudaStream_t s) {
-    if (n_groups == 0) return;
-    const size_t smem = (size_t)kRowWarps * SLOTS * 8;
+template <int MODE, class E>
+void launch_elem_packed_df(int64_t ne, int64_t e0, int64_t e1, const double *p, int64_t npts, const int32_t *t, int kind, const double *coef,
+                           int *misc, const PackedOut<E> &out, cudaStream_t s) {
+    constexpr int smem = kTile * 55 * (int)sizeof(E);
     if (smem > 48 * 1024)
-        SKG_CUDA(cudaFuncSetAttribute(k_rows_ke_f32<SLOTS, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned grid = (unsigned)((n_groups + kRowWarps - 1) / kRowWarps);
-    k_rows_ke_f32<SLOTS, P><<<grid, kRowWarps * 32, smem, s>>>(n_groups, groups, pat->indptr.get(), pat->inc_ptr.get(),
-                                                               pat->rec.get(), Ke, s_ptr, values);
-    SKG_LAUNCH_CHECK("rows_ke_f32");
+        SKG_CUDA(cudaFuncSetAttribute(k_elem_packed_df<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_elem_packed_df<MODE><<<grid_for(e1 - e0, kTile), kTile, smem, s>>>(ne, e0, e1, p, npts, t, kind, coef, misc,
+                                                                              out);
+    SKG_LAUNCH_CHECK("elem_packed_df");
 }
 
 // Fallback row pass (patterns without row blocks): thread per row, global
@@ -1484,6 +1151,96 @@ void launch_scale_exponent(const double *d_p, int64_t n, int *d_s, cudaStream_t 
     SKG_LAUNCH_CHECK("scale");
 }
 
+namespace {
+
+// Element pass and pair sums (see the head of the file).  FP32-pair modes:
+// scale exponent, element pass and sums, then the FP64 passes in their place
+// when a value left the FP32 range, decided on the device: no synchronisation
+// (waiting for the range flag left the GPU idle for 0.06 ms at 37 x 29 x 31
+// and 0.13 ms at 48^3).
+void affine_assemble_pairs(const skg_pattern *pat, const double *d_p, int64_t npts, const int32_t *d_t, int32_t nodes,
+                           int64_t ne, const std::vector<double> &T, bool exact_rule, int32_t coef_kind,
+                           const double *d_coef, int32_t precision, double *d_values, cudaStream_t s, cudaEvent_t *ev,
+                           double *h_values) {
+    const int np = nodes * (nodes + 1) / 2;
+    const int64_t tiles = (ne + kTile - 1) / kTile;
+    const bool maybe_lower = coef_kind != 0;  // a tensor may be nonsymmetric
+    // [0] scale exponent, [1] range flag (0x80808080: none, in range), [2] a tile holds a nonsymmetric coefficient
+    DevBuf<int> misc(3, s);
+    DevBuf<double> K((size_t)ne * np, s), lower(maybe_lower ? (size_t)ne * np : 0, s);
+    DevBuf<uint8_t> tile_flags(maybe_lower ? (size_t)tiles : 0, s);
+    int *any = maybe_lower ? misc.get() + 2 : nullptr;
+    if (maybe_lower) SKG_CUDA(cudaMemsetAsync(any, 0, 4, s));
+    const PackedOut<double> out64{K.get(), lower.get(), tile_flags.get(), any};
+    const double *Tg = nodes == 10 && !exact_rule ? device_table(T.data(), T.size(), s) : nullptr;
+    auto elem64 = [&](int64_t e0, int64_t e1, const int *redo) {
+        if (nodes == 4)
+            launch_elem_packed<4, false>(ne, e0, e1, d_p, npts, d_t, coef_kind, d_coef, T[0], nullptr, out64, redo, s);
+        else if (exact_rule)
+            launch_elem_packed<10, true>(ne, e0, e1, d_p, npts, d_t, coef_kind, d_coef, 1.0 / 30.0, nullptr, out64,
+                                         redo, s);
+        else
+            launch_elem_packed<10, false>(ne, e0, e1, d_p, npts, d_t, coef_kind, d_coef, 1.0, Tg, out64, redo, s);
+    };
+    if (ev) SKG_CUDA(cudaEventRecord(ev[0], s));
+    if (precision == SKG_FP64) {
+        run_pair_passes(
+            pat, ne, d_values, h_values, s,
+            [&](int64_t e0, int64_t e1) {
+                elem64(e0, e1, nullptr);
+                if (ev) SKG_CUDA(cudaEventRecord(ev[1], s));
+            },
+            [&](int s0, int s1, cudaStream_t st) {
+                pair_sum<double>(pat->pairs, s0, s1, K.get(), lower_of(out64), PairIdentity{}, nullptr, d_values, st);
+            });
+        if (ev) SKG_CUDA(cudaEventRecord(ev[2], s));
+        return;
+    }
+    SKG_CUDA(cudaMemsetAsync(misc.get(), 0x80, 2 * sizeof(int), s));
+    k_scale<<<2 * kSmCount, 256, 0, s>>>(d_p, 3 * npts, misc.get());
+    SKG_LAUNCH_CHECK("scale");
+    // The FP32-pair entries lie in scratch of their own: with a host output
+    // their sums and copies follow the element pass step by step, before the
+    // range flag is final.
+    const bool split = precision == SKG_SPLIT_FP32;
+    const size_t entry = split ? sizeof(float) : sizeof(float2);
+    DevBuf<unsigned char> Kf((size_t)ne * np * entry, s), lower_f(maybe_lower ? (size_t)ne * np * entry : 0, s);
+    const PackedOut<float2> out_df{reinterpret_cast<float2 *>(Kf.get()), reinterpret_cast<float2 *>(lower_f.get()),
+                                   tile_flags.get(), any};
+    const PackedOut<float> out_f{reinterpret_cast<float *>(Kf.get()), reinterpret_cast<float *>(lower_f.get()),
+                                 tile_flags.get(), any};
+    const PairUnscale unscale{misc.get()};
+    run_pair_passes(
+        pat, ne, d_values, h_values, s,
+        [&](int64_t e0, int64_t e1) {
+            if (split)
+                launch_elem_packed_df<MODE_SPLIT>(ne, e0, e1, d_p, npts, d_t, coef_kind, d_coef, misc.get(), out_f, s);
+            else
+                launch_elem_packed_df<MODE_DF64>(ne, e0, e1, d_p, npts, d_t, coef_kind, d_coef, misc.get(), out_df, s);
+            if (ev) SKG_CUDA(cudaEventRecord(ev[1], s));
+        },
+        [&](int s0, int s1, cudaStream_t st) {
+            if (split)
+                pair_sum<df64>(pat->pairs, s0, s1, out_f.upper, lower_of(out_f), unscale, nullptr, d_values, st);
+            else
+                pair_sum<df64>(pat->pairs, s0, s1, out_df.upper, lower_of(out_df), unscale, nullptr, d_values, st);
+        });
+    if (h_values) {  // the caller waits for the copies: the host decides
+        int h_misc[2];
+        SKG_CUDA(cudaMemcpyAsync(h_misc, misc.get(), sizeof(h_misc), cudaMemcpyDeviceToHost, s));
+        SKG_CUDA(cudaStreamSynchronize(s));
+        if (h_misc[1] != 1 && h_misc[0] >= -(1 << 20)) return;
+    }
+    if (ne) elem64(0, ne, misc.get());
+    pair_sum<double>(pat->pairs, 0, pat->pairs.n_slices, K.get(), lower_of(out64), PairIdentity{}, misc.get(), d_values,
+                     s);
+    if (ev) SKG_CUDA(cudaEventRecord(ev[2], s));
+    if (h_values && pat->nnz)
+        SKG_CUDA(cudaMemcpyAsync(h_values, d_values, (size_t)pat->nnz * sizeof(double), cudaMemcpyDeviceToHost, s));
+}
+
+}  // namespace
+
 // Shared by the C ABI entry points below.
 // h_values (optional, page-locked host): the values also go there, copied in
 // row chunks overlapping the row pass (run_row_pass).
@@ -1503,66 +1260,19 @@ void affine_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, co
     std::vector<double> T;
     Support sp{};
     affine_table(nodes, nq, h_X, h_W, T, sp);
+    const bool exact_rule = nodes == 10 && p2_rule_is_exact(T);
+    if (pat->pairs.block == 1 && pat->pairs.nodes == nodes && (precision == SKG_FP64 || exact_rule)) {
+        affine_assemble_pairs(pat, d_p, npts, d_t, nodes, ne, T, exact_rule, coef_kind, d_coef, precision, d_values, s,
+                              ev, h_values);
+        return;
+    }
     const double *Tg = device_table(T.data(), T.size(), s);
     DevBuf<double> G((size_t)ne * 16, s);  // 16 doubles or 16 df64 pairs per element
     const bool blocked = pat->max_row_len > 0;
-    const bool exact = nodes == 10 && blocked && precision != SKG_FP64 && p2_rule_is_exact(T);
+    const bool exact = exact_rule && blocked && precision != SKG_FP64;
     int mode = precision == SKG_FP64 ? MODE_FP64 : precision == SKG_SPLIT_FP32 ? MODE_SPLIT : MODE_DF64;
     if (!blocked) mode = MODE_FP64;
     DevBuf<int> misc(2, s);  // [0] scale exponent, [1] range flag
-    if (mode != MODE_FP64 && exact) {
-        // P2, exact rule, FP32 pairs: element matrices (double-float entries
-        // for SKG_FP64_EMULATED, FP32 entries summed in FP32 for
-        // SKG_SPLIT_FP32), then the row sums in double-float slots
-        const int init[2] = {INT_MIN, 0};
-        SKG_CUDA(cudaMemcpyAsync(misc.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
-        k_scale<<<2 * kSmCount, 256, 0, s>>>(d_p, 3 * npts, misc.get());
-        SKG_LAUNCH_CHECK("scale");
-        DevBuf<float2> Kf(mode == MODE_DF64 ? (size_t)ne * 100 : 0, s);
-        DevBuf<float> Kh(mode == MODE_SPLIT ? (size_t)ne * 100 : 0, s);
-        DevBuf<uint8_t> redo(mode == MODE_DF64 ? (size_t)grid_for(ne, kKeBlock) : 0, s);  // tiles left to k_elem_ke_df64
-        if (ev) SKG_CUDA(cudaEventRecord(ev[0], s));
-        if (ne) {
-            if (mode == MODE_DF64) {
-                const unsigned tiles = grid_for(ne, kKeBlock);
-                SKG_CUDA(cudaMemsetAsync(redo.get(), 0, tiles, s));
-                SKG_CUDA(cudaFuncSetAttribute(k_elem_ke_df64_packed, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              kPackedSmem));
-                k_elem_ke_df64_packed<<<tiles, kKeBlock, kPackedSmem, s>>>(
-                    ne, d_p, npts, d_t, coef_kind, d_coef, misc.get(), Kf.get(), misc.get() + 1, redo.get());
-                SKG_LAUNCH_CHECK("elem_ke_df64_packed");
-                k_elem_ke_df64<MODE_DF64><<<std::min<unsigned>((tiles + kKeBlock - 1) / kKeBlock, 2 * kSmCount),
-                                            kKeBlock, 0, s>>>(
-                    ne, d_p, npts, d_t, coef_kind, d_coef, misc.get(), Kf.get(), misc.get() + 1, redo.get());
-            }
-            else
-                k_elem_ke_split<<<grid_for(ne, kKeBlock), kKeBlock, 0, s>>>(ne, d_p, npts, d_t, coef_kind, d_coef,
-                                                                             misc.get(), Kh.get(), misc.get() + 1);
-            SKG_LAUNCH_CHECK("elem_ke_df64");
-        }
-        int h_misc[2];
-        SKG_CUDA(cudaMemcpyAsync(h_misc, misc.get(), sizeof(h_misc), cudaMemcpyDeviceToHost, s));
-        SKG_CUDA(cudaStreamSynchronize(s));
-        if (h_misc[1] == 0 && h_misc[0] != INT_MIN) {
-            if (ev) SKG_CUDA(cudaEventRecord(ev[1], s));
-            run_row_pass(pat, d_values, h_values, s, [&](const GroupSet &gs, cudaStream_t st) {
-                if (mode == MODE_DF64) {
-                    launch_ke_df_class<kGroupSlotsSmall, 1>(gs.n_small, gs.small, pat, Kf.get(), misc.get(), d_values,
-                                                            st);
-                    launch_ke_df_class<kGroupSlotsLarge, 2>(gs.n_large, gs.large, pat, Kf.get(), misc.get(), d_values,
-                                                            st);
-                } else {
-                    launch_ke_f32_class<kGroupSlotsSmall, 1>(gs.n_small, gs.small, pat, Kh.get(), misc.get(),
-                                                             d_values, st);
-                    launch_ke_f32_class<kGroupSlotsLarge, 2>(gs.n_large, gs.large, pat, Kh.get(), misc.get(),
-                                                             d_values, st);
-                }
-            });
-            if (ev) SKG_CUDA(cudaEventRecord(ev[2], s));
-            return;
-        }
-        mode = MODE_FP64;  // out of FP32 range: FP64 instead
-    }
     if (mode != MODE_FP64) {
         const int init[2] = {INT_MIN, 0};
         SKG_CUDA(cudaMemcpyAsync(misc.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
@@ -1579,28 +1289,6 @@ void affine_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, co
         SKG_CUDA(cudaMemcpyAsync(h_misc, misc.get(), sizeof(h_misc), cudaMemcpyDeviceToHost, s));
         SKG_CUDA(cudaStreamSynchronize(s));
         if (h_misc[1] != 0 || h_misc[0] == INT_MIN) mode = MODE_FP64;  // out of FP32 range: FP64 instead
-    }
-    if (mode == MODE_FP64 && nodes == 10 && blocked) {
-        // FP64 P2: element matrices, then row sums
-        // (with a host output the two passes interleave, see run_passes)
-        const bool exact_fp64 = p2_rule_is_exact(T);
-        DevBuf<double> Ke((size_t)ne * 100, s);
-        if (ev) SKG_CUDA(cudaEventRecord(ev[0], s));
-        run_passes(
-            pat, ne, d_values, h_values, s,
-            [&](int64_t e0, int64_t e1) {
-                if (exact_fp64)
-                    k_elem_ke_fp64_exact<<<grid_for(e1 - e0, kKeBlock), kKeBlock, 0, s>>>(ne, e0, e1, d_p, npts, d_t,
-                                                                                       coef_kind, d_coef, Ke.get());
-                else
-                    k_elem_ke_fp64<<<grid_for(e1 - e0, kKeBlock), kKeBlock, 0, s>>>(ne, e0, e1, d_p, npts, d_t,
-                                                                                 coef_kind, d_coef, Tg, Ke.get());
-                SKG_LAUNCH_CHECK("elem_ke_fp64");
-                if (ev) SKG_CUDA(cudaEventRecord(ev[1], s));
-            },
-            [&](const GroupSet &gs, cudaStream_t st) { add_element_rows<10>(pat, Ke.get(), d_values, st, gs); });
-        if (ev) SKG_CUDA(cudaEventRecord(ev[2], s));
-        return;
     }
     if (mode == MODE_FP64) {
         if (ev) SKG_CUDA(cudaEventRecord(ev[0], s));
@@ -1638,7 +1326,8 @@ void affine_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, co
                     if (exact) launch_rows_groups<10, MODE_SPLIT, true>(pat, G.get(), Tg, sp_ptr, d_values, st, gs);
                     else SKG_ROWS(10, MODE_SPLIT);
                 } else {
-                    SKG_ROWS(10, MODE_DF64);
+                    if (exact) launch_rows_groups<10, MODE_DF64, true>(pat, G.get(), Tg, sp_ptr, d_values, st, gs);
+                    else SKG_ROWS(10, MODE_DF64);
                 }
             }
         });

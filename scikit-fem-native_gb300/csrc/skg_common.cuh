@@ -190,6 +190,38 @@ constexpr int kHostChunks = 16;
 constexpr int64_t kHostChunkMinNnz = int64_t(1) << 22;  // 32 MiB of values
 }  // namespace skg
 
+namespace skg {
+// The slices below `slice` reference elements below `ready` only.
+struct PairStep {
+    int32_t slice = 0;
+    int64_t ready = 0;
+};
+
+// A host-output chunk: rows [row0, row1), CSR positions [slot0, slot1), complete
+// once the slices below `slice` are summed.
+struct PairCopy {
+    int32_t row0 = 0, row1 = 0, slot0 = 0, slot1 = 0, slice = 0;
+};
+
+// Contributions of the node pairs of a symmetric pattern (skg_pairs.cuh).
+struct PairPlan {
+    int32_t block = 0;  // components per node: 1 or 3; 0: no plan
+    int32_t nodes = 0;  // local nodes n
+    int32_t np = 0;     // n (n + 1) / 2 packed node blocks per element
+    int32_t n_slices = 0;
+    DevBuf<unsigned char> store;  // the arrays below
+    int32_t *slice_ptr = nullptr;  // (n_slices + 1), in units of 32 codes
+    uint32_t *codes = nullptr;     // element * np + packed position, contribution k of lane l at 32 k + l
+    uint32_t *orient = nullptr;    // per 32 codes, bit l: the pair's first node is the later local node
+    uint2 *slots = nullptr;        // block 1: CSR positions of (r, c) and (c, r) (the latter none when r = c)
+    uint4 *slots3 = nullptr;       // block 3: position of (3r, 3c), length of row 3r, the same for (3c, 3r)
+    // at least kHostChunkMinNnz values: up to kHostChunks copies, by `slice`, and
+    // the steps of the passes between them
+    std::vector<PairStep> steps;
+    std::vector<PairCopy> copies;
+};
+}  // namespace skg
+
 // Pattern handle (defined here so every translation unit sees the layout).
 struct skg_pattern {
     int64_t n_elements = 0, n_rows = 0, n_cols = 0, nnz = 0;
@@ -221,6 +253,9 @@ struct skg_pattern {
     // one int4 per incidence in `inc` order, x = e*row_local + i and the
     // bytes of y, z, w = column offset within the row of each local column.
     skg::DevBuf<int4> rec;
+    // Pair plan (row and column DOFs coincide), used by the assemblies of
+    // symmetric element matrices.
+    skg::PairPlan pairs;
 };
 
 

@@ -224,6 +224,8 @@ __global__ void k_element_span(int64_t n_rows, const int32_t *__restrict__ inc_p
     span[r] = i0 < i1 ? make_int2(inc[i0] / row_local, inc[i1 - 1] / row_local) : make_int2(INT_MAX, -1);
 }
 
+void build_pair_plan(skg_pattern *p, cudaStream_t s);
+
 // Incidence records for the warp-per-row assembly kernels; skipped when the
 // pattern is unsuitable (elements wider than 12 columns or rows of 256+
 // columns), in which case assemblies use the per-row global-memory gather.
@@ -295,50 +297,52 @@ void build_records(skg_pattern *p, cudaStream_t s) {
         for (size_t i = 0; i < vec->size(); ++i) key[i] = first_element((*vec)[i]);
         sort_by(*vec, key);
     }
-    // Host-output chunks: boundaries at group starts near equal slot counts.
-    const int64_t nnz = ip[p->n_rows];
-    p->hc_row.assign(1, 0);
-    for (int k = 1; k < kHostChunks; ++k) {
-        const int64_t target = nnz * k / kHostChunks;
-        const auto it = std::lower_bound(all.begin(), all.end(), target,
-                                         [&](const int2 &g, int64_t t) { return (int64_t)ip[g.x] < t; });
-        if (it != all.end() && it->x > p->hc_row.back()) p->hc_row.push_back(it->x);
-    }
-    p->hc_row.push_back((int32_t)p->n_rows);
-    const int n_chunks = (int)p->hc_row.size() - 1;
-    p->hc_slot.resize(n_chunks + 1);
-    for (int c = 0; c <= n_chunks; ++c) p->hc_slot[c] = ip[p->hc_row[c]];
-    p->hc_ready.assign(n_chunks, 0);
-    auto chunk_of = [&](int32_t row) {
-        return (int)(std::upper_bound(p->hc_row.begin(), p->hc_row.end(), row) - p->hc_row.begin()) - 1;
-    };
-    for (int c = 0; c < n_chunks; ++c)
-        for (int32_t q = p->hc_row[c]; q < p->hc_row[c + 1]; ++q)
-            p->hc_ready[c] = std::max(p->hc_ready[c], (int64_t)span[q].y + 1);
-    std::vector<int2> hc_small = small, hc_large = large;
-    for (auto *vec : {&hc_small, &hc_large}) {
-        std::vector<int64_t> key(vec->size());
-        for (size_t i = 0; i < vec->size(); ++i) key[i] = chunk_of((*vec)[i].x);
-        sort_by(*vec, key);  // stable: first-element order within a chunk
-    }
-    auto offsets = [&](const std::vector<int2> &vec, std::vector<int32_t> &off) {
-        off.assign(n_chunks + 1, 0);
-        for (const int2 &g : vec) ++off[chunk_of(g.x) + 1];
-        for (int c = 0; c < n_chunks; ++c) off[c + 1] += off[c];
-    };
-    offsets(hc_small, p->hc_small_off);
-    offsets(hc_large, p->hc_large_off);
     auto upload = [&](const std::vector<int2> &vec, DevBuf<int2> &dst) {
         dst = DevBuf<int2>::owned(vec.size());
         if (!vec.empty())
             SKG_CUDA(cudaMemcpyAsync(dst.get(), vec.data(), vec.size() * 8, cudaMemcpyHostToDevice, s));
     };
+    if (ip[p->n_rows] >= kHostChunkMinNnz) {
+        // Host-output chunks: boundaries at group starts near equal slot counts.
+        const int64_t nnz = ip[p->n_rows];
+        p->hc_row.assign(1, 0);
+        for (int k = 1; k < kHostChunks; ++k) {
+            const int64_t target = nnz * k / kHostChunks;
+            const auto it = std::lower_bound(all.begin(), all.end(), target,
+                                             [&](const int2 &g, int64_t t) { return (int64_t)ip[g.x] < t; });
+            if (it != all.end() && it->x > p->hc_row.back()) p->hc_row.push_back(it->x);
+        }
+        p->hc_row.push_back((int32_t)p->n_rows);
+        const int n_chunks = (int)p->hc_row.size() - 1;
+        p->hc_slot.resize(n_chunks + 1);
+        for (int c = 0; c <= n_chunks; ++c) p->hc_slot[c] = ip[p->hc_row[c]];
+        p->hc_ready.assign(n_chunks, 0);
+        auto chunk_of = [&](int32_t row) {
+            return (int)(std::upper_bound(p->hc_row.begin(), p->hc_row.end(), row) - p->hc_row.begin()) - 1;
+        };
+        for (int c = 0; c < n_chunks; ++c)
+            for (int32_t q = p->hc_row[c]; q < p->hc_row[c + 1]; ++q)
+                p->hc_ready[c] = std::max(p->hc_ready[c], (int64_t)span[q].y + 1);
+        std::vector<int2> hc_small = small, hc_large = large;
+        for (auto *vec : {&hc_small, &hc_large}) {
+            std::vector<int64_t> key(vec->size());
+            for (size_t i = 0; i < vec->size(); ++i) key[i] = chunk_of((*vec)[i].x);
+            sort_by(*vec, key);  // stable: first-element order within a chunk
+        }
+        auto offsets = [&](const std::vector<int2> &vec, std::vector<int32_t> &off) {
+            off.assign(n_chunks + 1, 0);
+            for (const int2 &g : vec) ++off[chunk_of(g.x) + 1];
+            for (int c = 0; c < n_chunks; ++c) off[c + 1] += off[c];
+        };
+        offsets(hc_small, p->hc_small_off);
+        offsets(hc_large, p->hc_large_off);
+        upload(hc_small, p->hc_small);
+        upload(hc_large, p->hc_large);
+    }
     p->n_groups_small = (int32_t)small.size();
     p->n_groups_large = (int32_t)large.size();
     upload(small, p->groups_small);
     upload(large, p->groups_large);
-    upload(hc_small, p->hc_small);
-    upload(hc_large, p->hc_large);
     SKG_CUDA(cudaStreamSynchronize(s));
     p->max_row_len = longest;
 }
@@ -425,6 +429,7 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
             SKG_LAUNCH_CHECK("row_columns_write");
             SKG_CUDA(cudaStreamSynchronize(s));
             build_records(p, s);
+            if (d_row_dofs == d_col_dofs && row_local == col_local && n_rows == n_cols) build_pair_plan(p, s);
         } catch (...) {
             delete p;
             throw;

@@ -1,0 +1,52 @@
+"""Pair sums against the oracle where tiles, windows and slices end: one cell, a tile of 64 elements
+and two more, whole tiles, an odd box; scalar, symmetric and partly nonsymmetric coefficients.
+
+Tolerances (largest error over the largest entry): an FP64 entry is at most 24 contributions of about 60
+roundings each, 2^-53 apiece relative to the contributions: 1e-12 holds with margin; double-float 1e-12 and
+split FP32 1e-7 are the modes' own bounds."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+sk = pytest.importorskip("skfemntv_gb300")
+import oracle as O  # noqa: E402
+from skfemntv_gb300.assembly import NativeTensorForm  # noqa: E402
+
+BOUND = {"fp64": 1e-12, "fp64_emulated": 1e-12, "split_fp32": 1e-7}
+
+
+def _mesh(cells, seed=3):
+    m = sk.MeshTet.init_tensor(*(np.linspace(0.0, 1.0, n + 1) for n in cells))
+    rng = np.random.default_rng(seed)
+    p = m.p + rng.uniform(-0.15, 0.15, m.p.shape) / np.array(cells)[:, None]
+    return sk.MeshTet(p, m.t)
+
+
+def _tensors(E, kind):
+    rng = np.random.default_rng(7)
+    B = rng.standard_normal((E, 3, 3))
+    A = np.einsum("eij,ekj->eik", B, B) + 2 * np.eye(3)
+    if kind == "mixed":  # the last element of the first tile and the mesh's last one
+        for e in {min(63, E - 1), E - 1}:
+            A[e, 0, 2] += 0.7
+            A[e, 2, 1] -= 0.4
+    return A
+
+
+@pytest.mark.parametrize("kind", ["symmetric", "mixed"])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (11, 1, 1), (4, 4, 4), (7, 5, 3)])
+@pytest.mark.parametrize("precision", sorted(BOUND))
+@pytest.mark.parametrize("order", [1, 2])
+def test_tensor_form(order, precision, cells, kind):
+    m = _mesh(cells)
+    if order == 2:
+        m = sk.MeshTet2.from_mesh(m)
+    elem = sk.ElementTetP2() if order == 2 else sk.ElementTetP1()
+    basis = sk.Basis(m, sk.ElementVector(elem, dim=1))
+    E, Q = basis._coefficient_shape
+    A = np.broadcast_to(np.moveaxis(_tensors(E, kind), 0, -1)[..., None], (3, 3, E, Q))
+    K = NativeTensorForm(basis).assemble(A, precision)
+    ob = O.make_basis(m.p, m.t, order == 2, quadrature=(basis.X, basis.W))
+    data, indptr, indices = O.cross_gradient_tensor_assemble(ob, O.anisotropic_tensor(A, ob.dx.shape))
+    assert np.array_equal(K.indptr, indptr) and np.array_equal(K.indices, indices)
+    assert np.max(np.abs(K.data - data)) <= BOUND[precision] * np.max(np.abs(data))
