@@ -45,6 +45,19 @@ __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p,
 
 namespace {
 
+// Full element matrices (E, 3n, 3n) from packed blocks: patterns without a
+// plan.  Thread per entry.
+__global__ void k_expand_blocks(int64_t ne, int64_t stride, int n, const double *__restrict__ K,
+                                double *__restrict__ full) {
+    const int L = 3 * n;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ne * L * L) return;
+    const int64_t e = i / (L * L);
+    const int q = (int)(i - e * L * L), r = q / L, c = q - r * L, a = r / 3, b = c / 3, x = r % 3, y = c % 3;
+    const int64_t t = a <= b ? tri_index(n, a, b) : tri_index(n, b, a);
+    full[i] = K[(t * stride + e) * 9 + (a <= b ? x * 3 + y : y * 3 + x)];
+}
+
 // Node-level view of a pattern with C components per node (C = 1: its DOFs).
 template <int C>
 struct NodeView {
@@ -204,7 +217,7 @@ template <int C>
 __global__ void __launch_bounds__(kPairWindow) k_pair_fill(NodeView<C> v, const int32_t *__restrict__ pair_ptr,
                                                            const int32_t *__restrict__ pair_row,
                                                            const int32_t *__restrict__ order,
-                                                           const int32_t *__restrict__ slice_ptr, int np,
+                                                           const int32_t *__restrict__ slice_ptr, int np, int64_t stride,
                                                            uint32_t *__restrict__ codes,
                                                            uint32_t *__restrict__ orient, uint2 *__restrict__ slots,
                                                            uint4 *__restrict__ slots3, int n_chunks,
@@ -222,8 +235,9 @@ __global__ void __launch_bounds__(kPairWindow) k_pair_fill(NodeView<C> v, const 
     if (j >= 0) {
         const int32_t r = pair_row[j], c = pair_column(v, r, j, pair_ptr);
         each_contribution(v, r, c, [&](int32_t e, int a, int b) {
+            const uint32_t t = (uint32_t)tri_index(v.n, min(a, b), max(a, b));
             codes[(int64_t)k * 32 + lane] =
-                (uint32_t)e * (uint32_t)np + (uint32_t)tri_index(v.n, min(a, b), max(a, b));
+                C == 1 ? (uint32_t)e * (uint32_t)np + t : t * (uint32_t)stride + (uint32_t)e;
             if (a > b) atomicOr(orient + k, 1u << lane);
             ++k;
         });
@@ -316,8 +330,8 @@ void build(skg_pattern *p, cudaStream_t s) {
         SKG_LAUNCH_CHECK("copy_rows");
     }
     k_pair_fill<C><<<n_windows, kPairWindow, 0, s>>>(v, pair_ptr.get(), pair_row.get(), order.get(),
-                                                    plan.slice_ptr, plan.np, plan.codes, plan.orient, plan.slots,
-                                                    plan.slots3, n_chunks, first, done);
+                                                    plan.slice_ptr, plan.np, block_stride(p->n_elements), plan.codes,
+                                                    plan.orient, plan.slots, plan.slots3, n_chunks, first, done);
     SKG_LAUNCH_CHECK("pair_fill");
     if (n_chunks) {
         download(h, chunk.get(), 3 * (kHostChunks + 1), s);
@@ -349,6 +363,12 @@ void build(skg_pattern *p, cudaStream_t s) {
 
 }  // namespace
 
+void expand_blocks(int64_t ne, int n, const double *K, double *full, cudaStream_t s) {
+    if (ne == 0) return;
+    k_expand_blocks<<<grid_for(ne * 9 * n * n, 256), 256, 0, s>>>(ne, block_stride(ne), n, K, full);
+    SKG_LAUNCH_CHECK("expand_blocks");
+}
+
 // Plan of a pattern whose row and column DOFs are the same array; none when
 // the packed positions exceed 32 bits (the assemblies then walk the rows).
 void build_pair_plan(skg_pattern *p, cudaStream_t s) {
@@ -357,7 +377,7 @@ void build_pair_plan(skg_pattern *p, cudaStream_t s) {
     // the element shapes that are assembled through a plan
     if (C == 1 && L != 4 && L != 6 && L != 10) return;
     const int64_t n = L / C, total = p->n_elements * L;
-    if (p->n_elements * (n * (n + 1) / 2) >= (int64_t)kPairNone) return;
+    if (block_stride(p->n_elements) * (n * (n + 1) / 2) >= (int64_t)kPairNone) return;
     if (C == 1) {
         build<1>(p, s);
         return;

@@ -218,12 +218,19 @@ inline void pair_sum(const PairPlan &plan, int s0, int s1, const E *K, const Pai
     SKG_LAUNCH_CHECK("pair_sum");
 }
 
-// Three components per node: packed blocks (E, np, 3, 3), a block of threads
-// per slice, nine threads per pair.
+// Three components per node: packed blocks (np, stride, 3, 3), block t of
+// element e at (t * stride + e) * 9; the blocks of 32 elements are one
+// contiguous, 16-byte aligned range for each t.  A block of threads per slice,
+// nine threads per pair.
+inline int64_t block_stride(int64_t ne) { return (ne + kTile - 1) / kTile * kTile; }
+
 constexpr int kPairBlock3 = 288;
 
 __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p, const double *__restrict__ K,
                                                            double *__restrict__ values);
+
+// Packed blocks to full matrices (E, 3n, 3n), for patterns without a plan.
+void expand_blocks(int64_t ne, int n, const double *K, double *full, cudaStream_t s);
 
 inline void pair_sum3(const PairPlan &plan, int s0, int s1, const double *K, double *values, cudaStream_t s) {
     if (s1 <= s0) return;
@@ -243,14 +250,21 @@ inline void pair_sum3(const PairPlan &plan, int s0, int s1, const double *K, dou
 // gains: P2 FP64 at 64^3 1.01 ms in one step, 1.10 in four and 1.22 in eight
 // on one stream, 1.60 in eight on two streams.)  Large host output: in steps on
 // s, each followed by the copies of the row chunks that it completes on the
-// copy stream, which hide the steps.
-template <class FE, class FS>
+// copy stream, which hide the steps.  tail(cs) queues what follows the sums on
+// s; what it copies to the host goes on cs (ordered after s when it is another
+// stream), before the values' last copies are waited for.
+struct NoTail {
+    void operator()(cudaStream_t) const {}
+};
+
+template <class FE, class FS, class FT = NoTail>
 void run_pair_passes(const skg_pattern *pat, int64_t ne, double *d_values, double *h_values, cudaStream_t s, FE &&elem,
-                     FS &&sums) {
+                     FS &&sums, FT &&tail = NoTail{}) {
     const PairPlan &plan = pat->pairs;
     if (!h_values || plan.copies.empty()) {
         if (ne) elem((int64_t)0, ne);
         sums(0, plan.n_slices, s);
+        tail(s);
         if (h_values && pat->nnz)
             SKG_CUDA(cudaMemcpyAsync(h_values, d_values, (size_t)pat->nnz * sizeof(double), cudaMemcpyDeviceToHost, s));
         return;
@@ -281,6 +295,7 @@ void run_pair_passes(const skg_pattern *pat, int64_t ne, double *d_values, doubl
             }
         }
         if (done < ne) elem(done, ne);  // elements no row references
+        tail(cs);
         ev.order(cs, s);
     } catch (...) {
         // scratch freed on s after this call must outlive the queued work
@@ -315,5 +330,40 @@ __device__ __forceinline__ void store_tile(const void *stage, void *dst, int byt
     }
     __syncthreads();
 }
+
+// One warp's blocks t of its 32 elements (n of them valid), 9 doubles per lane
+// at stage + 9 * lane, to global memory as one bulk copy.  Two stages per warp:
+// `turn` counts the copies issued, and the stage about to be written was last
+// read by the copy before the previous one.
+struct WarpStore {
+    double *stages;  // two of kStage doubles each, 16-byte aligned
+    int turn = 0;
+    static constexpr int kStage = 32 * 12;
+
+    __device__ __forceinline__ double *next() {
+        if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
+        return stages + (turn & 1) * kStage;
+    }
+    // `per` doubles per lane are in the stage
+    __device__ __forceinline__ void store(double *dst, int n, int per) {
+        const double *stage = stages + (turn & 1) * kStage;
+        ++turn;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        const int bytes = n * per * 8, bulk = bytes & ~15;
+        if ((threadIdx.x & 31) == 0) {
+            if (bulk)
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                             "r"((uint32_t)__cvta_generic_to_shared(stage)), "r"(bulk)
+                             : "memory");
+            if (bulk < bytes) dst[bulk / 8] = stage[bulk / 8];
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+    }
+    __device__ __forceinline__ void finish() {
+        if ((threadIdx.x & 31) == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
+};
 
 }  // namespace skg

@@ -6,12 +6,13 @@ Ownership follows the reference: the plain bilinear path returns one reused
 (form, basis); the tensor (anisotropic) path returns a fresh copy.  The CSR
 pattern is built once per (form, basis) on the device.
 
-Path selection for scalar P1/P2 on affine meshes with coefficients that are
-constant over each element's quadrature points: the fused affine kernel
-(geometry + contraction + fixed-order CSR sum from coordinates).  Anything
-else (vector fields, symmetric-gradient / divergence / mass terms, per-point
-coefficients, curved P2 geometry) goes through the tabulated path (device
-geometry tabulation, element matrices, the same fixed-order gather).
+Path selection on affine meshes with coefficients that are constant over
+each element's quadrature points: gradient and tensor forms of scalar bases
+take the fused diffusion path, every other form (vector fields,
+symmetric-gradient / divergence / mass terms) the fused forms path; both go
+straight from coordinates to the CSR values.  Per-point coefficients and curved
+P2 geometry go through the tabulated path (device geometry tabulation, element
+matrices, fixed-order sums).
 """
 from __future__ import annotations
 
@@ -335,9 +336,9 @@ class NativeBilinearForm:
             return self.target.d_values
         if prec != SKG_FP64:
             raise UnsupportedNativeForm("split precision is available on the affine scalar gradient path")
-        forms = self._p1_forms(value, gradient, symmetric_gradient, divergence)
+        forms = self._affine_forms(value, gradient, symmetric_gradient, divergence)
         if forms is not None:
-            self._p1_forms_launch(forms, dev.ptr(self.target.d_values), None)
+            self._affine_forms_launch(forms, dev.ptr(self.target.d_values), None)
             return self.target.d_values
         tab = b._device_tabulation()
         coefs = [self._point_coefficient(c, E, Q, n)
@@ -348,12 +349,12 @@ class NativeBilinearForm:
              dev.ptr(self.target.d_values), None, dev.stream_ptr())
         return self.target.d_values
 
-    def _p1_forms(self, value, gradient, symmetric_gradient, divergence):
+    def _affine_forms(self, value, gradient, symmetric_gradient, divergence):
         """The four coefficients as (E,) arrays, 0-d scalars or None when the
-        fused P1 path applies (affine P1 basis with 1 or 3 components, every
-        coefficient constant on each element, row-grouped pattern), else None."""
+        fused path applies (affine basis with 1 or 3 components, every
+        coefficient constant on each element), else None."""
         b = self.basis
-        if b._nodes != 4 or b._comp not in (1, 3) or not b.is_affine or not self.pattern.row_groups:
+        if b._comp not in (1, 3) or not b.is_affine:
             return None
         E, Q = b._coefficient_shape
         out = []
@@ -370,8 +371,8 @@ class NativeBilinearForm:
             out.append(pe)
         return out
 
-    def _p1_forms_launch(self, forms, d_values, h_values):
-        """skg_p1_assemble_affine_forms; per-element arrays are read in place
+    def _affine_forms_launch(self, forms, d_values, h_values):
+        """skg_h1_assemble_affine_forms; per-element arrays are read in place
         from host memory when `h_values` is given (the caller synchronises
         before the arrays go away), else uploaded.  Returns the uploads."""
         b = self.basis
@@ -388,8 +389,8 @@ class NativeBilinearForm:
                 ptr = dev.ptr(keep[-1])
             ptrs.append(ptr)
             consts.append(0.0)
-        call("skg_p1_assemble_affine_forms", self.pattern.h, dev.ptr(b.mesh._dev("p")), b.mesh.p.shape[1],
-             dev.ptr(b.mesh._dev("t")), E, b._comp, Q, dev.hptr(b.X), dev.hptr(b.W), *ptrs, *consts,
+        call("skg_h1_assemble_affine_forms", self.pattern.h, dev.ptr(b.mesh._dev("p")), b.mesh.p.shape[1],
+             dev.ptr(b.mesh._dev("t")), b._nodes, E, b._comp, Q, dev.hptr(b.X), dev.hptr(b.W), *ptrs, *consts,
              d_values, h_values, dev.stream_ptr())
         return keep
 
@@ -429,9 +430,9 @@ class NativeBilinearForm:
         if fast is not None:
             self._affine(fast, _precision(precision), self.target.pinned_ptr(), host=True)
             return self.target.finish_direct()
-        forms = self._p1_forms(value, gradient, symmetric_gradient, divergence)
+        forms = self._affine_forms(value, gradient, symmetric_gradient, divergence)
         if forms is not None and _precision(precision) == SKG_FP64:
-            self._p1_forms_launch(forms, dev.ptr(self.target.d_values), self.target.pinned_ptr())
+            self._affine_forms_launch(forms, dev.ptr(self.target.d_values), self.target.pinned_ptr())
             return self.target.finish_direct()
         self.assemble_device(value=value, gradient=gradient, symmetric_gradient=symmetric_gradient,
                              divergence=divergence, precision=precision)

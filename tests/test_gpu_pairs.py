@@ -50,3 +50,32 @@ def test_tensor_form(order, precision, cells, kind):
     data, indptr, indices = O.cross_gradient_tensor_assemble(ob, O.anisotropic_tensor(A, ob.dx.shape))
     assert np.array_equal(K.indptr, indptr) and np.array_equal(K.indices, indices)
     assert np.max(np.abs(K.data - data)) <= BOUND[precision] * np.max(np.abs(data))
+
+
+X1, W1 = np.full((3, 1), 0.25), np.array([1.0 / 6.0])
+KINDS = ("value", "gradient", "symmetric_gradient", "divergence")
+
+
+@pytest.mark.parametrize("one_point", [False, True])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (11, 1, 1), (4, 4, 4), (7, 5, 3)])
+@pytest.mark.parametrize("order,comp", [(1, 1), (1, 3), (2, 1), (2, 3)])
+def test_affine_forms(order, comp, cells, one_point):
+    """Every kind at once, per element and constant, on the default rules and on one that is not exact on
+    quadratics; bound as above (an entry of the vector P2 matrix takes about 60 roundings as well)."""
+    m = _mesh(cells)
+    if order == 2:
+        m = sk.MeshTet2.from_mesh(m)
+    elem = sk.ElementTetP2() if order == 2 else sk.ElementTetP1()
+    quadrature = (X1, W1) if one_point else None
+    basis = sk.Basis(m, sk.ElementVector(elem, dim=comp), quadrature=quadrature)
+    ob = O.make_basis(m.p, m.t, order == 2, comp=comp, quadrature=quadrature)
+    form = sk.NativeBilinearForm(basis)
+    rng = np.random.default_rng(1)
+    E, Q = basis._coefficient_shape
+    for co in ({k: rng.uniform(0.5, 2.0, (E, 1)) for k in KINDS}, dict(zip(KINDS, (0.5, 0.8, 1.6, 1.3)))):
+        K = form.assemble(**co)
+        assert basis._tab is None  # no tabulated point data
+        full = {k: np.broadcast_to(c, (E, Q)) for k, c in co.items()}
+        data, indptr, indices = O.bilinear_assemble(ob, **full)
+        assert np.array_equal(K.indptr, indptr) and np.array_equal(K.indices, indices)
+        assert np.max(np.abs(K.data - data)) <= 1e-12 * np.max(np.abs(data))
