@@ -184,6 +184,18 @@ int skg_cross_assemble_tabulated(const skg_pattern *pattern, int64_t n_elements,
                                  const double *d_dx, const double *d_coef,
                                  double *d_values, void *stream);
 
+/* The same element matrices from coordinates, for a coefficient that is constant
+ * on every element of an affine mesh (d_coef (E), or NULL: the constant c_coef)
+ * and the kinds of NativeCrossBilinearForm.assemble (bilinear_form.py:180-242):
+ * 0 value, 1 gradient, 2 row divergence (Ct 3, Cc 1), 3 column divergence
+ * (Ct 1, Cc 3).  nt / nc: 4 (P1) or 10 (P2) test / trial nodes.  No contraction
+ * tensor and no tabulated basis data is read.  Stream-ordered. */
+int skg_cross_assemble_affine(const skg_pattern *pattern, const double *d_p, int64_t npts,
+                              const int32_t *d_t, int64_t n_elements, int32_t nq,
+                              const double *h_X, const double *h_W, int32_t kind, int32_t nt,
+                              int32_t Ct, int32_t nc, int32_t Cc, const double *d_coef,
+                              double c_coef, double *d_values, void *stream);
+
 /* ------------------------------------------------------------------ */
 /* Fused scalar P1/P2 assembly straight from mesh coordinates.          */
 /* Replaces the whole `asm(BilinearForm, Basis)` chain for             */
@@ -415,6 +427,18 @@ int skg_linear_assemble_tabulated(const skg_pattern *pattern,
                                   const double *d_w, const double *d_value,
                                   const double *d_gradient, double *d_out,
                                   void *stream);
+
+/* The same vector on an affine mesh, from coordinates and the rule: nodes 4 (P1)
+ * or 10 (P2), comp 1 or 3.  d_value (element, point, component) and d_gradient
+ * (element, point, component, direction) are read by the given strides (in
+ * doubles; 0 for an axis the coefficient does not vary over); either may be
+ * NULL.  Stream-ordered. */
+int skg_linear_assemble_affine(const skg_pattern *pattern, const double *d_p, int64_t npts,
+                               const int32_t *d_t, int32_t nodes, int64_t n_elements,
+                               int32_t comp, int32_t nq, const double *h_X, const double *h_W,
+                               const double *d_value, int64_t ve, int64_t vq, int64_t vc,
+                               const double *d_gradient, int64_t ge, int64_t gq, int64_t gc,
+                               int64_t gd, double *d_out, void *stream);
 
 /* ------------------------------------------------------------------ */
 /* Adjoint of J = u^T K(kappa) v for P1 diffusion (no counterpart in    */

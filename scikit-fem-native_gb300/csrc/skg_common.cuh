@@ -256,6 +256,10 @@ struct skg_pattern {
     // Pair plan (row and column DOFs coincide), used by the assemblies of
     // symmetric element matrices.
     skg::PairPlan pairs;
+    // The same lists for whole element matrices (every slot its own pair, codes
+    // element * row_local * col_local + position), for the shapes without a pair
+    // plan or row groups.
+    skg::PairPlan whole;
 };
 
 

@@ -281,15 +281,6 @@ __global__ void __launch_bounds__(kTile) k_form_scalar(int64_t ne, int64_t e_beg
     store_tile(stage, Ke + tile * kTile * NP, (int)(e_end - e0 < kTile ? e_end - e0 : kTile) * NP * 8);
 }
 
-// Full matrices (E, n, n) from packed upper triangles: patterns without a plan.
-__global__ void k_expand_scalar(int64_t ne, int n, const double *__restrict__ K, double *__restrict__ full) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ne * n * n) return;
-    const int64_t e = i / (n * n);
-    const int q = (int)(i - e * n * n), a = q / n, b = q - a * n;
-    full[i] = K[e * (n * (n + 1) / 2) + (a <= b ? tri_index(n, a, b) : tri_index(n, b, a))];
-}
-
 std::vector<double> form_table(int nodes, int nq, const double *X, const double *W) {
     const int np = nodes * (nodes + 1) / 2;
     std::vector<double> T(nodes == 4 ? kP1Table : kP2Table, 0.0);
@@ -377,8 +368,7 @@ void affine_forms_assemble(const skg_pattern *pat, const double *d_p, int64_t np
     if (comp == 3) {
         expand_blocks(ne, nodes, Ke.get(), full.get(), s);
     } else {
-        k_expand_scalar<<<grid_for(ne * L * L, 256), 256, 0, s>>>(ne, nodes, Ke.get(), full.get());
-        SKG_LAUNCH_CHECK("expand_scalar");
+        expand_packed(ne, nodes, Ke.get(), full.get(), s);
     }
     gather_element_matrices(pat, full.get(), d_values, s);
     if (h_values && pat->nnz)

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "skg_common.cuh"
+#include "skg_pairs.cuh"
 #include "skg_rows.cuh"
 
 namespace skg {
@@ -341,6 +342,10 @@ void gather_element_matrices(const skg_pattern *pat, const double *Ke, double *v
             case 12: add_element_rows<12>(pat, Ke, values, s); return;
             default: break;
         }
+    }
+    if (pat->whole.block) {
+        pair_sum<double>(pat->whole, 0, pat->whole.n_slices, Ke, PairLower<double>{}, PairIdentity{}, nullptr, values, s);
+        return;
     }
     k_gather_rows<<<grid_for(pat->n_rows, 128), 128, 0, s>>>(pat->n_rows, pat->indptr.get(), pat->indices.get(),
                                                              pat->inc_ptr.get(), pat->inc.get(), pat->col_dofs.get(),

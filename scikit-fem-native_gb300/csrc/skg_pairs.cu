@@ -45,8 +45,16 @@ __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p,
 
 namespace {
 
-// Full element matrices (E, 3n, 3n) from packed blocks: patterns without a
-// plan.  Thread per entry.
+// Full matrices (E, n, n) from packed upper triangles: patterns without a plan.
+__global__ void k_expand_packed(int64_t ne, int n, const double *__restrict__ K, double *__restrict__ full) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ne * n * n) return;
+    const int64_t e = i / (n * n);
+    const int q = (int)(i - e * n * n), a = q / n, b = q - a * n;
+    full[i] = K[e * (n * (n + 1) / 2) + (a <= b ? tri_index(n, a, b) : tri_index(n, b, a))];
+}
+
+// Full element matrices (E, 3n, 3n) from packed blocks, likewise.
 __global__ void k_expand_blocks(int64_t ne, int64_t stride, int n, const double *__restrict__ K,
                                 double *__restrict__ full) {
     const int L = 3 * n;
@@ -58,12 +66,14 @@ __global__ void k_expand_blocks(int64_t ne, int64_t stride, int n, const double 
     full[i] = K[(t * stride + e) * 9 + (a <= b ? x * 3 + y : y * 3 + x)];
 }
 
-// Node-level view of a pattern with C components per node (C = 1: its DOFs).
-template <int C>
+// Node-level view of a pattern with C components per node (C = 1: its DOFs);
+// C = 0: the DOFs of a pattern whose element matrices are summed whole.
+template <int K>
 struct NodeView {
-    const int32_t *dofs, *indptr, *indices, *inc_ptr, *inc;
-    int32_t L, n;
-    __device__ int32_t node(int64_t e, int b) const { return dofs[e * L + C * b] / C; }
+    static constexpr int C = K == 0 ? 1 : K;
+    const int32_t *cols, *indptr, *indices, *inc_ptr, *inc;
+    int32_t L, Lc, n;  // local rows, local columns, local column nodes
+    __device__ int32_t node(int64_t e, int b) const { return cols[e * Lc + C * b] / C; }
     __device__ int32_t begin(int32_t r) const { return indptr[C * r]; }
     __device__ int32_t length(int32_t r) const { return indptr[C * r + 1] - indptr[C * r]; }  // DOF columns
     __device__ int32_t col(int32_t rb, int p) const { return indices[rb + C * p] / C; }
@@ -86,15 +96,15 @@ __global__ void k_block_check(int64_t total, const int32_t *__restrict__ dofs, i
     }
 }
 
-template <int C>
-__global__ void k_upper_count(NodeView<C> v, int32_t rows, int32_t *__restrict__ n_upper) {
+template <int K>
+__global__ void k_upper_count(NodeView<K> v, int32_t rows, int32_t *__restrict__ n_upper) {
     const int32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows) return;
-    n_upper[r] = v.length(r) / C - v.position(r, r);
+    n_upper[r] = v.length(r) / v.C - (K == 0 ? 0 : v.position(r, r));
 }
 
-template <int C>
-__global__ void k_pair_rows(NodeView<C> v, int32_t rows, const int32_t *__restrict__ pair_ptr,
+template <int K>
+__global__ void k_pair_rows(NodeView<K> v, int32_t rows, const int32_t *__restrict__ pair_ptr,
                             int32_t *__restrict__ pair_row) {
     const int32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= rows) return;
@@ -103,8 +113,9 @@ __global__ void k_pair_rows(NodeView<C> v, int32_t rows, const int32_t *__restri
 
 // Calls f(element, a, b) for every contribution of pair (r, c), in the order
 // of row r's incidences (ascending elements).
-template <int C, class F>
-__device__ __forceinline__ void each_contribution(const NodeView<C> &v, int32_t r, int32_t c, F &&f) {
+template <int K, class F>
+__device__ __forceinline__ void each_contribution(const NodeView<K> &v, int32_t r, int32_t c, F &&f) {
+    constexpr int C = NodeView<K>::C;
     for (int32_t it = v.inc_ptr[C * r]; it < v.inc_ptr[C * r + 1]; ++it) {
         const int32_t item = v.inc[it];
         const int32_t e = item / v.L;
@@ -114,15 +125,15 @@ __device__ __forceinline__ void each_contribution(const NodeView<C> &v, int32_t 
     }
 }
 
-template <int C>
-__device__ __forceinline__ int32_t pair_column(const NodeView<C> &v, int32_t r, int32_t j, const int32_t *pair_ptr) {
+template <int K>
+__device__ __forceinline__ int32_t pair_column(const NodeView<K> &v, int32_t r, int32_t j, const int32_t *pair_ptr) {
     // the pairs of row r are the last columns of the row
-    return v.col(v.begin(r), v.length(r) / C - (pair_ptr[r + 1] - j));
+    return v.col(v.begin(r), v.length(r) / v.C - (pair_ptr[r + 1] - j));
 }
 
 // Contributions of every pair; per window, the last element (+ 1) it needs.
-template <int C>
-__global__ void __launch_bounds__(256) k_pair_count(NodeView<C> v, int32_t n_pairs,
+template <int K>
+__global__ void __launch_bounds__(256) k_pair_count(NodeView<K> v, int32_t n_pairs,
                                                     const int32_t *__restrict__ pair_ptr,
                                                     const int32_t *__restrict__ pair_row, int32_t *__restrict__ count,
                                                     int32_t *__restrict__ ready) {
@@ -190,8 +201,8 @@ __global__ void __launch_bounds__(kPairWindow) k_window_sort(int32_t n_pairs, co
 }
 
 // First rows of the host-output chunks, of about equal slot counts.
-template <int C>
-__global__ void k_copy_rows(NodeView<C> v, int32_t rows, int64_t nnz, int n_chunks, int32_t *__restrict__ first,
+template <int K>
+__global__ void k_copy_rows(NodeView<K> v, int32_t rows, int64_t nnz, int n_chunks, int32_t *__restrict__ first,
                             int32_t *__restrict__ slot) {
     const int k = threadIdx.x;
     if (k > n_chunks) return;
@@ -202,7 +213,7 @@ __global__ void k_copy_rows(NodeView<C> v, int32_t rows, int64_t nnz, int n_chun
         if (v.begin(mid) < target) lo = mid + 1; else hi = mid;
     }
     first[k] = k == n_chunks ? rows : lo;
-    slot[k] = v.indptr[C * first[k]];
+    slot[k] = v.indptr[v.C * first[k]];
 }
 
 __device__ __forceinline__ int chunk_of(const int32_t *first, int n_chunks, int32_t row) {
@@ -213,8 +224,8 @@ __device__ __forceinline__ int chunk_of(const int32_t *first, int n_chunks, int3
 
 // Codes, orientations and targets of every slice lane; one block per window.
 // done[k]: windows after which host-output chunk k is complete.
-template <int C>
-__global__ void __launch_bounds__(kPairWindow) k_pair_fill(NodeView<C> v, const int32_t *__restrict__ pair_ptr,
+template <int K>
+__global__ void __launch_bounds__(kPairWindow) k_pair_fill(NodeView<K> v, const int32_t *__restrict__ pair_ptr,
                                                            const int32_t *__restrict__ pair_row,
                                                            const int32_t *__restrict__ order,
                                                            const int32_t *__restrict__ slice_ptr, int np, int64_t stride,
@@ -223,6 +234,7 @@ __global__ void __launch_bounds__(kPairWindow) k_pair_fill(NodeView<C> v, const 
                                                            uint4 *__restrict__ slots3, int n_chunks,
                                                            const int32_t *__restrict__ first,
                                                            int32_t *__restrict__ done) {
+    constexpr int C = NodeView<K>::C;
     __shared__ unsigned touched;
     if (threadIdx.x == 0) touched = 0;
     __syncthreads();
@@ -235,15 +247,15 @@ __global__ void __launch_bounds__(kPairWindow) k_pair_fill(NodeView<C> v, const 
     if (j >= 0) {
         const int32_t r = pair_row[j], c = pair_column(v, r, j, pair_ptr);
         each_contribution(v, r, c, [&](int32_t e, int a, int b) {
-            const uint32_t t = (uint32_t)tri_index(v.n, min(a, b), max(a, b));
+            const uint32_t t = (uint32_t)(K == 0 ? a * v.n + b : tri_index(v.n, min(a, b), max(a, b)));
             codes[(int64_t)k * 32 + lane] =
                 C == 1 ? (uint32_t)e * (uint32_t)np + t : t * (uint32_t)stride + (uint32_t)e;
-            if (a > b) atomicOr(orient + k, 1u << lane);
+            if (K != 0 && a > b) atomicOr(orient + k, 1u << lane);
             ++k;
         });
         to.x = (uint32_t)(v.begin(r) + v.length(r) - C * (pair_ptr[r + 1] - j));
         len.x = (uint32_t)v.length(r);
-        if (r != c) {
+        if (K != 0 && r != c) {
             to.y = (uint32_t)(v.begin(c) + C * v.position(c, r));
             len.y = (uint32_t)v.length(c);
         }
@@ -266,31 +278,32 @@ void download(std::vector<T> &h, const T *d, size_t n, cudaStream_t s) {
     SKG_CUDA(cudaStreamSynchronize(s));
 }
 
-template <int C>
-void build(skg_pattern *p, cudaStream_t s) {
-    const NodeView<C> v{p->row_dofs.get(), p->indptr.get(), p->indices.get(),    p->inc_ptr.get(),
-                        p->inc.get(),      p->row_local,    p->row_local / C};
+template <int K>
+PairPlan build(const skg_pattern *p, cudaStream_t s) {
+    constexpr int C = NodeView<K>::C;
+    const NodeView<K> v{p->col_dofs.get(), p->indptr.get(), p->indices.get(), p->inc_ptr.get(),
+                        p->inc.get(),      p->row_local,    p->col_local,     p->col_local / C};
     const int32_t rows = (int32_t)(p->n_rows / C);
     PairPlan plan;
     plan.nodes = v.n;
-    plan.np = v.n * (v.n + 1) / 2;
+    plan.np = K == 0 ? p->row_local * p->col_local : v.n * (v.n + 1) / 2;
     DevBuf<int32_t> n_upper(rows + 1, s), pair_ptr(rows + 1, s);
-    k_upper_count<C><<<grid_for(rows, 256), 256, 0, s>>>(v, rows, n_upper.get());
+    k_upper_count<K><<<grid_for(rows, 256), 256, 0, s>>>(v, rows, n_upper.get());
     SKG_LAUNCH_CHECK("upper_count");
     exclusive_scan_i32(n_upper.get(), pair_ptr.get(), rows, s);
     std::vector<int32_t> h;
     download(h, pair_ptr.get() + rows, 1, s);
     const int32_t n_pairs = h[0];
-    if (n_pairs <= 0) return;
+    if (n_pairs <= 0) return PairPlan{};
     const int32_t n_windows = (n_pairs - 1) / kPairWindow + 1;
     const int64_t n_lanes = (int64_t)n_windows * kPairWindow;
     plan.n_slices = (int32_t)(n_lanes / 32);
     DevBuf<int32_t> pair_row(n_pairs, s), count(n_pairs, s), ready(n_windows, s), windows(n_windows, s);
     DevBuf<int32_t> order(n_lanes, s), width(plan.n_slices + 1, s);
     SKG_CUDA(cudaMemsetAsync(ready.get(), 0, (size_t)n_windows * 4, s));
-    k_pair_rows<C><<<grid_for(rows, 256), 256, 0, s>>>(v, rows, pair_ptr.get(), pair_row.get());
+    k_pair_rows<K><<<grid_for(rows, 256), 256, 0, s>>>(v, rows, pair_ptr.get(), pair_row.get());
     SKG_LAUNCH_CHECK("pair_rows");
-    k_pair_count<C><<<grid_for(n_pairs, 256), 256, 0, s>>>(v, n_pairs, pair_ptr.get(), pair_row.get(), count.get(),
+    k_pair_count<K><<<grid_for(n_pairs, 256), 256, 0, s>>>(v, n_pairs, pair_ptr.get(), pair_row.get(), count.get(),
                                                           ready.get());
     SKG_LAUNCH_CHECK("pair_count");
     // windows by the elements they need
@@ -321,15 +334,15 @@ void build(skg_pattern *p, cudaStream_t s) {
     plan.slice_ptr = reinterpret_cast<int32_t *>(at += orient_bytes);
     SKG_CUDA(cudaMemcpyAsync(plan.slice_ptr, slice_ptr.get(), ptr_bytes, cudaMemcpyDeviceToDevice, s));
     SKG_CUDA(cudaMemsetAsync(plan.orient, 0, orient_bytes, s));
-    const int n_chunks = p->nnz >= kHostChunkMinNnz ? kHostChunks : 0;
+    const int n_chunks = K != 0 && p->nnz >= kHostChunkMinNnz ? kHostChunks : 0;
     DevBuf<int32_t> chunk(3 * (kHostChunks + 1), s);  // first rows, first slots, windows done
     int32_t *first = chunk.get(), *slot = first + kHostChunks + 1, *done = slot + kHostChunks + 1;
     if (n_chunks) {
         SKG_CUDA(cudaMemsetAsync(chunk.get(), 0, 3 * (kHostChunks + 1) * 4, s));
-        k_copy_rows<C><<<1, 32, 0, s>>>(v, rows, p->nnz, n_chunks, first, slot);
+        k_copy_rows<K><<<1, 32, 0, s>>>(v, rows, p->nnz, n_chunks, first, slot);
         SKG_LAUNCH_CHECK("copy_rows");
     }
-    k_pair_fill<C><<<n_windows, kPairWindow, 0, s>>>(v, pair_ptr.get(), pair_row.get(), order.get(),
+    k_pair_fill<K><<<n_windows, kPairWindow, 0, s>>>(v, pair_ptr.get(), pair_row.get(), order.get(),
                                                     plan.slice_ptr, plan.np, block_stride(p->n_elements), plan.codes,
                                                     plan.orient, plan.slots, plan.slots3, n_chunks, first, done);
     SKG_LAUNCH_CHECK("pair_fill");
@@ -358,10 +371,16 @@ void build(skg_pattern *p, cudaStream_t s) {
             plan.steps.push_back(PairStep{plan.n_slices, p->n_elements});
     }
     plan.block = C;
-    p->pairs = std::move(plan);
+    return plan;
 }
 
 }  // namespace
+
+void expand_packed(int64_t ne, int n, const double *K, double *full, cudaStream_t s) {
+    if (ne == 0) return;
+    k_expand_packed<<<grid_for(ne * n * n, 256), 256, 0, s>>>(ne, n, K, full);
+    SKG_LAUNCH_CHECK("expand_packed");
+}
 
 void expand_blocks(int64_t ne, int n, const double *K, double *full, cudaStream_t s) {
     if (ne == 0) return;
@@ -369,27 +388,33 @@ void expand_blocks(int64_t ne, int n, const double *K, double *full, cudaStream_
     SKG_LAUNCH_CHECK("expand_blocks");
 }
 
-// Plan of a pattern whose row and column DOFs are the same array; none when
-// the packed positions exceed 32 bits (the assemblies then walk the rows).
-void build_pair_plan(skg_pattern *p, cudaStream_t s) {
+// Plans of a pattern: the pair plan when its row and column DOFs are the same
+// array (`square`) and its shape is one that is assembled symmetric; the whole
+// sums for the shapes that no row group serves.  None when the positions exceed
+// 32 bits (the assemblies then walk the rows).
+void build_pair_plan(skg_pattern *p, bool square, cudaStream_t s) {
     if (p->n_rows == 0 || p->n_elements == 0) return;
     const int L = p->row_local, C = L == 12 || L == 30 ? 3 : 1;
-    // the element shapes that are assembled through a plan
-    if (C == 1 && L != 4 && L != 6 && L != 10) return;
     const int64_t n = L / C, total = p->n_elements * L;
-    if (block_stride(p->n_elements) * (n * (n + 1) / 2) >= (int64_t)kPairNone) return;
-    if (C == 1) {
-        build<1>(p, s);
-        return;
+    if (square && (C == 3 ? p->n_rows % 3 == 0 : L == 4 || L == 6 || L == 10) &&
+        block_stride(p->n_elements) * (n * (n + 1) / 2) < (int64_t)kPairNone) {
+        if (C == 1) {
+            p->pairs = build<1>(p, s);
+            return;
+        }
+        DevBuf<int32_t> bad(1, s);
+        SKG_CUDA(cudaMemsetAsync(bad.get(), 0, 4, s));
+        k_block_check<<<grid_for(total, 256), 256, 0, s>>>(total, p->row_dofs.get(), bad.get());
+        SKG_LAUNCH_CHECK("block_check");
+        std::vector<int32_t> h;
+        download(h, bad.get(), 1, s);
+        if (h[0] == 0) {
+            p->pairs = build<3>(p, s);
+            return;
+        }
     }
-    if (p->n_rows % 3) return;
-    DevBuf<int32_t> bad(1, s);
-    SKG_CUDA(cudaMemsetAsync(bad.get(), 0, 4, s));
-    k_block_check<<<grid_for(total, 256), 256, 0, s>>>(total, p->row_dofs.get(), bad.get());
-    SKG_LAUNCH_CHECK("block_check");
-    std::vector<int32_t> h;
-    download(h, bad.get(), 1, s);
-    if (h[0] == 0) build<3>(p, s);
+    const bool grouped = p->max_row_len > 0 && L == p->col_local && (L == 4 || L == 6 || L == 10 || L == 12);
+    if (!grouped && p->n_elements * L * (int64_t)p->col_local < (int64_t)kPairNone) p->whole = build<0>(p, s);
 }
 
 }  // namespace skg

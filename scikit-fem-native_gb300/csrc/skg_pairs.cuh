@@ -229,7 +229,8 @@ constexpr int kPairBlock3 = 288;
 __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p, const double *__restrict__ K,
                                                            double *__restrict__ values);
 
-// Packed blocks to full matrices (E, 3n, 3n), for patterns without a plan.
+// Packed triangles / blocks to full matrices, for patterns without a plan.
+void expand_packed(int64_t ne, int n, const double *K, double *full, cudaStream_t s);
 void expand_blocks(int64_t ne, int n, const double *K, double *full, cudaStream_t s);
 
 inline void pair_sum3(const PairPlan &plan, int s0, int s1, const double *K, double *values, cudaStream_t s) {

@@ -224,7 +224,7 @@ __global__ void k_element_span(int64_t n_rows, const int32_t *__restrict__ inc_p
     span[r] = i0 < i1 ? make_int2(inc[i0] / row_local, inc[i1 - 1] / row_local) : make_int2(INT_MAX, -1);
 }
 
-void build_pair_plan(skg_pattern *p, cudaStream_t s);
+void build_pair_plan(skg_pattern *p, bool square, cudaStream_t s);
 
 // Incidence records for the warp-per-row assembly kernels; skipped when the
 // pattern is unsuitable (elements wider than 12 columns or rows of 256+
@@ -429,7 +429,7 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
             SKG_LAUNCH_CHECK("row_columns_write");
             SKG_CUDA(cudaStreamSynchronize(s));
             build_records(p, s);
-            if (d_row_dofs == d_col_dofs && row_local == col_local && n_rows == n_cols) build_pair_plan(p, s);
+            build_pair_plan(p, d_row_dofs == d_col_dofs && row_local == col_local && n_rows == n_cols, s);
         } catch (...) {
             delete p;
             throw;

@@ -79,6 +79,8 @@ SIGNATURES = {
                                     _vp],
     "skg_cross_assemble_tabulated": [_vp, _i64, _i32, _i32, _i32, _i32, _vp, _vp, _i32, _i32, _i32, _vp, _vp, _vp,
                                      _vp, _vp, _vp],
+    "skg_cross_assemble_affine": [_vp, _vp, _i64, _vp, _i64, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp,
+                                  ctypes.c_double, _vp, _vp],
     "skg_n1_vector_load": [_vp, _vp, _i64, _vp, _vp, _i64, _i32, _vp, _vp, _vp, _vp, _vp],
     "skg_n1_element_matrices": [_vp, _i64, _vp, _vp, _i64, _i32, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _vp,
                                 _vp],
@@ -97,6 +99,8 @@ SIGNATURES = {
     "skg_p1_assemble_affine_forms": [_vp, _vp, _i64, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp,
                                      ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double, _vp, _vp,
                                      _vp],
+    "skg_linear_assemble_affine": [_vp, _vp, _i64, _vp, _i32, _i64, _i32, _i32, _vp, _vp, _vp, _i64, _i64, _i64,
+                                   _vp, _i64, _i64, _i64, _i64, _vp, _vp],
     "skg_linear_assemble_tabulated": [_vp, _vp, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp,
                                       _vp, _vp],
 }

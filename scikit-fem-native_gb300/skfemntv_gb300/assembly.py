@@ -565,6 +565,8 @@ class NativeCrossBilinearForm:
         coefficient = np.asarray(coefficient, dtype=np.float64)
         scalar = np.broadcast_to(coefficient, self.coefficient_shape)
         Ct, Cc, d = self.test_components, self.trial_components, self.dimension
+        if self._affine_kind(kind, scalar):
+            return self.target.copy_matrix()
         if kind in ("row_divergence", "column_divergence"):
             if kind == "row_divergence":
                 if Ct != d or Cc != 1:
@@ -591,6 +593,35 @@ class NativeCrossBilinearForm:
                 row_kind = column_kind = "value"
         full = scalar[(...,) + (None,) * tensor.ndim] * tensor
         return self.assemble_tensor(row_kind, column_kind, full)
+
+    def _affine_kind(self, kind, scalar):
+        """Assembles ``kind`` straight from coordinates into the host matrix when
+        its components fit, the bases share mesh and rule, the mesh is affine and the coefficient (broadcast
+        to (cell, point)) is constant on each element; else False."""
+        tb, cb = self.test_basis, self.trial_basis
+        Ct, Cc, d = self.test_components, self.trial_components, self.dimension
+        code = {"value": 0, "gradient": 1, "row_divergence": 2, "column_divergence": 3}.get(kind)
+        fits = (Ct, Cc) == {2: (d, 1), 3: (1, d)}.get(code, (Cc, Cc))
+        if (code is None or not fits or tb.mesh is not cb.mesh or not np.array_equal(tb.X, cb.X)
+                or not np.array_equal(tb.W, cb.W) or not tb.is_affine):
+            return False
+        E, Q = self.coefficient_shape
+        if Q == 0:
+            return False
+        d_coef, constant = None, 0.0
+        if E == 0 or scalar.strides == (0, 0):
+            constant = float(scalar[0, 0]) if E else 0.0
+        else:
+            pe = per_element(scalar, E, Q, kind)
+            if pe is None:
+                return False
+            d_coef = dev.to_device(pe, np.float64)
+        mesh = tb.mesh
+        call("skg_cross_assemble_affine", self.pattern.h, dev.ptr(mesh._dev("p")), mesh.p.shape[1],
+             dev.ptr(mesh._dev("t")), E, Q, dev.hptr(tb.X), dev.hptr(tb.W), code, tb._nodes, Ct, cb._nodes, Cc,
+             dev.ptr(d_coef), constant, dev.ptr(self.target.d_values), dev.stream_ptr())
+        self.target.download()
+        return True
 
     def assemble_kinds(self, row_kind, column_kind, coefficient=1.0, *, num_threads=0):
         """Value / gradient contractions with a scalar coefficient c
@@ -696,6 +727,22 @@ class NativeLinearForm:
         except ValueError as error:
             raise ValueError(f"{name} coefficient must broadcast to {shape}") from error
 
+    def _upload(self, c, ndim):
+        """(device copy, element strides) of a coefficient that broadcasts to
+        (E, Q, C) or (E, Q, C, 3): only what it stores is copied, in the order
+        in which it is stored (the public component-first layout needs no
+        transposition on the host), and the kernel reads it by strides."""
+        if c is None:
+            return None, (0,) * ndim
+        c = np.broadcast_to(c, (self._shape if ndim == 3 else self._gradient_shape))
+        c = c[tuple(slice(1) if st == 0 else slice(None) for st in c.strides)]  # broadcast axes once
+        order = sorted(range(ndim), key=lambda k: -abs(c.strides[k]))
+        packed = np.ascontiguousarray(c.transpose(order))
+        strides = [0] * ndim
+        for k, axis in enumerate(order):
+            strides[axis] = packed.strides[k] // 8 if packed.shape[k] > 1 else 0
+        return dev.host_tensor(packed).to(dev.device()), tuple(strides)
+
     def assemble(self, *, value=None, gradient=None, num_threads=0):
         start = time.perf_counter()
         b = self.basis
@@ -704,15 +751,22 @@ class NativeLinearForm:
         gradient = self._coefficient("gradient", gradient, self._gradient_shape)
         if value is None and gradient is None:
             raise ValueError("at least one coefficient is required")
-        dv = dg = None
-        if value is not None:
-            dv = dev.to_device(np.ascontiguousarray(np.broadcast_to(value, self._shape)), np.float64)
-        if gradient is not None:
-            dg = dev.to_device(np.ascontiguousarray(np.broadcast_to(gradient, self._gradient_shape)), np.float64)
-        tab = b._device_tabulation()
-        call("skg_linear_assemble_tabulated", self.pattern.h, dev.ptr(b._dev_dofs()), E, b._nodes, C, Q,
-             dev.ptr(tab["shape"]), dev.ptr(tab["grad"]), dev.ptr(tab["dx"]), dev.ptr(dv), dev.ptr(dg),
-             dev.ptr(self.d_out), dev.stream_ptr())
+        if E and Q and C in (1, 3) and b.is_affine:
+            dv, vs = self._upload(value, 3)
+            dg, gs = self._upload(gradient, 4)
+            call("skg_linear_assemble_affine", self.pattern.h, dev.ptr(b.mesh._dev("p")), b.mesh.p.shape[1],
+                 dev.ptr(b.mesh._dev("t")), b._nodes, E, C, Q, dev.hptr(b.X), dev.hptr(b.W), dev.ptr(dv), *vs,
+                 dev.ptr(dg), *gs, dev.ptr(self.d_out), dev.stream_ptr())
+        else:
+            dv = dg = None
+            if value is not None:
+                dv = dev.to_device(np.ascontiguousarray(np.broadcast_to(value, self._shape)), np.float64)
+            if gradient is not None:
+                dg = dev.to_device(np.ascontiguousarray(np.broadcast_to(gradient, self._gradient_shape)), np.float64)
+            tab = b._device_tabulation()
+            call("skg_linear_assemble_tabulated", self.pattern.h, dev.ptr(b._dev_dofs()), E, b._nodes, C, Q,
+                 dev.ptr(tab["shape"]), dev.ptr(tab["grad"]), dev.ptr(tab["dx"]), dev.ptr(dv), dev.ptr(dg),
+                 dev.ptr(self.d_out), dev.stream_ptr())
         result = self.d_out[: b.N].cpu().numpy()
         return result, LinearFormDiagnostics(E, Q, time.perf_counter() - start)
 
