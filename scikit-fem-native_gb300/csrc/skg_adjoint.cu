@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "skg_common.cuh"
+#include "skg_fp64.cuh"
 
 namespace skg {
 namespace {
@@ -30,11 +31,12 @@ namespace {
 // C is det J times the gradient of lambda_{k+1}); the kernels apply the
 // powers of 1 / det J to a few scalars instead of forming J^-1.
 struct ElemAdj {
-    double C[9], det, id;  // id = 1 / det J
+    double C[4][3], id, aid;  // rows 1..3; id = 1 / det J, aid = 1 / |det J|
 };
 
-__device__ __forceinline__ bool elem_geom(const double *__restrict__ p, int64_t npts, const int32_t *__restrict__ t,
-                                          int64_t ne, int64_t e, int32_t v[4], ElemAdj &g) {
+__device__ __forceinline__ void elem_geom(const double *__restrict__ p, int64_t npts, const int32_t *__restrict__ t,
+                                          int64_t ne, int64_t e, const Fp64 &F, ElemAdj &g) {
+    int32_t v[4];
     bool ok = true;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -47,29 +49,41 @@ __device__ __forceinline__ bool elem_geom(const double *__restrict__ p, int64_t 
     for (int i = 0; i < 3; ++i) {
         const double x0 = p[i * npts + v[0]];
 #pragma unroll
-        for (int r = 0; r < 3; ++r) J[i * 3 + r] = p[i * npts + v[r + 1]] - x0;
+        for (int r = 0; r < 3; ++r) J[i * 3 + r] = F.sub(p[i * npts + v[r + 1]], x0);
     }
-    double *C = g.C;
-    C[0] = J[4] * J[8] - J[5] * J[7]; C[1] = J[2] * J[7] - J[1] * J[8]; C[2] = J[1] * J[5] - J[2] * J[4];
-    C[3] = J[5] * J[6] - J[3] * J[8]; C[4] = J[0] * J[8] - J[2] * J[6]; C[5] = J[2] * J[3] - J[0] * J[5];
-    C[6] = J[3] * J[7] - J[4] * J[6]; C[7] = J[1] * J[6] - J[0] * J[7]; C[8] = J[0] * J[4] - J[1] * J[3];
-    g.det = J[0] * C[0] + J[1] * C[3] + J[2] * C[6];
-    g.id = 1.0 / g.det;
-    return ok;
+    g.id = 1.0 / F.adjugate(J, g.C);
+    g.aid = fabs(g.id);
 }
 
-// C^T y: out_j = sum_k C[k][j] y_k  (det J times J^-T y)
-__device__ __forceinline__ void mul_CT(const double C[9], const double y[3], double out[3]) {
+// The element's differences of u and v, and a~ = det J grad u_e, b~ = det J grad v_e.
+__device__ __forceinline__ void elem_fields(const ElemAdj &g, const int32_t *__restrict__ dofs,
+                                            const double *__restrict__ u, const double *__restrict__ v, int64_t e,
+                                            const Fp64 &F, double a[3], double b[3]) {
+    const int32_t d0 = dofs[e * 4], d1 = dofs[e * 4 + 1], d2 = dofs[e * 4 + 2], d3 = dofs[e * 4 + 3];
+    const double u0 = u[d0], v0 = v[d0];
+    const double gu[3] = {F.sub(u[d1], u0), F.sub(u[d2], u0), F.sub(u[d3], u0)};
+    const double gv[3] = {F.sub(v[d1], v0), F.sub(v[d2], v0), F.sub(v[d3], v0)};
 #pragma unroll
-    for (int j = 0; j < 3; ++j) out[j] = C[0 * 3 + j] * y[0] + C[1 * 3 + j] * y[1] + C[2 * 3 + j] * y[2];
+    for (int j = 0; j < 3; ++j) {
+        a[j] = fma(g.C[3][j], gu[2], fma(g.C[2][j], gu[1], F.mul(g.C[1][j], gu[0])));
+        b[j] = fma(g.C[3][j], gv[2], fma(g.C[2][j], gv[1], F.mul(g.C[1][j], gv[0])));
+    }
 }
-// C y: out_i = sum_j C[i][j] y_j  (det J times J^-1 y)
-__device__ __forceinline__ void mul_C(const double C[9], const double y[3], double out[3]) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) out[i] = C[i * 3 + 0] * y[0] + C[i * 3 + 1] * y[1] + C[i * 3 + 2] * y[2];
+
+// 32-byte accesses: one full sector per thread.
+__device__ __forceinline__ void store4(double *p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+__device__ __forceinline__ void load4(const double *p, double x[4]) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3]) : "l"(p));
 }
 
 constexpr int kRed = 256;
+
+// One element's energy, the same expression in both passes (identical bits).
+__device__ __forceinline__ double elem_energy(double k, double wsum, double aid, double phi, const Fp64 &F) {
+    return F.mul(F.mul(F.mul(k, wsum), aid), phi);
+}
 
 // Forward: per-element energies reduced per block (fixed tree order).
 __global__ void __launch_bounds__(kRed) k_energy(int64_t ne, const double *__restrict__ p, int64_t npts,
@@ -81,17 +95,13 @@ __global__ void __launch_bounds__(kRed) k_energy(int64_t ne, const double *__res
     const int64_t e = (int64_t)blockIdx.x * kRed + threadIdx.x;
     double f = 0.0;
     if (e < ne) {
-        int32_t vt[4];
+        const Fp64 F = Fp64::load();
         ElemAdj g;
-        elem_geom(p, npts, t, ne, e, vt, g);
-        const int32_t d0 = dofs[e * 4], d1 = dofs[e * 4 + 1], d2 = dofs[e * 4 + 2], d3 = dofs[e * 4 + 3];
-        const double gu[3] = {u[d1] - u[d0], u[d2] - u[d0], u[d3] - u[d0]};
-        const double gv[3] = {v[d1] - v[d0], v[d2] - v[d0], v[d3] - v[d0]};
-        double a[3], b[3];  // det J times grad u_e, grad v_e
-        mul_CT(g.C, gu, a);
-        mul_CT(g.C, gv, b);
-        // kappa |det J| wsum (grad u_e . grad v_e) = kappa wsum (a . b) / |det J|
-        f = (kappa ? kappa[e] : 1.0) * wsum * fabs(g.id) * (a[0] * b[0] + a[1] * b[1] + a[2] * b[2]);
+        elem_geom(p, npts, t, ne, e, F, g);
+        double a[3], b[3];
+        elem_fields(g, dofs, u, v, e, F, a, b);
+        // kappa |det J| wsum (grad u_e . grad v_e) = kappa wsum (a~ . b~) / |det J|
+        f = elem_energy(kappa ? kappa[e] : 1.0, wsum, g.aid, F.dot(a, b), F);
     }
     red[threadIdx.x] = f;
     __syncthreads();
@@ -102,15 +112,20 @@ __global__ void __launch_bounds__(kRed) k_energy(int64_t ne, const double *__res
     if (threadIdx.x == 0) block_sums[blockIdx.x] = red[0];
 }
 
-// One warp, fixed order: lane l sums the block sums l, l + 32, ... in turn,
-// then the lanes are combined by a fixed shuffle tree.
-__global__ void k_sum_blocks(const double *__restrict__ in, int64_t n, double *__restrict__ out) {
-    const int lane = threadIdx.x & 31;
+// One block, fixed order: thread i sums the block sums i, i + 1024, ... in
+// turn, then the threads are combined by a fixed tree.
+__global__ void __launch_bounds__(1024) k_sum_blocks(const double *__restrict__ in, int64_t n,
+                                                     double *__restrict__ out) {
+    __shared__ double red[1024];
     double s = 0.0;
-    for (int64_t i = lane; i < n; i += 32) s += in[i];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
-    if (lane == 0) *out = s;
+    for (int64_t i = threadIdx.x; i < n; i += 1024) s += in[i];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int off = 512; off > 0; off >>= 1) {
+        if (threadIdx.x < off) red[threadIdx.x] += red[threadIdx.x + off];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *out = red[0];
 }
 
 // Element e's adjoint contributions (see k_energy_grad_elem); returns its energy.
@@ -118,65 +133,66 @@ __device__ __forceinline__ double elem_adjoint(int64_t ne, const double *__restr
                                                const int32_t *__restrict__ t, const int32_t *__restrict__ dofs,
                                                const double *__restrict__ kappa, const double *__restrict__ u,
                                                const double *__restrict__ v, double wsum, double gout,
-                                               double *__restrict__ gkappa, double *__restrict__ contrib,
-                                               int64_t e) {
-    int32_t vt[4];
+                                               double *__restrict__ gkappa, double *__restrict__ cx,
+                                               double *__restrict__ cv, int64_t e) {
+    const Fp64 F = Fp64::load();
     ElemAdj g;
-    elem_geom(p, npts, t, ne, e, vt, g);
-    const int32_t d0 = dofs[e * 4], d1 = dofs[e * 4 + 1], d2 = dofs[e * 4 + 2], d3 = dofs[e * 4 + 3];
-    const double gu[3] = {u[d1] - u[d0], u[d2] - u[d0], u[d3] - u[d0]};
-    const double gv[3] = {v[d1] - v[d0], v[d2] - v[d0], v[d3] - v[d0]};
+    elem_geom(p, npts, t, ne, e, F, g);
     // with tildes for the scaled quantities:  a = a~ / det, b = b~ / det,
     // c = J^-1 b = c~ / det^2, d = J^-1 a = d~ / det^2, phi = a . b = phi~ / det^2
     double a[3], b[3], c[3], d[3];
-    mul_CT(g.C, gu, a);
-    mul_CT(g.C, gv, b);
-    mul_C(g.C, b, c);
-    mul_C(g.C, a, d);
-    const double phi = a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
-    const double aid = fabs(g.id);
-    const double k = kappa ? kappa[e] : 1.0;
-    if (gkappa) gkappa[e] = gout * wsum * aid * phi;  // V phi = wsum phi~ / |det|
-    const double s2 = gout * k * wsum * aid;           // s / det^2 with s = gout kappa V
-    const double s3 = s2 * g.id;                       // s / det^3
-    double *out = contrib + e * 20;
-    // dJ/dJ_ij = s (phi Ji[j][i] - a_i c_j - b_i d_j) = s / det^3 (phi~ C[j][i] - a~_i c~_j - b~_i d~_j)
-    const double ph = s3 * phi;
-    double as[3], bs[3];
+    elem_fields(g, dofs, u, v, e, F, a, b);
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        as[i] = s3 * a[i];
-        bs[i] = s3 * b[i];
+    for (int k = 0; k < 3; ++k) {
+        c[k] = F.dot(g.C[k + 1], b);
+        d[k] = F.dot(g.C[k + 1], a);
     }
-    double col_sum[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            const double gJ = ph * g.C[j * 3 + i] - as[i] * c[j] - bs[i] * d[j];
-            out[(j + 1) * 3 + i] = gJ;  // vertex j+1, coordinate i
-            col_sum[i] += gJ;
-        }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) out[i] = -col_sum[i];
+    const double phi = F.dot(a, b);
+    const double k = kappa ? kappa[e] : 1.0;
+    if (gkappa) gkappa[e] = gout * wsum * g.aid * phi;  // V phi = wsum phi~ / |det|
+    const double s2 = F.mul(F.mul(F.mul(gout, k), wsum), g.aid);  // s / det^2 with s = gout kappa V
+    const double s3 = F.mul(s2, g.id);                            // s / det^3
     // dJ/du_m = s grad lambda_m . b = s c_{m-1} (m = 1..3), dJ/dv_m = s d_{m-1};
     // lambda_0's gradient is minus the sum of the others
-    double du[3], dv[3];
+    double du[4] = {0.0, 0.0, 0.0, 0.0};
+    if (cv) {
+        double dv[4];
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
-        du[m] = s2 * c[m];
-        dv[m] = s2 * d[m];
-        out[13 + m] = du[m];
-        out[17 + m] = dv[m];
+        for (int m = 0; m < 3; ++m) {
+            du[m + 1] = F.mul(s2, c[m]);
+            dv[m + 1] = F.mul(s2, d[m]);
+        }
+        du[0] = -F.add3(du[1], du[2], du[3]);
+        dv[0] = -F.add3(dv[1], dv[2], dv[3]);
+        store4(cv + e * 4, dv[0], dv[1], dv[2], dv[3]);
     }
-    out[12] = -(du[0] + du[1] + du[2]);
-    out[16] = -(dv[0] + dv[1] + dv[2]);
-    return k * wsum * aid * phi;  // the element energy, as k_energy forms it
+    // dJ/dJ_ij = s (phi Ji[j][i] - a_i c_j - b_i d_j) = s / det^3 (phi~ C[j][i] - a~_i c~_j - b~_i d~_j)
+    const double ph = F.mul(s3, phi);
+    double as[3], bs[3], sum[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        as[i] = F.mul(s3, a[i]);
+        bs[i] = F.mul(s3, b[i]);
+    }
+    double *out = cx + e * 16;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        double gJ[3];  // vertex j + 1
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            gJ[i] = fma(-bs[i], d[j], fma(-as[i], c[j], F.mul(ph, g.C[j + 1][i])));
+            sum[i] = j == 0 ? gJ[i] : F.add(sum[i], gJ[i]);
+        }
+        store4(out + (j + 1) * 4, gJ[0], gJ[1], gJ[2], du[j + 1]);
+    }
+    store4(out, -sum[0], -sum[1], -sum[2], du[0]);
+    return elem_energy(k, wsum, g.aid, phi, F);  // as k_energy forms it
 }
 
 // Backward, element pass: dJ/dkappa and the per-element vertex / DOF
-// contributions (scaled by the upstream gradient).  contrib layout per
-// element: 12 doubles dx (vertex k, coordinate i at k*3+i), 4 du, 4 dv.
+// contributions (scaled by the upstream gradient).  cx: per element and vertex
+// one 32-byte record (dx, dy, dz, du), stored and loaded as whole sectors; cv
+// (only when dJ/du or dJ/dv is wanted): 4 dv per element.
 // WITH_J: the element energies are also reduced per block exactly as
 // k_energy does (same expression, same tree), so that one pass gives J and
 // its gradients.
@@ -187,11 +203,12 @@ __global__ void __launch_bounds__(kRed) k_energy_grad_elem(int64_t ne, const dou
                                                            const double *__restrict__ kappa,
                                                            const double *__restrict__ u,
                                                            const double *__restrict__ v, double wsum, double gout,
-                                                           double *__restrict__ gkappa, double *__restrict__ contrib,
+                                                           double *__restrict__ gkappa, double *__restrict__ cx,
+                                                           double *__restrict__ cv,
                                                            double *__restrict__ block_sums) {
     const int64_t e = (int64_t)blockIdx.x * kRed + threadIdx.x;
     double f = 0.0;
-    if (e < ne) f = elem_adjoint(ne, p, npts, t, dofs, kappa, u, v, wsum, gout, gkappa, contrib, e);
+    if (e < ne) f = elem_adjoint(ne, p, npts, t, dofs, kappa, u, v, wsum, gout, gkappa, cx, cv, e);
     if constexpr (WITH_J) {
         __shared__ double red[kRed];
         red[threadIdx.x] = f;
@@ -209,32 +226,42 @@ __global__ void __launch_bounds__(kRed) k_energy_grad_elem(int64_t ne, const dou
 //   coordinates (out_x, (3, n_rows), component-major like mesh.p) and / or
 //   u / v DOFs (out_u, out_v (n_rows)); both in one walk when the vertex and
 //   DOF incidence lists coincide (scalar P1 with every vertex a DOF).
-__global__ void k_energy_grad_gather(int64_t n_rows, const int32_t *__restrict__ inc_ptr,
-                                     const int32_t *__restrict__ inc, const double *__restrict__ contrib,
-                                     double *__restrict__ out_x, double *__restrict__ out_u,
-                                     double *__restrict__ out_v) {
+__global__ void __launch_bounds__(128) k_energy_grad_gather(int64_t n_rows, const int32_t *__restrict__ inc_ptr,
+                                                            const int32_t *__restrict__ inc,
+                                                            const double *__restrict__ cx,
+                                                            const double *__restrict__ cv,
+                                                            double *__restrict__ out_x, double *__restrict__ out_u,
+                                                            double *__restrict__ out_v) {
     const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n_rows) return;
-    double s0 = 0.0, s1 = 0.0, s2 = 0.0, su = 0.0, sv = 0.0;
-    for (int32_t it = inc_ptr[r]; it < inc_ptr[r + 1]; ++it) {
-        const int32_t item = inc[it];
-        const int64_t e = item >> 2;
-        const int k = item & 3;
-        const double *c = contrib + e * 20;
-        if (out_x) {
-            s0 += c[k * 3];
-            s1 += c[k * 3 + 1];
-            s2 += c[k * 3 + 2];
+    double s[4] = {0.0, 0.0, 0.0, 0.0}, sv = 0.0;
+    const int32_t end = inc_ptr[r + 1];
+    for (int32_t it = inc_ptr[r]; it < end; it += 4) {  // four records in flight
+        double x[4][4], y[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int32_t item = it + j < end ? inc[it + j] : -1;  // element * 4 + vertex
+            y[j] = -0.0;  // leaves the sums unchanged
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[j][i] = -0.0;
+            if (item >= 0) {
+                load4(cx + (int64_t)item * 4, x[j]);
+                if (cv) y[j] = __ldg(cv + item);
+            }
         }
-        if (out_u) su += c[12 + k];
-        if (out_v) sv += c[16 + k];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[i] += x[j][i];
+            sv += y[j];
+        }
     }
     if (out_x) {
-        out_x[r] = s0;
-        out_x[n_rows + r] = s1;
-        out_x[2 * n_rows + r] = s2;
+        out_x[r] = s[0];
+        out_x[n_rows + r] = s[1];
+        out_x[2 * n_rows + r] = s[2];
     }
-    if (out_u) out_u[r] = su;
+    if (out_u) out_u[r] = s[3];
     if (out_v) out_v[r] = sv;
 }
 
@@ -257,7 +284,7 @@ extern "C" int skg_p1_energy(const double *d_p, int64_t npts, const int32_t *d_t
         } else {
             SKG_CUDA(cudaMemsetAsync(partial.get(), 0, 8, s));
         }
-        k_sum_blocks<<<1, 32, 0, s>>>(partial.get(), nb, d_out);
+        k_sum_blocks<<<1, 1024, 0, s>>>(partial.get(), nb, d_out);
         SKG_LAUNCH_CHECK("energy_sum");
     });
 }
@@ -274,43 +301,44 @@ void energy_grad(const skg_pattern *vertex_inc, const skg_pattern *dof_inc, cons
                 "coordinate gradients need the vertex incidence handle of this mesh");
         require((!d_gu && !d_gv) || (dof_inc && dof_inc->row_local == 4 && dof_inc->n_elements == ne),
                 "DOF gradients need the DOF incidence handle of this basis");
-        DevBuf<double> contrib((size_t)(ne ? ne : 1) * 20, s);
+        const bool fields = d_gu || d_gv;
+        DevBuf<double> cx((size_t)(ne ? ne : 1) * 16, s), cv(fields ? (size_t)(ne ? ne : 1) * 4 : 0, s);
         const int64_t nb = ne ? (ne + kRed - 1) / kRed : 1;
         DevBuf<double> partial(d_energy ? nb : 0, s);
         if (ne) {
             if (d_energy)
                 k_energy_grad_elem<true><<<(unsigned)nb, kRed, 0, s>>>(ne, d_p, npts, d_t, d_dofs, d_kappa, d_u, d_v,
-                                                                       wsum, grad_out, d_gkappa, contrib.get(),
+                                                                       wsum, grad_out, d_gkappa, cx.get(), cv.get(),
                                                                        partial.get());
             else
                 k_energy_grad_elem<false><<<(unsigned)nb, kRed, 0, s>>>(ne, d_p, npts, d_t, d_dofs, d_kappa, d_u,
-                                                                        d_v, wsum, grad_out, d_gkappa, contrib.get(),
-                                                                        nullptr);
+                                                                        d_v, wsum, grad_out, d_gkappa, cx.get(),
+                                                                        cv.get(), nullptr);
             SKG_LAUNCH_CHECK("energy_grad_elem");
         } else if (d_energy) {
             SKG_CUDA(cudaMemsetAsync(partial.get(), 0, 8, s));
         }
         if (d_energy) {
-            k_sum_blocks<<<1, 32, 0, s>>>(partial.get(), nb, d_energy);
+            k_sum_blocks<<<1, 1024, 0, s>>>(partial.get(), nb, d_energy);
             SKG_LAUNCH_CHECK("energy_sum");
         }
         const bool shared = vertex_inc == dof_inc;  // one incidence structure for both
         if (d_gp && shared) {
             k_energy_grad_gather<<<grid_for(npts, 128), 128, 0, s>>>(npts, vertex_inc->inc_ptr.get(),
-                                                                     vertex_inc->inc.get(), contrib.get(), d_gp, d_gu,
-                                                                     d_gv);
+                                                                     vertex_inc->inc.get(), cx.get(), cv.get(), d_gp,
+                                                                     d_gu, d_gv);
             SKG_LAUNCH_CHECK("energy_grad_xuv");
             return;
         }
         if (d_gp) {
             k_energy_grad_gather<<<grid_for(npts, 128), 128, 0, s>>>(npts, vertex_inc->inc_ptr.get(),
-                                                                     vertex_inc->inc.get(), contrib.get(), d_gp,
+                                                                     vertex_inc->inc.get(), cx.get(), nullptr, d_gp,
                                                                      nullptr, nullptr);
             SKG_LAUNCH_CHECK("energy_grad_x");
         }
         if (d_gu || d_gv) {
             k_energy_grad_gather<<<grid_for(dof_inc->n_rows, 128), 128, 0, s>>>(
-                dof_inc->n_rows, dof_inc->inc_ptr.get(), dof_inc->inc.get(), contrib.get(), nullptr, d_gu, d_gv);
+                dof_inc->n_rows, dof_inc->inc_ptr.get(), dof_inc->inc.get(), cx.get(), cv.get(), nullptr, d_gu, d_gv);
             SKG_LAUNCH_CHECK("energy_grad_uv");
         }
     }
