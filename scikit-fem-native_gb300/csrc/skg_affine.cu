@@ -18,9 +18,8 @@
 // Passes.
 //  1. element pass (thread per element): G (4x4) from coordinates and the
 //     coefficient, then the packed upper triangle of the element matrix (10
-//     entries for P1, 55 for P2), staged in shared memory and stored as one
-//     bulk copy per tile.  Tiles with a nonsymmetric
-//     coefficient also leave the lower triangles.
+//     entries for P1, 55 for P2), entry by entry in whole lines.  Tiles with a
+//     nonsymmetric coefficient also leave the lower triangles.
 //  2. pair sums (skg_pairs.cuh): one thread per pair of DOFs sums its
 //     contributions in ascending element order and writes the values of
 //     (r, c) and (c, r).  Every value is written by one thread from sums in a
@@ -51,6 +50,7 @@
 
 #include "skg_common.cuh"
 #include "skg_df64.cuh"
+#include "skg_fp64.cuh"
 #include "skg_pairs.cuh"
 #include "skg_rows.cuh"
 
@@ -150,7 +150,7 @@ __device__ __forceinline__ bool coef_symmetric(const double A[9]) {
 __device__ __forceinline__ bool elem_g_fp64(int64_t ne, const double *__restrict__ p, int64_t npts,
                                             const int32_t *__restrict__ t, int coef_kind,
                                             const double *__restrict__ coef, int64_t e, double g[16],
-                                            double gscale = 1.0) {
+                                            const Fp64 &F, double gscale = 1.0) {
     int32_t v[4];
     const bool ok = load_vertices(t, ne, e, npts, v);
     double J[9];
@@ -158,28 +158,19 @@ __device__ __forceinline__ bool elem_g_fp64(int64_t ne, const double *__restrict
     for (int i = 0; i < 3; ++i) {
         const double x0 = p[i * npts + v[0]];
 #pragma unroll
-        for (int r = 0; r < 3; ++r) J[i * 3 + r] = p[i * npts + v[r + 1]] - x0;
+        for (int r = 0; r < 3; ++r) J[i * 3 + r] = F.sub(p[i * npts + v[r + 1]], x0);
     }
     double b[4][3];
-    b[1][0] = J[4] * J[8] - J[5] * J[7];
-    b[1][1] = J[2] * J[7] - J[1] * J[8];
-    b[1][2] = J[1] * J[5] - J[2] * J[4];
-    b[2][0] = J[5] * J[6] - J[3] * J[8];
-    b[2][1] = J[0] * J[8] - J[2] * J[6];
-    b[2][2] = J[2] * J[3] - J[0] * J[5];
-    b[3][0] = J[3] * J[7] - J[4] * J[6];
-    b[3][1] = J[1] * J[6] - J[0] * J[7];
-    b[3][2] = J[0] * J[4] - J[1] * J[3];
-    const double det = J[0] * b[1][0] + J[1] * b[2][0] + J[2] * b[3][0];
+    const double det = F.adjugate(J, b);
     const double inv = ok ? gscale / fabs(det) : __longlong_as_double(0x7ff8000000000000LL);
     bool sym = true;
     if (coef_kind == 0) {
-        const double sc = (coef ? coef[e] : 1.0) * inv;
+        const double sc = coef ? F.mul(coef[e], inv) : inv;
 #pragma unroll
         for (int k = 1; k < 4; ++k)
 #pragma unroll
             for (int l = k; l < 4; ++l) {
-                const double val = sc * (b[k][0] * b[l][0] + b[k][1] * b[l][1] + b[k][2] * b[l][2]);
+                const double val = F.mul(sc, F.dot(b[k], b[l]));
                 g[k * 4 + l] = val;
                 g[l * 4 + k] = val;
             }
@@ -192,11 +183,11 @@ __device__ __forceinline__ bool elem_g_fp64(int64_t ne, const double *__restrict
         for (int l = 1; l < 4; ++l) {
             double Ab[3];
 #pragma unroll
-            for (int i = 0; i < 3; ++i) Ab[i] = A[i * 3] * b[l][0] + A[i * 3 + 1] * b[l][1] + A[i * 3 + 2] * b[l][2];
+            for (int i = 0; i < 3; ++i) Ab[i] = F.dot(A + i * 3, b[l]);
 #pragma unroll
             for (int k = 1; k < 4; ++k) {
                 if (k > l && sym) continue;  // mirrored below
-                g[k * 4 + l] = inv * (b[k][0] * Ab[0] + b[k][1] * Ab[1] + b[k][2] * Ab[2]);
+                g[k * 4 + l] = F.mul(inv, F.dot(b[k], Ab));
             }
         }
         if (sym) {
@@ -207,15 +198,15 @@ __device__ __forceinline__ bool elem_g_fp64(int64_t ne, const double *__restrict
         }
     }
 #pragma unroll
-    for (int l = 1; l < 4; ++l) g[l] = -(g[4 + l] + g[8 + l] + g[12 + l]);
+    for (int l = 1; l < 4; ++l) g[l] = -F.add3(g[4 + l], g[8 + l], g[12 + l]);
     if (sym) {
 #pragma unroll
         for (int k = 1; k < 4; ++k) g[k * 4] = g[k];
     } else {
 #pragma unroll
-        for (int k = 1; k < 4; ++k) g[k * 4] = -(g[k * 4 + 1] + g[k * 4 + 2] + g[k * 4 + 3]);
+        for (int k = 1; k < 4; ++k) g[k * 4] = -F.add3(g[k * 4 + 1], g[k * 4 + 2], g[k * 4 + 3]);
     }
-    g[0] = -(g[1] + g[2] + g[3]);
+    g[0] = -F.add3(g[1], g[2], g[3]);
     return sym;
 }
 
@@ -227,7 +218,7 @@ __global__ void __launch_bounds__(kElemBlock) k_elem_fp64(int64_t ne, const doub
     const int64_t e = e0 + threadIdx.x;
     if (e < ne) {
         double g[16];
-        elem_g_fp64(ne, p, npts, t, coef_kind, coef, e, g);
+        elem_g_fp64(ne, p, npts, t, coef_kind, coef, e, g, Fp64::load());
         double2 *st = reinterpret_cast<double2 *>(stage + threadIdx.x * kStagePad);
 #pragma unroll
         for (int m = 0; m < 8; ++m) st[m] = make_double2(g[2 * m], g[2 * m + 1]);
@@ -809,108 +800,112 @@ __device__ __forceinline__ bool shared_entries_ok(const double g[16]) {
 }
 
 template <int A, int BB>
-__device__ __forceinline__ double shared_entry(const double g[16], const double S[4][6]) {
+__device__ __forceinline__ double shared_entry(const double g[16], const double S[4][6], const Fp64 &F) {
     if constexpr (A < 4 && BB < 4) {
-        if constexpr (A == BB) return 3.0 * g[A * 4 + A];
+        if constexpr (A == BB) return F.mul(F.three_, g[A * 4 + A]);
         else return neg_bits(g[A * 4 + BB]);
     } else if constexpr (A < 4) {
         constexpr int lo = sup_lo(BB), hi = sup_hi(BB);
         if constexpr (A != lo && A != hi) return neg_bits(S[A][BB - 4]);
-        else if constexpr (A == lo) return fma(3.0, g[A * 4 + hi], -g[A * 4 + lo]);
-        else return fma(3.0, g[A * 4 + lo], -g[A * 4 + hi]);
+        else if constexpr (A == lo) return fma(F.three_, g[A * 4 + hi], -g[A * 4 + lo]);
+        else return fma(F.three_, g[A * 4 + lo], -g[A * 4 + hi]);
     } else {
         constexpr int i = sup_lo(A), j = sup_hi(A), lb = sup_lo(BB), hb = sup_hi(BB);
         if constexpr (A == BB) {
             // 4 (S_i + S_j + g_ii + g_jj) over edge (i, j) = 8 (g_ii + g_jj + g_ij): g is symmetric here
-            return times8_bits((g[i * 4 + i] + g[j * 4 + j]) + g[i * 4 + j]);
+            return times8_bits(F.add3(g[i * 4 + i], g[j * 4 + j], g[i * 4 + j]));
         }
         if constexpr (i == lb || i == hb || j == lb || j == hb) {
             // shared vertex sv, other ends na (of a) and nb (of b), fourth vertex n: with the zero row sum
             // G_sv,sv + G_sv,na + G_sv,nb + G_sv,n = 0 the entry is 4 (2 G_na,nb - G_sv,n)
             constexpr int sv = (i == lb || i == hb) ? i : j;
             constexpr int na = sv == i ? j : i, nb = (lb == sv) ? hb : lb, n = 6 - sv - na - nb;
-            return times4_bits(times2_bits(g[na * 4 + nb]) - g[sv * 4 + n]);
+            return times4_bits(F.sub(times2_bits(g[na * 4 + nb]), g[sv * 4 + n]));
         } else {
-            return times4_bits(S[i][BB - 4] + S[j][BB - 4]);
+            return times4_bits(F.add(S[i][BB - 4], S[j][BB - 4]));
         }
     }
 }
 
-__device__ __forceinline__ void shared_entries(const double g[16], double *U) {
+template <class Out>
+__device__ __forceinline__ void shared_entries(const double g[16], const Out &U, const Fp64 &F) {
     double S[4][6];  // S_v(b) for vertex v off edge b only (the others are not used)
     static_for<0, 24>([&](auto kk) {
         constexpr int k = decltype(kk)::value, v = k / 6, e = k % 6;
         if constexpr (v != sup_lo(4 + e) && v != sup_hi(4 + e))
-            S[v][e] = g[v * 4 + sup_lo(4 + e)] + g[v * 4 + sup_hi(4 + e)];
+            S[v][e] = F.add(g[v * 4 + sup_lo(4 + e)], g[v * 4 + sup_hi(4 + e)]);
     });
     static_for<0, 100>([&](auto kk) {
         constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
-        if constexpr (A <= BB) U[tri10(A, BB)] = shared_entry<A, BB>(g, S);
+        if constexpr (A <= BB) U[tri10(A, BB)] = shared_entry<A, BB>(g, S, F);
     });
 }
 
-// Where the element pass leaves the packed matrices of a tile, and the lower
-// triangles of the tiles that hold a nonsymmetric coefficient.
+// Where the element pass leaves the packed matrices (entry t of element e at
+// t * stride + e), and the lower triangles of the tiles that hold a nonsymmetric
+// coefficient.
 template <class E>
 struct PackedOut {
     E *upper, *lower;
     uint8_t *tiles;  // per tile: the lower triangles are there too
     int *any;        // set when a tile is flagged
+    int64_t stride;
 };
 
-// Writes the block's stage (`n` packed matrices of NP entries) to `upper`, and
-// for a tile with a nonsymmetric element the lower triangles (`entry_ba` of
-// the nonsymmetric elements; a symmetric one's stage already holds them) to
-// `lower`.
-template <int NP, class E, class F>
-__device__ __forceinline__ void store_packed(E *stage, int64_t tile, int n, bool sym, const PackedOut<E> &out,
-                                             F &&lower_entries) {
-    const int64_t at = tile * kTile * NP;
-    store_tile(stage, out.upper + at, n * NP * (int)sizeof(E));
+// Element e's entries as an array.
+template <class E>
+struct PackedEntries {
+    E *at;
+    int64_t stride;
+    __device__ __forceinline__ E &operator[](int t) const { return at[t * stride]; }
+};
+
+// The block's vote on its tile: true when every coefficient is symmetric.
+template <class E>
+__device__ __forceinline__ bool tile_symmetric(bool sym, int64_t tile, const PackedOut<E> &out) {
     const bool all = __syncthreads_and(sym);
-    if (out.tiles && threadIdx.x == 0) out.tiles[tile] = all ? 0 : 1;
-    if (all) return;
-    if (threadIdx.x == 0) *out.any = 1;
-    if (!sym) lower_entries();
-    store_tile(stage, out.lower + at, n * NP * (int)sizeof(E));
+    if (out.tiles && threadIdx.x == 0) {
+        out.tiles[tile] = all ? 0 : 1;
+        if (!all) *out.any = 1;
+    }
+    return all;
 }
 
 // FP64 element pass, thread per element: the packed upper triangle of K_e.
 // P1: the 10 entries wsum G (RULE unused).  P2: the 55 entries from G, for a
 // rule exact on quadratics (EXACT; the 4-point and the 11-point Keast rule)
 // from the integer table with compile-time factors and shared sums
-// (shared_entry), else from the rule's table in shared memory.  Each entry
-// goes to the shared-memory stage as it is computed (an odd or 10-double
-// stride per thread: at most two-way bank conflicts), so no entry array is
-// held in registers.  Bound by the FP64 pipe: about 105 instructions for G
-// and 58 for the P2 entries.
+// (shared_entry), else from the rule's table in shared memory.  Each entry is
+// stored as it is computed, so no entry array is held in registers or staged.
+// Bound by the FP64 pipe: 169 instructions per element, about 110 of them for
+// G: 469 us at 64^3, 90 % of the pipe's rate (with DADD / DMUL instead of
+// skg_fp64.cuh 507 us; with the 64 registers of an unbounded launch, which
+// recomputes, 534 us; four blocks per SM leave it 128).
 //
 // With `redo`, the pass runs only when the FP32-pair pass before it left its
 // range (its blocks then walk the tiles: the launch that finds nothing to do
 // is small).
 template <int NN, bool EXACT>
-__global__ void __launch_bounds__(kTile) k_elem_packed(int64_t ne, int64_t e_begin, int64_t e_end,
+__global__ void __launch_bounds__(kTile, 4) k_elem_packed(int64_t ne, int64_t e_begin, int64_t e_end,
                                                           const double *__restrict__ p, int64_t npts,
                                                           const int32_t *__restrict__ t, int coef_kind,
                                                           const double *__restrict__ coef, double gscale,
                                                           const double *__restrict__ Tg, PackedOut<double> out,
                                                           const int *__restrict__ redo) {
-    constexpr int NP = NN * (NN + 1) / 2;
-    extern __shared__ __align__(16) unsigned char smem[];
-    double *stage = reinterpret_cast<double *>(smem);  // kTile x NP, then the table
-    double *Ts = stage + kTile * NP;
+    __shared__ double Ts[NN == 10 && !EXACT ? 400 : 1];
     if (redo && !out_of_range(redo)) return;
+    const Fp64 F = Fp64::load();
     if constexpr (NN == 10 && !EXACT) {
         for (int i = threadIdx.x; i < 400; i += kTile) Ts[i] = Tg[i];
         __syncthreads();
     }
     const int64_t last = (e_end + kTile - 1) / kTile;
     for (int64_t tile = e_begin / kTile + blockIdx.x; tile < last; tile += gridDim.x) {
-        const int64_t e0 = tile * kTile, e = e0 + threadIdx.x;
-        double *st = stage + threadIdx.x * NP;
+        const int64_t e = tile * kTile + threadIdx.x;
+        const PackedEntries<double> st{out.upper + e, out.stride};
         double g[16];
         bool sym = true;
-        if (e < e_end) sym = elem_g_fp64(ne, p, npts, t, coef_kind, coef, e, g, gscale);
+        if (e < e_end) sym = elem_g_fp64(ne, p, npts, t, coef_kind, coef, e, g, F, gscale);
         auto table_entry = [&](int a, int bb) -> double {
             const int ka0 = sup_lo(a), ka1 = sup_hi(a), kb0 = sup_lo(bb), kb1 = sup_hi(bb);
             const double *T = Ts + (a * 10 + bb) * 4;
@@ -930,7 +925,7 @@ __global__ void __launch_bounds__(kTile) k_elem_packed(int64_t ne, int64_t e_beg
                     for (int b = a; b < 4; ++b) st[tri_index(4, a, b)] = g[a * 4 + b];
             } else if constexpr (EXACT) {
                 if (sym && shared_entries_ok(g)) {
-                    shared_entries(g, st);
+                    shared_entries(g, st, F);
                 } else {
                     static_for<0, 100>([&](auto kk) {
                         constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
@@ -944,25 +939,28 @@ __global__ void __launch_bounds__(kTile) k_elem_packed(int64_t ne, int64_t e_beg
                     for (int b = a; b < 10; ++b) st[tri10(a, b)] = table_entry(a, b);
             }
         }
-        const int n = (int)(e_end - e0 < kTile ? e_end - e0 : kTile);
-        store_packed<NP>(stage, tile, n, sym, out, [&] {
-            if constexpr (NN == 4) {
+        if (tile_symmetric(sym, tile, out) || e >= e_end) continue;
+        const PackedEntries<double> lo{out.lower + e, out.stride};
+        if constexpr (NN == 4) {
 #pragma unroll
-                for (int a = 0; a < 4; ++a)
+            for (int a = 0; a < 4; ++a)
 #pragma unroll
-                    for (int b = a; b < 4; ++b) st[tri_index(4, a, b)] = g[b * 4 + a];
-            } else if constexpr (EXACT) {
+                for (int b = a; b < 4; ++b) lo[tri_index(4, a, b)] = g[b * 4 + a];
+        } else if constexpr (EXACT) {
+            if (sym) {  // the mirrored entries, bit for bit
+                for (int q = 0; q < 55; ++q) lo[q] = st[q];
+            } else {
                 static_for<0, 100>([&](auto kk) {
                     constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
-                    if constexpr (A <= BB) st[tri10(A, BB)] = exact_entry_fp64<BB, A>(g);
+                    if constexpr (A <= BB) lo[tri10(A, BB)] = exact_entry_fp64<BB, A>(g);
                 });
-            } else {
-#pragma unroll
-                for (int a = 0; a < 10; ++a)
-#pragma unroll
-                    for (int b = a; b < 10; ++b) st[tri10(a, b)] = table_entry(b, a);
             }
-        });
+        } else {
+#pragma unroll
+            for (int a = 0; a < 10; ++a)
+#pragma unroll
+                for (int b = a; b < 10; ++b) lo[tri10(a, b)] = sym ? st[tri10(a, b)] : table_entry(b, a);
+        }
     }
 }
 
@@ -977,10 +975,8 @@ __global__ void __launch_bounds__(kTile) k_elem_packed_df(
     const double *__restrict__ coef, int *__restrict__ misc,
     PackedOut<typename std::conditional<MODE == MODE_DF64, float2, float>::type> out) {
     using E = typename std::conditional<MODE == MODE_DF64, float2, float>::type;
-    extern __shared__ __align__(16) unsigned char smem[];
-    E *stage = reinterpret_cast<E *>(smem);  // kTile x 55
-    const int64_t tile = e_begin / kTile + blockIdx.x, e0 = tile * kTile, e = e0 + threadIdx.x;
-    E *st = stage + threadIdx.x * 55;
+    const int64_t tile = e_begin / kTile + blockIdx.x, e = tile * kTile + threadIdx.x;
+    PackedEntries<E> st{out.upper + e, out.stride};
     auto store = [&](int k, df64 v) {
         if constexpr (MODE == MODE_DF64) st[k] = make_float2(v.hi, v.lo);
         else st[k] = v.hi + v.lo;
@@ -1002,41 +998,39 @@ __global__ void __launch_bounds__(kTile) k_elem_packed_df(
             });
         }
     }
-    store_packed<55>(stage, tile, (int)(e_end - e0 < kTile ? e_end - e0 : kTile), sym, out, [&] {
-        static_for<0, 100>([&](auto kk) {
-            constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
-            if constexpr (A <= BB) store(tri10(A, BB), exact_entry<BB, A, MODE>(g));
-        });
+    if (tile_symmetric(sym, tile, out) || e >= e_end) return;
+    const PackedEntries<E> up = st;
+    st.at = out.lower + e;
+    if (sym) {  // the mirrored entries, bit for bit
+        for (int q = 0; q < 55; ++q) st[q] = up[q];
+        return;
+    }
+    static_for<0, 100>([&](auto kk) {
+        constexpr int k = decltype(kk)::value, A = k / 10, BB = k % 10;
+        if constexpr (A <= BB) store(tri10(A, BB), exact_entry<BB, A, MODE>(g));
     });
 }
 
 // Packed matrices of one assembly: scratch, launches and the sums.
 template <class E>
 PairLower<E> lower_of(const PackedOut<E> &o) {
-    return o.lower ? PairLower<E>{o.lower, o.any, o.tiles} : PairLower<E>{};
+    return o.lower ? PairLower<E>{o.lower, o.any, o.tiles, (uint32_t)o.stride} : PairLower<E>{};
 }
 
 template <int NN, bool EXACT>
 void launch_elem_packed(int64_t ne, int64_t e0, int64_t e1, const double *p, int64_t npts, const int32_t *t, int kind,
                         const double *coef, double gscale, const double *Tg, const PackedOut<double> &out,
                         const int *redo, cudaStream_t s) {
-    constexpr int smem = kTile * NN * (NN + 1) / 2 * 8 + (NN == 10 && !EXACT ? 400 * 8 : 0);
-    if (smem > 48 * 1024)
-        SKG_CUDA(cudaFuncSetAttribute(k_elem_packed<NN, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     unsigned grid = grid_for(e1 - e0, kTile);
     if (redo) grid = std::min(grid, 2u * kSmCount);
-    k_elem_packed<NN, EXACT><<<grid, kTile, smem, s>>>(ne, e0, e1, p, npts, t, kind, coef, gscale, Tg, out, redo);
+    k_elem_packed<NN, EXACT><<<grid, kTile, 0, s>>>(ne, e0, e1, p, npts, t, kind, coef, gscale, Tg, out, redo);
     SKG_LAUNCH_CHECK("elem_packed");
 }
 
 template <int MODE, class E>
 void launch_elem_packed_df(int64_t ne, int64_t e0, int64_t e1, const double *p, int64_t npts, const int32_t *t, int kind, const double *coef,
                            int *misc, const PackedOut<E> &out, cudaStream_t s) {
-    constexpr int smem = kTile * 55 * (int)sizeof(E);
-    if (smem > 48 * 1024)
-        SKG_CUDA(cudaFuncSetAttribute(k_elem_packed_df<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    k_elem_packed_df<MODE><<<grid_for(e1 - e0, kTile), kTile, smem, s>>>(ne, e0, e1, p, npts, t, kind, coef, misc,
-                                                                              out);
+    k_elem_packed_df<MODE><<<grid_for(e1 - e0, kTile), kTile, 0, s>>>(ne, e0, e1, p, npts, t, kind, coef, misc, out);
     SKG_LAUNCH_CHECK("elem_packed_df");
 }
 
@@ -1167,11 +1161,12 @@ void affine_assemble_pairs(const skg_pattern *pat, const double *d_p, int64_t np
     const bool maybe_lower = coef_kind != 0;  // a tensor may be nonsymmetric
     // [0] scale exponent, [1] range flag (0x80808080: none, in range), [2] a tile holds a nonsymmetric coefficient
     DevBuf<int> misc(3, s);
-    DevBuf<double> K((size_t)ne * np, s), lower(maybe_lower ? (size_t)ne * np : 0, s);
+    const int64_t stride = block_stride(ne);
+    DevBuf<double> K((size_t)stride * np, s), lower(maybe_lower ? (size_t)stride * np : 0, s);
     DevBuf<uint8_t> tile_flags(maybe_lower ? (size_t)tiles : 0, s);
     int *any = maybe_lower ? misc.get() + 2 : nullptr;
     if (maybe_lower) SKG_CUDA(cudaMemsetAsync(any, 0, 4, s));
-    const PackedOut<double> out64{K.get(), lower.get(), tile_flags.get(), any};
+    const PackedOut<double> out64{K.get(), lower.get(), tile_flags.get(), any, stride};
     const double *Tg = nodes == 10 && !exact_rule ? device_table(T.data(), T.size(), s) : nullptr;
     auto elem64 = [&](int64_t e0, int64_t e1, const int *redo) {
         if (nodes == 4)
@@ -1204,11 +1199,11 @@ void affine_assemble_pairs(const skg_pattern *pat, const double *d_p, int64_t np
     // range flag is final.
     const bool split = precision == SKG_SPLIT_FP32;
     const size_t entry = split ? sizeof(float) : sizeof(float2);
-    DevBuf<unsigned char> Kf((size_t)ne * np * entry, s), lower_f(maybe_lower ? (size_t)ne * np * entry : 0, s);
+    DevBuf<unsigned char> Kf((size_t)stride * np * entry, s), lower_f(maybe_lower ? (size_t)stride * np * entry : 0, s);
     const PackedOut<float2> out_df{reinterpret_cast<float2 *>(Kf.get()), reinterpret_cast<float2 *>(lower_f.get()),
-                                   tile_flags.get(), any};
+                                   tile_flags.get(), any, stride};
     const PackedOut<float> out_f{reinterpret_cast<float *>(Kf.get()), reinterpret_cast<float *>(lower_f.get()),
-                                 tile_flags.get(), any};
+                                 tile_flags.get(), any, stride};
     const PairUnscale unscale{misc.get()};
     run_pair_passes(
         pat, ne, d_values, h_values, s,

@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "skg_common.cuh"
+#include "skg_fp64.cuh"
 #include "skg_pairs.cuh"
 
 namespace skg {
@@ -50,7 +51,7 @@ struct Element {
 };
 
 __device__ __forceinline__ Element load_element(int64_t ne, int64_t e, const double *__restrict__ p, int64_t npts,
-                                                const int32_t *__restrict__ t, const FormCoefs &fc) {
+                                                const int32_t *__restrict__ t, const FormCoefs &fc, const Fp64 &F) {
     Element el;
     int32_t v[4];
     bool ok = true;
@@ -65,52 +66,43 @@ __device__ __forceinline__ Element load_element(int64_t ne, int64_t e, const dou
     for (int i = 0; i < 3; ++i) {
         const double x0 = p[i * npts + v[0]];
 #pragma unroll
-        for (int r = 0; r < 3; ++r) J[i * 3 + r] = p[i * npts + v[r + 1]] - x0;
+        for (int r = 0; r < 3; ++r) J[i * 3 + r] = F.sub(p[i * npts + v[r + 1]], x0);
     }
     double (*B)[3] = el.B;
-    B[1][0] = J[4] * J[8] - J[5] * J[7];
-    B[1][1] = J[2] * J[7] - J[1] * J[8];
-    B[1][2] = J[1] * J[5] - J[2] * J[4];
-    B[2][0] = J[5] * J[6] - J[3] * J[8];
-    B[2][1] = J[0] * J[8] - J[2] * J[6];
-    B[2][2] = J[2] * J[3] - J[0] * J[5];
-    B[3][0] = J[3] * J[7] - J[4] * J[6];
-    B[3][1] = J[1] * J[6] - J[0] * J[7];
-    B[3][2] = J[0] * J[4] - J[1] * J[3];
-    el.ad = fabs(J[0] * B[1][0] + J[1] * B[2][0] + J[2] * B[3][0]);
+    el.ad = fabs(F.adjugate(J, B));
 #pragma unroll
-    for (int i = 0; i < 3; ++i) B[0][i] = -(B[1][i] + B[2][i] + B[3][i]);
+    for (int i = 0; i < 3; ++i) B[0][i] = -F.add3(B[1][i], B[2][i], B[3][i]);
     const auto coef = [&](int k) { return fc.arr[k] ? fc.arr[k][e] : fc.cst[k]; };
     const double inv = ok ? 1.0 / el.ad : __longlong_as_double(0x7ff8000000000000LL);
-    el.vm = coef(0) * el.ad;
-    el.hs = 0.5 * coef(2) * inv;
-    el.dv = coef(3) * inv;
-    el.dg = coef(1) * inv + el.hs;
+    el.vm = F.mul(coef(0), el.ad);
+    el.hs = F.mul(0.5 * coef(2), inv);
+    el.dv = F.mul(coef(3), inv);
+    el.dg = fma(coef(1), inv, el.hs);
     return el;
 }
 
 // Gram products dg B_k . B_l: dot products for k, l >= 1, the rest from the
 // zero row sums.
-__device__ __forceinline__ void gram(const Element &el, double G[4][4]) {
+__device__ __forceinline__ void gram(const Element &el, double G[4][4], const Fp64 &F) {
 #pragma unroll
     for (int k = 1; k < 4; ++k)
 #pragma unroll
         for (int l = k; l < 4; ++l) {
-            G[k][l] = el.dg * (el.B[k][0] * el.B[l][0] + el.B[k][1] * el.B[l][1] + el.B[k][2] * el.B[l][2]);
+            G[k][l] = F.mul(el.dg, F.dot(el.B[k], el.B[l]));
             G[l][k] = G[k][l];
         }
 #pragma unroll
     for (int l = 1; l < 4; ++l) {
-        G[0][l] = -(G[1][l] + G[2][l] + G[3][l]);
+        G[0][l] = -F.add3(G[1][l], G[2][l], G[3][l]);
         G[l][0] = G[0][l];
     }
-    G[0][0] = -(G[0][1] + G[0][2] + G[0][3]);
+    G[0][0] = -F.add3(G[0][1], G[0][2], G[0][3]);
 }
 
 // Vector block (k, l), k <= l: H[c][d] = pk_d B_l,c + qk_c B_l,d (c != d),
 // tk_c B_l,c + diag (c == d), with pk = hs B_k, qk = dv B_k, tk = pk + qk.
 __device__ __forceinline__ void vector_block(const double pk[3], const double qk[3], const double tk[3],
-                                             const double Bl[3], bool same, double diag, double H[9]) {
+                                             const double Bl[3], bool same, double diag, double H[9], const Fp64 &F) {
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
@@ -118,9 +110,9 @@ __device__ __forceinline__ void vector_block(const double pk[3], const double qk
             if (c == d) {
                 H[c * 3 + d] = fma(tk[c], Bl[c], diag);
             } else if (!same) {
-                H[c * 3 + d] = fma(pk[d], Bl[c], qk[c] * Bl[d]);
+                H[c * 3 + d] = fma(pk[d], Bl[c], F.mul(qk[c], Bl[d]));
             } else if (d > c) {
-                const double x = tk[d] * Bl[c];  // diagonal block: symmetric
+                const double x = F.mul(tk[d], Bl[c]);  // diagonal block: symmetric
                 H[c * 3 + d] = x;
                 H[d * 3 + c] = x;
             }
@@ -138,26 +130,27 @@ __global__ void __launch_bounds__(kFormBlock) k_form_p1v(int64_t ne, int64_t e_b
     const int n = (int)(e_end - e0 < 32 ? e_end - e0 : 32);
     if (n <= 0) return;
     WarpStore out{stages + (threadIdx.x >> 5) * 2 * WarpStore::kStage};
-    Element el = load_element(ne, lane < n ? e0 + lane : e0, p, npts, t, fc);  // lanes past the end: unwritten
+    const Fp64 F = Fp64::load();
+    Element el = load_element(ne, lane < n ? e0 + lane : e0, p, npts, t, fc, F);  // lanes past the end: unwritten
     const double sw = __ldg(tab);
     el.hs *= sw;
     el.dv *= sw;
     el.dg *= sw;
     double G[4][4];
-    gram(el, G);
+    gram(el, G, F);
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
         double pk[3], qk[3], tk[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            pk[c] = el.hs * el.B[a][c];
-            qk[c] = el.dv * el.B[a][c];
-            tk[c] = pk[c] + qk[c];
+            pk[c] = F.mul(el.hs, el.B[a][c]);
+            qk[c] = F.mul(el.dv, el.B[a][c]);
+            tk[c] = F.add(pk[c], qk[c]);
         }
 #pragma unroll
         for (int b = a; b < 4; ++b) {
             double H[9];
-            vector_block(pk, qk, tk, el.B[b], a == b, fma(el.vm, __ldg(tab + 1 + tri_index(4, a, b)), G[a][b]), H);
+            vector_block(pk, qk, tk, el.B[b], a == b, fma(el.vm, __ldg(tab + 1 + tri_index(4, a, b)), G[a][b]), H, F);
             double *st = out.next() + 9 * lane;
 #pragma unroll
             for (int x = 0; x < 9; ++x) st[x] = H[x];
@@ -181,24 +174,25 @@ __global__ void __launch_bounds__(kFormBlock, 4) k_form_p2v(int64_t ne, int64_t 
     const int n = (int)(e_end - e0 < 32 ? e_end - e0 : 32);
     if (n <= 0) return;
     WarpStore out{stages + (threadIdx.x >> 5) * 2 * WarpStore::kStage};
+    const Fp64 F = Fp64::load();
     double H[10][9], vm;
     {
-        const Element el = load_element(ne, lane < n ? e0 + lane : e0, p, npts, t, fc);
+        const Element el = load_element(ne, lane < n ? e0 + lane : e0, p, npts, t, fc, F);
         vm = el.vm;
         double G[4][4];
-        gram(el, G);
+        gram(el, G, F);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             double pk[3], qk[3], tk[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                pk[c] = el.hs * el.B[k][c];
-                qk[c] = el.dv * el.B[k][c];
-                tk[c] = pk[c] + qk[c];
+                pk[c] = F.mul(el.hs, el.B[k][c]);
+                qk[c] = F.mul(el.dv, el.B[k][c]);
+                tk[c] = F.add(pk[c], qk[c]);
             }
 #pragma unroll
             for (int l = k; l < 4; ++l)
-                vector_block(pk, qk, tk, el.B[l], k == l, G[k][l], H[tri_index(4, k, l)]);
+                vector_block(pk, qk, tk, el.B[l], k == l, G[k][l], H[tri_index(4, k, l)], F);
         }
     }
 #pragma unroll
@@ -222,36 +216,34 @@ __global__ void __launch_bounds__(kFormBlock, 4) k_form_p2v(int64_t ne, int64_t 
                     for (int d = 0; d < 3; ++d) {
                         if (a == b && d < c) continue;  // diagonal block: symmetric
                         const double x = h[k <= l ? c * 3 + d : d * 3 + c];
-                        v[c * 3 + d] = first ? T * x : fma(T, x, v[c * 3 + d]);
+                        v[c * 3 + d] = first ? F.mul(T, x) : fma(T, x, v[c * 3 + d]);
                     }
                 first = false;
             }
-            const double m = vm * Ts[220 + t4];
+            const double m = F.mul(vm, Ts[220 + t4]);
             double *st = out.next() + 9 * lane;
 #pragma unroll
             for (int c = 0; c < 3; ++c)
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
-                    st[c * 3 + d] = c == d ? v[c * 3 + d] + m : a == b && d < c ? v[d * 3 + c] : v[c * 3 + d];
+                    st[c * 3 + d] = c == d ? F.add(v[c * 3 + d], m) : a == b && d < c ? v[d * 3 + c] : v[c * 3 + d];
             out.store(Ke + ((int64_t)t4 * stride + e0) * 9, n, 9);
         }
     out.finish();
 }
 
-// Scalar P1 / P2: packed upper triangles (E, np).
+// Scalar P1 / P2: packed upper triangles (np, stride).
 template <int NN>
-__global__ void __launch_bounds__(kTile) k_form_scalar(int64_t ne, int64_t e_begin, int64_t e_end,
+__global__ void __launch_bounds__(kTile) k_form_scalar(int64_t ne, int64_t e_begin, int64_t e_end, int64_t stride,
                                                        const double *__restrict__ p, int64_t npts,
                                                        const int32_t *__restrict__ t, FormCoefs fc,
                                                        const double *__restrict__ tab, double *__restrict__ Ke) {
-    constexpr int NP = NN * (NN + 1) / 2;
-    __shared__ __align__(16) double stage[kTile * NP];
-    const int64_t tile = e_begin / kTile + blockIdx.x, e0 = tile * kTile, e = e0 + threadIdx.x;
-    double *st = stage + threadIdx.x * NP;
+    const int64_t e = e_begin + (int64_t)blockIdx.x * kTile + threadIdx.x;
     if (e < e_end) {
-        const Element el = load_element(ne, e, p, npts, t, fc);
+        const Fp64 F = Fp64::load();
+        const Element el = load_element(ne, e, p, npts, t, fc, F);
         double G[4][4];
-        gram(el, G);
+        gram(el, G, F);
         const double x = el.hs + el.dv;  // the one component's symmetric-gradient and divergence terms
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -266,19 +258,18 @@ __global__ void __launch_bounds__(kTile) k_form_scalar(int64_t ne, int64_t e_beg
             for (int b = a; b < NN; ++b) {
                 const int q = tri_index(NN, a, b);
                 if constexpr (NN == 4) {
-                    st[q] = fma(el.vm, __ldg(tab + 1 + q), __ldg(tab) * G[a][b]);
+                    Ke[q * stride + e] = fma(el.vm, __ldg(tab + 1 + q), F.mul(__ldg(tab), G[a][b]));
                 } else {
-                    double v = el.vm * __ldg(tab + 220 + q);
+                    double v = F.mul(el.vm, __ldg(tab + 220 + q));
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
                         if ((u & 2 && a < 4) || (u & 1 && b < 4)) continue;
                         v = fma(__ldg(tab + q * 4 + u), G[u & 2 ? hi_of(a) : lo_of(a)][u & 1 ? hi_of(b) : lo_of(b)], v);
                     }
-                    st[q] = v;
+                    Ke[q * stride + e] = v;
                 }
             }
     }
-    store_tile(stage, Ke + tile * kTile * NP, (int)(e_end - e0 < kTile ? e_end - e0 : kTile) * NP * 8);
 }
 
 std::vector<double> form_table(int nodes, int nq, const double *X, const double *W) {
@@ -343,7 +334,7 @@ void affine_forms_assemble(const skg_pattern *pat, const double *d_p, int64_t np
         fc.cst[k] = coef[k] ? 0.0 : cst[k];
     }
     const int64_t stride = block_stride(ne);
-    DevBuf<double> Ke(comp == 3 ? (size_t)stride * np * 9 : (size_t)ne * np, s);
+    DevBuf<double> Ke((size_t)stride * np * (comp == 3 ? 9 : 1), s);
     auto elem = [&](int64_t e0, int64_t e1) {
         const unsigned grid = grid_for(e1 - e0, kFormBlock);
         if (comp == 3 && nodes == 4)
@@ -351,9 +342,9 @@ void affine_forms_assemble(const skg_pattern *pat, const double *d_p, int64_t np
         else if (comp == 3)
             k_form_p2v<<<grid, kFormBlock, 0, s>>>(ne, e0, e1, stride, d_p, npts, d_t, fc, tab, Ke.get());
         else if (nodes == 4)
-            k_form_scalar<4><<<grid_for(e1 - e0, kTile), kTile, 0, s>>>(ne, e0, e1, d_p, npts, d_t, fc, tab, Ke.get());
+            k_form_scalar<4><<<grid_for(e1 - e0, kTile), kTile, 0, s>>>(ne, e0, e1, stride, d_p, npts, d_t, fc, tab, Ke.get());
         else
-            k_form_scalar<10><<<grid_for(e1 - e0, kTile), kTile, 0, s>>>(ne, e0, e1, d_p, npts, d_t, fc, tab, Ke.get());
+            k_form_scalar<10><<<grid_for(e1 - e0, kTile), kTile, 0, s>>>(ne, e0, e1, stride, d_p, npts, d_t, fc, tab, Ke.get());
         SKG_LAUNCH_CHECK("form");
     };
     if (pat->pairs.block == comp && pat->pairs.nodes == nodes) {

@@ -20,13 +20,17 @@
 //   M_ab = mass * s_a s_b sum_{k,l} (b_k.b_l / |det|) Tm^{kl}_ab,
 //   Tm^{kl}_ab = sum_q w_q d^k_a(xi_q) d^l_b(xi_q)   (host table, per rule)
 //   C_ab = curl * s_a s_b (sum_q w_q) (J c_a).(J c_b) / |det|.
-// Per-point coefficients use the explicit quadrature loop.  The 6x6 element
-// matrices then go through the same fixed-order row-owner gather as H1.
+// The 21 distinct entries then go through the pair sums (skg_pairs.cuh).
+// Per-point coefficients use the explicit quadrature loop, and the fixed-order
+// row-owner gather as H1.
+#include <algorithm>
 #include <climits>
 #include <vector>
 
 #include "skg_common.cuh"
 #include "skg_df64.cuh"
+#include "skg_fp64.cuh"
+#include "skg_pairs.cuh"
 #include "skg_rows.cuh"
 
 namespace skg {
@@ -161,92 +165,126 @@ __host__ __device__ constexpr double ref_curl(int a, int i) {
     return c[a][i];
 }
 
-constexpr int kN1Block = 128;
+constexpr int kN1Block = kTile;
 
 // Per-element coefficients, closed form: K_ac = s_a s_c (mu sum_uv G T + nu
 // (J c_a . J c_c) wsum / |det|) with G = b_k . b_l / |det|; the 21 entries of
-// the symmetric 6 x 6 matrix, stores staged through shared memory (FP64).
+// the symmetric 6 x 6 matrix, packed (21, stride) for the pair sums or full (E,
+// 6, 6), staged through shared memory (FP64).  With `redo`, the pass runs
+// only when the split-precision pass before it left its range (its blocks then
+// walk the tiles).
 // The curl term as c_a^T H c_c with H = 4 nu wsum J^T J / |det| (the
 // reference curls c_a have entries 0 and +-2): signed sums of H's entries.
+template <bool PACKED>
 __global__ void __launch_bounds__(kN1Block) k_n1_elem_fast(int64_t ne, int64_t e_begin, int64_t e_end,
                                                             const double *__restrict__ p, int64_t npts,
                                                             const int32_t *__restrict__ t,
                                                             const int8_t *__restrict__ signs, N1Table tab,
                                                             const double *__restrict__ mass,
                                                             const double *__restrict__ curl, int inc_mass,
-                                                            int inc_curl, double *__restrict__ Ke) {
-    __shared__ double stage[kN1Block * 37];
-    const int64_t e0 = e_begin + (int64_t)blockIdx.x * kN1Block;
-    const int64_t e = e0 + threadIdx.x;
-    if (e < e_end) {
-        double J[9], b[4][3], det;
-        n1_geometry(p, npts, t, ne, e, J, b, det);
-        const double inv = 1.0 / fabs(det);
-        const double mu = inc_mass ? (mass ? mass[e] : 1.0) : 0.0;
-        const double nu = inc_curl ? (curl ? curl[e] : 1.0) * inv * tab.wsum : 0.0;
-        // mu b_k . b_l / |det J|: dot products for k, l >= 1, row 0 from
-        // b_0 = -(b_1 + b_2 + b_3); mu / |det J| scales the six products once
-        const double mi = mu * inv;
-        double Gm[4][4];
-#pragma unroll
-        for (int k = 1; k < 4; ++k)
-#pragma unroll
-            for (int l = k; l < 4; ++l) {
-                Gm[k][l] = (b[k][0] * b[l][0] + b[k][1] * b[l][1] + b[k][2] * b[l][2]) * mi;
-                Gm[l][k] = Gm[k][l];
-            }
-#pragma unroll
-        for (int l = 1; l < 4; ++l) {
-            Gm[0][l] = -(Gm[1][l] + Gm[2][l] + Gm[3][l]);
-            Gm[l][0] = Gm[0][l];
-        }
-        Gm[0][0] = -(Gm[0][1] + Gm[0][2] + Gm[0][3]);
-        // curl term nu (J c_a).(J c_c) = c_a^T (nu J^T J) c_c: with H = 4 nu J^T J (6 entries) and the
-        // reference curls' entries +-2, each entry is a signed sum of 1 to 4 entries of H
-        double H[3][3];
-        const double nu4 = 4.0 * nu;
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-            for (int q = r; q < 3; ++q) {
-                H[r][q] = nu4 * (J[r] * J[q] + J[3 + r] * J[3 + q] + J[6 + r] * J[6 + q]);
-                H[q][r] = H[r][q];
-            }
-        // orientation signs (+1 / -1) applied as a sign-bit flip of the FP64 value
-        uint32_t neg[6];
-#pragma unroll
-        for (int a = 0; a < 6; ++a) neg[a] = signs[a * ne + e] < 0 ? 1u : 0u;
-        double *st = stage + threadIdx.x * 37;
-#pragma unroll
-        for (int a = 0; a < 6; ++a)
-#pragma unroll
-            for (int c = a; c < 6; ++c) {
-                double val = 0.0;
-                bool first = true;
-#pragma unroll
-                for (int r = 0; r < 3; ++r)
-#pragma unroll
-                    for (int q = 0; q < 3; ++q)
-                        if (ref_curl(a, r) != 0.0 && ref_curl(c, q) != 0.0) {
-                            const double h = (ref_curl(a, r) > 0.0) == (ref_curl(c, q) > 0.0) ? H[r][q] : -H[r][q];
-                            val = first ? h : val + h;
-                            first = false;
-                        }
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
-#pragma unroll
-                    for (int v = 0; v < 2; ++v) val += Gm[edge_v(a, u)][edge_v(c, v)] * tab.Tm[a][c][u * 2 + v];
-                const unsigned long long flip = (unsigned long long)(neg[a] ^ neg[c]) << 63;
-                val = __longlong_as_double((long long)((unsigned long long)__double_as_longlong(val) ^ flip));
-                st[a * 6 + c] = val;
-                st[c * 6 + a] = val;
-            }
-    }
+                                                            int inc_curl, const int *__restrict__ redo,
+                                                            int64_t stride, double *__restrict__ Ke) {
+    __shared__ double stage[PACKED ? 1 : kN1Block * 37];
+    __shared__ double Tm[6 * 6 * 4];  // operands from shared memory: see skg_fp64.cuh
+    if (redo && !out_of_range(redo)) return;
+    const Fp64 F = Fp64::load();
+    for (int i = threadIdx.x; i < 144; i += kN1Block) Tm[i] = (&tab.Tm[0][0][0])[i];
     __syncthreads();
-    const int nvalid = (int)(e_end - e0 < kN1Block ? e_end - e0 : kN1Block);
-    for (int i = threadIdx.x; i < nvalid * 36; i += kN1Block) {
-        const int el = i / 36, q = i - el * 36;
-        Ke[(e0 + el) * 36 + q] = stage[el * 37 + q];
+    for (int64_t e0 = e_begin + (int64_t)blockIdx.x * kN1Block; e0 < e_end; e0 += (int64_t)gridDim.x * kN1Block) {
+        const int64_t e = e0 + threadIdx.x;
+        if (e < e_end) {
+            int32_t v[4];
+            bool ok = true;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                v[q] = t[q * ne + e];
+                ok = ok && v[q] >= 0 && v[q] < npts;
+            }
+            // out-of-range vertex ids never reach memory: the element becomes NaN
+            if (!ok) v[0] = v[1] = v[2] = v[3] = 0;
+            double J[9], b[4][3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const double x0 = ok ? p[i * npts + v[0]] : __longlong_as_double(0x7ff8000000000000LL);
+#pragma unroll
+                for (int r = 0; r < 3; ++r) J[i * 3 + r] = F.sub(p[i * npts + v[r + 1]], x0);
+            }
+            const double det = F.adjugate(J, b);
+            const double inv = 1.0 / fabs(det);
+            const double mu = inc_mass ? (mass ? mass[e] : 1.0) : 0.0;
+            const double nu = inc_curl ? (curl ? curl[e] : 1.0) * inv * tab.wsum : 0.0;
+            // mu b_k . b_l / |det J|: dot products for k, l >= 1, row 0 from
+            // b_0 = -(b_1 + b_2 + b_3); mu / |det J| scales the six products once
+            const double mi = mu * inv;
+            double Gm[4][4];
+#pragma unroll
+            for (int k = 1; k < 4; ++k)
+#pragma unroll
+                for (int l = k; l < 4; ++l) {
+                    Gm[k][l] = F.mul(F.dot(b[k], b[l]), mi);
+                    Gm[l][k] = Gm[k][l];
+                }
+#pragma unroll
+            for (int l = 1; l < 4; ++l) {
+                Gm[0][l] = -F.add3(Gm[1][l], Gm[2][l], Gm[3][l]);
+                Gm[l][0] = Gm[0][l];
+            }
+            Gm[0][0] = -F.add3(Gm[0][1], Gm[0][2], Gm[0][3]);
+            // curl term nu (J c_a).(J c_c) = c_a^T (nu J^T J) c_c: with H = 4 nu J^T J (6 entries) and the
+            // reference curls' entries +-2, each entry is a signed sum of 1 to 4 entries of H
+            double H[3][3];
+            const double nu4 = 4.0 * nu;
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int q = r; q < 3; ++q) {
+                    H[r][q] = F.mul(nu4, fma(J[6 + r], J[6 + q], fma(J[3 + r], J[3 + q], F.mul(J[r], J[q]))));
+                    H[q][r] = H[r][q];
+                }
+            // orientation signs (+1 / -1) applied as a sign-bit flip of the FP64 value
+            uint32_t neg[6];
+#pragma unroll
+            for (int a = 0; a < 6; ++a) neg[a] = signs[a * ne + e] < 0 ? 1u : 0u;
+            double *st = stage + (PACKED ? 0 : threadIdx.x * 37);
+#pragma unroll
+            for (int a = 0; a < 6; ++a)
+#pragma unroll
+                for (int c = a; c < 6; ++c) {
+                    double val = 0.0;
+                    bool first = true;
+#pragma unroll
+                    for (int r = 0; r < 3; ++r)
+#pragma unroll
+                        for (int q = 0; q < 3; ++q)
+                            if (ref_curl(a, r) != 0.0 && ref_curl(c, q) != 0.0) {
+                                const double h = (ref_curl(a, r) > 0.0) == (ref_curl(c, q) > 0.0) ? H[r][q] : -H[r][q];
+                                val = first ? h : F.add(val, h);
+                                first = false;
+                            }
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+#pragma unroll
+                        for (int w = 0; w < 2; ++w)
+                            val = fma(Gm[edge_v(a, u)][edge_v(c, w)], Tm[(a * 6 + c) * 4 + u * 2 + w], val);
+                    const unsigned long long flip = (unsigned long long)(neg[a] ^ neg[c]) << 63;
+                    val = __longlong_as_double((long long)((unsigned long long)__double_as_longlong(val) ^ flip));
+                    if constexpr (PACKED) {
+                        Ke[tri_index(6, a, c) * stride + e] = val;
+                    } else {
+                        st[a * 6 + c] = val;
+                        st[c * 6 + a] = val;
+                    }
+                }
+        }
+        if constexpr (!PACKED) {
+            const int nvalid = (int)(e_end - e0 < kN1Block ? e_end - e0 : kN1Block);
+            __syncthreads();
+            for (int i = threadIdx.x; i < nvalid * 36; i += kN1Block) {
+                const int el = i / 36, q = i - el * 36;
+                Ke[(e0 + el) * 36 + q] = stage[el * 37 + q];
+            }
+            __syncthreads();
+        }
     }
 }
 
@@ -265,8 +303,8 @@ __global__ void __launch_bounds__(kN1Block) k_n1_elem_df(int64_t ne, int64_t e_b
                                                           const double *__restrict__ mass,
                                                           const double *__restrict__ curl, int inc_mass,
                                                           int inc_curl, const int *__restrict__ s_ptr,
-                                                          int *__restrict__ range_bad, double *__restrict__ Ke) {
-    __shared__ double stage[kN1Block * 37];
+                                                          int *__restrict__ range_bad, int64_t stride,
+                                                          double *__restrict__ Ke) {
     const int sc = *s_ptr;
     const int64_t e0 = e_begin + (int64_t)blockIdx.x * kN1Block;
     const int64_t e = e0 + threadIdx.x;
@@ -334,7 +372,6 @@ __global__ void __launch_bounds__(kN1Block) k_n1_elem_df(int64_t ne, int64_t e_b
         float sg[6];
 #pragma unroll
         for (int a = 0; a < 6; ++a) sg[a] = (float)signs[a * ne + e];
-        double *st = stage + threadIdx.x * 37;
 #pragma unroll
         for (int a = 0; a < 6; ++a)
 #pragma unroll
@@ -373,16 +410,9 @@ __global__ void __launch_bounds__(kN1Block) k_n1_elem_df(int64_t ne, int64_t e_b
                 // unscaled in the FP64 exponent (exact), then one FP64 add
                 double dv = df_to_double(mt, sc) + df_to_double(ct, -sc);
                 if (sg[a] * sg[c] < 0.f) dv = -dv;
-                st[a * 6 + c] = dv;
-                st[c * 6 + a] = dv;
+                Ke[tri_index(6, a, c) * stride + e] = dv;
             }
         if (!ok) *range_bad = 1;
-    }
-    __syncthreads();
-    const int nvalid = (int)(e_end - e0 < kN1Block ? e_end - e0 : kN1Block);
-    for (int i = threadIdx.x; i < nvalid * 36; i += kN1Block) {
-        const int el = i / 36, q = i - el * 36;
-        Ke[(e0 + el) * 36 + q] = stage[el * 37 + q];
     }
 }
 
@@ -557,28 +587,28 @@ static void n1_table(int nq, const double *X, const double *W, N1Table &tab) {
 namespace skg {
 namespace {
 
-// Element matrices by the closed form, then CSR row sums.  h_values
-// (optional, page-locked host): the values are also copied there; on a
-// row-grouped pattern the element and row passes then interleave over row
-// chunks so that the copies overlap them (run_passes).
+// Element matrices by the closed form (packed), then the pair sums.  h_values
+// (optional, page-locked host): the values are also copied there.  Split
+// precision: the double-float element pass, then the FP64 one in its place when
+// a value left the FP32 range, decided on the device (no synchronisation).
 void n1_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, const int32_t *d_t, const int8_t *d_signs,
                  int64_t ne, int32_t nq, const double *h_X, const double *h_W, const double *d_mass,
                  const double *d_curl, int32_t include_mass, int32_t include_curl, int32_t precision,
                  double *d_values, double *h_values, cudaStream_t s) {
     N1Table tab;
     n1_table(nq, h_X, h_W, tab);
-    DevBuf<double> Ke((size_t)ne * 36, s);
-    auto elem64 = [&](int64_t e0, int64_t e1) {
-        k_n1_elem_fast<<<grid_for(e1 - e0, kN1Block), kN1Block, 0, s>>>(ne, e0, e1, d_p, npts, d_t, d_signs, tab,
-                                                                      d_mass, d_curl, include_mass, include_curl,
-                                                                      Ke.get());
+    const int64_t stride = block_stride(ne);
+    DevBuf<double> Ke((size_t)stride * 21, s);
+    DevBuf<int> misc(2, s);  // [0] scale exponent, [1] range flag (split precision)
+    auto elem64 = [&](int64_t e0, int64_t e1, const int *redo) {
+        const unsigned grid = grid_for(e1 - e0, kN1Block);
+        k_n1_elem_fast<true><<<redo ? std::min(grid, 4u * kSmCount) : grid, kN1Block, 0, s>>>(
+            ne, e0, e1, d_p, npts, d_t, d_signs, tab, d_mass, d_curl, include_mass, include_curl, redo, stride,
+            Ke.get());
         SKG_LAUNCH_CHECK("n1_element");
     };
-    auto rows = [&](const GroupSet &gs, cudaStream_t st) { add_element_rows<6>(pat, Ke.get(), d_values, st, gs); };
-    const bool groups = pat->max_row_len > 0;
-    if (precision == SKG_SPLIT_FP32 && ne) {
-        // element pass in split precision over all elements first (its range
-        // check decides whether the FP64 pass replaces it), then the row pass
+    const bool split = precision == SKG_SPLIT_FP32 && ne;
+    if (split) {
         N1TableF tf;
         for (int a = 0; a < 6; ++a)
             for (int c = 0; c < 6; ++c)
@@ -589,29 +619,26 @@ void n1_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, const 
                 }
         const float wh = (float)tab.wsum;
         tf.wsum = make_float2(wh, (float)(tab.wsum - (double)wh));
-        DevBuf<int> misc(2, s);  // [0] scale exponent, [1] range flag
-        const int init[2] = {INT_MIN, 0};
-        SKG_CUDA(cudaMemcpyAsync(misc.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
+        SKG_CUDA(cudaMemsetAsync(misc.get(), 0x80, 2 * sizeof(int), s));
         launch_scale_exponent(d_p, 3 * npts, misc.get(), s);
         k_n1_elem_df<<<grid_for(ne, kN1Block), kN1Block, 0, s>>>(ne, 0, ne, d_p, npts, d_t, d_signs, tf, d_mass,
                                                                  d_curl, include_mass, include_curl, misc.get(),
-                                                                 misc.get() + 1, Ke.get());
+                                                                 misc.get() + 1, stride, Ke.get());
         SKG_LAUNCH_CHECK("n1_element_df");
-        int h_misc[2];
-        SKG_CUDA(cudaMemcpyAsync(h_misc, misc.get(), sizeof(h_misc), cudaMemcpyDeviceToHost, s));
-        SKG_CUDA(cudaStreamSynchronize(s));
-        if (h_misc[1] != 0 || h_misc[0] == INT_MIN) elem64(0, ne);  // out of FP32 range: FP64 instead
-        if (groups) {
-            run_row_pass(pat, d_values, h_values, s, rows);
-            return;
-        }
-    } else if (h_values && groups) {
-        run_passes(pat, ne, d_values, h_values, s, elem64, rows);
-        return;
-    } else if (ne) {
-        elem64(0, ne);
+        elem64(0, ne, misc.get());
     }
-    gather_element_matrices(pat, Ke.get(), d_values, s);
+    if (pat->pairs.block == 1 && pat->pairs.nodes == 6) {
+        run_pair_passes(
+            pat, split ? 0 : ne, d_values, h_values, s, [&](int64_t e0, int64_t e1) { elem64(e0, e1, nullptr); },
+            [&](int s0, int s1, cudaStream_t st) {
+                pair_sum<double>(pat->pairs, s0, s1, Ke.get(), PairLower<double>{}, PairIdentity{}, nullptr, d_values, st);
+            });
+        return;
+    }
+    if (!split && ne) elem64(0, ne, nullptr);
+    DevBuf<double> full((size_t)ne * 36, s);
+    expand_packed(ne, 6, Ke.get(), full.get(), s);
+    gather_element_matrices(pat, full.get(), d_values, s);
     if (h_values && pat->nnz)
         SKG_CUDA(cudaMemcpyAsync(h_values, d_values, (size_t)pat->nnz * sizeof(double), cudaMemcpyDeviceToHost, s));
 }
@@ -803,9 +830,9 @@ extern "C" int skg_n1_element_matrices(const double *d_p, int64_t npts, const in
         N1Table tab;
         n1_table(nq, h_X, h_W, tab);
         if (!coef_per_point) {
-            k_n1_elem_fast<<<grid_for(ne, kN1Block), kN1Block, 0, s>>>(ne, 0, ne, d_p, npts, d_t, d_signs, tab,
-                                                                      d_mass, d_curl, include_mass, include_curl,
-                                                                      d_out);
+            k_n1_elem_fast<false><<<grid_for(ne, kN1Block), kN1Block, 0, s>>>(ne, 0, ne, d_p, npts, d_t, d_signs, tab,
+                                                                             d_mass, d_curl, include_mass,
+                                                                             include_curl, nullptr, 0, d_out);
             SKG_LAUNCH_CHECK("n1_element_matrices");
             return;
         }

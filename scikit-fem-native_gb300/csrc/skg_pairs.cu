@@ -46,12 +46,13 @@ __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p,
 namespace {
 
 // Full matrices (E, n, n) from packed upper triangles: patterns without a plan.
-__global__ void k_expand_packed(int64_t ne, int n, const double *__restrict__ K, double *__restrict__ full) {
+__global__ void k_expand_packed(int64_t ne, int64_t stride, int n, const double *__restrict__ K,
+                                double *__restrict__ full) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ne * n * n) return;
     const int64_t e = i / (n * n);
     const int q = (int)(i - e * n * n), a = q / n, b = q - a * n;
-    full[i] = K[e * (n * (n + 1) / 2) + (a <= b ? tri_index(n, a, b) : tri_index(n, b, a))];
+    full[i] = K[(a <= b ? tri_index(n, a, b) : tri_index(n, b, a)) * stride + e];
 }
 
 // Full element matrices (E, 3n, 3n) from packed blocks, likewise.
@@ -249,7 +250,7 @@ __global__ void __launch_bounds__(kPairWindow) k_pair_fill(NodeView<K> v, const 
         each_contribution(v, r, c, [&](int32_t e, int a, int b) {
             const uint32_t t = (uint32_t)(K == 0 ? a * v.n + b : tri_index(v.n, min(a, b), max(a, b)));
             codes[(int64_t)k * 32 + lane] =
-                C == 1 ? (uint32_t)e * (uint32_t)np + t : t * (uint32_t)stride + (uint32_t)e;
+                K == 0 ? (uint32_t)e * (uint32_t)np + t : t * (uint32_t)stride + (uint32_t)e;
             if (K != 0 && a > b) atomicOr(orient + k, 1u << lane);
             ++k;
         });
@@ -378,7 +379,7 @@ PairPlan build(const skg_pattern *p, cudaStream_t s) {
 
 void expand_packed(int64_t ne, int n, const double *K, double *full, cudaStream_t s) {
     if (ne == 0) return;
-    k_expand_packed<<<grid_for(ne * n * n, 256), 256, 0, s>>>(ne, n, K, full);
+    k_expand_packed<<<grid_for(ne * n * n, 256), 256, 0, s>>>(ne, block_stride(ne), n, K, full);
     SKG_LAUNCH_CHECK("expand_packed");
 }
 

@@ -37,10 +37,14 @@ namespace skg {
 
 constexpr int kPairWindow = 1024;
 constexpr uint32_t kPairNone = 0xffffffffu;
-// Elements per tile (one block) of the element passes: small blocks keep the
-// FP64 pipe fed while others load or store (P2 element pass at 64^3: 509 us,
-// 534 us with tiles of 128).
-constexpr int kTile = 64;
+// Elements per tile (one block) of the element passes.
+constexpr int kTile = 128;
+
+// Packed element matrices lie entry by entry: entry (block) t of element e at
+// t * stride + e, so that the threads of an element pass (one element each)
+// store whole lines without a stage in shared memory, whose size would limit
+// the warps that keep the FP64 pipe fed.
+inline int64_t block_stride(int64_t ne) { return (ne + kTile - 1) / kTile * kTile; }
 
 // Packed upper triangle of an n x n (block) matrix, a <= b.
 __host__ __device__ constexpr int tri_index(int n, int a, int b) { return a * n - a * (a - 1) / 2 + (b - a); }
@@ -90,6 +94,7 @@ struct PairLower {
     const E *K = nullptr;
     const int *any = nullptr;
     const uint8_t *tiles = nullptr;
+    uint32_t stride = 1;
 };
 
 struct PairArrays {
@@ -97,11 +102,10 @@ struct PairArrays {
     const uint32_t *codes, *orient;
     const uint2 *slots;
     const uint4 *slots3;
-    int np;
 };
 
 inline PairArrays pair_arrays(const PairPlan &p) {
-    return PairArrays{p.slice_ptr, p.codes, p.orient, p.slots, p.slots3, p.np};
+    return PairArrays{p.slice_ptr, p.codes, p.orient, p.slots, p.slots3};
 }
 
 struct PairIdentity {
@@ -149,7 +153,7 @@ __global__ void __launch_bounds__(kPairWarps * 32) k_pair_sum(int w0, int w1, Pa
                     T a, b;
                     pair_load(K, c, a);
                     b = a;
-                    if (lower.tiles[c / (uint32_t)p.np / (uint32_t)kTile]) pair_load(lower.K, c, b);
+                    if (lower.tiles[c % lower.stride / (uint32_t)kTile]) pair_load(lower.K, c, b);
                     pair_add(up, turned ? b : a);
                     pair_add(lo, turned ? a : b);
                 }
@@ -218,12 +222,9 @@ inline void pair_sum(const PairPlan &plan, int s0, int s1, const E *K, const Pai
     SKG_LAUNCH_CHECK("pair_sum");
 }
 
-// Three components per node: packed blocks (np, stride, 3, 3), block t of
-// element e at (t * stride + e) * 9; the blocks of 32 elements are one
-// contiguous, 16-byte aligned range for each t.  A block of threads per slice,
-// nine threads per pair.
-inline int64_t block_stride(int64_t ne) { return (ne + kTile - 1) / kTile * kTile; }
-
+// Three components per node: packed blocks (np, stride, 3, 3); the blocks t of
+// 32 elements are one contiguous, 16-byte aligned range.  A block of threads
+// per slice, nine threads per pair.
 constexpr int kPairBlock3 = 288;
 
 __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p, const double *__restrict__ K,
@@ -310,7 +311,7 @@ void run_pair_passes(const skg_pattern *pat, int64_t ne, double *d_values, doubl
     }
 }
 
-// A block's packed matrices, staged in shared memory (16-byte aligned), to
+// A block's element vectors, staged in shared memory (16-byte aligned), to
 // global memory as one bulk copy: the tile is one contiguous range, and the
 // copy engine writes it without load / store instructions of the threads.
 // Every thread of the block calls it after its last store to the stage; the

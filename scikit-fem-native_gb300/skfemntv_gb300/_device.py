@@ -57,11 +57,7 @@ _TORCH_DTYPES = {
 
 def to_device(a, dtype):
     """Copy a host array to a new contiguous device tensor of ``dtype``."""
-    t = require_cuda()
-    a = np.ascontiguousarray(np.asarray(a, dtype=dtype))
-    if not a.flags.writeable:
-        a = a.copy()
-    return t.from_numpy(a).to(device(), non_blocking=False)
+    return host_tensor(np.asarray(a, dtype=dtype)).to(device(), non_blocking=False)
 
 
 def empty(shape, dtype):
