@@ -232,10 +232,14 @@ __host__ __device__ constexpr int tri10(int a, int b) { return tri_index(10, a, 
 // The largest |x| is found on the bit patterns (for non-negative doubles the
 // integer order of the bits is the numeric order), so the scan runs on the
 // integer pipes; only the winner's exponent is decoded.
-__global__ void k_scale(const double *__restrict__ p, int64_t n, int *__restrict__ s_out) {
+constexpr int kScaleBlock = 512;
+
+__global__ void __launch_bounds__(kScaleBlock) k_scale(const double *__restrict__ p, int64_t n,
+                                                       int *__restrict__ s_out) {
+    __shared__ unsigned long long best[kScaleBlock / 32];
     unsigned long long m = 0;
-#pragma unroll 8
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+#pragma unroll 16
+    for (int64_t i = (int64_t)blockIdx.x * kScaleBlock + threadIdx.x; i < n; i += (int64_t)gridDim.x * kScaleBlock) {
         const unsigned long long b = (unsigned long long)__double_as_longlong(p[i]) & 0x7fffffffffffffffULL;
         if (b < 0x7ff0000000000000ULL) m = b > m ? b : m;  // finite values only
     }
@@ -244,9 +248,11 @@ __global__ void k_scale(const double *__restrict__ p, int64_t n, int *__restrict
         const unsigned long long q = __shfl_xor_sync(0xffffffffu, m, o);
         m = q > m ? q : m;
     }
-    if ((threadIdx.x & 31) == 0 && m != 0) {
-        const double a = __longlong_as_double((long long)m);
-        atomicMax(s_out, ilogb(a) + 1);
+    if ((threadIdx.x & 31) == 0) best[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {  // one atomic per block: they queue at one address
+        for (int w = 1; w < kScaleBlock / 32; ++w) m = best[w] > m ? best[w] : m;
+        if (m != 0) atomicMax(s_out, ilogb(__longlong_as_double((long long)m)) + 1);
     }
 }
 
@@ -848,7 +854,7 @@ template <class E>
 struct PackedOut {
     E *upper, *lower;
     uint8_t *tiles;  // per tile: the lower triangles are there too
-    int *any;        // set when a tile is flagged
+    int *any;        // set to 1 when a tile is flagged
     int64_t stride;
 };
 
@@ -1141,7 +1147,7 @@ bool p2_rule_is_exact(const std::vector<double> &T) {
 }  // namespace
 
 void launch_scale_exponent(const double *d_p, int64_t n, int *d_s, cudaStream_t stream) {
-    k_scale<<<2 * kSmCount, 256, 0, stream>>>(d_p, n, d_s);
+    k_scale<<<2 * kSmCount, kScaleBlock, 0, stream>>>(d_p, n, d_s);
     SKG_LAUNCH_CHECK("scale");
 }
 
@@ -1159,13 +1165,13 @@ void affine_assemble_pairs(const skg_pattern *pat, const double *d_p, int64_t np
     const int np = nodes * (nodes + 1) / 2;
     const int64_t tiles = (ne + kTile - 1) / kTile;
     const bool maybe_lower = coef_kind != 0;  // a tensor may be nonsymmetric
-    // [0] scale exponent, [1] range flag (0x80808080: none, in range), [2] a tile holds a nonsymmetric coefficient
+    // [0] scale exponent, [1] range flag, [2] a tile holds a nonsymmetric coefficient (1); 0x80808080: none of it
     DevBuf<int> misc(3, s);
     const int64_t stride = block_stride(ne);
     DevBuf<double> K((size_t)stride * np, s), lower(maybe_lower ? (size_t)stride * np : 0, s);
     DevBuf<uint8_t> tile_flags(maybe_lower ? (size_t)tiles : 0, s);
     int *any = maybe_lower ? misc.get() + 2 : nullptr;
-    if (maybe_lower) SKG_CUDA(cudaMemsetAsync(any, 0, 4, s));
+    if (maybe_lower || precision != SKG_FP64) SKG_CUDA(cudaMemsetAsync(misc.get(), 0x80, 3 * sizeof(int), s));
     const PackedOut<double> out64{K.get(), lower.get(), tile_flags.get(), any, stride};
     const double *Tg = nodes == 10 && !exact_rule ? device_table(T.data(), T.size(), s) : nullptr;
     auto elem64 = [&](int64_t e0, int64_t e1, const int *redo) {
@@ -1191,9 +1197,7 @@ void affine_assemble_pairs(const skg_pattern *pat, const double *d_p, int64_t np
         if (ev) SKG_CUDA(cudaEventRecord(ev[2], s));
         return;
     }
-    SKG_CUDA(cudaMemsetAsync(misc.get(), 0x80, 2 * sizeof(int), s));
-    k_scale<<<2 * kSmCount, 256, 0, s>>>(d_p, 3 * npts, misc.get());
-    SKG_LAUNCH_CHECK("scale");
+    launch_scale_exponent(d_p, 3 * npts, misc.get(), s);
     // The FP32-pair entries lie in scratch of their own: with a host output
     // their sums and copies follow the element pass step by step, before the
     // range flag is final.
@@ -1271,7 +1275,7 @@ void affine_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, co
     if (mode != MODE_FP64) {
         const int init[2] = {INT_MIN, 0};
         SKG_CUDA(cudaMemcpyAsync(misc.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
-        k_scale<<<2 * kSmCount, 256, 0, s>>>(d_p, 3 * npts, misc.get());
+        k_scale<<<2 * kSmCount, kScaleBlock, 0, s>>>(d_p, 3 * npts, misc.get());
         SKG_LAUNCH_CHECK("scale");
         if (ev) SKG_CUDA(cudaEventRecord(ev[0], s));
         if (ne) {
@@ -1499,7 +1503,7 @@ extern "C" int skg_h1_assemble_affine_noalloc(const skg_pattern *pat, const doub
             // the array keeps the previous call's contents: reset the scale and the flag
             const int init[2] = {INT_MIN, 0};
             SKG_CUDA(cudaMemcpyAsync(misc, init, sizeof(init), cudaMemcpyHostToDevice, s));
-            k_scale<<<2 * kSmCount, 256, 0, s>>>(d_p, 3 * npts, misc);
+            k_scale<<<2 * kSmCount, kScaleBlock, 0, s>>>(d_p, 3 * npts, misc);
             SKG_LAUNCH_CHECK("scale");
             if (ne) {
                 k_elem_df64<<<grid_for(ne, kElemBlock), kElemBlock, 0, s>>>(ne, d_p, npts, d_t, coef_kind, d_coef, misc,

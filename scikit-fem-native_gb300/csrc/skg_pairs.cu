@@ -9,34 +9,33 @@
 namespace skg {
 
 // Nine threads per pair; a contribution is 72 contiguous bytes, so that the
-// nine loads of a pair share its sectors.
+// nine loads of a pair share its sectors.  One slice per block and four
+// contributions together keep 32 pairs' loads in flight per block at 44
+// registers; two or four slices per block measured 1.3 and 4 times as long
+// (vector P1 48^3: 158 us; 215, 727).
 __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p, const double *__restrict__ K,
                                                            double *__restrict__ values) {
-    constexpr int kAhead = 4;  // contributions loaded together
+    constexpr int kAhead = 4;
     const int s = s0 + blockIdx.x;
     const int l = threadIdx.x / 9, en = threadIdx.x - l * 9, i = en / 3, k = en - i * 3;
     const int at = i * 3 + k, turned = k * 3 + i;
     const int32_t k0 = p.slice_ptr[s], n = p.slice_ptr[s + 1] - k0;
-    const uint32_t *cs = p.codes + (int64_t)k0 * 32 + l;
     const uint4 to = p.slots3[(int64_t)s * 32 + l];
     double sum = -0.0;  // leaves any sum unchanged
-    for (int q = 0; q < n; q += kAhead) {
+    for (int f = 0; f < n; f += kAhead) {
         uint32_t c[kAhead], o[kAhead];
         double v[kAhead];
 #pragma unroll
         for (int j = 0; j < kAhead; ++j) {
-            c[j] = q + j < n ? __ldg(cs + (q + j) * 32) : kPairNone;
-            o[j] = q + j < n ? __ldg(p.orient + k0 + q + j) : 0u;
+            c[j] = f + j < n ? __ldg(p.codes + (int64_t)(k0 + f + j) * 32 + l) : kPairNone;
+            o[j] = f + j < n ? __ldg(p.orient + k0 + f + j) : 0u;
         }
 #pragma unroll
         for (int j = 0; j < kAhead; ++j)
             v[j] = c[j] != kPairNone ? __ldg(K + (int64_t)c[j] * 9 + ((o[j] >> l) & 1u ? turned : at)) : -0.0;
 #pragma unroll
         for (int j = 0; j < kAhead; ++j)
-            if (q + j < n) {
-                if (q + j == 0) sum = v[0];
-                else sum += v[j];
-            }
+            if (f + j < n) sum = f + j == 0 ? v[j] : sum + v[j];
     }
     if (to.x == kPairNone) return;
     values[to.x + i * to.y + k] = sum;

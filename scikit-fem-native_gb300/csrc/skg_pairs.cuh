@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kPairWarps * 32) k_pair_sum(int w0, int w1, Pa
                                                              const int *__restrict__ redo,
                                                              double *__restrict__ values) {
     if (redo && !out_of_range(redo)) return;
-    const bool general = lower.any && *lower.any != 0;
+    const bool general = lower.any && *lower.any == 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int w = w0 + blockIdx.x; w < w1; w += gridDim.x) {
         const int s = w * (kPairWindow / 32) + warp;
