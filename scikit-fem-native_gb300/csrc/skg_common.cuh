@@ -212,7 +212,7 @@ struct PairPlan {
     DevBuf<unsigned char> store;  // the arrays below
     int32_t *slice_ptr = nullptr;  // (n_slices + 1), in units of 32 codes
     uint32_t *codes = nullptr;     // position in the packed matrices, contribution k of lane l at 32 k + l
-    uint32_t *orient = nullptr;    // per 32 codes, bit l: the pair's first node is the later local node
+    uint32_t *orient = nullptr;    // block 1: per 32 codes, bit l: the pair's first node is the later local node
     uint2 *slots = nullptr;        // block 1: CSR positions of (r, c) and (c, r) (the latter none when r = c)
     uint4 *slots3 = nullptr;       // block 3: position of (3r, 3c), length of row 3r, the same for (3c, 3r)
     // at least kHostChunkMinNnz values: up to kHostChunks copies, by `slice`, and

@@ -23,6 +23,11 @@ struct Fp64 {
         asm volatile("ld.global.f64 %0, [%1];" : "=d"(f.three_) : "l"(g_fp64_units + 2));
         return f;
     }
+    static __device__ __forceinline__ double unit() {
+        double one;
+        asm volatile("ld.global.f64 %0, [%1];" : "=d"(one) : "l"(g_fp64_units));
+        return one;
+    }
     __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
     __device__ __forceinline__ double sub(double a, double b) const { return fma(a, one, -b); }
     __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, none); }

@@ -1,42 +1,58 @@
 // Builds the pair plan of a pattern (see skg_pairs.cuh) and holds the sums of
 // plans with three components per node.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "skg_common.cuh"
+#include "skg_fp64.cuh"
 #include "skg_pairs.cuh"
 
 namespace skg {
 
 // Nine threads per pair; a contribution is 72 contiguous bytes, so that the
-// nine loads of a pair share its sectors.  One slice per block and four
-// contributions together keep 32 pairs' loads in flight per block at 44
-// registers; two or four slices per block measured 1.3 and 4 times as long
-// (vector P1 48^3: 158 us; 215, 727).
+// nine loads of a pair share its sectors.  Bound by the FP64 pipe (three
+// quarters busy; an addition costs the same for a partly filled warp), the
+// reads and issue together: additions are fused multiply-adds, the orientation
+// is the top bit of the code, and the contributions come in whole batches (one
+// slice per block: its count is the same for every thread).  Vector P1 48^3:
+// 158 -> 139 us; batches of 2 or 8 instead of 4: 154, 142; predicated batches of
+// 4, 8, 12: 149, 173, 242; codes staged in shared memory: no faster.
 __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p, const double *__restrict__ K,
                                                            double *__restrict__ values) {
-    constexpr int kAhead = 4;
+    const double one = Fp64::unit();
     const int s = s0 + blockIdx.x;
     const int l = threadIdx.x / 9, en = threadIdx.x - l * 9, i = en / 3, k = en - i * 3;
-    const int at = i * 3 + k, turned = k * 3 + i;
     const int32_t k0 = p.slice_ptr[s], n = p.slice_ptr[s + 1] - k0;
     const uint4 to = p.slots3[(int64_t)s * 32 + l];
-    double sum = -0.0;  // leaves any sum unchanged
-    for (int f = 0; f < n; f += kAhead) {
-        uint32_t c[kAhead], o[kAhead];
-        double v[kAhead];
+    const uint32_t *cs = p.codes + (int64_t)k0 * 32 + l;
+    const double *at = K + en, *turned = K + k * 3 + i;
+    double sum = -0.0;
+    // the next N contributions, the first of all without an addition: whole
+    // batches, so that no instruction is issued for nothing
+    const auto batch = [&](auto count, bool first) {
+        constexpr int N = decltype(count)::value;
+        uint32_t c[N];
+        double v[N];
 #pragma unroll
-        for (int j = 0; j < kAhead; ++j) {
-            c[j] = f + j < n ? __ldg(p.codes + (int64_t)(k0 + f + j) * 32 + l) : kPairNone;
-            o[j] = f + j < n ? __ldg(p.orient + k0 + f + j) : 0u;
-        }
+        for (int j = 0; j < N; ++j) c[j] = __ldg(cs + 32 * j);
 #pragma unroll
-        for (int j = 0; j < kAhead; ++j)
-            v[j] = c[j] != kPairNone ? __ldg(K + (int64_t)c[j] * 9 + ((o[j] >> l) & 1u ? turned : at)) : -0.0;
+        for (int j = 0; j < N; ++j)  // -0.0 leaves any sum unchanged
+            v[j] = c[j] != kPairNone ? __ldg((c[j] & kPairTurned ? turned : at) + (uint64_t)(c[j] & ~kPairTurned) * 9)
+                                     : -0.0;
+        sum = first ? v[0] : fma(sum, one, v[0]);
 #pragma unroll
-        for (int j = 0; j < kAhead; ++j)
-            if (f + j < n) sum = f + j == 0 ? v[j] : sum + v[j];
+        for (int j = 1; j < N; ++j) sum = fma(sum, one, v[j]);
+        cs += 32 * N;
+    };
+    switch (n & 3) {
+        case 1: batch(std::integral_constant<int, 1>{}, true); break;
+        case 2: batch(std::integral_constant<int, 2>{}, true); break;
+        case 3: batch(std::integral_constant<int, 3>{}, true); break;
+        default:
+            if (n) batch(std::integral_constant<int, 4>{}, true);
     }
+    for (int f = (n - 1) >> 2; f > 0; --f) batch(std::integral_constant<int, 4>{}, false);
     if (to.x == kPairNone) return;
     values[to.x + i * to.y + k] = sum;
     if (to.z != kPairNone) values[to.z + k * to.w + i] = sum;
@@ -249,8 +265,9 @@ __global__ void __launch_bounds__(kPairWindow) k_pair_fill(NodeView<K> v, const 
         each_contribution(v, r, c, [&](int32_t e, int a, int b) {
             const uint32_t t = (uint32_t)(K == 0 ? a * v.n + b : tri_index(v.n, min(a, b), max(a, b)));
             codes[(int64_t)k * 32 + lane] =
-                K == 0 ? (uint32_t)e * (uint32_t)np + t : t * (uint32_t)stride + (uint32_t)e;
-            if (K != 0 && a > b) atomicOr(orient + k, 1u << lane);
+                K == 0 ? (uint32_t)e * (uint32_t)np + t
+                       : (t * (uint32_t)stride + (uint32_t)e) | (K == 3 && a > b ? kPairTurned : 0u);
+            if (K == 1 && a > b) atomicOr(orient + k, 1u << lane);
             ++k;
         });
         to.x = (uint32_t)(v.begin(r) + v.length(r) - C * (pair_ptr[r + 1] - j));
@@ -322,7 +339,7 @@ PairPlan build(const skg_pattern *p, cudaStream_t s) {
     exclusive_scan_i32(width.get(), slice_ptr.get(), plan.n_slices, s);
     download(h, slice_ptr.get() + plan.n_slices, 1, s);
     const int32_t total = h[0];
-    const size_t ptr_bytes = ((size_t)plan.n_slices + 1) * 4, orient_bytes = (size_t)total * 4;
+    const size_t ptr_bytes = ((size_t)plan.n_slices + 1) * 4, orient_bytes = K == 1 ? (size_t)total * 4 : 0;
     const size_t slot_bytes = (size_t)n_lanes * (C == 1 ? sizeof(uint2) : sizeof(uint4));
     const size_t code_bytes = (size_t)total * 32 * 4;
     plan.store = DevBuf<unsigned char>::owned(slot_bytes + code_bytes + orient_bytes + ptr_bytes);
@@ -333,7 +350,7 @@ PairPlan build(const skg_pattern *p, cudaStream_t s) {
     plan.orient = reinterpret_cast<uint32_t *>(at += code_bytes);
     plan.slice_ptr = reinterpret_cast<int32_t *>(at += orient_bytes);
     SKG_CUDA(cudaMemcpyAsync(plan.slice_ptr, slice_ptr.get(), ptr_bytes, cudaMemcpyDeviceToDevice, s));
-    SKG_CUDA(cudaMemsetAsync(plan.orient, 0, orient_bytes, s));
+    if (orient_bytes) SKG_CUDA(cudaMemsetAsync(plan.orient, 0, orient_bytes, s));
     const int n_chunks = K != 0 && p->nnz >= kHostChunkMinNnz ? kHostChunks : 0;
     DevBuf<int32_t> chunk(3 * (kHostChunks + 1), s);  // first rows, first slots, windows done
     int32_t *first = chunk.get(), *slot = first + kHostChunks + 1, *done = slot + kHostChunks + 1;
@@ -397,7 +414,7 @@ void build_pair_plan(skg_pattern *p, bool square, cudaStream_t s) {
     const int L = p->row_local, C = L == 12 || L == 30 ? 3 : 1;
     const int64_t n = L / C, total = p->n_elements * L;
     if (square && (C == 3 ? p->n_rows % 3 == 0 : L == 4 || L == 6 || L == 10) &&
-        block_stride(p->n_elements) * (n * (n + 1) / 2) < (int64_t)kPairNone) {
+        block_stride(p->n_elements) * (n * (n + 1) / 2) < (int64_t)(C == 3 ? kPairTurned - 1 : kPairNone)) {
         if (C == 1) {
             p->pairs = build<1>(p, s);
             return;

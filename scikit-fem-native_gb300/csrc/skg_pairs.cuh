@@ -27,6 +27,7 @@
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "skg_common.cuh"
@@ -37,6 +38,9 @@ namespace skg {
 
 constexpr int kPairWindow = 1024;
 constexpr uint32_t kPairNone = 0xffffffffu;
+// Plans of three components: set in the codes of the contributions whose first
+// node is the later local node (the stored block is read transposed).
+constexpr uint32_t kPairTurned = 0x80000000u;
 // Elements per tile (one block) of the element passes.
 constexpr int kTile = 128;
 
@@ -188,21 +192,27 @@ __global__ void __launch_bounds__(kPairWarps * 32) k_pair_sum(int w0, int w1, Pa
         for (int q = 0; q < kPairSlices; ++q) {
             T sum = v[q][0];
             if (n[q] > 1) pair_add(sum, v[q][1]);
-            const uint32_t *cs = p.codes + (int64_t)k0[q] * 32 + lane;
-            for (int k = 2; k < n[q]; k += 4) {
-                uint32_t d[4];
-                T x[4];
+            const uint32_t *cs = p.codes + (int64_t)(k0[q] + 2) * 32 + lane;
+            const auto batch = [&](auto count) {  // whole batches: no instruction is issued for nothing
+                constexpr int N = decltype(count)::value;
+                uint32_t d[N];
+                T x[N];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) d[j] = k + j < n[q] ? __ldcs(cs + (k + j) * 32) : kPairNone;
+                for (int j = 0; j < N; ++j) d[j] = __ldcs(cs + j * 32);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int j = 0; j < N; ++j) {
                     x[j] = pair_zero<T>();
                     if (d[j] != kPairNone) pair_load(K, d[j], x[j]);
                 }
 #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (k + j < n[q]) pair_add(sum, x[j]);
-            }
+                for (int j = 0; j < N; ++j) pair_add(sum, x[j]);
+                cs += N * 32;
+            };
+            int left = n[q] - 2;
+            for (; left >= 4; left -= 4) batch(std::integral_constant<int, 4>{});
+            if (left == 3) batch(std::integral_constant<int, 3>{});
+            if (left == 2) batch(std::integral_constant<int, 2>{});
+            if (left == 1) batch(std::integral_constant<int, 1>{});
             const double r = finish(sum);
             if (to[q].x != kPairNone) values[to[q].x] = r;
             if (to[q].y != kPairNone) values[to[q].y] = r;
@@ -226,6 +236,7 @@ inline void pair_sum(const PairPlan &plan, int s0, int s1, const E *K, const Pai
 // 32 elements are one contiguous, 16-byte aligned range.  A block of threads
 // per slice, nine threads per pair.
 constexpr int kPairBlock3 = 288;
+constexpr int kPairStage = 32;  // contributions per pair whose codes are staged together
 
 __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p, const double *__restrict__ K,
                                                            double *__restrict__ values);
