@@ -33,7 +33,7 @@
 
 #include "skg_common.cuh"
 #include "skg_nh.cuh"
-#include "skg_nh_rows.cuh"
+#include "skg_pairs.cuh"
 #include "skg_tc.cuh"
 
 namespace skg {
@@ -512,29 +512,29 @@ __device__ __forceinline__ void normalised_input(const SurState &s, const float 
     for (int m = 0; m < 3; ++m) x[m] = (fr[m] - Nrm[m]) / Nrm[3 + m];
 }
 
-// From the network's derivatives (gx, Hx, normalised units) to the stress,
-// the per-element check against the plain law (FP32) and the tangent.
-// Returns false when the element must fall back to the plain law.  FUSED:
-// writes the surrogate record `out`; otherwise the element tangent Ke and
-// residual re (already offset to the element).
-template <bool FUSED>
-__device__ __forceinline__ bool surrogate_finish(const SurState &st, const float *__restrict__ Nrm, const float gx[3],
-                                                 const float Hx[9], double mu, double lmbda, float tol, float Vf,
-                                                 const float ga[4][3], float4 *__restrict__ out, double *__restrict__ Ke,
-                                                 double *__restrict__ re, double V, int i_begin = 0, int i_end = 3,
-                                                 bool tail = true) {
-    const float *F = st.F, *C = st.C, *FiT = st.FiT;
-    const float I1 = st.I1, J = st.J, iJ = 1.f / st.J;
-    // derivatives of W with respect to the features f
+constexpr int kFinishElems = 64;                // elements per block of the finish kernel
+constexpr int kFinishStage = kFinishElems * 9;  // floats of one packed block of its elements
+
+// Derivatives of W with respect to the features from the network's (gx, Hx, in
+// normalised units); the stress-free reference state is shifted out.
+__device__ __forceinline__ void feature_derivatives(const float *__restrict__ Nrm, const float gx[3],
+                                                    const float Hx[9], float Wf[3], float Wff[9]) {
     const float ys = Nrm[6];
-    float Wf[3], Wff[9];
 #pragma unroll
     for (int m = 0; m < 3; ++m) Wf[m] = ys * gx[m] / Nrm[3 + m];
-    Wf[2] -= Nrm[8];  // stress-free reference state
+    Wf[2] -= Nrm[8];
 #pragma unroll
     for (int m = 0; m < 3; ++m)
 #pragma unroll
         for (int l = 0; l < 3; ++l) Wff[m * 3 + l] = ys * Hx[m * 3 + l] / (Nrm[3 + m] * Nrm[3 + l]);
+}
+
+template <class FB, class FR>
+__device__ __forceinline__ bool surrogate_finish(const SurState &st, const float Wf[3], const float Wff[9], double mu,
+                                                 double lmbda, float tol, float V, const float ga[4][3], FB &&block,
+                                                 FR &&residual) {
+    const float *F = st.F, *C = st.C, *FiT = st.FiT;
+    const float I1 = st.I1, J = st.J, iJ = 1.f / st.J;
     // features -> invariants: f3 = ln J: dW/dJ = W3 / J, d2W/dJ2 = (W33 - W3) / J^2, d2W/dIa dJ = Wa3 / J
     float Wa[3], Wab[9];
     Wa[0] = Wf[0]; Wa[1] = Wf[1]; Wa[2] = Wf[2] * iJ;
@@ -545,23 +545,18 @@ __device__ __forceinline__ bool surrogate_finish(const SurState &st, const float
     Wab[0 * 3 + 2] = Wab[2 * 3 + 0] = Wff[0 * 3 + 2] * iJ;
     Wab[1 * 3 + 2] = Wab[2 * 3 + 1] = Wff[1 * 3 + 2] * iJ;
     Wab[8] = (Wff[8] - Wf[2]) * iJ * iJ;
-    float FC[9], FFt[9], dI[3][9], Pm[9];
+    float dI2[9], FFt[9], Pm[9];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            FC[i * 3 + j] = F[i * 3] * C[j] + F[i * 3 + 1] * C[3 + j] + F[i * 3 + 2] * C[6 + j];
+            dI2[i * 3 + j] = 2.f * (I1 * F[i * 3 + j] -
+                                    (F[i * 3] * C[j] + F[i * 3 + 1] * C[3 + j] + F[i * 3 + 2] * C[6 + j]));
             FFt[i * 3 + j] = F[i * 3] * F[j * 3] + F[i * 3 + 1] * F[j * 3 + 1] + F[i * 3 + 2] * F[j * 3 + 2];
         }
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        dI[0][k] = 2.f * F[k];
-        dI[1][k] = 2.f * (I1 * F[k] - FC[k]);
-        dI[2][k] = J * FiT[k];
-    }
-#pragma unroll
-    for (int k = 0; k < 9; ++k) Pm[k] = Wa[0] * dI[0][k] + Wa[1] * dI[1][k] + Wa[2] * dI[2][k];
-    // per-element check against the plain law in FP32: the stresses must agree
+    for (int k = 0; k < 9; ++k) Pm[k] = Wa[0] * (2.f * F[k]) + Wa[1] * dI2[k] + Wa[2] * (J * FiT[k]);
+    // the stresses must agree with the plain law's
     float diff = 0.f, nrm = 0.f;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
@@ -570,136 +565,121 @@ __device__ __forceinline__ bool surrogate_finish(const SurState &st, const float
         nrm = fmaxf(nrm, fabsf(pl));
     }
     if (!(diff <= tol * fmaxf(nrm, 1e-3f))) return false;
-    // tangent A_iJkL, one row block i (27 entries) at a time; the row-i
-    // quantities are selected once so that the block body is compiled once
-#pragma unroll 1
-    for (int i = i_begin; i < i_end; ++i) {
-        float dIr[3][3], Fr[3], FiTr[3], FFtr[3];
+    float Fg[4][3], Dg[4][3], hg[4][3];  // F g, (dI2/dF) g, (dJ/dF) g
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int m = 0; m < 3; ++m) dIr[m][c] = i == 0 ? dI[m][c] : i == 1 ? dI[m][3 + c] : dI[m][6 + c];
-            Fr[c] = i == 0 ? F[c] : i == 1 ? F[3 + c] : F[6 + c];
-            FiTr[c] = i == 0 ? FiT[c] : i == 1 ? FiT[3 + c] : FiT[6 + c];
-            FFtr[c] = i == 0 ? FFt[c] : i == 1 ? FFt[3 + c] : FFt[6 + c];
+        for (int i = 0; i < 3; ++i) {
+            Fg[a][i] = F[i * 3] * ga[a][0] + F[i * 3 + 1] * ga[a][1] + F[i * 3 + 2] * ga[a][2];
+            Dg[a][i] = dI2[i * 3] * ga[a][0] + dI2[i * 3 + 1] * ga[a][1] + dI2[i * 3 + 2] * ga[a][2];
+            hg[a][i] = J * (FiT[i * 3] * ga[a][0] + FiT[i * 3 + 1] * ga[a][1] + FiT[i * 3 + 2] * ga[a][2]);
+            residual(a, i, V * (Pm[i * 3] * ga[a][0] + Pm[i * 3 + 1] * ga[a][1] + Pm[i * 3 + 2] * ga[a][2]));
         }
-        // sum_ml Wab[m][l] dI_m[iJ] dI_l[kL] = sum_l U[l][J] dI_l[kL] with U[l][J] = sum_m Wab[m][l] dI_m[iJ],
-        // formed once per row block
-        float U[3][3];
+    const float w0 = 2.f * V * Wa[0], w1 = 2.f * V * Wa[1], w2 = V * Wa[2] * iJ;
 #pragma unroll
-        for (int l = 0; l < 3; ++l)
+    for (int k = 0; k < 9; ++k) Wab[k] *= V;
 #pragma unroll
-            for (int Jj = 0; Jj < 3; ++Jj)
-                U[l][Jj] = Wab[l] * dIr[0][Jj] + Wab[3 + l] * dIr[1][Jj] + Wab[6 + l] * dIr[2][Jj];
-        float Ai[28];
+    for (int a = 0; a < 4; ++a) {
+        // sum_ml Wab[m][l] (dI_m g_a)_i (dI_l g_b)_k = sum_l U_l,i (dI_l g_b)_k, and the products with F g_b
+        // and F^-T g_b of the second derivatives
+        float X[3], Y[3], Z[3];
 #pragma unroll
-        for (int Jj = 0; Jj < 3; ++Jj)
+        for (int i = 0; i < 3; ++i) {
+            const float d0 = 2.f * Fg[a][i];
+            X[i] = 2.f * (Wab[0] * d0 + Wab[3] * Dg[a][i] + Wab[6] * hg[a][i] + w1 * Fg[a][i]);
+            Y[i] = Wab[1] * d0 + Wab[4] * Dg[a][i] + Wab[7] * hg[a][i];
+            Z[i] = Wab[2] * d0 + Wab[5] * Dg[a][i] + Wab[8] * hg[a][i] + w2 * hg[a][i];
+        }
 #pragma unroll
-            for (int k = 0; k < 3; ++k)
+        for (int b = a; b < 4; ++b) {
+            const float gg = ga[a][0] * ga[b][0] + ga[a][1] * ga[b][1] + ga[a][2] * ga[b][2];
+            const float ff = Fg[a][0] * Fg[b][0] + Fg[a][1] * Fg[b][1] + Fg[a][2] * Fg[b][2];
+            const float diag = w0 * gg + w1 * (I1 * gg - ff), q = w1 * gg;
 #pragma unroll
-                for (int L = 0; L < 3; ++L) {
-                    const int b = k * 3 + L;
-                    float v = U[0][Jj] * dI[0][b] + U[1][Jj] * dI[1][b] + U[2][Jj] * dI[2][b];
-                    const float dik = i == k ? 1.f : 0.f, dJL = Jj == L ? 1.f : 0.f;
-                    v += Wa[0] * 2.f * dik * dJL;
-                    v += Wa[1] * 2.f * (2.f * Fr[Jj] * F[b] + I1 * dik * dJL - dik * C[L * 3 + Jj] -
-                                        Fr[L] * F[k * 3 + Jj] - FFtr[k] * dJL);
-                    v += Wa[2] * J * (FiTr[Jj] * FiT[b] - FiTr[L] * FiT[k * 3 + Jj]);
-                    Ai[Jj * 9 + b] = v;
+            for (int i = 0; i < 3; ++i) {
+                const float f = w1 * Fg[b][i], h = w2 * hg[b][i];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    float v = X[i] * Fg[b][k] + Y[i] * Dg[b][k] + Z[i] * hg[b][k];
+                    v -= f * Fg[a][k] + h * hg[a][k] + q * FFt[i * 3 + k];
+                    block(a, b, i, k, i == k ? v + diag : v);
                 }
-        Ai[27] = 0.f;
-        if constexpr (FUSED) {
-            // tangent rows (a, i) of the element matrix, V folded in
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                float w[9];
-#pragma unroll
-                for (int kL = 0; kL < 9; ++kL)
-                    w[kL] = Vf * (ga[a][0] * Ai[kL] + ga[a][1] * Ai[9 + kL] + ga[a][2] * Ai[18 + kL]);
-                float row[12];
-#pragma unroll
-                for (int b = 0; b < 4; ++b)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        row[b * 3 + k] = w[k * 3] * ga[b][0] + w[k * 3 + 1] * ga[b][1] + w[k * 3 + 2] * ga[b][2];
-                float4 *dst = out + (a * 3 + i) * 3;
-#pragma unroll
-                for (int q = 0; q < 3; ++q)
-                    dst[q] = make_float4(row[4 * q], row[4 * q + 1], row[4 * q + 2], row[4 * q + 3]);
-            }
-        } else if (Ke) {
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                // row (a, i): sum_JL ga[a][J] A[iJ][kL] ga[b][L]
-                float tmp[9];
-#pragma unroll
-                for (int kL = 0; kL < 9; ++kL)
-                    tmp[kL] = ga[a][0] * Ai[kL] + ga[a][1] * Ai[9 + kL] + ga[a][2] * Ai[18 + kL];
-#pragma unroll
-                for (int b = 0; b < 4; ++b)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        Ke[(a * 3 + i) * 12 + b * 3 + k] =
-                            V * (double)(tmp[k * 3] * ga[b][0] + tmp[k * 3 + 1] * ga[b][1] + tmp[k * 3 + 2] * ga[b][2]);
             }
         }
-    }
-    if (!tail) return true;
-    if constexpr (FUSED) {
-        // residual r_(a,c) = V sum_j P_cj g_a,j
-        float r[12];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                r[a * 3 + c] = Vf * (Pm[c * 3] * ga[a][0] + Pm[c * 3 + 1] * ga[a][1] + Pm[c * 3 + 2] * ga[a][2]);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) out[36 + q] = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
-    } else if (re) {
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-                re[a * 3 + c] = V * (double)(Pm[c * 3] * ga[a][0] + Pm[c * 3 + 1] * ga[a][1] + Pm[c * 3 + 2] * ga[a][2]);
     }
     return true;
 }
 
-// Plain-law fallback of one element (FP64 geometry and law).
-template <bool FUSED>
+// Plain-law fallback of one element (FP64 geometry and law): element tangent
+// and residual (Ke, re, already offset to the element).
 __device__ __forceinline__ void surrogate_fallback(int64_t e, const double *__restrict__ p, int64_t npts,
                                                    const int32_t *__restrict__ t, int64_t ne,
                                                    const int32_t *__restrict__ dofs, const double *__restrict__ u,
                                                    double mu, double lmbda, double wsum, double *__restrict__ Ke,
-                                                   double *__restrict__ re, double *__restrict__ recd,
-                                                   unsigned char *__restrict__ flags,
-                                                   unsigned long long *__restrict__ fallback) {
+                                                   double *__restrict__ re) {
     NhGeom g;
     nh_geometry(p, npts, t, ne, e, wsum, g);
     double Gu[9];
     displacement_gradient(g, dofs + e * 12, u, Gu);
     NhLaw law;
     nh_plain_law(Gu, mu, lmbda, law);
-    if constexpr (FUSED) {
-        write_plain_record(g, law, mu, lmbda, recd + e * kNhRecD);
-        flags[e] = 1;
-    } else {
-        write_nh_element(g, law, mu, lmbda, Ke ? Ke + e * 144 : nullptr, re ? re + e * 12 : nullptr);
-    }
-    atomicAdd(fallback, 1ULL);
+    write_nh_element(g, law, mu, lmbda, Ke, re);
 }
 
-// One thread per element, network on the CUDA cores (mlp_eval).  FUSED:
-// writes the surrogate record (recf) or, for a fallback element, the plain
-// FP64 record (recd) and sets flags[e]; otherwise the element tangent and
-// residual (Ke, re) for the gathers.
-template <bool FUSED>
+// The same as packed blocks, every value split into two FP32 parts: the high
+// parts to `out` (see surrogate_finish) and r + 12 e, the low parts to block t
+// of element e of b.K_low and b.r_low.
+__device__ __forceinline__ void surrogate_fallback_packed(int64_t e, int64_t stride, const double *__restrict__ p,
+                                                          int64_t npts, const int32_t *__restrict__ t, int64_t ne,
+                                                          const int32_t *__restrict__ dofs,
+                                                          const double *__restrict__ u, double mu, double lmbda,
+                                                          double wsum, float *__restrict__ out,
+                                                          const ClosureBlocks &blk) {
+    NhGeom g;
+    nh_geometry(p, npts, t, ne, e, wsum, g);
+    double Gu[9];
+    displacement_gradient(g, dofs + e * 12, u, Gu);
+    NhLaw law;
+    nh_plain_law(Gu, mu, lmbda, law);
+    double h[4][3];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            h[a][i] = law.FiT[i * 3] * g.g[a][0] + law.FiT[i * 3 + 1] * g.g[a][1] + law.FiT[i * 3 + 2] * g.g[a][2];
+            const double r =
+                g.V * (law.P[i * 3] * g.g[a][0] + law.P[i * 3 + 1] * g.g[a][1] + law.P[i * 3 + 2] * g.g[a][2]);
+            const float hi = (float)r;
+            blk.r[e * 12 + a * 3 + i] = hi;
+            blk.r_low[e * 12 + a * 3 + i] = (float)(r - (double)hi);
+        }
+    const double c2 = mu - lmbda * law.lnJ;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = a; b < 4; ++b) {
+            const double gg = g.g[a][0] * g.g[b][0] + g.g[a][1] * g.g[b][1] + g.g[a][2] * g.g[b][2];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const double v =
+                        g.V * ((i == k ? mu * gg : 0.0) + c2 * h[b][i] * h[a][k] + lmbda * h[a][i] * h[b][k]);
+                    const float hi = (float)v;
+                    out[tri_index(4, a, b) * kFinishStage + i * 3 + k] = hi;
+                    blk.K_low[(tri_index(4, a, b) * stride + e) * 9 + i * 3 + k] = (float)(v - (double)hi);
+                }
+        }
+}
+
+// One thread per element, network on the CUDA cores (mlp_eval): element
+// tangent and residual (Ke, re) for the gathers (patterns without a pair plan,
+// residual alone).
 __global__ void __launch_bounds__(kEvalBlock) k_nh_surrogate_element(
     int64_t ne, const double *__restrict__ p, int64_t npts, const int32_t *__restrict__ t,
     const int32_t *__restrict__ dofs, const double *__restrict__ u, double mu, double lmbda, double wsum,
     const float *__restrict__ params, const float *__restrict__ box, float tol, double *__restrict__ Ke,
-    double *__restrict__ re, float *__restrict__ recf, double *__restrict__ recd, unsigned char *__restrict__ flags,
-    unsigned long long *__restrict__ fallback) {
+    double *__restrict__ re, unsigned long long *__restrict__ fallback) {
     extern __shared__ __align__(16) unsigned char smem[];
     const EvalShared ev = eval_shared(smem);
     load_eval_shared(params, ev);
@@ -724,14 +704,23 @@ __global__ void __launch_bounds__(kEvalBlock) k_nh_surrogate_element(
         for (int q = 0; q < 4; ++q)
 #pragma unroll
             for (int j = 0; j < 3; ++j) ga[q][j] = (float)g.g[q][j];
-        use = surrogate_finish<FUSED>(st, Nrm, gx, Hx, mu, lmbda, tol, (float)g.V, ga,
-                                      FUSED ? reinterpret_cast<float4 *>(recf + e * kNhRecF) : nullptr,
-                                      Ke ? Ke + e * 144 : nullptr, re ? re + e * 12 : nullptr, g.V);
+        float Wf[3], Wff[9];
+        feature_derivatives(Nrm, gx, Hx, Wf, Wff);
+        use = surrogate_finish(
+            st, Wf, Wff, mu, lmbda, tol, 1.f, ga,
+            [&](int a, int b, int i, int k, float v) {
+                if (!Ke) return;
+                Ke[e * 144 + (a * 3 + i) * 12 + b * 3 + k] = g.V * (double)v;
+                if (a != b) Ke[e * 144 + (b * 3 + k) * 12 + a * 3 + i] = g.V * (double)v;
+            },
+            [&](int a, int i, float v) {
+                if (re) re[e * 12 + a * 3 + i] = g.V * (double)v;
+            });
     }
     if (!use) {
-        surrogate_fallback<FUSED>(e, p, npts, t, ne, dofs, u, mu, lmbda, wsum, Ke, re, recd, flags, fallback);
-    } else if (FUSED) {
-        flags[e] = 0;
+        surrogate_fallback(e, p, npts, t, ne, dofs, u, mu, lmbda, wsum, Ke ? Ke + e * 144 : nullptr,
+                           re ? re + e * 12 : nullptr);
+        atomicAdd(fallback, 1ULL);
     }
 }
 
@@ -741,31 +730,38 @@ __global__ void __launch_bounds__(kEvalBlock) k_nh_surrogate_element(
 // element row r = tensor-memory lane r.  The two 64 x 64 layers are tcgen05
 // MMAs (kind::tf32) with FP32-accurate products: every operand is split
 // x = hi + lo in tf32 and D = A_hi B_hi + A_hi B_lo + A_lo B_hi.
-//   GEMM 1: [a2 | B0 | B1 | B2] = [Z1 | Q0 | Q1 | Q2] W2^T    (TMEM columns 0..255)
-//           with Q_m[e][j] = s1[e][j] W1[j][m]  (B = W2 diag(s1) W1 per element)
-//   GEMM 2: u1 = D2 W2                                          (TMEM columns 0..63)
+//   a2 = Z1 W2^T                       (64 columns)
+//   B_m = S1 (W2 diag(W1[:, m]))^T     (m = 0..2, one product of 192 columns)
+//   u1 = D2 W2                         (64 columns)
+// with Z1 the first layer's outputs, S1 = 1 - Z1^2 and D2 the second layer's
+// derivatives.  The A operands lie in tensor memory, written by the threads
+// that computed them; with them in shared memory (five operands: Q_m = S1
+// diag(W1[:, m]) instead of S1 alone) the tile's writes and the MMAs' reads of
+// them, serialised by one buffer pair, took most of the time.
 // Two threads per element row (warps w and w + 4 share the row's lane
 // quarter): each owns half of the hidden units for the elementwise work
 // (tanh, operand writes, Hessian contractions); their partial gradient and
-// Hessian sums are exchanged through shared memory and added in the same
-// order by both.  The tangent's row blocks are split between the two.
-// Shared memory: W2 and W2^T (hi, lo) as B operands, two 128 x 64 A-operand
-// buffers (hi, lo), small vectors, the partial sums.
+// Hessian sums are exchanged through shared memory.  The products run behind
+// the elementwise work: a2 behind S1, B behind the second layer, u1 behind the
+// Hessian's second term and the next tile's first layer.
+// 48^3 x 6 elements: 351 us -> 248 us.
 constexpr int kTcRows = 128;
 constexpr int kTcThreads = 2 * kTcRows;
 constexpr int kHalf = H / 2;
-constexpr uint32_t kTcCols = 256;
-constexpr int kOpBytes = kTcRows * H * 4;  // one 128 x 64 tf32 operand
-constexpr int kWBytes = H * H * 4;
+// tensor-memory columns: A operands Z1 / D2 and S1 (hi, lo), results a2 / u1 and B
+constexpr uint32_t kTcCols = 512, TM_Z = 0, TM_S = 128, TM_A2 = 256, TM_B = 320;
+constexpr int kBn = 3 * H;  // columns of B
+constexpr int kWBytes = H * H * 4, kWdBytes = kBn * H * 4;
 constexpr int SM_W2B_HI = 0, SM_W2B_LO = kWBytes, SM_W2T_HI = 2 * kWBytes, SM_W2T_LO = 3 * kWBytes;
-constexpr int SM_OPA_HI = 4 * kWBytes, SM_OPA_LO = SM_OPA_HI + kOpBytes;
-constexpr int SM_OPB_HI = SM_OPA_LO + kOpBytes, SM_OPB_LO = SM_OPB_HI + kOpBytes;
-constexpr int SM_Q = SM_OPB_LO + kOpBytes;
-constexpr int kPart = 9;  // gx (3) + H (6)
-constexpr int SM_PART = SM_Q + QSIZE * 4;
-constexpr size_t kTcSmem = SM_PART + sizeof(float) * 2 * kTcRows * kPart;
+constexpr int SM_W2D_HI = 4 * kWBytes, SM_W2D_LO = SM_W2D_HI + kWdBytes;
+constexpr int SM_L1 = SM_W2D_LO + kWdBytes;    // float4 per unit: W1[j][0..2], b1[j]
+constexpr int SM_L2 = SM_L1 + H * 16;          // float2 per unit: b2[i], w3[i]
+constexpr int SM_WW = SM_L2 + H * 8;           // 8 floats per unit: the products W1[j][m] W1[j][l], m <= l
+constexpr int kPart = 9;                       // gx (3) + H (6)
+constexpr int SM_PART = SM_WW + H * 32;
+constexpr size_t kTcSmem = SM_PART + sizeof(float) * kTcRows * kPart;
 constexpr uint32_t kTcWaitLimit = 1u << 24;
-constexpr int kNetOut = 10;  // per element: d psi / dx (3), d2 psi / dx2 (6 upper entries), usable flag
+constexpr int kNetOut = 12;  // per element: dW / df (3), d2W / df2 (6 upper entries), usable flag, padding
 constexpr int kFinishBlock = 128;
 constexpr int kGeoRec = 24;  // floats per element: F (9), grad lambda (12), V, padding
 
@@ -775,37 +771,39 @@ __device__ __forceinline__ float tanh_fast(float a) {
     return 1.f - __fdividef(2.f, __expf(2.f * a) + 1.f);
 }
 
-// Writes 4 consecutive k of row `row` into an A operand (tf32 hi and lo parts).
-__device__ __forceinline__ void put_op4(unsigned char *hi, unsigned char *lo, int row, int k, float a, float b,
-                                        float c, float d) {
-    const uint32_t off = tc::operand_offset(kTcRows, row, k);
-    const float ha = tc::to_tf32(a), hb = tc::to_tf32(b), hc = tc::to_tf32(c), hd = tc::to_tf32(d);
-    *reinterpret_cast<float4 *>(hi + off) = make_float4(ha, hb, hc, hd);
-    *reinterpret_cast<float4 *>(lo + off) =
-        make_float4(tc::to_tf32(a - ha), tc::to_tf32(b - hb), tc::to_tf32(c - hc), tc::to_tf32(d - hd));
+// Writes 16 columns of this thread's row of an A operand: tf32 high parts at
+// column `col`, low parts 64 columns further.
+__device__ __forceinline__ void put_operand(uint32_t taddr, const float v[16]) {
+    float hi[16], lo[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        hi[k] = tc::to_tf32(v[k]);
+        lo[k] = tc::to_tf32(v[k] - hi[k]);
+    }
+    tc::tmem_st16(taddr, hi);
+    tc::tmem_st16(taddr + H, lo);
 }
 
-// D[tmem] = A (128 x 64) * B^T (B: 64 x 64), 3xTF32, single issuing thread.
-__device__ __forceinline__ void issue_gemm(uint32_t d_tmem, const unsigned char *a_hi, const unsigned char *a_lo,
-                                           const unsigned char *b_hi, const unsigned char *b_lo) {
-    const uint32_t idesc = tc::idesc_tf32(kTcRows, H);
-    const uint32_t ah0 = tc::smem_addr(a_hi), al0 = tc::smem_addr(a_lo);
+// D[tmem] = A (128 x 64, tensor memory) * B^T (B: N x 64), 3xTF32, single issuing thread.
+template <int N>
+__device__ __forceinline__ void issue_gemm(uint32_t d_tmem, uint32_t a_tmem, const unsigned char *b_hi,
+                                           const unsigned char *b_lo) {
+    const uint32_t idesc = tc::idesc_tf32(kTcRows, N);
     const uint32_t bh0 = tc::smem_addr(b_hi), bl0 = tc::smem_addr(b_lo);
 #pragma unroll
     for (int s = 0; s < H / 8; ++s) {
-        const uint32_t ao = s * 2 * (kTcRows * 16), bo = s * 2 * (H * 16);
-        const uint64_t ah = tc::smem_desc(ah0 + ao, kTcRows * 16, 128), al = tc::smem_desc(al0 + ao, kTcRows * 16, 128);
-        const uint64_t bh = tc::smem_desc(bh0 + bo, H * 16, 128), bl = tc::smem_desc(bl0 + bo, H * 16, 128);
-        tc::mma_tf32(d_tmem, ah, bh, idesc, s > 0);
-        tc::mma_tf32(d_tmem, ah, bl, idesc, true);
-        tc::mma_tf32(d_tmem, al, bh, idesc, true);
+        const uint32_t bo = s * 2 * (N * 16);
+        const uint64_t bh = tc::smem_desc(bh0 + bo, N * 16, 128), bl = tc::smem_desc(bl0 + bo, N * 16, 128);
+        tc::mma_tf32(d_tmem, a_tmem + 8 * s, bh, idesc, s > 0);
+        tc::mma_tf32(d_tmem, a_tmem + 8 * s, bl, idesc, true);
+        tc::mma_tf32(d_tmem, a_tmem + H + 8 * s, bh, idesc, true);
     }
 }
 
 // Operand writes -> tensor cores; tensor-memory reads of the previous phase
 // are ordered before the next MMAs.
 __device__ __forceinline__ void sync_for_mma() {
-    tc::fence_proxy_async();
+    tc::tmem_st_wait();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -866,178 +864,196 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_nh_surrogate_tc(int64_t e_beg
                                                                    float *__restrict__ net,
                                                                    unsigned long long *__restrict__ counters) {
     extern __shared__ __align__(1024) unsigned char smem_tc[];  // own name: the other kernels' dynamic arrays are 16-aligned
-    __shared__ uint64_t mbar;
+    __shared__ uint64_t mbars[2];  // [0] a2 and u1, [1] B
     __shared__ uint32_t tslot;
+    __shared__ float scale[kPart + 1], shift[kPart];  // network -> feature units; the reference state's shift; linear skip
     const int tid = threadIdx.x, warp = tid >> 5;
     const int row = tid & (kTcRows - 1), half = tid / kTcRows, jb = half * kHalf;
-    float *Q = reinterpret_cast<float *>(smem_tc + SM_Q);
-    float *part = reinterpret_cast<float *>(smem_tc + SM_PART);  // [half][kPart][row]
-    unsigned char *opa_hi = smem_tc + SM_OPA_HI, *opa_lo = smem_tc + SM_OPA_LO;
-    unsigned char *opb_hi = smem_tc + SM_OPB_HI, *opb_lo = smem_tc + SM_OPB_LO;
-    const unsigned char *w2b_hi = smem_tc + SM_W2B_HI, *w2b_lo = smem_tc + SM_W2B_LO;
-    const unsigned char *w2t_hi = smem_tc + SM_W2T_HI, *w2t_lo = smem_tc + SM_W2T_LO;
+    const float4 *L1 = reinterpret_cast<const float4 *>(smem_tc + SM_L1);
+    const float2 *L2 = reinterpret_cast<const float2 *>(smem_tc + SM_L2);
+    const float4 *WW = reinterpret_cast<const float4 *>(smem_tc + SM_WW);
+    float *part = reinterpret_cast<float *>(smem_tc + SM_PART);  // [kPart][row], of the second half
     for (int k = tid; k < H * H; k += kTcThreads) {
         const int i = k / H, j = k - (k / H) * H;
-        const float w = params[OW2 + k], hi = tc::to_tf32(w), lo = tc::to_tf32(w - hi);
-        *reinterpret_cast<float *>(smem_tc + SM_W2B_HI + tc::operand_offset(H, i, j)) = hi;
-        *reinterpret_cast<float *>(smem_tc + SM_W2B_LO + tc::operand_offset(H, i, j)) = lo;
-        *reinterpret_cast<float *>(smem_tc + SM_W2T_HI + tc::operand_offset(H, j, i)) = hi;
-        *reinterpret_cast<float *>(smem_tc + SM_W2T_LO + tc::operand_offset(H, j, i)) = lo;
+        const auto put = [&](int at_hi, int at_lo, uint32_t off, float w) {
+            const float hi = tc::to_tf32(w);
+            *reinterpret_cast<float *>(smem_tc + at_hi + off) = hi;
+            *reinterpret_cast<float *>(smem_tc + at_lo + off) = tc::to_tf32(w - hi);
+        };
+        const float w = params[OW2 + k];
+        put(SM_W2B_HI, SM_W2B_LO, tc::operand_offset(H, i, j), w);
+        put(SM_W2T_HI, SM_W2T_LO, tc::operand_offset(H, j, i), w);
+#pragma unroll
+        for (int m = 0; m < 3; ++m)
+            put(SM_W2D_HI, SM_W2D_LO, tc::operand_offset(kBn, m * H + i, j), w * params[OW1 + 3 * j + m]);
     }
-    for (int k = tid; k < QSIZE; k += kTcThreads) {
-        float v = 0.f;
-        if (k < QB2) v = params[OW1 + k];
-        else if (k < QB3 + 1) v = params[OB2 + (k - QB2)];
-        else if (k < QNORM) v = params[OC + (k - QC)];
-        else if (k < QNORM + 9) v = params[ONORM + (k - QNORM)];
-        Q[k] = v;
+    for (int j = tid; j < H; j += kTcThreads) {
+        const float w[3] = {params[OW1 + 3 * j], params[OW1 + 3 * j + 1], params[OW1 + 3 * j + 2]};
+        reinterpret_cast<float4 *>(smem_tc + SM_L1)[j] = make_float4(w[0], w[1], w[2], params[OB1 + j]);
+        reinterpret_cast<float2 *>(smem_tc + SM_L2)[j] = make_float2(params[OB2 + j], params[OW3 + j]);
+        float4 *q = reinterpret_cast<float4 *>(smem_tc + SM_WW) + 2 * j;
+        q[0] = make_float4(w[0] * w[0], w[0] * w[1], w[0] * w[2], w[1] * w[1]);
+        q[1] = make_float4(w[1] * w[2], w[2] * w[2], 0.f, 0.f);
     }
     if (tid == 0) {
-        tc::mbar_init(&mbar, 1);
+        const float *Nrm = params + ONORM;
+        for (int m = 0, k = 3; m < 3; ++m) {
+            scale[m] = Nrm[6] / Nrm[3 + m];
+            shift[m] = params[OC + m];
+            for (int l = m; l < 3; ++l, ++k) {
+                scale[k] = Nrm[6] / (Nrm[3 + m] * Nrm[3 + l]);
+                shift[k] = 0.f;
+            }
+        }
+        scale[kPart] = Nrm[8];
+        tc::mbar_init(&mbars[0], 1);
+        tc::mbar_init(&mbars[1], 1);
         tc::fence_mbar_init();
     }
     if (warp == 0) tc::tmem_alloc(&tslot, kTcCols);
-    sync_for_mma();
+    tc::fence_proxy_async();  // the weights, for the MMAs
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
     const uint32_t tmem = tslot;
-    const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16);  // this warp's lane quarter
-    uint32_t phase = 0;
+    const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + jb;  // this warp's lane quarter, its half
+    uint32_t phase[2] = {0, 0};
     bool tc_ok = true;
+    const auto wait_for = [&](int k) {
+        tc_ok = __syncthreads_and(tc::mbar_wait(&mbars[k], phase[k], kTcWaitLimit));
+        phase[k] ^= 1;
+        tc::fence_after_sync();
+    };
+    const auto input = [&](int64_t tile) {
+        const int64_t e = e_begin + tile * kTcRows + row;
+        return e < e_end ? xin[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    const auto layer1 = [&](const float4 &x, float z[kHalf]) {
+#pragma unroll
+        for (int c = 0; c < kHalf; ++c) {
+            const float4 w = L1[jb + c];
+            z[c] = tanh_fast(w.w + w.x * x.x + w.y * x.y + w.z * x.z);
+        }
+    };
+    float4 x = input(blockIdx.x);
+    float z1[kHalf];  // hidden units jb .. jb + 31
+    layer1(x, z1);
     for (int64_t tile = blockIdx.x; e_begin + tile * kTcRows < e_end; tile += gridDim.x) {
         const int64_t e = e_begin + tile * kTcRows + row;
-        const bool valid = e < e_end;
-        const float4 xe = valid ? xin[e] : make_float4(0.f, 0.f, 0.f, 0.f);
-        bool use = xe.w != 0.f;
-        const float x[3] = {xe.x, xe.y, xe.z};
-        float z1[kHalf];  // hidden units jb .. jb + 31
-        if (tc_ok) {
-            // ---- layer 1; A operands Z1 and Q0 (own half of the columns)
-#pragma unroll
-            for (int c0 = 0; c0 < kHalf; c0 += 4) {
-                float zz[4], q0[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int j = jb + c0 + c;
-                    const float a = Q[QB1 + j] + Q[QW1 + 3 * j] * x[0] + Q[QW1 + 3 * j + 1] * x[1] +
-                                    Q[QW1 + 3 * j + 2] * x[2];
-                    z1[c0 + c] = tanh_fast(a);
-                    zz[c] = z1[c0 + c];
-                    q0[c] = (1.f - zz[c] * zz[c]) * Q[QW1 + 3 * j];
-                }
-                put_op4(opa_hi, opa_lo, row, jb + c0, zz[0], zz[1], zz[2], zz[3]);
-                put_op4(opb_hi, opb_lo, row, jb + c0, q0[0], q0[1], q0[2], q0[3]);
-            }
-            sync_for_mma();
-            if (tid == 0) {
-                issue_gemm(tmem + 0, opa_hi, opa_lo, w2b_hi, w2b_lo);
-                issue_gemm(tmem + 64, opb_hi, opb_lo, w2b_hi, w2b_lo);
-                tc::mma_commit(&mbar);
-            }
-            tc_ok = __syncthreads_and(tc::mbar_wait(&mbar, phase, kTcWaitLimit));
-            phase ^= 1;
-        }
-        if (tc_ok) {
-            // ---- A operands Q1 and Q2
-#pragma unroll
-            for (int c0 = 0; c0 < kHalf; c0 += 4) {
-                float q1[4], q2[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int j = jb + c0 + c;
-                    const float s1 = 1.f - z1[c0 + c] * z1[c0 + c];
-                    q1[c] = s1 * Q[QW1 + 3 * j + 1];
-                    q2[c] = s1 * Q[QW1 + 3 * j + 2];
-                }
-                put_op4(opa_hi, opa_lo, row, jb + c0, q1[0], q1[1], q1[2], q1[3]);
-                put_op4(opb_hi, opb_lo, row, jb + c0, q2[0], q2[1], q2[2], q2[3]);
-            }
-            sync_for_mma();
-            if (tid == 0) {
-                issue_gemm(tmem + 128, opa_hi, opa_lo, w2b_hi, w2b_lo);
-                issue_gemm(tmem + 192, opb_hi, opb_lo, w2b_hi, w2b_lo);
-                tc::mma_commit(&mbar);
-            }
-            tc_ok = __syncthreads_and(tc::mbar_wait(&mbar, phase, kTcWaitLimit));
-            phase ^= 1;
-        }
+        bool use = x.w != 0.f;
         float pr[kPart];  // gx (3), H (6) partial sums of this half
 #pragma unroll
         for (int k = 0; k < kPart; ++k) pr[k] = 0.f;
+        float z1n[kHalf], t2[kHalf];
+        const float4 xn = input(tile + gridDim.x);
         if (tc_ok) {
-            // ---- layer 2 (own half of the outputs) and the second Hessian term; A operand D2
-            tc::fence_after_sync();
+            // ---- A operands Z1, then S1 (own half of the columns)
+            put_operand(tl + TM_Z, z1);
+            put_operand(tl + TM_Z + 16, z1 + 16);
+            sync_for_mma();
+            if (tid == 0) {
+                issue_gemm<H>(tmem + TM_A2, tmem + TM_Z, smem_tc + SM_W2B_HI, smem_tc + SM_W2B_LO);
+                tc::mma_commit(&mbars[0]);
+            }
+            __syncwarp();
 #pragma unroll
             for (int ch = 0; ch < kHalf / 16; ++ch) {
-                const int c0 = jb + ch * 16;
-                float a2[16], b0[16], b1[16], b2[16], dv[16];
-                tc::tmem_ld16(tl + c0, a2);
-                tc::tmem_ld16(tl + 64 + c0, b0);
-                tc::tmem_ld16(tl + 128 + c0, b1);
-                tc::tmem_ld16(tl + 192 + c0, b2);
+                float s1[16];
 #pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    const int i = c0 + q;
-                    const float z2 = tanh_fast(a2[q] + Q[QB2 + i]), w3 = Q[QW3 + i];
-                    const float d2 = (1.f - z2 * z2) * w3;
-                    dv[q] = d2;
-                    const float t2 = -2.f * z2 * d2;
-                    const float tb0 = t2 * b0[q], tb1 = t2 * b1[q];
-                    pr[3] += tb0 * b0[q]; pr[4] += tb0 * b1[q]; pr[5] += tb0 * b2[q];
-                    pr[6] += tb1 * b1[q]; pr[7] += tb1 * b2[q]; pr[8] += t2 * b2[q] * b2[q];
-                }
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-                    put_op4(opa_hi, opa_lo, row, c0 + 4 * r, dv[4 * r], dv[4 * r + 1], dv[4 * r + 2], dv[4 * r + 3]);
+                for (int q = 0; q < 16; ++q) s1[q] = 1.f - z1[ch * 16 + q] * z1[ch * 16 + q];
+                put_operand(tl + TM_S + ch * 16, s1);
             }
             sync_for_mma();
             if (tid == 0) {
-                issue_gemm(tmem + 0, opa_hi, opa_lo, w2t_hi, w2t_lo);
-                tc::mma_commit(&mbar);
+                issue_gemm<kBn>(tmem + TM_B, tmem + TM_S, smem_tc + SM_W2D_HI, smem_tc + SM_W2D_LO);
+                tc::mma_commit(&mbars[1]);
             }
-            tc_ok = __syncthreads_and(tc::mbar_wait(&mbar, phase, kTcWaitLimit));
-            phase ^= 1;
+            __syncwarp();
+            wait_for(0);
+        }
+        if (tc_ok) {
+            // ---- layer 2 (own half of the outputs); A operand D2 in the place of Z1
+#pragma unroll
+            for (int ch = 0; ch < kHalf / 16; ++ch) {
+                float a2[16];
+                tc::tmem_ld16(tl + TM_A2 + ch * 16, a2);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    const float2 bw = L2[jb + ch * 16 + q];
+                    const float z2 = tanh_fast(a2[q] + bw.x);
+                    a2[q] = (1.f - z2 * z2) * bw.y;
+                    t2[ch * 16 + q] = -2.f * z2 * a2[q];
+                }
+                put_operand(tl + TM_Z + ch * 16, a2);
+            }
+            sync_for_mma();
+            if (tid == 0) {
+                issue_gemm<H>(tmem + TM_A2, tmem + TM_Z, smem_tc + SM_W2T_HI, smem_tc + SM_W2T_LO);
+                tc::mma_commit(&mbars[0]);
+            }
+            __syncwarp();
+            layer1(xn, z1n);
+            wait_for(1);
+        }
+        if (tc_ok) {
+            // ---- second Hessian term
+#pragma unroll
+            for (int ch = 0; ch < kHalf / 16; ++ch) {
+                float b0[16], b1[16], b2[16];
+                tc::tmem_ld16(tl + TM_B + ch * 16, b0);
+                tc::tmem_ld16(tl + TM_B + H + ch * 16, b1);
+                tc::tmem_ld16(tl + TM_B + 2 * H + ch * 16, b2);
+#pragma unroll
+                for (int q = 0; q < 16; ++q) {
+                    const float t = t2[ch * 16 + q], tb0 = t * b0[q], tb1 = t * b1[q];
+                    pr[3] += tb0 * b0[q]; pr[4] += tb0 * b1[q]; pr[5] += tb0 * b2[q];
+                    pr[6] += tb1 * b1[q]; pr[7] += tb1 * b2[q]; pr[8] += t * b2[q] * b2[q];
+                }
+            }
+            wait_for(0);
         }
         if (tc_ok) {
             // ---- u1 = W2^T d2 (own half): gradient and first Hessian term
-            tc::fence_after_sync();
 #pragma unroll
             for (int ch = 0; ch < kHalf / 16; ++ch) {
                 float u1[16];
-                tc::tmem_ld16(tl + jb + ch * 16, u1);
+                tc::tmem_ld16(tl + TM_A2 + ch * 16, u1);
 #pragma unroll
                 for (int q = 0; q < 16; ++q) {
                     const int jl = ch * 16 + q, j = jb + jl;
                     const float d1 = (1.f - z1[jl] * z1[jl]) * u1[q];
-                    const float w0 = Q[QW1 + 3 * j], w1 = Q[QW1 + 3 * j + 1], w2 = Q[QW1 + 3 * j + 2];
-                    pr[0] += w0 * d1;
-                    pr[1] += w1 * d1;
-                    pr[2] += w2 * d1;
+                    const float4 w = L1[j], wa = WW[2 * j], wb = WW[2 * j + 1];
+                    pr[0] += w.x * d1;
+                    pr[1] += w.y * d1;
+                    pr[2] += w.z * d1;
                     const float rr = -2.f * z1[jl] * d1;
-                    pr[3] += rr * w0 * w0; pr[4] += rr * w0 * w1; pr[5] += rr * w0 * w2;
-                    pr[6] += rr * w1 * w1; pr[7] += rr * w1 * w2; pr[8] += rr * w2 * w2;
+                    pr[3] += rr * wa.x; pr[4] += rr * wa.y; pr[5] += rr * wa.z;
+                    pr[6] += rr * wa.w; pr[7] += rr * wb.x; pr[8] += rr * wb.y;
                 }
             }
         } else {
             use = false;  // tensor-core phase gave up: plain law for the rest
         }
-        // ---- combine the two halves (same order in both: bitwise equal sums)
+        // ---- combine the two halves
+        if (half == 1) {
 #pragma unroll
-        for (int k = 0; k < kPart; ++k) part[(half * kPart + k) * kTcRows + row] = pr[k];
-        __syncthreads();
-        float tot[kPart];
-#pragma unroll
-        for (int k = 0; k < kPart; ++k)
-            tot[k] = part[(0 * kPart + k) * kTcRows + row] + part[(1 * kPart + k) * kTcRows + row];
-        // network result of the element: feature gradient (3), Hessian (6), usable flag
-        if (valid && half == 0) {
-            float *o = net + e * kNetOut;
-            o[0] = Q[QC] + tot[0]; o[1] = Q[QC + 1] + tot[1]; o[2] = Q[QC + 2] + tot[2];
-#pragma unroll
-            for (int k = 3; k < 9; ++k) o[k] = tot[k];
-            o[9] = use ? 1.f : 0.f;
+            for (int k = 0; k < kPart; ++k) part[k * kTcRows + row] = pr[k];
         }
-        // tensor-memory reads, operand buffers and partial sums are free for the next tile
-        tc::fence_before_sync();
         __syncthreads();
+        // network result of the element in feature units
+        if (e < e_end && half == 0) {
+            float4 *o = reinterpret_cast<float4 *>(net + e * kNetOut);
+#pragma unroll
+            for (int k = 0; k < kPart; ++k) pr[k] = scale[k] * (shift[k] + pr[k] + part[k * kTcRows + row]);
+            o[0] = make_float4(pr[0], pr[1], pr[2] - scale[kPart], pr[3]);
+            o[1] = make_float4(pr[4], pr[5], pr[6], pr[7]);
+            o[2] = make_float4(pr[8], use ? 1.f : 0.f, 0.f, 0.f);
+        }
+        // the next tile's barriers separate these reads from its partial sums,
+        // and the tensor-memory reads above from its MMAs
+        x = xn;
+#pragma unroll
+        for (int c = 0; c < kHalf; ++c) z1[c] = z1n[c];
     }
     if (!tc_ok && tid == 0) atomicAdd(counters + 1, 1ULL);
     tc::fence_before_sync();
@@ -1046,16 +1062,17 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_nh_surrogate_tc(int64_t e_beg
     if (warp == 0) tc::tmem_dealloc(tmem, kTcCols);
 }
 
-// The surrogate element pass runs in three kernels: k_nh_surrogate_prep
+// The surrogate element pass runs in three kernels (48^3: 49, 248 and 79 us): k_nh_surrogate_prep
 // (thread per element: FP32 geometry, deformation gradient, invariants, the
 // network input and whether the network may serve the element), the
 // tensor-core network k_nh_surrogate_tc (feature gradient and Hessian), and
-// k_nh_surrogate_finish (three threads per element, one per tangent row
-// block i: stress from the invariant derivatives, the check against the plain
-// law, tangent rows and, for the last block, the residual entries; elements
-// the network may not serve, or whose check fails, get the FP64 plain record).
-// The two CUDA-core kernels have no tensor-memory or shared-memory budget and
-// run at full occupancy, which hides the gathers' latency.
+// k_nh_surrogate_finish (thread per element: stress from the invariant
+// derivatives, the check against the plain law, the ten upper blocks and the
+// residual entries; elements the network may not serve, or whose check fails,
+// get the plain law's FP64 values in two FP32 parts).  The two CUDA-core
+// kernels have no tensor-memory budget and run at high occupancy, which hides
+// the gathers' latency; the finish kernel's blocks leave through a stage in
+// shared memory, as whole lines.
 __global__ void __launch_bounds__(kFinishBlock) k_nh_surrogate_prep(
     int64_t ne, int64_t e_begin, int64_t e_end, const double *__restrict__ p, int64_t npts,
     const int32_t *__restrict__ t, const int32_t *__restrict__ dofs, const double *__restrict__ u, double wsum,
@@ -1085,36 +1102,63 @@ __global__ void __launch_bounds__(kFinishBlock) k_nh_surrogate_prep(
     g[5] = make_float4(ga[3][2], Vf, 0.f, 0.f);
 }
 
-__global__ void __launch_bounds__(kFinishBlock, 4) k_nh_surrogate_finish(
-    int64_t ne, int64_t e_begin, int64_t e_end, const double *__restrict__ p, int64_t npts,
+__global__ void __launch_bounds__(kFinishElems, 8) k_nh_surrogate_finish(
+    int64_t ne, int64_t e_begin, int64_t e_end, int64_t stride, const double *__restrict__ p, int64_t npts,
     const int32_t *__restrict__ t, const int32_t *__restrict__ dofs, const double *__restrict__ u, double mu,
-    double lmbda, double wsum, const float *__restrict__ params, const float *__restrict__ net,
-    const float4 *__restrict__ geo_in, float tol, float *__restrict__ recf, double *__restrict__ recd,
-    unsigned char *__restrict__ flags, unsigned long long *__restrict__ counters) {
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t e = e_begin + k / 3;
-    const int i = (int)(k % 3);  // tangent row block of this thread; block 2 also does the tail
-    if (e >= e_end) return;
-    const float *o = net + e * kNetOut;
-    bool use = o[9] != 0.f;
-    if (use) {
-        const float4 *g = geo_in + e * (kGeoRec / 4);
-        const float4 g0 = g[0], g1 = g[1], g2 = g[2], g3 = g[3], g4 = g[4], g5 = g[5];
-        const float F[9] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w, g2.x};
-        const float ga[4][3] = {{g2.y, g2.z, g2.w}, {g3.x, g3.y, g3.z}, {g3.w, g4.x, g4.y}, {g4.z, g4.w, g5.x}};
-        const float Vf = g5.y;
-        SurState st;
-        surrogate_state(F, st);
-        const float gx[3] = {o[0], o[1], o[2]};
-        const float Hx[9] = {o[3], o[4], o[5], o[4], o[6], o[7], o[5], o[7], o[8]};
-        use = surrogate_finish<true>(st, params + ONORM, gx, Hx, mu, lmbda, tol, Vf, ga,
-                                     reinterpret_cast<float4 *>(recf + e * kNhRecF), nullptr, nullptr, 0.0, i, i + 1,
-                                     i == 2);
+    double lmbda, double wsum, const float *__restrict__ net, const float4 *__restrict__ geo_in, float tol,
+    ClosureBlocks blk) {
+    __shared__ __align__(16) float stage[10 * kFinishStage];
+    const int64_t e0 = e_begin + (int64_t)blockIdx.x * kFinishElems;
+    const int n = (int)(e_end - e0 < kFinishElems ? e_end - e0 : kFinishElems);
+    const int el = threadIdx.x;
+    const int64_t e = e0 + el;
+    if (el < n) {
+        float *out = stage + el * 9;
+        const float4 *o = reinterpret_cast<const float4 *>(net + e * kNetOut);
+        const float4 o0 = o[0], o1 = o[1], o2 = o[2];
+        bool use = o2.y != 0.f;
+        if (use) {
+            const float4 *g = geo_in + e * (kGeoRec / 4);
+            const float4 g0 = g[0], g1 = g[1], g2 = g[2], g3 = g[3], g4 = g[4], g5 = g[5];
+            const float F[9] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w, g2.x};
+            const float ga[4][3] = {{g2.y, g2.z, g2.w}, {g3.x, g3.y, g3.z}, {g3.w, g4.x, g4.y}, {g4.z, g4.w, g5.x}};
+            const float Vf = g5.y;
+            SurState st;
+            surrogate_state(F, st);
+            const float Wf[3] = {o0.x, o0.y, o0.z};
+            const float Wff[9] = {o0.w, o1.x, o1.y, o1.x, o1.z, o1.w, o1.y, o1.w, o2.x};
+            float r[12];
+            use = surrogate_finish(
+                st, Wf, Wff, mu, lmbda, tol, Vf, ga,
+                [&](int a, int b, int i, int k, float v) { out[tri_index(4, a, b) * kFinishStage + i * 3 + k] = v; },
+                [&](int a, int i, float v) { r[a * 3 + i] = v; });
+            if (use) {
+                float4 *rf = reinterpret_cast<float4 *>(blk.r + e * 12);
+#pragma unroll
+                for (int q = 0; q < 3; ++q) rf[q] = make_float4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+            }
+        }
+        if (!use) {
+            surrogate_fallback_packed(e, stride, p, npts, t, ne, dofs, u, mu, lmbda, wsum, out, blk);
+            atomicAdd(blk.fallbacks, 1ULL);
+        }
+        blk.flags[e] = use ? 0 : 1;
     }
-    if (i != 2) return;
-    if (!use) surrogate_fallback<true>(e, p, npts, t, ne, dofs, u, mu, lmbda, wsum, nullptr, nullptr, recd, flags,
-                                       counters);
-    else flags[e] = 0;
+    __syncthreads();
+    // the elements' blocks t are one contiguous range
+    if (n == kFinishElems) {
+        constexpr int kVec = kFinishStage / 4;
+        for (int x = threadIdx.x; x < 10 * kVec; x += kFinishElems) {
+            const int tb = x / kVec, q = x - tb * kVec;
+            reinterpret_cast<float4 *>(blk.K + (tb * stride + e0) * 9)[q] =
+                reinterpret_cast<const float4 *>(stage + tb * kFinishStage)[q];
+        }
+    } else {
+        for (int x = threadIdx.x; x < 10 * kFinishStage; x += kFinishElems) {
+            const int tb = x / kFinishStage, q = x - tb * kFinishStage;
+            if (q < n * 9) blk.K[(tb * stride + e0) * 9 + q] = stage[x];
+        }
+    }
 }
 
 }  // namespace
@@ -1331,13 +1375,15 @@ void nh_assemble_surrogate(const skg_pattern *pat, const double *d_p, int64_t np
     d_u = device_resident(d_u, pat->n_rows, u_stage, s);
     DevBuf<unsigned long long> fb(2, s);  // [0] fallback elements, [1] tensor-core waits given up
     SKG_CUDA(cudaMemsetAsync(fb.get(), 0, 16, s));
-    if (d_values && pat->max_row_len > 0) {  // fused path, network on the tensor cores
-        DevBuf<float> recf((size_t)ne * kNhRecF, s), net((size_t)ne * kNetOut, s), geo((size_t)ne * kGeoRec, s);
+    if (d_values && pat->pairs.block == 3) {  // network on the tensor cores, pair sums
+        const int64_t stride = block_stride(ne);
+        DevBuf<float> K((size_t)stride * 90, s), K_low((size_t)stride * 90, s), re((size_t)ne * 24, s);
+        DevBuf<float> net((size_t)ne * kNetOut, s), geo((size_t)ne * kGeoRec, s);
         DevBuf<float4> xin((size_t)ne, s);
-        DevBuf<double> recd((size_t)ne * kNhRecD, s);
         DevBuf<unsigned char> flags((size_t)ne, s);
+        const ClosureBlocks blk{K.get(), K_low.get(), re.get(), re.get() + ne * 12, flags.get(), fb.get()};
         SKG_CUDA(cudaFuncSetAttribute(k_nh_surrogate_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem));
-        run_passes(
+        run_pair_passes(
             pat, ne, d_values, h_values, s,
             [&](int64_t e0, int64_t e1) {
                 k_nh_surrogate_prep<<<grid_for(e1 - e0, kFinishBlock), kFinishBlock, 0, s>>>(
@@ -1348,23 +1394,24 @@ void nh_assemble_surrogate(const skg_pattern *pat, const double *d_p, int64_t np
                 const unsigned grid = (unsigned)(tiles < kSmCount ? tiles : kSmCount);
                 k_nh_surrogate_tc<<<grid, kTcThreads, kTcSmem, s>>>(e0, e1, d_params, xin.get(), net.get(), fb.get());
                 SKG_LAUNCH_CHECK("nh_surrogate_tc");
-                k_nh_surrogate_finish<<<grid_for(3 * (e1 - e0), kFinishBlock), kFinishBlock, 0, s>>>(
-                    ne, e0, e1, d_p, npts, d_t, pat->row_dofs.get(), d_u, mu, lmbda, wsum, d_params, net.get(),
-                    reinterpret_cast<const float4 *>(geo.get()), tol, recf.get(), recd.get(), flags.get(), fb.get());
+                k_nh_surrogate_finish<<<grid_for(e1 - e0, kFinishElems), kFinishElems, 0, s>>>(
+                    ne, e0, e1, stride, d_p, npts, d_t, pat->row_dofs.get(), d_u, mu, lmbda, wsum,
+                    net.get(), reinterpret_cast<const float4 *>(geo.get()), tol, blk);
                 SKG_LAUNCH_CHECK("nh_surrogate_finish");
             },
-            [&](const GroupSet &gs, cudaStream_t st) {
-                nh_rows(pat, gs, recd.get(), recf.get(), flags.get(), fb.get(), d_residual, d_values, st);
-            },
-            d_residual, h_residual);
+            [&](int s0, int s1, cudaStream_t st) { closure_sums(pat, s0, s1, blk, d_values, st); },
+            [&](cudaStream_t cs) {
+                if (d_residual) closure_residual(pat, blk, d_residual, s);
+                residual_to_host(pat, d_residual, h_residual, s, cs);
+            });
     } else {
         DevBuf<double> Ke(d_values ? (size_t)ne * 144 : 0, s), re(d_residual ? (size_t)ne * 12 : 0, s);
         if (ne) {
-            SKG_CUDA(cudaFuncSetAttribute(k_nh_surrogate_element<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            SKG_CUDA(cudaFuncSetAttribute(k_nh_surrogate_element, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kEvalSmem));
-            k_nh_surrogate_element<false><<<grid_for(ne, kEvalBlock), kEvalBlock, kEvalSmem, s>>>(
+            k_nh_surrogate_element<<<grid_for(ne, kEvalBlock), kEvalBlock, kEvalSmem, s>>>(
                 ne, d_p, npts, d_t, pat->row_dofs.get(), d_u, mu, lmbda, wsum, d_params, d_box, tol, Ke.get(),
-                re.get(), nullptr, nullptr, nullptr, fb.get());
+                re.get(), fb.get());
             SKG_LAUNCH_CHECK("nh_surrogate_element");
         }
         nh_gather(pat, Ke.get(), re.get(), d_residual, d_values, s);

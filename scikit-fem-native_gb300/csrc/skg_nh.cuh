@@ -120,4 +120,28 @@ __device__ __forceinline__ void write_nh_element(const NhGeom &g, const NhLaw &L
         }
 }
 
+// What the learned law's element pass writes and its sums read: packed FP32
+// blocks of the tangent (skg_pairs.cuh) and residual entries (E, 12); the low
+// parts of the FP64 values of the elements that the plain law served, which are
+// flagged and counted.
+struct ClosureBlocks {
+    float *K, *K_low, *r, *r_low;
+    unsigned char *flags;
+    unsigned long long *fallbacks;
+};
+
+// Tangent values of the slices [s0, s1) of the pair plan; residual per DOF.
+void closure_sums(const skg_pattern *pat, int s0, int s1, const ClosureBlocks &b, double *values, cudaStream_t s);
+void closure_residual(const skg_pattern *pat, const ClosureBlocks &b, double *residual, cudaStream_t s);
+
+// Residual and tangent from per-element arrays.
+void nh_gather(const skg_pattern *pat, const double *Ke, const double *re, double *d_residual, double *d_values,
+               cudaStream_t s);
+
+// Whole-array copies of the results to the host; the residual on cs, ordered after s.
+void nh_download(const skg_pattern *pat, const double *d_residual, const double *d_values, double *h_residual,
+                 double *h_values, cudaStream_t s);
+void residual_to_host(const skg_pattern *pat, const double *d_residual, double *h_residual, cudaStream_t s,
+                      cudaStream_t cs);
+
 }  // namespace skg

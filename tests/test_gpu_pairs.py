@@ -132,3 +132,32 @@ def test_affine_loads_in_every_layout(order, comp, cells):
                 for c, tail in ((value, ()), (gradient, (3,)))]
         want = O.linear_assemble(ob, value=full[0], gradient=full[1])
         assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("law", ["plain", "learned", "learned, all elements by the plain law"])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (11, 1, 1), (4, 4, 4), (7, 5, 3)])
+def test_neo_hookean(cells, law, surrogate):
+    """Residual and tangent.  FP64 entries, and FP64 entries carried in two FP32 parts (2^-48 apiece), as above;
+    the learned law's own error is 1e-4 at this deformation, 1e-3 holds with margin."""
+    m = _mesh(cells)
+    b = sk.Basis(m, sk.ElementVector(sk.ElementTetP1(), dim=3), quadrature=(X1, W1))
+    rng = np.random.default_rng(11)
+    G = rng.uniform(-0.08, 0.08, (3, 3))
+    u = (G @ m.p + 0.01 * np.sin(np.pi * m.p[::-1]) / max(cells)).T.ravel()
+    r, K = sk.NeoHookean(b, 1.0, 10.0).assemble(
+        u, **({} if law == "plain" else dict(surrogate=surrogate, tol=1e-2 if law == "learned" else -1.0)))
+    x = m.p[:, m.t]
+    J = np.moveaxis(x[:, 1:] - x[:, :1], -1, 0)
+    g = np.linalg.inv(J)
+    g = np.concatenate([-g.sum(axis=1, keepdims=True), g], axis=1)  # (E, 4, 3)
+    V = np.abs(np.linalg.det(J)) / 6.0
+    Gu = np.einsum("eac,eaj->ecj", u.reshape(-1, 3)[m.t.T], g)
+    re = np.einsum("e,ecj,eaj->eac", V, O.nh_first_piola(Gu, 1.0, 10.0), g).reshape(len(V), 12)
+    Ke = np.einsum("e,ericj,eai,ebj->earbc", V, O.nh_tangent(Gu, 1.0, 10.0), g, g).reshape(len(V), 12, 12)
+    dofs = (3 * m.t.T[:, :, None] + np.arange(3)).reshape(len(V), 12)
+    res, tan = np.zeros(b.N), np.zeros((b.N, b.N))
+    np.add.at(res, dofs, re)
+    np.add.at(tan, (dofs[:, :, None], dofs[:, None, :]), Ke)
+    bound = 1e-3 if law == "learned" else 1e-12
+    assert np.max(np.abs(r - res)) <= bound * np.max(np.abs(res))
+    assert np.max(np.abs(K.toarray() - tan)) <= bound * np.max(np.abs(tan))
