@@ -82,7 +82,7 @@ __global__ void k_check_range(const int32_t *v, int64_t n, int64_t hi, int32_t *
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int32_t x = v[i];
-        if (x < 0 || x >= hi) atomicMin(err, (int32_t)(i < (int64_t)INT_MAX - 1 ? i : (int64_t)INT_MAX - 1));
+        if (x < 0 || x >= hi) *err = 1;
     }
 }
 
@@ -102,20 +102,18 @@ __global__ void k_fill_incidence(const int32_t *row_dofs, int64_t total, const i
     }
 }
 
-// Thread per row: insertion sort of the (short) incidence list.
-__global__ void k_sort_incidence(const int32_t *inc_ptr, int32_t *inc, int64_t n_rows) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_rows) return;
-    const int32_t b = inc_ptr[r], e = inc_ptr[r + 1];
-    for (int32_t k = b + 1; k < e; ++k) {
-        const int32_t x = inc[k];
-        int32_t j = k - 1;
-        while (j >= b && inc[j] > x) {
-            inc[j + 1] = inc[j];
-            --j;
-        }
-        inc[j + 1] = x;
-    }
+// Orders every row's (short) incidence list: thread per incidence, which goes to
+// its rank among the row's.  (Thread per row, by insertion: 25 us at 6^3 cells,
+// a chain of dependent loads; 7 us this way.)
+__global__ void k_order_incidence(const int32_t *__restrict__ row_dofs, int64_t total,
+                                  const int32_t *__restrict__ inc_ptr, const int32_t *__restrict__ from,
+                                  int32_t *__restrict__ inc) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total) return;
+    const int32_t x = from[i], r = row_dofs[x], b = inc_ptr[r], e = inc_ptr[r + 1];
+    int32_t rank = 0;
+    for (int32_t k = b; k < e; ++k) rank += from[k] < x;
+    inc[b + rank] = x;
 }
 
 constexpr int kWarpsPerBlock = 4;
@@ -191,57 +189,69 @@ __global__ void k_row_columns(const int32_t *inc_ptr, const int32_t *inc, const 
     if (mode == 0 && lane == 0) counts[r] = written;
 }
 
-// Thread per row: column offsets of every incidence's local columns.
-__global__ void k_records(int64_t n_rows, const int32_t *__restrict__ indptr, const int32_t *__restrict__ indices,
-                          const int32_t *__restrict__ inc_ptr, const int32_t *__restrict__ inc,
+// Thread per incidence: column offsets of its local columns in its row.
+__global__ void k_records(int64_t total, const int32_t *__restrict__ indptr, const int32_t *__restrict__ indices,
+                          const int32_t *__restrict__ inc, const int32_t *__restrict__ row_dofs,
                           const int32_t *__restrict__ col_dofs, int32_t row_local, int32_t col_local,
                           int4 *__restrict__ rec) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_rows) return;
+    const int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (it >= total) return;
+    const int32_t item = inc[it], r = row_dofs[item];
     const int32_t rb = indptr[r], rn = indptr[r + 1] - rb;
-    const int32_t *cols = indices + rb;
-    for (int32_t it = inc_ptr[r]; it < inc_ptr[r + 1]; ++it) {
-        const int32_t item = inc[it];
-        const int64_t e = item / row_local;
-        unsigned w[3] = {0u, 0u, 0u};
-        for (int k = 0; k < col_local; ++k) {
-            const int pos = lower_bound_i32(cols, rn, col_dofs[e * col_local + k]);
-            w[k >> 2] |= (unsigned)(pos & 0xff) << (8 * (k & 3));
-        }
-        rec[it] = make_int4(item, (int)w[0], (int)w[1], (int)w[2]);
+    const int64_t e = item / row_local;
+    unsigned w[3] = {0u, 0u, 0u};
+    for (int k = 0; k < col_local; ++k) {
+        const int pos = lower_bound_i32(indices + rb, rn, col_dofs[e * col_local + k]);
+        const unsigned v = (unsigned)(pos & 0xff) << (8 * (k & 3));
+        if (k < 4) w[0] |= v;
+        else if (k < 8) w[1] |= v;
+        else w[2] |= v;
     }
+    rec[it] = make_int4(item, (int)w[0], (int)w[1], (int)w[2]);
 }
 
 }  // namespace
 
-// First and last element referenced by each row (incidences are in ascending
-// element order; rows without incidences: INT_MAX and -1).
-__global__ void k_element_span(int64_t n_rows, const int32_t *__restrict__ inc_ptr, const int32_t *__restrict__ inc,
-                               int32_t row_local, int2 *__restrict__ span) {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_rows) return;
-    const int32_t i0 = inc_ptr[r], i1 = inc_ptr[r + 1];
-    span[r] = i0 < i1 ? make_int2(inc[i0] / row_local, inc[i1 - 1] / row_local) : make_int2(INT_MAX, -1);
+// First and last element referenced by the rows [x, y) of each group
+// (incidences are in ascending element order; rows without incidences: INT_MAX
+// and -1); one warp per group.
+__global__ void k_group_span(int n, const int2 *__restrict__ groups, const int32_t *__restrict__ inc_ptr,
+                             const int32_t *__restrict__ inc, int32_t row_local, int2 *__restrict__ span) {
+    const int g = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    if (g >= n) return;
+    int lo = INT_MAX, hi = -1;
+    for (int32_t r = groups[g].x + (threadIdx.x & 31); r < groups[g].y; r += 32) {
+        const int32_t i0 = inc_ptr[r], i1 = inc_ptr[r + 1];
+        if (i0 < i1) {
+            lo = min(lo, inc[i0] / row_local);
+            hi = max(hi, inc[i1 - 1] / row_local);
+        }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) span[g] = make_int2(lo, hi);
 }
+
+// Groups that are resident together whatever their order.
+constexpr int kGroupsAtOnce = 4 * kSmCount;
 
 void build_pair_plan(skg_pattern *p, bool square, cudaStream_t s);
 
 // Incidence records for the warp-per-row assembly kernels; skipped when the
 // pattern is unsuitable (elements wider than 12 columns or rows of 256+
 // columns), in which case assemblies use the per-row global-memory gather.
-void build_records(skg_pattern *p, cudaStream_t s) {
+// `ip`: indptr on the host.
+void build_records(skg_pattern *p, const std::vector<int32_t> &ip, cudaStream_t s) {
     if (p->col_local > 12 || p->n_rows == 0) return;
-    std::vector<int32_t> ip(p->n_rows + 1);
-    SKG_CUDA(cudaMemcpyAsync(ip.data(), p->indptr.get(), ip.size() * 4, cudaMemcpyDeviceToHost, s));
-    SKG_CUDA(cudaStreamSynchronize(s));
     int32_t longest = 0;
     for (int64_t r = 0; r < p->n_rows; ++r) longest = std::max(longest, ip[r + 1] - ip[r]);
     if (longest > 255) return;
     const int64_t n_inc = p->n_elements * p->row_local;
     p->rec = DevBuf<int4>::owned(n_inc);
-    k_records<<<grid_for(p->n_rows, 128), 128, 0, s>>>(p->n_rows, p->indptr.get(), p->indices.get(),
-                                                       p->inc_ptr.get(), p->inc.get(), p->col_dofs.get(),
-                                                       p->row_local, p->col_local, p->rec.get());
+    if (n_inc)
+        k_records<<<grid_for(n_inc, 256), 256, 0, s>>>(n_inc, p->indptr.get(), p->indices.get(), p->inc.get(),
+                                                       p->row_dofs.get(), p->col_dofs.get(), p->row_local,
+                                                       p->col_local, p->rec.get());
     SKG_LAUNCH_CHECK("records");
     // Row groups.  A group first takes up to 32 consecutive rows within
     // kGroupSlotsSmall slots (one thread per row); when fewer than 24 rows
@@ -249,6 +259,7 @@ void build_records(skg_pattern *p, cudaStream_t s) {
     // kGroupSlotsLarge / 2 slots, served by two threads per row with one
     // accumulator copy each.
     std::vector<int2> small, large, all;  // `all`: every group, in row order
+    std::vector<int32_t> small_at, large_at;  // positions in `all`
     int64_t r = 0;
     while (r < p->n_rows) {
         const int64_t r0 = r;
@@ -257,33 +268,38 @@ void build_records(skg_pattern *p, cudaStream_t s) {
         if (r1 - r0 >= 24 || r1 == p->n_rows) {
             if (r1 == r0) r1 = r0 + 1;
             small.push_back(make_int2((int)r0, (int)r1));
+            small_at.push_back((int32_t)all.size());
         } else {
             r1 = r0;
             while (r1 < p->n_rows && r1 - r0 < 16 && ip[r1 + 1] - ip[r0] <= kGroupSlotsLarge / 2) ++r1;
             if (r1 == r0) r1 = r0 + 1;  // single row above the budget (cannot happen below 256 columns)
             large.push_back(make_int2((int)r0, (int)r1));
+            large_at.push_back((int32_t)all.size());
         }
         all.push_back(make_int2((int)r0, (int)r1));
         r = r1;
     }
-    std::vector<int2> span(p->n_rows);
-    {
-        DevBuf<int2> d_span(p->n_rows, s);
-        k_element_span<<<grid_for(p->n_rows, 256), 256, 0, s>>>(p->n_rows, p->inc_ptr.get(), p->inc.get(),
-                                                              p->row_local, d_span.get());
-        SKG_LAUNCH_CHECK("element_span");
-        SKG_CUDA(cudaMemcpyAsync(span.data(), d_span.get(), span.size() * 8, cudaMemcpyDeviceToHost, s));
+    auto upload = [&](const std::vector<int2> &vec, DevBuf<int2> &dst) {
+        dst = DevBuf<int2>::owned(vec.size());
+        if (!vec.empty())
+            SKG_CUDA(cudaMemcpyAsync(dst.get(), vec.data(), vec.size() * 8, cudaMemcpyHostToDevice, s));
+    };
+    std::vector<int2> span;  // per group of `all`
+    if ((int)all.size() > kGroupsAtOnce || ip[p->n_rows] >= kHostChunkMinNnz) {
+        const int n = (int)all.size();
+        DevBuf<int2> d_all(n, s), d_span(n, s);
+        span.resize(n);
+        SKG_CUDA(cudaMemcpyAsync(d_all.get(), all.data(), (size_t)n * 8, cudaMemcpyHostToDevice, s));
+        k_group_span<<<grid_for(n, 4), 128, 0, s>>>(n, d_all.get(), p->inc_ptr.get(), p->inc.get(), p->row_local,
+                                                    d_span.get());
+        SKG_LAUNCH_CHECK("group_span");
+        SKG_CUDA(cudaMemcpyAsync(span.data(), d_span.get(), (size_t)n * 8, cudaMemcpyDeviceToHost, s));
         SKG_CUDA(cudaStreamSynchronize(s));
     }
     // Order the groups by the first element they reference, so that groups
     // running at the same time touch a compact band of elements (their
     // per-element data stays in L2).  Each group still owns a contiguous
     // slot range, so the output writes stay coalesced.
-    auto first_element = [&](const int2 &g) {
-        int32_t m = INT_MAX;
-        for (int32_t q = g.x; q < g.y; ++q) m = std::min(m, span[q].x);
-        return m;
-    };
     auto sort_by = [](std::vector<int2> &vec, const std::vector<int64_t> &key) {
         std::vector<size_t> order(vec.size());
         for (size_t i = 0; i < order.size(); ++i) order[i] = i;
@@ -292,16 +308,13 @@ void build_records(skg_pattern *p, cudaStream_t s) {
         for (size_t i = 0; i < order.size(); ++i) out[i] = vec[order[i]];
         vec.swap(out);
     };
-    for (auto *vec : {&small, &large}) {
-        std::vector<int64_t> key(vec->size());
-        for (size_t i = 0; i < vec->size(); ++i) key[i] = first_element((*vec)[i]);
-        sort_by(*vec, key);
-    }
-    auto upload = [&](const std::vector<int2> &vec, DevBuf<int2> &dst) {
-        dst = DevBuf<int2>::owned(vec.size());
-        if (!vec.empty())
-            SKG_CUDA(cudaMemcpyAsync(dst.get(), vec.data(), vec.size() * 8, cudaMemcpyHostToDevice, s));
-    };
+    if (!span.empty())
+        for (int k = 0; k < 2; ++k) {
+            const std::vector<int32_t> &at = k ? large_at : small_at;
+            std::vector<int64_t> key(at.size());
+            for (size_t i = 0; i < at.size(); ++i) key[i] = span[at[i]].x;
+            sort_by(k ? large : small, key);
+        }
     if (ip[p->n_rows] >= kHostChunkMinNnz) {
         // Host-output chunks: boundaries at group starts near equal slot counts.
         const int64_t nnz = ip[p->n_rows];
@@ -320,9 +333,10 @@ void build_records(skg_pattern *p, cudaStream_t s) {
         auto chunk_of = [&](int32_t row) {
             return (int)(std::upper_bound(p->hc_row.begin(), p->hc_row.end(), row) - p->hc_row.begin()) - 1;
         };
-        for (int c = 0; c < n_chunks; ++c)
-            for (int32_t q = p->hc_row[c]; q < p->hc_row[c + 1]; ++q)
-                p->hc_ready[c] = std::max(p->hc_ready[c], (int64_t)span[q].y + 1);
+        for (size_t g = 0; g < all.size(); ++g) {  // a chunk is a range of whole groups
+            int64_t &ready = p->hc_ready[chunk_of(all[g].x)];
+            ready = std::max(ready, (int64_t)span[g].y + 1);
+        }
         std::vector<int2> hc_small = small, hc_large = large;
         for (auto *vec : {&hc_small, &hc_large}) {
             std::vector<int64_t> key(vec->size());
@@ -343,7 +357,6 @@ void build_records(skg_pattern *p, cudaStream_t s) {
     p->n_groups_large = (int32_t)large.size();
     upload(small, p->groups_small);
     upload(large, p->groups_large);
-    SKG_CUDA(cudaStreamSynchronize(s));
     p->max_row_len = longest;
 }
 
@@ -380,15 +393,14 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
             if (tc) SKG_CUDA(cudaMemcpyAsync(p->col_dofs.get(), d_col_dofs, tc * 4, cudaMemcpyDeviceToDevice, s));
             // range checks (the reference raises "element DOF index is out of bounds")
             DevBuf<int32_t> err(2, s);
-            const int32_t init[2] = {INT_MAX, INT_MAX};
-            SKG_CUDA(cudaMemcpyAsync(err.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
+            SKG_CUDA(cudaMemsetAsync(err.get(), 0, 8, s));
             if (tr) k_check_range<<<grid_for(tr, 256), 256, 0, s>>>(p->row_dofs.get(), tr, n_rows, err.get());
             if (tc) k_check_range<<<grid_for(tc, 256), 256, 0, s>>>(p->col_dofs.get(), tc, n_cols, err.get() + 1);
             SKG_LAUNCH_CHECK("check_range");
             int32_t herr[2];
             SKG_CUDA(cudaMemcpyAsync(herr, err.get(), sizeof(herr), cudaMemcpyDeviceToHost, s));
             SKG_CUDA(cudaStreamSynchronize(s));
-            require(herr[0] == INT_MAX && herr[1] == INT_MAX, "element DOF index is out of bounds", SKG_ERANGE);
+            require(!herr[0] && !herr[1], "element DOF index is out of bounds", SKG_ERANGE);
 
             DevBuf<int32_t> cnt(n_rows + 1, s), cursor(n_rows + 1, s);
             SKG_CUDA(cudaMemsetAsync(cnt.get(), 0, (n_rows + 1) * 4, s));
@@ -398,10 +410,15 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
             p->inc_ptr = DevBuf<int32_t>::owned(n_rows + 1);
             exclusive_scan_i32(cnt.get(), p->inc_ptr.get(), n_rows, s);
             p->inc = DevBuf<int32_t>::owned(tr);
-            if (tr) k_fill_incidence<<<grid_for(tr, 256), 256, 0, s>>>(p->row_dofs.get(), tr, p->inc_ptr.get(), cursor.get(), p->inc.get());
+            DevBuf<int32_t> unordered(tr, s);
+            if (tr)
+                k_fill_incidence<<<grid_for(tr, 256), 256, 0, s>>>(p->row_dofs.get(), tr, p->inc_ptr.get(),
+                                                                   cursor.get(), unordered.get());
             SKG_LAUNCH_CHECK("fill_incidence");
-            if (n_rows) k_sort_incidence<<<grid_for(n_rows, 128), 128, 0, s>>>(p->inc_ptr.get(), p->inc.get(), n_rows);
-            SKG_LAUNCH_CHECK("sort_incidence");
+            if (tr)
+                k_order_incidence<<<grid_for(tr, 256), 256, 0, s>>>(p->row_dofs.get(), tr, p->inc_ptr.get(),
+                                                                    unordered.get(), p->inc.get());
+            SKG_LAUNCH_CHECK("order_incidence");
             if (!with_csr) {
                 p->indptr = DevBuf<int32_t>::owned(n_rows + 1);
                 SKG_CUDA(cudaMemsetAsync(p->indptr.get(), 0, (n_rows + 1) * 4, s));
@@ -416,9 +433,12 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
             SKG_LAUNCH_CHECK("row_columns_count");
             p->indptr = DevBuf<int32_t>::owned(n_rows + 1);
             exclusive_scan_i32(cnt.get(), p->indptr.get(), n_rows, s);
-            int32_t nnz = 0;
-            SKG_CUDA(cudaMemcpyAsync(&nnz, p->indptr.get() + n_rows, 4, cudaMemcpyDeviceToHost, s));
+            // the row groups are formed from all of indptr, the rest needs its last entry
+            std::vector<int32_t> ip(col_local <= 12 ? n_rows + 1 : 1);
+            SKG_CUDA(cudaMemcpyAsync(ip.data(), p->indptr.get() + (n_rows + 1 - ip.size()), ip.size() * 4,
+                                     cudaMemcpyDeviceToHost, s));
             SKG_CUDA(cudaStreamSynchronize(s));
+            const int32_t nnz = ip.back();
             require(nnz >= 0, "pattern too large for 32-bit CSR offsets");
             p->nnz = nnz;
             p->indices = DevBuf<int32_t>::owned(nnz);
@@ -427,9 +447,9 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
                                                                  row_local, col_local, n_rows, 1, nullptr, p->indptr.get(),
                                                                  p->indices.get());
             SKG_LAUNCH_CHECK("row_columns_write");
-            SKG_CUDA(cudaStreamSynchronize(s));
-            build_records(p, s);
+            build_records(p, ip, s);
             build_pair_plan(p, d_row_dofs == d_col_dofs && row_local == col_local && n_rows == n_cols, s);
+            SKG_CUDA(cudaStreamSynchronize(s));  // the handle may be used on any stream
         } catch (...) {
             delete p;
             throw;

@@ -216,7 +216,7 @@ def _pattern_bytes(E, Lr, Lc, rows, nnz):
     csr = (_I32 * (rows + 1) + (_I32 + _F64) * nnz  # device CSR and values
            + 2 * ((_F64 + _I32) * nnz + _I64 * (rows + 1)))  # page-locked host matrix and one copy
     incidence = 20 * tr + _I32 * (rows + 1) + 2 * 8 * rows
-    temporary = 128 * (rows + 1) + _I32 * nnz
+    temporary = 128 * (rows + 1) + _I32 * (nnz + tr)
     if Lr == Lc:  # pair plan: padded positions and targets; pair rows, counts and order while it is built
         incidence += 2 * _I32 * E * (Lr * (Lr + 1) // 2) + 8 * (nnz // 2 + rows + 1024)
         temporary += 3 * _I32 * (nnz // 2 + rows + 1024)
