@@ -13,10 +13,11 @@
 // H_kl^T), so only the blocks a <= b are evaluated, and the pair sums
 // (skg_pairs.cuh) write both places.  No point data is read or tabulated.
 //
-// Bound by the FP64 pipe: about 240 FP64 instructions per vector P1 element,
-// 1,500 per vector P2 element (142 table terms of 9 products and the 10 blocks
-// H_kl).
+// Bound by the FP64 pipe: about 230 FP64 instructions per vector P1 element,
+// 980 to 1,870 per vector P2 element (142 terms of 9 products and the 10 blocks
+// H_kl; fewer for exact rules and without a value coefficient).
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "skg_common.cuh"
@@ -119,7 +120,9 @@ __device__ __forceinline__ void vector_block(const double pk[3], const double qk
         }
 }
 
-// Vector P1: blocks (np, stride, 3, 3), see skg_pairs.cuh.
+// Vector P1: blocks (np, stride, 3, 3), see skg_pairs.cuh.  MASS: there is a
+// value coefficient.
+template <bool MASS>
 __global__ void __launch_bounds__(kFormBlock) k_form_p1v(int64_t ne, int64_t e_begin, int64_t e_end, int64_t stride,
                                                         const double *__restrict__ p, int64_t npts,
                                                         const int32_t *__restrict__ t, FormCoefs fc,
@@ -150,7 +153,8 @@ __global__ void __launch_bounds__(kFormBlock) k_form_p1v(int64_t ne, int64_t e_b
 #pragma unroll
         for (int b = a; b < 4; ++b) {
             double H[9];
-            vector_block(pk, qk, tk, el.B[b], a == b, fma(el.vm, __ldg(tab + 1 + tri_index(4, a, b)), G[a][b]), H, F);
+            vector_block(pk, qk, tk, el.B[b], a == b,
+                         MASS ? fma(el.vm, __ldg(tab + 1 + tri_index(4, a, b)), G[a][b]) : G[a][b], H, F);
             double *st = out.next() + 9 * lane;
 #pragma unroll
             for (int x = 0; x < 9; ++x) st[x] = H[x];
@@ -160,25 +164,49 @@ __global__ void __launch_bounds__(kFormBlock) k_form_p1v(int64_t ne, int64_t e_b
     out.finish();
 }
 
-// Vector P2: the 10 blocks H_kl in registers, the 55 blocks from the table.
+// Coefficients of an exact rule, in units of -1/30: term (k, l) of the entry
+// (a, b), with k, l among the support vertices of a, b.  The gradient of vertex
+// shape a is (4 lambda_a - 1) B_a, that of edge shape (i, j) is 4 (lambda_j B_i +
+// lambda_i B_j), and the integrals of lambda_m lambda_n are (1 + [m = n]) / 120.
+__host__ __device__ constexpr int other_of(int b, int k) { return lo_of(b) == k ? hi_of(b) : lo_of(b); }
+__host__ __device__ constexpr int exact_term(int a, int k, int b, int l) {
+    const bool same = (a < 4 ? a : other_of(a, k)) == (b < 4 ? b : other_of(b, l));
+    return a < 4 || b < 4 ? (same ? -3 : 1) : (same ? -8 : -4);
+}
+
+// Vector P2: the 10 blocks H_kl in registers, the 55 blocks from the rule's
+// table, or for a rule exact on quadratics (EXACT) as small multiples of H / -30
+// (of -4 times that between edges): 1 to 3 operations per entry instead of 1 to
+// 4, and none for the blocks between vertices.  Bound by the FP64 pipe: about
+// 1870 instructions per element from the table with the mass term, 980 EXACT
+// without (MASS: there is a value coefficient); 19x17x18 cells 110 -> 80 us.
+template <bool EXACT, bool MASS>
 __global__ void __launch_bounds__(kFormBlock, 4) k_form_p2v(int64_t ne, int64_t e_begin, int64_t e_end,
                                                            int64_t stride, const double *__restrict__ p, int64_t npts,
                                                            const int32_t *__restrict__ t, FormCoefs fc,
                                                            const double *__restrict__ tab, double *__restrict__ Ke) {
     __shared__ __align__(16) double stages[kFormBlock / 32 * 2 * WarpStore::kStage];
-    __shared__ double Ts[kP2Table];
-    for (int i = threadIdx.x; i < kP2Table; i += kFormBlock) Ts[i] = tab[i];
-    __syncthreads();
+    __shared__ double Ts[EXACT && !MASS ? 1 : kP2Table];
+    if (!EXACT || MASS) {
+        for (int i = threadIdx.x; i < kP2Table; i += kFormBlock) Ts[i] = tab[i];
+        __syncthreads();
+    }
     const int lane = threadIdx.x & 31;
     const int64_t e0 = e_begin + (int64_t)blockIdx.x * kFormBlock + (threadIdx.x & ~31);
     const int n = (int)(e_end - e0 < 32 ? e_end - e0 : 32);
     if (n <= 0) return;
     WarpStore out{stages + (threadIdx.x >> 5) * 2 * WarpStore::kStage};
     const Fp64 F = Fp64::load();
+    const double two = F.add(F.one, F.one), four = F.add(two, two);  // in registers
     double H[10][9], vm;
     {
-        const Element el = load_element(ne, lane < n ? e0 + lane : e0, p, npts, t, fc, F);
+        Element el = load_element(ne, lane < n ? e0 + lane : e0, p, npts, t, fc, F);
         vm = el.vm;
+        if (EXACT) {
+            el.hs *= -1.0 / 30.0;
+            el.dv *= -1.0 / 30.0;
+            el.dg *= -1.0 / 30.0;
+        }
         double G[4][4];
         gram(el, G, F);
 #pragma unroll
@@ -196,7 +224,13 @@ __global__ void __launch_bounds__(kFormBlock, 4) k_form_p2v(int64_t ne, int64_t 
         }
     }
 #pragma unroll
-    for (int a = 0; a < 10; ++a)
+    for (int a = 0; a < 10; ++a) {
+        if (EXACT && a == 4) {  // from here on between edges only
+#pragma unroll
+            for (int q = 0; q < 10; ++q)
+#pragma unroll
+                for (int x = 0; x < 9; ++x) H[q][x] = F.mul(-four, H[q][x]);
+        }
 #pragma unroll
         for (int b = a; b < 10; ++b) {
             constexpr int kSup = 4;
@@ -208,7 +242,8 @@ __global__ void __launch_bounds__(kFormBlock, 4) k_form_p2v(int64_t ne, int64_t 
             for (int u = 0; u < kSup; ++u) {
                 if ((u & 2 && a < 4) || (u & 1 && b < 4)) continue;  // one support vertex
                 const int k = ka[u >> 1], l = kb[u & 1];
-                const double T = Ts[t4 * 4 + u];
+                const double T = EXACT ? 0.0 : Ts[EXACT ? 0 : t4 * 4 + u];
+                const int times = a < 4 ? exact_term(a, k, b, l) : exact_term(a, k, b, l) / -4;  // -3, 1 or 2
                 const double *h = H[k <= l ? tri_index(4, k, l) : tri_index(4, l, k)];
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
@@ -216,19 +251,26 @@ __global__ void __launch_bounds__(kFormBlock, 4) k_form_p2v(int64_t ne, int64_t 
                     for (int d = 0; d < 3; ++d) {
                         if (a == b && d < c) continue;  // diagonal block: symmetric
                         const double x = h[k <= l ? c * 3 + d : d * 3 + c];
-                        v[c * 3 + d] = first ? F.mul(T, x) : fma(T, x, v[c * 3 + d]);
+                        double &r = v[c * 3 + d];
+                        if (!EXACT) r = first ? F.mul(T, x) : fma(T, x, r);
+                        else if (times == 1) r = first ? x : F.add(x, r);
+                        else if (times == 2) r = first ? F.mul(two, x) : fma(two, x, r);
+                        else r = first ? F.mul(-F.three_, x) : fma(-F.three_, x, r);
                     }
                 first = false;
             }
-            const double m = F.mul(vm, Ts[220 + t4]);
+            const double m = MASS ? F.mul(vm, Ts[MASS ? 220 + t4 : 0]) : 0.0;
             double *st = out.next() + 9 * lane;
 #pragma unroll
             for (int c = 0; c < 3; ++c)
 #pragma unroll
-                for (int d = 0; d < 3; ++d)
-                    st[c * 3 + d] = c == d ? F.add(v[c * 3 + d], m) : a == b && d < c ? v[d * 3 + c] : v[c * 3 + d];
+                for (int d = 0; d < 3; ++d) {
+                    const double x = a == b && d < c ? v[d * 3 + c] : v[c * 3 + d];
+                    st[c * 3 + d] = MASS && c == d ? F.add(x, m) : x;
+                }
             out.store(Ke + ((int64_t)t4 * stride + e0) * 9, n, 9);
         }
+    }
     out.finish();
 }
 
@@ -306,6 +348,18 @@ std::vector<double> form_table(int nodes, int nq, const double *X, const double 
     return T;
 }
 
+// True when the rule's table of gradient products is that of exact integration.
+bool p2_form_is_exact(const std::vector<double> &T) {
+    for (int a = 0; a < 10; ++a)
+        for (int b = a; b < 10; ++b)
+            for (int u = 0; u < 4; ++u) {
+                if ((u & 2 && a < 4) || (u & 1 && b < 4)) continue;
+                const int k = u & 2 ? hi_of(a) : lo_of(a), l = u & 1 ? hi_of(b) : lo_of(b);
+                if (!(std::fabs(T[tri_index(10, a, b) * 4 + u] + exact_term(a, k, b, l) / 30.0) <= 1e-13)) return false;
+            }
+    return true;
+}
+
 }  // namespace
 
 void affine_forms_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, const int32_t *d_t, int nodes,
@@ -335,12 +389,15 @@ void affine_forms_assemble(const skg_pattern *pat, const double *d_p, int64_t np
     }
     const int64_t stride = block_stride(ne);
     DevBuf<double> Ke((size_t)stride * np * (comp == 3 ? 9 : 1), s);
+    const bool mass = fc.arr[0] || fc.cst[0] != 0.0;
+    const bool exact = comp == 3 && nodes == 10 && p2_form_is_exact(T);
+    const auto vector_form = nodes == 4 ? (mass ? k_form_p1v<true> : k_form_p1v<false>)
+                             : exact    ? (mass ? k_form_p2v<true, true> : k_form_p2v<true, false>)
+                                        : (mass ? k_form_p2v<false, true> : k_form_p2v<false, false>);
     auto elem = [&](int64_t e0, int64_t e1) {
-        const unsigned grid = grid_for(e1 - e0, kFormBlock);
-        if (comp == 3 && nodes == 4)
-            k_form_p1v<<<grid, kFormBlock, 0, s>>>(ne, e0, e1, stride, d_p, npts, d_t, fc, tab, Ke.get());
-        else if (comp == 3)
-            k_form_p2v<<<grid, kFormBlock, 0, s>>>(ne, e0, e1, stride, d_p, npts, d_t, fc, tab, Ke.get());
+        if (comp == 3)
+            vector_form<<<grid_for(e1 - e0, kFormBlock), kFormBlock, 0, s>>>(ne, e0, e1, stride, d_p, npts, d_t, fc, tab,
+                                                                            Ke.get());
         else if (nodes == 4)
             k_form_scalar<4><<<grid_for(e1 - e0, kTile), kTile, 0, s>>>(ne, e0, e1, stride, d_p, npts, d_t, fc, tab, Ke.get());
         else

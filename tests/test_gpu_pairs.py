@@ -81,6 +81,26 @@ def test_affine_forms(order, comp, cells, one_point):
         assert np.max(np.abs(K.data - data)) <= 1e-12 * np.max(np.abs(data))
 
 
+@pytest.mark.parametrize("one_point", [False, True])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (11, 1, 1), (7, 5, 3)])
+@pytest.mark.parametrize("order", [1, 2])
+def test_vector_forms_without_a_value_term(order, cells, one_point):
+    """As above, without the mass term."""
+    m = _mesh(cells)
+    if order == 2:
+        m = sk.MeshTet2.from_mesh(m)
+    quadrature = (X1, W1) if one_point else None
+    basis = sk.Basis(m, sk.ElementVector(sk.ElementTetP2() if order == 2 else sk.ElementTetP1(), dim=3),
+                     quadrature=quadrature)
+    ob = O.make_basis(m.p, m.t, order == 2, comp=3, quadrature=quadrature)
+    E, Q = basis._coefficient_shape
+    rng = np.random.default_rng(4)
+    co = {"gradient": 0.8, "symmetric_gradient": rng.uniform(0.5, 2.0, (E, 1)), "divergence": 1.3}
+    K = sk.NativeBilinearForm(basis).assemble(**co)
+    data, _, _ = O.bilinear_assemble(ob, **{k: np.broadcast_to(c, (E, Q)) for k, c in co.items()})
+    assert np.max(np.abs(K.data - data)) <= 1e-12 * np.max(np.abs(data))
+
+
 def _affine_pair(cells, orders, comps):
     m = sk.MeshTet2.from_mesh(_mesh(cells))
     elem = {1: sk.ElementTetP1(), 2: sk.ElementTetP2()}
