@@ -25,6 +25,7 @@
 // row-owner gather as H1.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <vector>
 
 #include "skg_common.cuh"
@@ -173,10 +174,18 @@ constexpr int kN1Block = kTile;
 // 6, 6), staged through shared memory (FP64).  With `redo`, the pass runs
 // only when the split-precision pass before it left its range (its blocks then
 // walk the tiles).
-// The curl term as c_a^T H c_c with H = 4 nu wsum J^T J / |det| (the
-// reference curls c_a have entries 0 and +-2): signed sums of H's entries.
-template <bool PACKED>
-__global__ void __launch_bounds__(kN1Block) k_n1_elem_fast(int64_t ne, int64_t e_begin, int64_t e_end,
+//
+// Bound by the FP64 pipe, hence the curl term from the entries of H = 4 nu wsum
+// J^T J / |det|: the reference curls 1, 4 and 5 are +-2 times a unit vector and
+// the others sums of two of them, one addition per further entry.  EXACT (the
+// rule integrates quadratics): the integrals of lambda_m lambda_n are (1 + [m =
+// n]) / 120, so with G in units of mu / 120 the mass terms of two edges (s, x),
+// (s, y) that share s are 2 (G_xy + G_ss) + G_sm, m the fourth vertex (from 2
+// G_xy - G_sx - G_sy + G_ss and the zero row sums of G); three operations
+// instead of four from the table.  48^3: 242 -> 204 us (4 blocks per
+// SM; 5 and 6: 203, 224).
+template <bool PACKED, bool EXACT>
+__global__ void __launch_bounds__(kN1Block, EXACT ? 4 : 2) k_n1_elem_fast(int64_t ne, int64_t e_begin, int64_t e_end,
                                                             const double *__restrict__ p, int64_t npts,
                                                             const int32_t *__restrict__ t,
                                                             const int8_t *__restrict__ signs, N1Table tab,
@@ -185,11 +194,14 @@ __global__ void __launch_bounds__(kN1Block) k_n1_elem_fast(int64_t ne, int64_t e
                                                             int inc_curl, const int *__restrict__ redo,
                                                             int64_t stride, double *__restrict__ Ke) {
     __shared__ double stage[PACKED ? 1 : kN1Block * 37];
-    __shared__ double Tm[6 * 6 * 4];  // operands from shared memory: see skg_fp64.cuh
+    __shared__ double Tm[EXACT ? 1 : 6 * 6 * 4];  // operands from shared memory: see skg_fp64.cuh
     if (redo && !out_of_range(redo)) return;
     const Fp64 F = Fp64::load();
-    for (int i = threadIdx.x; i < 144; i += kN1Block) Tm[i] = (&tab.Tm[0][0][0])[i];
-    __syncthreads();
+    const double two = F.add(F.one, F.one);  // in a register
+    if constexpr (!EXACT) {
+        for (int i = threadIdx.x; i < 144; i += kN1Block) Tm[i] = (&tab.Tm[0][0][0])[i];
+        __syncthreads();
+    }
     for (int64_t e0 = e_begin + (int64_t)blockIdx.x * kN1Block; e0 < e_end; e0 += (int64_t)gridDim.x * kN1Block) {
         const int64_t e = e0 + threadIdx.x;
         if (e < e_end) {
@@ -215,7 +227,7 @@ __global__ void __launch_bounds__(kN1Block) k_n1_elem_fast(int64_t ne, int64_t e
             const double nu = inc_curl ? (curl ? curl[e] : 1.0) * inv * tab.wsum : 0.0;
             // mu b_k . b_l / |det J|: dot products for k, l >= 1, row 0 from
             // b_0 = -(b_1 + b_2 + b_3); mu / |det J| scales the six products once
-            const double mi = mu * inv;
+            const double mi = EXACT ? mu * inv * (1.0 / 120.0) : mu * inv;
             double Gm[4][4];
 #pragma unroll
             for (int k = 1; k < 4; ++k)
@@ -230,8 +242,7 @@ __global__ void __launch_bounds__(kN1Block) k_n1_elem_fast(int64_t ne, int64_t e
                 Gm[l][0] = Gm[0][l];
             }
             Gm[0][0] = -F.add3(Gm[0][1], Gm[0][2], Gm[0][3]);
-            // curl term nu (J c_a).(J c_c) = c_a^T (nu J^T J) c_c: with H = 4 nu J^T J (6 entries) and the
-            // reference curls' entries +-2, each entry is a signed sum of 1 to 4 entries of H
+            // curl term nu (J c_a).(J c_c) = c_a^T (nu J^T J) c_c, with H = 4 nu J^T J
             double H[3][3];
             const double nu4 = 4.0 * nu;
 #pragma unroll
@@ -241,6 +252,29 @@ __global__ void __launch_bounds__(kN1Block) k_n1_elem_fast(int64_t ne, int64_t e
                     H[r][q] = F.mul(nu4, fma(J[6 + r], J[6 + q], fma(J[3 + r], J[3 + q], F.mul(J[r], J[q]))));
                     H[q][r] = H[r][q];
                 }
+            // unit curls u_1 = z, u_4 = -y, u_5 = x; u_0 = u_1 + u_4, u_2 = u_1 - u_5, u_3 = -u_4 - u_5
+            double C[6][6];
+            C[1][1] = H[2][2];
+            C[1][4] = -H[1][2];
+            C[1][5] = H[0][2];
+            C[4][4] = H[1][1];
+            C[4][5] = -H[0][1];
+            C[5][5] = H[0][0];
+            C[0][1] = F.add(C[1][1], C[1][4]);
+            C[0][4] = F.add(C[1][4], C[4][4]);
+            C[0][5] = F.add(C[1][5], C[4][5]);
+            C[1][2] = F.sub(C[1][1], C[1][5]);
+            C[2][4] = F.sub(C[1][4], C[4][5]);
+            C[2][5] = F.sub(C[1][5], C[5][5]);
+            C[1][3] = F.sub(-C[1][4], C[1][5]);
+            C[3][4] = F.sub(-C[4][4], C[4][5]);
+            C[3][5] = F.sub(-C[4][5], C[5][5]);
+            C[0][0] = F.add(C[0][1], C[0][4]);
+            C[0][2] = F.add(C[1][2], C[2][4]);
+            C[0][3] = F.add(C[1][3], C[3][4]);
+            C[2][2] = F.sub(C[1][2], C[2][5]);
+            C[2][3] = F.sub(C[1][3], C[3][5]);
+            C[3][3] = F.sub(-C[3][4], C[3][5]);
             // orientation signs (+1 / -1) applied as a sign-bit flip of the FP64 value
             uint32_t neg[6];
 #pragma unroll
@@ -250,22 +284,24 @@ __global__ void __launch_bounds__(kN1Block) k_n1_elem_fast(int64_t ne, int64_t e
             for (int a = 0; a < 6; ++a)
 #pragma unroll
                 for (int c = a; c < 6; ++c) {
-                    double val = 0.0;
-                    bool first = true;
+                    double val = C[a][c];
+                    const int i = edge_v(a, 0), j = edge_v(a, 1), k = edge_v(c, 0), l = edge_v(c, 1);
+                    if constexpr (!EXACT) {
 #pragma unroll
-                    for (int r = 0; r < 3; ++r)
+                        for (int u = 0; u < 2; ++u)
 #pragma unroll
-                        for (int q = 0; q < 3; ++q)
-                            if (ref_curl(a, r) != 0.0 && ref_curl(c, q) != 0.0) {
-                                const double h = (ref_curl(a, r) > 0.0) == (ref_curl(c, q) > 0.0) ? H[r][q] : -H[r][q];
-                                val = first ? h : F.add(val, h);
-                                first = false;
-                            }
-#pragma unroll
-                    for (int u = 0; u < 2; ++u)
-#pragma unroll
-                        for (int w = 0; w < 2; ++w)
-                            val = fma(Gm[edge_v(a, u)][edge_v(c, w)], Tm[(a * 6 + c) * 4 + u * 2 + w], val);
+                            for (int w = 0; w < 2; ++w)
+                                val = fma(Gm[edge_v(a, u)][edge_v(c, w)], Tm[(a * 6 + c) * 4 + u * 2 + w], val);
+                    } else if (a == c) {
+                        val = fma(two, F.sub(F.add(Gm[i][i], Gm[j][j]), Gm[i][j]), val);
+                    } else if (i == k || i == l || j == k || j == l) {
+                        const int sh = i == k || i == l ? i : j, x = i + j - sh, y = k + l - sh, m = 6 - sh - x - y;
+                        const double twice = F.add(Gm[x][y], Gm[sh][sh]);
+                        if ((sh == i) == (sh == k)) val = fma(two, twice, F.add(val, Gm[sh][m]));
+                        else val = fma(-two, twice, F.sub(val, Gm[sh][m]));
+                    } else {
+                        val = F.add(F.add(F.sub(F.sub(val, Gm[j][k]), Gm[i][l]), Gm[j][l]), Gm[i][k]);
+                    }
                     const unsigned long long flip = (unsigned long long)(neg[a] ^ neg[c]) << 63;
                     val = __longlong_as_double((long long)((unsigned long long)__double_as_longlong(val) ^ flip));
                     if constexpr (PACKED) {
@@ -587,6 +623,18 @@ static void n1_table(int nq, const double *X, const double *W, N1Table &tab) {
 namespace skg {
 namespace {
 
+// True when the rule reproduces the exact integrals of lambda_m lambda_n.
+bool n1_rule_is_exact(const N1Table &tab) {
+    for (int a = 0; a < 6; ++a)
+        for (int c = 0; c < 6; ++c)
+            for (int u = 0; u < 2; ++u)
+                for (int w = 0; w < 2; ++w) {
+                    const double want = (edge_v(a, 1 - u) == edge_v(c, 1 - w) ? 2.0 : 1.0) / (u == w ? 120.0 : -120.0);
+                    if (!(std::fabs(tab.Tm[a][c][u * 2 + w] - want) <= 1e-15)) return false;
+                }
+    return true;
+}
+
 // Element matrices by the closed form (packed), then the pair sums.  h_values
 // (optional, page-locked host): the values are also copied there.  Split
 // precision: the double-float element pass, then the FP64 one in its place when
@@ -597,12 +645,14 @@ void n1_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, const 
                  double *d_values, double *h_values, cudaStream_t s) {
     N1Table tab;
     n1_table(nq, h_X, h_W, tab);
+    const bool exact = n1_rule_is_exact(tab);
     const int64_t stride = block_stride(ne);
     DevBuf<double> Ke((size_t)stride * 21, s);
     DevBuf<int> misc(2, s);  // [0] scale exponent, [1] range flag (split precision)
     auto elem64 = [&](int64_t e0, int64_t e1, const int *redo) {
         const unsigned grid = grid_for(e1 - e0, kN1Block);
-        k_n1_elem_fast<true><<<redo ? std::min(grid, 4u * kSmCount) : grid, kN1Block, 0, s>>>(
+        (exact ? k_n1_elem_fast<true, true> : k_n1_elem_fast<true, false>)<<<redo ? std::min(grid, 4u * kSmCount) : grid,
+                                                                             kN1Block, 0, s>>>(
             ne, e0, e1, d_p, npts, d_t, d_signs, tab, d_mass, d_curl, include_mass, include_curl, redo, stride,
             Ke.get());
         SKG_LAUNCH_CHECK("n1_element");
@@ -830,7 +880,7 @@ extern "C" int skg_n1_element_matrices(const double *d_p, int64_t npts, const in
         N1Table tab;
         n1_table(nq, h_X, h_W, tab);
         if (!coef_per_point) {
-            k_n1_elem_fast<false><<<grid_for(ne, kN1Block), kN1Block, 0, s>>>(ne, 0, ne, d_p, npts, d_t, d_signs, tab,
+            k_n1_elem_fast<false, false><<<grid_for(ne, kN1Block), kN1Block, 0, s>>>(ne, 0, ne, d_p, npts, d_t, d_signs, tab,
                                                                              d_mass, d_curl, include_mass,
                                                                              include_curl, nullptr, 0, d_out);
             SKG_LAUNCH_CHECK("n1_element_matrices");

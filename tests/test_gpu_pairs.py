@@ -154,6 +154,22 @@ def test_affine_loads_in_every_layout(order, comp, cells):
         assert np.max(np.abs(got - want)) <= 1e-12 * np.max(np.abs(want))
 
 
+@pytest.mark.parametrize("terms", ["both", "mass", "curl"])
+@pytest.mark.parametrize("cells", [(1, 1, 1), (11, 1, 1), (4, 4, 4), (7, 5, 3)])
+@pytest.mark.parametrize("intorder", [1, 2, 4])
+def test_n1_rules(intorder, cells, terms):
+    """Coefficients per element on a rule that is not exact for the mass term and on two that are; about 24
+    contributions of 60 roundings: 1e-12 of the largest entry."""
+    m = _mesh(cells)
+    rng = np.random.default_rng(5)
+    mass, curl = rng.uniform(0.5, 2.0, (2, m.t.shape[1], 1)) * np.array([terms != "curl", terms != "mass"])[:, None, None]
+    K = sk.TetN1Assembler(sk.AffineTetN1Basis(m, intorder=intorder)).assemble_maxwell(mass_coefficient=mass,
+                                                                                      curl_coefficient=curl)
+    data, indptr, indices = O.n1_assemble_maxwell(O.make_n1_basis(m.p, m.t, intorder), mass, curl)
+    assert np.array_equal(K.indptr, indptr) and np.array_equal(K.indices, indices)
+    assert np.max(np.abs(K.data - data)) <= 1e-12 * np.max(np.abs(data))
+
+
 @pytest.mark.parametrize("law", ["plain", "learned", "learned, all elements by the plain law"])
 @pytest.mark.parametrize("cells", [(1, 1, 1), (11, 1, 1), (4, 4, 4), (7, 5, 3)])
 def test_neo_hookean(cells, law, surrogate):
