@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(kFormBlock) k_form_p1v(int64_t ne, int64_t e_b
     el.hs *= sw;
     el.dv *= sw;
     el.dg *= sw;
+    const double ht = F.add(el.hs, el.dv);
     double G[4][4];
     gram(el, G, F);
 #pragma unroll
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(kFormBlock) k_form_p1v(int64_t ne, int64_t e_b
         for (int c = 0; c < 3; ++c) {
             pk[c] = F.mul(el.hs, el.B[a][c]);
             qk[c] = F.mul(el.dv, el.B[a][c]);
-            tk[c] = F.add(pk[c], qk[c]);
+            tk[c] = F.mul(ht, el.B[a][c]);
         }
 #pragma unroll
         for (int b = a; b < 4; ++b) {
@@ -207,6 +208,7 @@ __global__ void __launch_bounds__(kFormBlock, 4) k_form_p2v(int64_t ne, int64_t 
             el.dv *= -1.0 / 30.0;
             el.dg *= -1.0 / 30.0;
         }
+        const double ht = F.add(el.hs, el.dv);
         double G[4][4];
         gram(el, G, F);
 #pragma unroll
@@ -216,7 +218,7 @@ __global__ void __launch_bounds__(kFormBlock, 4) k_form_p2v(int64_t ne, int64_t 
             for (int c = 0; c < 3; ++c) {
                 pk[c] = F.mul(el.hs, el.B[k][c]);
                 qk[c] = F.mul(el.dv, el.B[k][c]);
-                tk[c] = F.add(pk[c], qk[c]);
+                tk[c] = F.mul(ht, el.B[k][c]);
             }
 #pragma unroll
             for (int l = k; l < 4; ++l)

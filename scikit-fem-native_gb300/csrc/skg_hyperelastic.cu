@@ -39,7 +39,8 @@ constexpr int kNhBlock = 64;
 // skg_pairs.cuh) and residual (E, 12) of the plain law, thread per element.
 //
 // The kernel is bound by the FP64 pipe, so the law is evaluated in the form
-// with the fewest FP64 instructions (535 -> about 365 per element):
+// with the fewest FP64 instructions (535 -> about 360 per element; 64^3: 1543 ->
+// 922 us, 1001 at the 80 registers that the compiler takes by itself):
 // * h_a = F^-T grad lambda_a is the gradient of lambda_a on the displaced
 //   tetrahedron (edges j_k = J_k + u_k - u_0): its cofactors over its
 //   determinant, without F, its inverse or the products with it; det F is the
@@ -51,7 +52,7 @@ constexpr int kNhBlock = 64;
 //   the entries are p_a,k h_b,i + q_a,i h_b,k (i != k), t_a,i h_b,i + G_ab
 //   (i = k), and t_a,k h_a,i in the diagonal blocks (symmetric).
 // Ke or re may be NULL (that output is skipped).
-__global__ void __launch_bounds__(kNhBlock) k_nh_packed(int64_t ne, int64_t e_begin, int64_t e_end, int64_t stride,
+__global__ void __launch_bounds__(kNhBlock, 8) k_nh_packed(int64_t ne, int64_t e_begin, int64_t e_end, int64_t stride,
                                                        const double *__restrict__ p, int64_t npts,
                                                        const int32_t *__restrict__ t, const int32_t *__restrict__ dofs,
                                                        const double *__restrict__ u, double mu, double lmbda,
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(kNhBlock) k_nh_packed(int64_t ne, int64_t e_be
     const double idj = 1.0 / detj;
     const double lnJ = log(detj * id);
     const double V = fabs(det) * wsum;
-    const double c2V = (mu - lmbda * lnJ) * V, lamV = lmbda * V;
+    const double c2V = (mu - lmbda * lnJ) * V, lamV = lmbda * V, tV = c2V + lamV;
     double G[4][4];
     const double gs = mu * V * id * id;
 #pragma unroll
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kNhBlock) k_nh_packed(int64_t ne, int64_t e_be
             for (int i = 0; i < 3; ++i) {
                 pa[i] = F.mul(c2V, h[a][i]);
                 qa[i] = F.mul(lamV, h[a][i]);
-                ta[i] = F.add(pa[i], qa[i]);
+                ta[i] = F.mul(tV, h[a][i]);
             }
 #pragma unroll
             for (int b = a; b < 4; ++b) {
