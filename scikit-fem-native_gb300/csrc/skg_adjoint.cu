@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kRed) k_energy_grad_elem(int64_t ne, const dou
 //   coordinates (out_x, (3, n_rows), component-major like mesh.p) and / or
 //   u / v DOFs (out_u, out_v (n_rows)); both in one walk when the vertex and
 //   DOF incidence lists coincide (scalar P1 with every vertex a DOF).
-__global__ void __launch_bounds__(128) k_energy_grad_gather(int64_t n_rows, const int32_t *__restrict__ inc_ptr,
+__global__ void __launch_bounds__(128, 4) k_energy_grad_gather(int64_t n_rows, const int32_t *__restrict__ inc_ptr,
                                                             const int32_t *__restrict__ inc,
                                                             const double *__restrict__ cx,
                                                             const double *__restrict__ cv,

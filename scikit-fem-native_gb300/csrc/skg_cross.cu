@@ -34,7 +34,7 @@ __host__ __device__ constexpr int sup1(int b) { return b < 4 ? b : (b == 4 ? 1 :
 // (E, nt Ct, nc Cc).  tab (nt, nc, 4): value tables in entry 0; gradient T^kl
 // over the supports; divergences R^l over the differentiated function's
 // supports.
-__global__ void __launch_bounds__(128) k_cross_affine(int64_t ne, const double *__restrict__ p, int64_t npts,
+__global__ void __launch_bounds__(128, 4) k_cross_affine(int64_t ne, const double *__restrict__ p, int64_t npts,
                                                       const int32_t *__restrict__ t, int kind, int nt, int Ct, int nc,
                                                       int Cc, const double *__restrict__ tab,
                                                       const double *__restrict__ coef, double cst,
