@@ -242,12 +242,10 @@ struct skg_pattern {
     skg::DevBuf<int2> groups_small, groups_large;
     // Host-output row chunks: up to kHostChunks row ranges of about equal
     // slot counts whose boundaries are group starts.  Chunk c covers rows
-    // [hc_row[c], hc_row[c+1]) = slots [hc_slot[c], hc_slot[c+1]); its rows
-    // reference elements below hc_ready[c] only.  The same groups as above,
-    // ordered by chunk (then by first element), are hc_small / hc_large, and
+    // [hc_row[c], hc_row[c+1]) = slots [hc_slot[c], hc_slot[c+1]).  The same
+    // groups as above, ordered by chunk (then by first element), are hc_small / hc_large, and
     // chunk c's groups of a class start at hc_small_off[c] / hc_large_off[c].
     std::vector<int32_t> hc_row, hc_slot, hc_small_off, hc_large_off;
-    std::vector<int64_t> hc_ready;
     skg::DevBuf<int2> hc_small, hc_large;
     // Incidence records (col_local <= 12 and every row shorter than 256):
     // one int4 per incidence in `inc` order, x = e*row_local + i and the

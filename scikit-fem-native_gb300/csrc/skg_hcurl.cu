@@ -648,7 +648,6 @@ void n1_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, const 
     const bool exact = n1_rule_is_exact(tab);
     const int64_t stride = block_stride(ne);
     DevBuf<double> Ke((size_t)stride * 21, s);
-    DevBuf<int> misc(2, s);  // [0] scale exponent, [1] range flag (split precision)
     auto elem64 = [&](int64_t e0, int64_t e1, const int *redo) {
         const unsigned grid = grid_for(e1 - e0, kN1Block);
         (exact ? k_n1_elem_fast<true, true> : k_n1_elem_fast<true, false>)<<<redo ? std::min(grid, 4u * kSmCount) : grid,
@@ -658,6 +657,7 @@ void n1_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, const 
         SKG_LAUNCH_CHECK("n1_element");
     };
     const bool split = precision == SKG_SPLIT_FP32 && ne;
+    DevBuf<int> misc(split ? 2 : 0, s);  // [0] scale exponent, [1] range flag
     if (split) {
         N1TableF tf;
         for (int a = 0; a < 6; ++a)

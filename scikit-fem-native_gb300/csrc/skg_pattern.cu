@@ -212,24 +212,17 @@ __global__ void k_records(int64_t total, const int32_t *__restrict__ indptr, con
 
 }  // namespace
 
-// First and last element referenced by the rows [x, y) of each group
-// (incidences are in ascending element order; rows without incidences: INT_MAX
-// and -1); one warp per group.
-__global__ void k_group_span(int n, const int2 *__restrict__ groups, const int32_t *__restrict__ inc_ptr,
-                             const int32_t *__restrict__ inc, int32_t row_local, int2 *__restrict__ span) {
+// First element referenced by the rows [x, y) of each group (incidences are in
+// ascending element order; INT_MAX without incidences); one warp per group.
+__global__ void k_group_first(int n, const int2 *__restrict__ groups, const int32_t *__restrict__ inc_ptr,
+                              const int32_t *__restrict__ inc, int32_t row_local, int32_t *__restrict__ first) {
     const int g = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
     if (g >= n) return;
-    int lo = INT_MAX, hi = -1;
-    for (int32_t r = groups[g].x + (threadIdx.x & 31); r < groups[g].y; r += 32) {
-        const int32_t i0 = inc_ptr[r], i1 = inc_ptr[r + 1];
-        if (i0 < i1) {
-            lo = min(lo, inc[i0] / row_local);
-            hi = max(hi, inc[i1 - 1] / row_local);
-        }
-    }
+    int lo = INT_MAX;
+    for (int32_t r = groups[g].x + (threadIdx.x & 31); r < groups[g].y; r += 32)
+        if (inc_ptr[r] < inc_ptr[r + 1]) lo = min(lo, inc[inc_ptr[r]] / row_local);
     lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if ((threadIdx.x & 31) == 0) span[g] = make_int2(lo, hi);
+    if ((threadIdx.x & 31) == 0) first[g] = lo;
 }
 
 // Groups that are resident together whatever their order.
@@ -284,16 +277,17 @@ void build_records(skg_pattern *p, const std::vector<int32_t> &ip, cudaStream_t 
         if (!vec.empty())
             SKG_CUDA(cudaMemcpyAsync(dst.get(), vec.data(), vec.size() * 8, cudaMemcpyHostToDevice, s));
     };
-    std::vector<int2> span;  // per group of `all`
-    if ((int)all.size() > kGroupsAtOnce || ip[p->n_rows] >= kHostChunkMinNnz) {
+    std::vector<int32_t> first;  // per group of `all`
+    if ((int)all.size() > kGroupsAtOnce) {
         const int n = (int)all.size();
-        DevBuf<int2> d_all(n, s), d_span(n, s);
-        span.resize(n);
+        DevBuf<int2> d_all(n, s);
+        DevBuf<int32_t> d_first(n, s);
+        first.resize(n);
         SKG_CUDA(cudaMemcpyAsync(d_all.get(), all.data(), (size_t)n * 8, cudaMemcpyHostToDevice, s));
-        k_group_span<<<grid_for(n, 4), 128, 0, s>>>(n, d_all.get(), p->inc_ptr.get(), p->inc.get(), p->row_local,
-                                                    d_span.get());
-        SKG_LAUNCH_CHECK("group_span");
-        SKG_CUDA(cudaMemcpyAsync(span.data(), d_span.get(), (size_t)n * 8, cudaMemcpyDeviceToHost, s));
+        k_group_first<<<grid_for(n, 4), 128, 0, s>>>(n, d_all.get(), p->inc_ptr.get(), p->inc.get(), p->row_local,
+                                                     d_first.get());
+        SKG_LAUNCH_CHECK("group_first");
+        SKG_CUDA(cudaMemcpyAsync(first.data(), d_first.get(), (size_t)n * 4, cudaMemcpyDeviceToHost, s));
         SKG_CUDA(cudaStreamSynchronize(s));
     }
     // Order the groups by the first element they reference, so that groups
@@ -308,11 +302,11 @@ void build_records(skg_pattern *p, const std::vector<int32_t> &ip, cudaStream_t 
         for (size_t i = 0; i < order.size(); ++i) out[i] = vec[order[i]];
         vec.swap(out);
     };
-    if (!span.empty())
+    if (!first.empty())
         for (int k = 0; k < 2; ++k) {
             const std::vector<int32_t> &at = k ? large_at : small_at;
             std::vector<int64_t> key(at.size());
-            for (size_t i = 0; i < at.size(); ++i) key[i] = span[at[i]].x;
+            for (size_t i = 0; i < at.size(); ++i) key[i] = first[at[i]];
             sort_by(k ? large : small, key);
         }
     if (ip[p->n_rows] >= kHostChunkMinNnz) {
@@ -329,14 +323,9 @@ void build_records(skg_pattern *p, const std::vector<int32_t> &ip, cudaStream_t 
         const int n_chunks = (int)p->hc_row.size() - 1;
         p->hc_slot.resize(n_chunks + 1);
         for (int c = 0; c <= n_chunks; ++c) p->hc_slot[c] = ip[p->hc_row[c]];
-        p->hc_ready.assign(n_chunks, 0);
         auto chunk_of = [&](int32_t row) {
             return (int)(std::upper_bound(p->hc_row.begin(), p->hc_row.end(), row) - p->hc_row.begin()) - 1;
         };
-        for (size_t g = 0; g < all.size(); ++g) {  // a chunk is a range of whole groups
-            int64_t &ready = p->hc_ready[chunk_of(all[g].x)];
-            ready = std::max(ready, (int64_t)span[g].y + 1);
-        }
         std::vector<int2> hc_small = small, hc_large = large;
         for (auto *vec : {&hc_small, &hc_large}) {
             std::vector<int64_t> key(vec->size());

@@ -9,9 +9,7 @@
 // at the record's column offsets (the first incidence stores instead: an
 // element's columns are distinct slots, so no slot is touched twice); the
 // warp sums the copies in copy order and writes the group's slot range with
-// coalesced stores.  No atomics: bitwise reproducible.  Optionally the same
-// walk sums a per-incidence vector re (E * row_local, e.g. element residual
-// entries) into residual[row], the P parts combined in part order.
+// coalesced stores.  No atomics: bitwise reproducible.
 #pragma once
 
 #include <algorithm>
@@ -31,7 +29,6 @@ template <int N, int SLOTS, int P>
 __device__ __forceinline__ void rows_ke_warp(int2 grp, const int32_t *__restrict__ indptr,
                                              const int32_t *__restrict__ inc_ptr, const int4 *__restrict__ rec,
                                              const double *__restrict__ Ke, double *__restrict__ values,
-                                             const double *__restrict__ re, double *__restrict__ residual,
                                              double *acc) {
     static_assert(N % 2 == 0 && N <= 12, "rows are loaded as 16-byte pairs, at most 12 columns");
     static_assert(P == 1 || P == 2, "one or two accumulator copies");
@@ -43,7 +40,6 @@ __device__ __forceinline__ void rows_ke_warp(int2 grp, const int32_t *__restrict
     const int ridx = lane / P, part = lane - (lane / P) * P;
     const int32_t r = grp.x + ridx;
     const bool live = ridx < 32 / P && r < grp.y;
-    double rsum = 0.0;
     if (live) {
         const int base = indptr[r] - s0 + part * nslots;
         const int32_t it1 = inc_ptr[r + 1];
@@ -68,7 +64,6 @@ __device__ __forceinline__ void rows_ke_warp(int2 grp, const int32_t *__restrict
                     for (int q = 0; q < N / 2; ++q) nxt[q] = __ldg(src + q);
                 }
                 const int4 rcnn = it + 2 * P < it1 ? rec[it + 2 * P] : make_int4(0, 0, 0, 0);
-                if (re) rsum += __ldg(re + rc.x);
                 const unsigned ow[3] = {(unsigned)rc.y, (unsigned)rc.z, (unsigned)rc.w};
                 int off[N];
 #pragma unroll
@@ -100,10 +95,6 @@ __device__ __forceinline__ void rows_ke_warp(int2 grp, const int32_t *__restrict
             }
         }
     }
-    if (re) {  // uniform across the warp: every lane takes part in the shuffle
-        if constexpr (P == 2) rsum += __shfl_down_sync(0xffffffffu, rsum, 1);
-        if (live && part == 0) residual[r] = rsum;
-    }
     __syncwarp();
     for (int j = lane; j < nslots; j += 32) {
         double v = acc[j];
@@ -118,20 +109,18 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_rows_ke(int n_groups, const 
                                                            const int32_t *__restrict__ indptr,
                                                            const int32_t *__restrict__ inc_ptr,
                                                            const int4 *__restrict__ rec, const double *__restrict__ Ke,
-                                                           double *__restrict__ values, const double *__restrict__ re,
-                                                           double *__restrict__ residual) {
+                                                           double *__restrict__ values) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5;
     const int gi = blockIdx.x * kRowWarps + warp;
     if (gi >= n_groups) return;
     double *acc = reinterpret_cast<double *>(smem + (size_t)warp * SLOTS * 8);
-    rows_ke_warp<N, SLOTS, P>(groups[gi], indptr, inc_ptr, rec, Ke, values, re, residual, acc);
+    rows_ke_warp<N, SLOTS, P>(groups[gi], indptr, inc_ptr, rec, Ke, values, acc);
 }
 
 template <int N, int SLOTS, int P>
 inline void launch_ke_class(int n_groups, const int2 *groups, const skg_pattern *pat, const double *Ke,
-                            double *values, cudaStream_t s, const double *re = nullptr,
-                            double *residual = nullptr) {
+                            double *values, cudaStream_t s) {
     if (n_groups == 0) return;
     const size_t smem = (size_t)kRowWarps * SLOTS * 8;
     if (smem > 48 * 1024)
@@ -139,8 +128,7 @@ inline void launch_ke_class(int n_groups, const int2 *groups, const skg_pattern 
                                       (int)smem));
     const unsigned grid = (unsigned)((n_groups + kRowWarps - 1) / kRowWarps);
     k_rows_ke<N, SLOTS, P><<<grid, kRowWarps * 32, smem, s>>>(n_groups, groups, pat->indptr.get(),
-                                                              pat->inc_ptr.get(), pat->rec.get(), Ke, values, re,
-                                                              residual);
+                                                              pat->inc_ptr.get(), pat->rec.get(), Ke, values);
     SKG_LAUNCH_CHECK("rows_ke");
 }
 
@@ -159,9 +147,9 @@ inline GroupSet chunk_groups(const skg_pattern *pat, int c) {
 // row groups (pat->max_row_len > 0, square N x N element blocks).
 template <int N>
 inline void add_element_rows(const skg_pattern *pat, const double *Ke, double *values, cudaStream_t s,
-                             const GroupSet &gs, const double *re = nullptr, double *residual = nullptr) {
-    launch_ke_class<N, kGroupSlotsSmall, 1>(gs.n_small, gs.small, pat, Ke, values, s, re, residual);
-    launch_ke_class<N, kGroupSlotsLarge, 2>(gs.n_large, gs.large, pat, Ke, values, s, re, residual);
+                             const GroupSet &gs) {
+    launch_ke_class<N, kGroupSlotsSmall, 1>(gs.n_small, gs.small, pat, Ke, values, s);
+    launch_ke_class<N, kGroupSlotsLarge, 2>(gs.n_large, gs.large, pat, Ke, values, s);
 }
 
 // Per-device non-blocking side streams of the assembly passes.
@@ -214,66 +202,36 @@ inline void add_element_rows(const skg_pattern *pat, const double *Ke, double *v
             [&](const GroupSet &gs, cudaStream_t st) { add_element_rows<N>(pat, Ke, values, st, gs); });
 }
 
-// Element pass and row pass of a pattern with row groups; elem(e0, e1)
-// launches the element pass over elements [e0, e1) on s, rows(groups, st)
-// the row pass of a group set on stream st.  The values optionally go to
-// the page-locked host array h_values as well.
+// Row pass of a pattern with row groups over element data that the work queued
+// on s computes: rows(groups, st) launches it for a group set on stream st.  The
+// values optionally go to the page-locked host array h_values as well.
 //
 // Device output, or a host output of fewer than kHostChunkMinNnz values
 // (where the chunks' launches and events would cost more than the overlap
-// gains): elem(0, ne), the row pass of all groups on s, then one copy.
-// Host output: the row chunks are taken in the order in which their elements
-// are complete (hc_ready).  The element pass runs on s in steps of at least
-// ne / kHostChunks elements, so launches stay large; each chunk's row pass
-// runs on the rows side stream once the element steps it needs are done,
-// overlapping the following element steps, and its slot range is then copied
-// to h_values on the copy stream.  Every group lies inside one chunk, so each
-// copied range is complete.  d_rowvec / h_rowvec (optional): a per-row vector
-// the row pass also writes (a residual), copied with each chunk's rows.  At
-// the end s waits for the copies, which waited for every row pass.
-template <class FE, class FR>
-void run_passes(const skg_pattern *pat, int64_t ne, double *d_values, double *h_values, cudaStream_t s, FE &&elem,
-                FR &&rows, const double *d_rowvec = nullptr, double *h_rowvec = nullptr) {
+// gains): the rows of all groups on s, then one copy.  Host output: each row
+// chunk on the rows side stream, its slot range then copied to h_values on the
+// copy stream.  Every group lies inside one chunk, so each copied range is
+// complete.  At the end s waits for the copies, which waited for every row pass.
+template <class FR>
+void run_row_pass(const skg_pattern *pat, double *d_values, double *h_values, cudaStream_t s, FR &&rows) {
     EventSet ev;
     if (!h_values || pat->nnz < kHostChunkMinNnz) {
-        if (ne) elem((int64_t)0, ne);
         rows_on(all_groups(pat), s, ev, rows);
         if (h_values && pat->nnz)
             SKG_CUDA(cudaMemcpyAsync(h_values, d_values, (size_t)pat->nnz * sizeof(double), cudaMemcpyDeviceToHost, s));
-        if (h_values && d_rowvec && h_rowvec && pat->n_rows)
-            SKG_CUDA(cudaMemcpyAsync(h_rowvec, d_rowvec, (size_t)pat->n_rows * sizeof(double), cudaMemcpyDeviceToHost,
-                                     s));
         return;
     }
-    const int n_chunks = (int)pat->hc_ready.size();
-    std::vector<int> order(n_chunks);
-    for (int c = 0; c < n_chunks; ++c) order[c] = c;
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return pat->hc_ready[a] < pat->hc_ready[b]; });
-    const int64_t step = std::max<int64_t>(1, ne / kHostChunks);
     cudaStream_t rs = side_stream(Side::rows), cs = side_stream(Side::copy);
     try {
-        ev.order(s, rs);  // inputs written earlier on s
-        int64_t done = 0;
-        for (int c : order) {
-            const int64_t need = std::min(ne, pat->hc_ready[c]);
-            if (need > done) {
-                const int64_t to = std::min(ne, std::max(need, done + step));
-                elem(done, to);
-                done = to;
-                ev.order(s, rs);
-            }
+        ev.order(s, rs);
+        for (int c = 0; c + 1 < (int)pat->hc_slot.size(); ++c) {
             rows_on(chunk_groups(pat, c), rs, ev, rows);
             ev.order(rs, cs);
             const int64_t s0 = pat->hc_slot[c], n = pat->hc_slot[c + 1] - s0;
             if (n)
                 SKG_CUDA(cudaMemcpyAsync(h_values + s0, d_values + s0, (size_t)n * sizeof(double),
                                          cudaMemcpyDeviceToHost, cs));
-            const int64_t r0 = pat->hc_row[c], nr = pat->hc_row[c + 1] - r0;
-            if (d_rowvec && h_rowvec && nr)
-                SKG_CUDA(cudaMemcpyAsync(h_rowvec + r0, d_rowvec + r0, (size_t)nr * sizeof(double),
-                                         cudaMemcpyDeviceToHost, cs));
         }
-        if (done < ne) elem(done, ne);  // elements no row references
         ev.order(rs, cs);
         ev.order(cs, s);
     } catch (...) {
@@ -287,12 +245,6 @@ void run_passes(const skg_pattern *pat, int64_t ne, double *d_values, double *h_
             }
         throw;
     }
-}
-
-// Row pass alone (element data already computed), as run_passes.
-template <class FR>
-void run_row_pass(const skg_pattern *pat, double *d_values, double *h_values, cudaStream_t s, FR &&rows) {
-    run_passes(pat, 0, d_values, h_values, s, [](int64_t, int64_t) {}, rows);
 }
 
 }  // namespace skg

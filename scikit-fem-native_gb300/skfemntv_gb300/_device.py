@@ -57,7 +57,10 @@ _TORCH_DTYPES = {
 
 def to_device(a, dtype):
     """Copy a host array to a new contiguous device tensor of ``dtype``."""
-    return host_tensor(np.asarray(a, dtype=dtype)).to(device(), non_blocking=False)
+    a = np.asarray(a, dtype=dtype)
+    if not a.flags.writeable and a.nbytes < 1 << 16:
+        a = a.copy()  # cheaper than viewing a read-only array
+    return host_tensor(a).to(device(), non_blocking=False)
 
 
 def empty(shape, dtype):
@@ -106,9 +109,12 @@ def host_tensor(a):
     import warnings
 
     t = require_cuda()
+    a = np.ascontiguousarray(a)
+    if a.flags.writeable:
+        return t.from_numpy(a)
     with warnings.catch_warnings():
         warnings.simplefilter("ignore")
-        return t.from_numpy(np.ascontiguousarray(a))
+        return t.from_numpy(a)
 
 
 def host_copy(a):

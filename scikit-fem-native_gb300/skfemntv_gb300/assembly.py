@@ -734,14 +734,15 @@ class NativeLinearForm:
         transposition on the host), and the kernel reads it by strides."""
         if c is None:
             return None, (0,) * ndim
-        c = np.broadcast_to(c, (self._shape if ndim == 3 else self._gradient_shape))
+        if c.ndim != ndim:
+            c = np.broadcast_to(c, (self._shape if ndim == 3 else self._gradient_shape))
         c = c[tuple(slice(1) if st == 0 else slice(None) for st in c.strides)]  # broadcast axes once
         order = sorted(range(ndim), key=lambda k: -abs(c.strides[k]))
         packed = np.ascontiguousarray(c.transpose(order))
         strides = [0] * ndim
         for k, axis in enumerate(order):
             strides[axis] = packed.strides[k] // 8 if packed.shape[k] > 1 else 0
-        return dev.host_tensor(packed).to(dev.device()), tuple(strides)
+        return dev.to_device(packed, np.float64), tuple(strides)
 
     def assemble(self, *, value=None, gradient=None, num_threads=0):
         start = time.perf_counter()
