@@ -14,7 +14,7 @@
 // (skg_pairs.cuh) write both places.  No point data is read or tabulated.
 //
 // Bound by the FP64 pipe: about 230 FP64 instructions per vector P1 element,
-// 980 to 1,870 per vector P2 element (142 terms of 9 products and the 10 blocks
+// 1,160 to 1,870 per vector P2 element (142 terms of 9 products and the 10 blocks
 // H_kl; fewer for exact rules and without a value coefficient).
 #include <algorithm>
 #include <cmath>
@@ -179,7 +179,7 @@ __host__ __device__ constexpr int exact_term(int a, int k, int b, int l) {
 // table, or for a rule exact on quadratics (EXACT) as small multiples of H / -30
 // (of -4 times that between edges): 1 to 3 operations per entry instead of 1 to
 // 4, and none for the blocks between vertices.  Bound by the FP64 pipe: about
-// 1870 instructions per element from the table with the mass term, 980 EXACT
+// 1870 instructions per element from the table with the mass term, 1160 EXACT
 // without (MASS: there is a value coefficient); 19x17x18 cells 110 -> 80 us.
 template <bool EXACT, bool MASS>
 __global__ void __launch_bounds__(kFormBlock, 4) k_form_p2v(int64_t ne, int64_t e_begin, int64_t e_end,

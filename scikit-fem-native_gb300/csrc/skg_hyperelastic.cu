@@ -186,15 +186,14 @@ __device__ __forceinline__ double closure_value(df64 v) {
 // double-float in element order.  The elements that the plain law served
 // (flags, read when the call's count `fallbacks` is set) have the low parts of
 // their FP64 entries at the same positions of `low`.  Bound by the blocks'
-// reads and the values' writes; nine threads per pair as in k_pair_sum3 (whole
-// batches instead of predicated ones: 174 us, against 144 at 48^3).
+// reads and the values' writes; nine threads per pair as in k_pair_sum3.  The
+// two cases are walked apart: with the flags' test between them the loads of a
+// batch wait for one another (48^3: 144 and 174 us, 116 apart).
 __global__ void __launch_bounds__(kPairBlock3) k_closure_sum3(int s0, PairArrays p, const float *__restrict__ K,
                                                               const float *__restrict__ low,
                                                               const unsigned char *__restrict__ flags, uint32_t stride,
                                                               const unsigned long long *__restrict__ fallbacks,
                                                               double *__restrict__ values) {
-    constexpr int kAhead = 4;
-    const bool any = *fallbacks != 0;
     const int s = s0 + blockIdx.x;
     const int l = threadIdx.x / 9, en = threadIdx.x - l * 9, i = en / 3, k = en - i * 3;
     const int turned = k * 3 + i;
@@ -202,24 +201,31 @@ __global__ void __launch_bounds__(kPairBlock3) k_closure_sum3(int s0, PairArrays
     const uint4 to = p.slots3[(int64_t)s * 32 + l];
     const uint32_t *cs = p.codes + (int64_t)k0 * 32 + l;
     df64 sum = pair_zero<df64>();
-    for (int f = 0; f < n; f += kAhead, cs += 32 * kAhead) {
-        uint32_t c[kAhead];
-        df64 v[kAhead];
+    const auto batch = [&](auto count, auto any) {
+        constexpr int N = decltype(count)::value;
+        uint32_t c[N];
+        df64 v[N];
 #pragma unroll
-        for (int j = 0; j < kAhead; ++j) c[j] = f + j < n ? __ldg(cs + 32 * j) : kPairNone;
+        for (int j = 0; j < N; ++j) c[j] = __ldg(cs + 32 * j);
 #pragma unroll
-        for (int j = 0; j < kAhead; ++j) {
+        for (int j = 0; j < N; ++j) {
             v[j] = pair_zero<df64>();
-            if (c[j] == kPairNone) continue;
-            const uint32_t b = c[j] & ~kPairTurned;
-            const int64_t pos = (int64_t)b * 9 + (c[j] & kPairTurned ? turned : en);
-            v[j].hi = __ldg(K + pos);
-            if (any && flags[b % stride]) v[j].lo = __ldg(low + pos);
+            const int64_t pos = (int64_t)(c[j] & ~kPairTurned) * 9 + (c[j] & kPairTurned ? turned : en);
+            if (c[j] != kPairNone) v[j].hi = __ldg(K + pos);
+            if (decltype(any)::value && c[j] != kPairNone && flags[(c[j] & ~kPairTurned) % stride])
+                v[j].lo = __ldg(low + pos);
         }
 #pragma unroll
-        for (int j = 0; j < kAhead; ++j)
-            if (f + j < n) pair_add(sum, v[j]);
-    }
+        for (int j = 0; j < N; ++j) pair_add(sum, v[j]);
+        cs += 32 * N;
+    };
+    const auto walk = [&](auto any) {
+        for (int f = n >> 2; f > 0; --f) batch(std::integral_constant<int, 4>{}, any);
+        if (n & 2) batch(std::integral_constant<int, 2>{}, any);
+        if (n & 1) batch(std::integral_constant<int, 1>{}, any);
+    };
+    if (*fallbacks == 0) walk(std::false_type{});
+    else walk(std::true_type{});
     if (to.x == kPairNone) return;
     const double r = closure_value(sum);
     values[to.x + i * to.y + k] = r;

@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(kEvalBlock) k_nh_surrogate_element(
 // Hessian sums are exchanged through shared memory.  The products run behind
 // the elementwise work: a2 behind S1, B behind the second layer, u1 behind the
 // Hessian's second term and the next tile's first layer.
-// 48^3 x 6 elements: 351 us -> 248 us.
+// 48^3 x 6 elements: 351 us -> 229 us.
 constexpr int kTcRows = 128;
 constexpr int kTcThreads = 2 * kTcRows;
 constexpr int kHalf = H / 2;
@@ -777,8 +777,8 @@ __device__ __forceinline__ void put_operand(uint32_t taddr, const float v[16]) {
     float hi[16], lo[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
-        hi[k] = tc::to_tf32(v[k]);
-        lo[k] = tc::to_tf32(v[k] - hi[k]);
+        hi[k] = tc::round_tf32(v[k]);
+        lo[k] = tc::round_tf32(v[k] - hi[k]);
     }
     tc::tmem_st16(taddr, hi);
     tc::tmem_st16(taddr + H, lo);
@@ -1062,7 +1062,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_nh_surrogate_tc(int64_t e_beg
     if (warp == 0) tc::tmem_dealloc(tmem, kTcCols);
 }
 
-// The surrogate element pass runs in three kernels (48^3: 49, 248 and 79 us): k_nh_surrogate_prep
+// The surrogate element pass runs in three kernels (48^3: 49, 229 and 79 us): k_nh_surrogate_prep
 // (thread per element: FP32 geometry, deformation gradient, invariants, the
 // network input and whether the network may serve the element), the
 // tensor-core network k_nh_surrogate_tc (feature gradient and Hessian), and

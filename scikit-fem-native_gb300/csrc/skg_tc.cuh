@@ -47,6 +47,13 @@ __device__ __forceinline__ float to_tf32(float x) {
     return __uint_as_float(r);
 }
 
+// The same rounding (to nearest, ties away) of a finite value by integer
+// instructions, which the conversion's lower rate does not limit (the closure's
+// network 247 -> 229 us at 48^3).
+__device__ __forceinline__ float round_tf32(float x) {
+    return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+}
+
 // Tensor-memory allocation (one full warp), result written to *slot.
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)),
