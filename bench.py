@@ -271,14 +271,14 @@ def measured_peak():
 # dram__bytes_write.sum of one launch at 48^3, scaled to 64^3 by the element
 # count) of each FP64 pass of the headline workload.
 FP64_PROFILE = {
-    "source": "ncu --metrics ... --clock-control none on python bench.py --cells 32 (instructions) / --cells 48 "
-              "(DRAM) --steps 2 --warmup 3 --no-cpu-baseline --modes fp64, GB300",
-    "commit": "a327ee2",
-    "ops_per_element": {"k_elem_ke_fp64_exact": 163.0, "k_rows_ke": 95.3},
-    "dram_bytes_64": {"k_elem_ke_fp64_exact": 1262200000.0, "k_rows_ke": 2229800000.0},
+    "source": "ncu --metrics ... --clock-control none on one assembly at 32^3 (instructions) / 48^3 (DRAM), "
+              "profiles/pair_passes_32.md, GB300",
+    "commit": "fb2a138",
+    "ops_per_element": {"k_elem_packed": 166.0, "k_pair_sum": 42.0},
+    "dram_bytes_64": {"k_elem_packed": 693509233.8, "k_pair_sum": 1790956278.5},
 }
-# The plain neo-Hookean call: element matrices k_nh_ke + row pass k_rows_ke<12>.
-NH_FP64_OPS_PER_ELEMENT = 535.1 + 180.0
+# The plain neo-Hookean call: element blocks k_nh_packed, pair sums k_pair_sum3, residual gather.
+NH_FP64_OPS_PER_ELEMENT = 352.0 + 81.3 + 12.0
 
 
 def fp64_roof(call, passes, elements):
@@ -386,7 +386,7 @@ def run_gpu(args, rank, world):
     value = head["value"]
 
     # ---- e2e (native FP64) through the assembler's host API: A from host memory in,
-    # the CSR values out into the host matrix (chunked copies overlapping the row pass)
+    # the CSR values out into the host matrix (chunked copies overlapping the pair sums)
     for _ in range(2):
         form.assemble(A_pub, copy=False)
     barrier()
@@ -402,14 +402,13 @@ def run_gpu(args, rank, world):
     npts_vertex = (args.cells + 1) ** 3
     # compulsory bytes, each counted once: vertex coordinates, 10 int32 DOF
     # ids per element (4 vertex ids read by the element pass, 6 edge ids
-    # charged to the row pass), A (9 float64 per element), the CSR values
+    # charged to the sums), A (9 float64 per element), the CSR values
     bytes_elem = 24 * npts_vertex + 16 * E + 72 * E
     bytes_rows = 24 * E + 8 * nnz
     head_mode = args.modes[0]
     # the workload's 4-point rule integrates quadratics exactly: the integer-factor element kernel runs
-    names = {"fp64": ("k_elem_ke_fp64_exact", "k_rows_ke"), "fp64_emulated": ("k_elem_ke_df64_packed", "k_rows_ke_df"),
-             "split_fp32": ("k_elem_ke_split", "k_rows_ke_f32")}[head_mode]
-    passes = [q for q in [(names[0], "element", bytes_elem, t_el), (names[1], "row", bytes_rows, t_rows)] if q[3] > 0]
+    names = ("k_elem_packed" if head_mode == "fp64" else "k_elem_packed_df", "k_pair_sum")
+    passes = [q for q in [(names[0], "element", bytes_elem, t_el), (names[1], "sums", bytes_rows, t_rows)] if q[3] > 0]
     dominant = max(passes, key=lambda q: q[3])
     achieved = dominant[2] / (dominant[3] * 1e-3) / 1e9
     traffic = (FP64_PROFILE["dram_bytes_64"].get(dominant[0])
@@ -429,15 +428,15 @@ def run_gpu(args, rank, world):
         "roofline": {"bound": "hbm", "kernel": dominant[0], "achieved": achieved, "peak": peak,
                      "peak_kind": f"{peak_kind} hbm_gbs", "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "algorithmic_bytes_per_launch": dominant[2],
-                     "limiter": ("FP64 pipe in the element pass; load latency and the FP64 pipe in the row pass"
-                                 if head_mode == "fp64" else "load latency of the row pass"),
+                     "limiter": ("FP64 pipe in the element pass; load latency and L2 in the pair sums"
+                                 if head_mode == "fp64" else "load latency and L2 in the pair sums"),
                      "passes": {q[0]: {"ms": q[3], "algorithmic_bytes": q[2],
                                        "achieved_gbs": q[2] / (q[3] * 1e-3) / 1e9} for q in passes},
                      "whole_assembly_bytes": bytes_elem + bytes_rows,
                      "whole_assembly_hbm_frac": (bytes_elem + bytes_rows) / ((t_el + t_rows) * 1e-3) / 1e9 / peak,
                      "fp64_pipe": fp64_roof(call, passes, E) if head_mode == "fp64" else None},
         "precision_variants": results,
-        "gpu_launches": 3 * args.steps,  # element pass + one row pass per group class
+        "gpu_launches": 2 * args.steps,  # element pass + pair sums (FP64; the FP32-pair modes are not counted)
         "clocks": head["clocks"],
     }
     if rank == 0 and not args.no_cpu_baseline:
@@ -608,7 +607,7 @@ def wl_p1_laplace(args, world, timed, wall):
         roofline=_roofline(alg, head["ms_per_step"]), precision_variants=variants,
         cuda_graph={"value": world * nnz / (ms_g * 1e-3), "ms_per_step": ms_g, "max_rel_err_vs_fp64": graph_err,
                     "clocks": clk_g, "note": "NativeBilinearForm.capture_gradient, replay() per step"},
-        gpu_launches=3 * args.steps)
+        gpu_launches=2 * args.steps)  # element pass + pair sums
 
 
 def wl_n1_maxwell(args, world, timed, wall):
@@ -661,7 +660,7 @@ def wl_n1_maxwell(args, world, timed, wall):
         precision_variants={"fp64": {"value": world * nnz / (ms * 1e-3), "ms_per_step": ms},
                             "split_fp32": {"value": world * nnz / (ms_s * 1e-3), "ms_per_step": ms_s,
                                            "max_rel_err_vs_fp64": err_s, "clocks": clk_s}},
-        gpu_launches=3 * args.steps)
+        gpu_launches=2 * args.steps)  # element pass + pair sums
 
 
 def wl_p1_adjoint(args, world, timed, wall):
@@ -804,7 +803,7 @@ def wl_nh(args, world, timed, wall):
                          "training_seconds": t_train, "training_history": sur.history[-2:],
                          "roofline": _roofline(alg, ms_sur), "clocks": clk_s,
                          "integer_wavevectors": int3},
-        gpu_launches=3 * args.steps)
+        gpu_launches=3 * args.steps)  # element pass, pair sums, residual gather
 
 
 def wl_vp1_elasticity(args, world, timed, wall):
@@ -850,7 +849,7 @@ def wl_vp1_elasticity(args, world, timed, wall):
                              "note": "same form, coefficients as device (E, Q) arrays: tabulated kernels"},
         e2e={"value": world * nnz / e2e_s, "unit": "nnz/s", "h2d_bytes_per_step": 0,
              "d2h_bytes_per_step": 8 * nnz, "ms_per_step": 1e3 * e2e_s},
-        roofline=_roofline(alg, ms), gpu_launches=3 * args.steps)  # element pass + one row pass per group class
+        roofline=_roofline(alg, ms), gpu_launches=2 * args.steps)  # element pass + pair sums
 
 
 AUX_WORKLOADS = {"p1_laplace": wl_p1_laplace, "n1_maxwell": wl_n1_maxwell, "p1_adjoint": wl_p1_adjoint,

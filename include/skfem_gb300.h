@@ -224,7 +224,7 @@ int skg_h1_assemble_affine(const skg_pattern *pattern, const double *d_p,
                            double *d_values, void *stream);
 
 /* Same as skg_h1_assemble_affine, and writes the duration of its two
- * kernels (element pass, row pass) in milliseconds to h_kernel_ms[0..1],
+ * kernels (element pass, sums) in milliseconds to h_kernel_ms[0..1],
  * measured with CUDA events on `stream`.  Synchronous. */
 int skg_h1_assemble_affine_profiled(const skg_pattern *pattern, const double *d_p,
                                     int64_t npts, const int32_t *d_t, int32_t nodes,
@@ -233,8 +233,8 @@ int skg_h1_assemble_affine_profiled(const skg_pattern *pattern, const double *d_
                                     const double *d_coef, int32_t precision,
                                     double *d_values, float *h_kernel_ms, void *stream);
 /* As skg_h1_assemble_affine, the values also delivered to page-locked host
- * memory h_values (nnz): the row pass runs in row chunks and each chunk's
- * values are copied while the next chunk is assembled (d_values is the
+ * memory h_values (nnz): the sums run in steps and each chunk of rows is
+ * copied while the next ones are assembled (d_values is the
  * device staging buffer).  Stream-ordered; h_values is complete when the
  * stream is.  No counterpart in the reference (host-only). */
 int skg_h1_assemble_affine_host(const skg_pattern *pattern, const double *d_p,
@@ -345,9 +345,9 @@ int skg_n1_assemble(const skg_pattern *pattern, const double *d_p, int64_t npts,
 /* skg_n1_assemble with the values also written to the page-locked host
  * array h_values (nnz), for callers that want the host CSR matrix
  * (TetN1Assembler.assemble_maxwell returns one, hcurl_assembler.py:160-215).
- * d_values (nnz, device) is the staging array.  On a row-grouped pattern the
- * element and row passes run over row chunks and each chunk's values are
- * copied while later chunks run; the stream has the host values once it
+ * d_values (nnz, device) is the staging array.  The passes of a large
+ * matrix run in steps and each chunk of rows is
+ * copied while later steps run; the stream has the host values once it
  * reaches the end of the call's work. */
 int skg_n1_assemble_host(const skg_pattern *pattern, const double *d_p, int64_t npts,
                          const int32_t *d_t, const int32_t *d_elem_edges,
@@ -497,9 +497,9 @@ int skg_nh_assemble(const skg_pattern *pattern, const double *d_p, int64_t npts,
                     double *d_values, void *stream);
 /* skg_nh_assemble with the residual and tangent values also written to the
  * page-locked host arrays h_residual (N) and h_values (nnz); d_residual and
- * d_values are the device staging arrays (both required).  On a row-grouped
- * pattern the element and row passes run over row chunks and each chunk's
- * rows are copied while later chunks run. */
+ * d_values are the device staging arrays (both required).  The passes of a
+ * large matrix run in steps and each chunk of rows is copied while later steps
+ * run. */
 int skg_nh_assemble_host(const skg_pattern *pattern, const double *d_p, int64_t npts,
                          const int32_t *d_t, int64_t n_elements, const double *d_u,
                          double mu, double lmbda, double wsum, double *d_residual,
