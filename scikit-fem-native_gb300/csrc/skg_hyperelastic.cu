@@ -38,16 +38,26 @@ constexpr int kNhBlock = 64;
 // Element tangent (packed 3 x 3 blocks of the node pairs a <= b, see
 // skg_pairs.cuh) and residual (E, 12) of the plain law, thread per element.
 //
-// The kernel is bound by the FP64 pipe, so the law is evaluated in the form
-// with the fewest FP64 instructions (535 -> about 360 per element; 64^3: 1543 ->
-// 922 us, 1001 at the 80 registers that the compiler takes by itself):
+// The kernel is bound by the FP64 pipe, so the law is evaluated in a form with
+// few FP64 instructions that keeps the stress of small strains:
 // * h_a = F^-T grad lambda_a is the gradient of lambda_a on the displaced
-//   tetrahedron (edges j_k = J_k + u_k - u_0): its cofactors over its
-//   determinant, without F, its inverse or the products with it; det F is the
-//   ratio of the two determinants.
-// * With G_ab = mu V g_a . g_b (from the cofactors' products, row 0 from the
-//   zero sum of the g_a) the residual is r_a = V P g_a = sum_k j_k G_ka -
-//   (mu - lambda ln J) V h_a, since F = sum_k j_k g_k^T; r_0 from the zero sum.
+//   tetrahedron (edges j_k = e_k + d_k, d_k = u_k - u_0): its cofactors over its
+//   determinant, without F, its inverse or the products with it.
+// * det F - 1 is made of terms with one displacement difference each, exchanging
+//   one edge at a time: (d_1 . j_2 x j_3 + d_2 . j_3 x e_1 + d_3 . e_1 x e_2) / det,
+//   and ln J = log1p of it (of the determinants' ratio itself where it is far
+//   from 1).
+// * With H = grad u = sum_k d_k g_k^T: F g_a = g_a + H g_a and g_a - h_a = H^T h_a
+//   (g_a = F^T h_a), so the residual is r_a = V P g_a = mu V (H g_a + H^T h_a) +
+//   lambda ln J V h_a = sum_k (d_k G_ka + mu V g_k (d_k . h_a)) + lambda ln J V h_a
+//   with G_ab = mu V g_a . g_b; r_0 from the zero sum.  Every term carries a
+//   displacement difference: the residual is zero without displacement, and its
+//   error is relative to the strain (formed as F - F^-T, or from the displaced
+//   edges whole, it is a difference of numbers of size one: at strain 1e-6 on
+//   elements of aspect ratio 1000 5e-9 or 2e-6 of the largest entry instead of
+//   4e-11, and 1e-11 instead of zero at the undeformed state).  Residual and
+//   tangent at 64^3, the whole call: 1476 us; 1290 us by the displaced edges
+//   whole, 2259 us by the stress and tangent tensors.
 // * With p_a = (mu - lambda ln J) V h_a, q_a = lambda V h_a, t_a = p_a + q_a
 //   the entries are p_a,k h_b,i + q_a,i h_b,k (i != k), t_a,i h_b,i + G_ab
 //   (i = k), and t_a,k h_a,i in the diagonal blocks (symmetric).
@@ -73,22 +83,37 @@ __global__ void __launch_bounds__(kNhBlock, 8) k_nh_packed(int64_t ne, int64_t e
         ok = ok && v[k] >= 0 && v[k] < npts;
     }
     if (!ok) v[0] = v[1] = v[2] = v[3] = 0;
-    double J[9], j[9];  // [coordinate * 3 + edge]: edges of the element, and displaced
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const double x0 = p[i * npts + v[0]], u0 = u[dofs[e * 12 + i]];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            J[i * 3 + k] = F.sub(p[i * npts + v[k + 1]], x0);
-            j[i * 3 + k] = F.add(J[i * 3 + k], F.sub(u[dofs[e * 12 + 3 * (k + 1) + i]], u0));
-        }
-    }
+    double d[9];              // [coordinate * 3 + edge]: displacement differences
     double c[4][3], h[4][3];  // rows 1..3 of the adjugates: the determinant times grad lambda_k
-    const double det = F.adjugate(J, c);
+    double det, detj, grown;  // grown: det (det F - 1)
+    {
+        double J[9], j[9];  // edges of the element, and displaced
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double x0 = p[i * npts + v[0]], u0 = u[dofs[e * 12 + i]];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                J[i * 3 + k] = F.sub(p[i * npts + v[k + 1]], x0);
+                d[i * 3 + k] = F.sub(u[dofs[e * 12 + 3 * (k + 1) + i]], u0);
+                j[i * 3 + k] = F.add(J[i * 3 + k], d[i * 3 + k]);
+            }
+        }
+        det = F.adjugate(J, c);
+        detj = F.adjugate(j, h);
+        // row 2 of the adjugate with the first edge as it was and the third displaced
+        const double m[3] = {F.cross(j[5], J[6], J[3], j[8]), F.cross(J[0], j[8], j[2], J[6]),
+                             F.cross(j[2], J[3], J[0], j[5])};
+        grown = F.mul(d[0], h[1][0]);
+        grown = fma(d[3], h[1][1], grown);
+        grown = fma(d[6], h[1][2], grown);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) grown = fma(d[i * 3 + 2], c[3][i], fma(d[i * 3 + 1], m[i], grown));
+    }
     const double id = ok ? 1.0 / det : __longlong_as_double(0x7ff8000000000000LL);
-    const double detj = F.adjugate(j, h);
     const double idj = 1.0 / detj;
-    const double lnJ = log(detj * id);
+    const double rise = grown * id;
+    // far from 1 the ratio of the determinants has the smaller relative error
+    const double lnJ = fabs(rise) < 0.5 ? log1p(rise) : log(detj * id);
     const double V = fabs(det) * wsum;
     const double c2V = (mu - lmbda * lnJ) * V, lamV = lmbda * V, tV = c2V + lamV;
     double G[4][4];
@@ -111,18 +136,28 @@ __global__ void __launch_bounds__(kNhBlock, 8) k_nh_packed(int64_t ne, int64_t e
     }
     if (re) {
         double *st = out.next() + 12 * lane;
+        const double gV = mu * V * id, lnV = lmbda * lnJ * V;
+        double sum[3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            double sum = 0.0;
+        for (int a = 1; a < 4; ++a) {
+            double r[3];
 #pragma unroll
-            for (int a = 1; a < 4; ++a) {
-                const double r = fma(j[i * 3 + 2], G[3][a],
-                                     fma(j[i * 3 + 1], G[2][a], fma(j[i * 3], G[1][a], -F.mul(c2V, h[a][i]))));
-                st[a * 3 + i] = r;
-                sum = a == 1 ? r : F.add(sum, r);
+            for (int i = 0; i < 3; ++i) r[i] = F.mul(lnV, h[a][i]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                // d_k . h_a
+                const double dh = F.mul(gV, fma(d[6 + k], h[a][2], fma(d[3 + k], h[a][1], F.mul(d[k], h[a][0]))));
+#pragma unroll
+                for (int i = 0; i < 3; ++i) r[i] = fma(d[i * 3 + k], G[k + 1][a], fma(c[k + 1][i], dh, r[i]));
             }
-            st[i] = -sum;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                st[a * 3 + i] = r[i];
+                sum[i] = a == 1 ? r[i] : F.add(sum[i], r[i]);
+            }
         }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) st[i] = -sum[i];
         out.store(re + e0 * 12, n, 12);
     }
     if (Ke) {
