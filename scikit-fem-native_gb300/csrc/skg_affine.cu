@@ -1198,15 +1198,13 @@ void affine_assemble_pairs(const skg_pattern *pat, const double *d_p, int64_t np
         return;
     }
     launch_scale_exponent(d_p, 3 * npts, misc.get(), s);
-    // The FP32-pair entries lie in scratch of their own: with a host output
-    // their sums and copies follow the element pass step by step, before the
-    // range flag is final.
+    // The FP32-pair entries lie in the first half or the whole of the FP64
+    // matrices' memory (4 or 8 bytes each): the FP64 passes, if they follow, are
+    // queued behind the last sums that read them.
     const bool split = precision == SKG_SPLIT_FP32;
-    const size_t entry = split ? sizeof(float) : sizeof(float2);
-    DevBuf<unsigned char> Kf((size_t)stride * np * entry, s), lower_f(maybe_lower ? (size_t)stride * np * entry : 0, s);
-    const PackedOut<float2> out_df{reinterpret_cast<float2 *>(Kf.get()), reinterpret_cast<float2 *>(lower_f.get()),
+    const PackedOut<float2> out_df{reinterpret_cast<float2 *>(K.get()), reinterpret_cast<float2 *>(lower.get()),
                                    tile_flags.get(), any, stride};
-    const PackedOut<float> out_f{reinterpret_cast<float *>(Kf.get()), reinterpret_cast<float *>(lower_f.get()),
+    const PackedOut<float> out_f{reinterpret_cast<float *>(K.get()), reinterpret_cast<float *>(lower.get()),
                                  tile_flags.get(), any, stride};
     const PairUnscale unscale{misc.get()};
     run_pair_passes(

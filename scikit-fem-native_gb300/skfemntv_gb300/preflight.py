@@ -256,7 +256,7 @@ def estimate_bilinear_memory(basis, trial_basis=None):
         assumptions=(
             "int32 device DOF maps, CSR offsets and columns; float64 values",
             "CSR nnz is an adjacency-free upper bound, not an exact count",
-            "element matrices are float64 (the FP32-pair precisions write as much or less)",
+            "element matrices are float64 (the FP32-pair precisions use the same memory)",
             "per-point coefficients of every kind are staged (page-locked and device copies)",
             "the CUDA sparse tensor of assemble_torch (int64 offsets and columns) is not counted",
             "Python objects and allocator rounding are excluded",
