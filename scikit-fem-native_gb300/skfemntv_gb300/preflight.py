@@ -23,19 +23,21 @@ csr_bytes_upper_bound
     page-locked host matrix (float64 values, int32 columns, int64 offsets)
     and one returned copy of it.
 scatter_bytes
-    the element matrices one assembly writes and then sums by rows, float64
-    E x Lr x Lc.  They are released after each call into the device's memory
+    the element matrices one assembly writes and then sums, float64 E x Lr x Lc
+    (the packed triangles, with their lower twins for a tensor coefficient,
+    take as much with the geometry below, or less).  They are released after each call into the device's memory
     pool, which keeps them reserved, so they count as persistent.
 coloring_bytes_upper_bound
-    the row-incidence structure that takes the place of the reference's
-    element colouring: the int32 incidence list and offsets, one 16-byte
-    record per incidence and the row groups (at most R, in two orders).
+    the structures that take the place of the reference's element colouring:
+    the int32 incidence list and offsets, one 16-byte record per incidence, the
+    row groups (at most R, in two orders) and the plan of the sums (4 bytes per
+    contribution, padded, and 8 or 16 per pair).
 pattern_temporary_bytes_upper_bound
     device counters and host row lists of the pattern build, and the
     temporaries of the CSR export.
 staging_bytes_upper_bound
-    per call: the per-element geometry of the scalar affine path (16 float64
-    per element) and the page-locked and device copies of per-point
+    per call: the per-element geometry of the scalar affine path without packed
+    triangles (16 float64 per element) and the page-locked and device copies of per-point
     coefficients.  The reference has no such field: its kernels read the
     caller's arrays.
 """
@@ -208,18 +210,41 @@ def _validate_basis(basis, label):
         raise TypeError(f"{label} is not a nodal tetrahedral Basis of this backend")
 
 
-def _pattern_bytes(E, Lr, Lc, rows, nnz):
+_PAIR_WINDOW = 1024  # pairs are padded to whole windows
+
+
+def _pair_plan_bytes(E, Lr, Lc, comp, rows, nnz, square):
+    """(arrays, temporaries) of the plan of the sums: of the node pairs r <= c
+    of a symmetric pattern (``square``) in one of the shapes that are assembled
+    symmetric, else of every CSR entry (not made where rows of fewer than 256
+    columns are summed in groups, but counted).  The positions are padded to the
+    largest count of 32 neighbours in the order of their counts: at most twice
+    as many on the meshes in use."""
+    n = Lr // comp
+    if square and comp in (1, 3) and n in (4, 6, 10):
+        contributions = E * (n * (n + 1) // 2)
+        pairs, nodes = (nnz // comp ** 2 + rows // comp) // 2 + 1, rows // comp
+    else:
+        comp, contributions, pairs, nodes = 1, E * Lr * Lc, nnz, rows
+    lanes = pairs + _PAIR_WINDOW
+    # positions, one word per 32 of them, targets, slices
+    arrays = 2 * contributions * _I32 + contributions // 16 * _I32 + (8 if comp == 1 else 16) * lanes + lanes // 8
+    # row, count and order of every pair, the nodes' pair counts and offsets
+    temporary = 3 * _I32 * lanes + 2 * _I32 * (nodes + 1)
+    return arrays, temporary
+
+
+def _pattern_bytes(E, Lr, Lc, rows, nnz, comp=1, square=True):
     """(DOF-map copies, CSR, row incidence, temporaries) of one pattern and
-    its matrix target, in bytes."""
+    its matrix target, in bytes; ``comp`` components per node, ``square``: rows
+    and columns are the same DOFs."""
     tr, tc = E * Lr, E * Lc
     dof_copies = _I32 * (tr + tc)
     csr = (_I32 * (rows + 1) + (_I32 + _F64) * nnz  # device CSR and values
            + 2 * ((_F64 + _I32) * nnz + _I64 * (rows + 1)))  # page-locked host matrix and one copy
-    incidence = 20 * tr + _I32 * (rows + 1) + 2 * 8 * rows
-    temporary = 128 * (rows + 1) + _I32 * (nnz + tr)
-    if Lr == Lc:  # pair plan: padded positions and targets; pair rows, counts and order while it is built
-        incidence += 2 * _I32 * E * (Lr * (Lr + 1) // 2) + 8 * (nnz // 2 + rows + 1024)
-        temporary += 3 * _I32 * (nnz // 2 + rows + 1024)
+    plan, plan_temporary = _pair_plan_bytes(E, Lr, Lc, comp, rows, nnz, square)
+    incidence = 20 * tr + _I32 * (rows + 1) + 2 * 8 * rows + plan
+    temporary = 128 * (rows + 1) + _I32 * (nnz + tr) + plan_temporary
     return dof_copies, csr, incidence, temporary
 
 
@@ -243,7 +268,7 @@ def estimate_bilinear_memory(basis, trial_basis=None):
     if not same:  # the cross form compares the bases' dx and points on the host
         tabulation += sum(4 * E * Q * _F64 for b in distinct if "x" not in getattr(b, "_tab_host", {}))
     dof_maps = sum(E * b._nodes * b._comp * _I32 for b in distinct if not hasattr(b, "_dofs_dev"))
-    dof_copies, csr, incidence, temporary = _pattern_bytes(E, Lr, Lc, rows, nnz)
+    dof_copies, csr, incidence, temporary = _pattern_bytes(E, Lr, Lc, rows, nnz, basis._comp, same)
     per_point = (9 if basis._comp == 1 else 4) if same else 9 * basis._comp * trial._comp
     geometry = 16 * _F64 * E if same and basis._comp == 1 else 0
     return AssemblyMemoryEstimate(
