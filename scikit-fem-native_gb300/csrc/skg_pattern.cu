@@ -233,8 +233,11 @@ void build_pair_plan(skg_pattern *p, bool square, cudaStream_t s);
 // Incidence records for the warp-per-row assembly kernels; skipped when the
 // pattern is unsuitable (elements wider than 12 columns or rows of 256+
 // columns), in which case assemblies use the per-row global-memory gather.
-// `ip`: indptr on the host.
-void build_records(skg_pattern *p, const std::vector<int32_t> &ip, cudaStream_t s) {
+// `ip`: indptr on the host.  `keep` takes the host arrays whose copies to the
+// device are queued: they have to live until s is waited for (a device that
+// reads pageable memory need not stage it).
+void build_records(skg_pattern *p, const std::vector<int32_t> &ip, std::vector<std::vector<int2>> &keep,
+                   cudaStream_t s) {
     if (p->col_local > 12 || p->n_rows == 0) return;
     int32_t longest = 0;
     for (int64_t r = 0; r < p->n_rows; ++r) longest = std::max(longest, ip[r + 1] - ip[r]);
@@ -272,10 +275,11 @@ void build_records(skg_pattern *p, const std::vector<int32_t> &ip, cudaStream_t 
         all.push_back(make_int2((int)r0, (int)r1));
         r = r1;
     }
-    auto upload = [&](const std::vector<int2> &vec, DevBuf<int2> &dst) {
+    auto upload = [&](std::vector<int2> &&vec, DevBuf<int2> &dst) {
         dst = DevBuf<int2>::owned(vec.size());
-        if (!vec.empty())
-            SKG_CUDA(cudaMemcpyAsync(dst.get(), vec.data(), vec.size() * 8, cudaMemcpyHostToDevice, s));
+        if (vec.empty()) return;
+        keep.push_back(std::move(vec));
+        SKG_CUDA(cudaMemcpyAsync(dst.get(), keep.back().data(), keep.back().size() * 8, cudaMemcpyHostToDevice, s));
     };
     std::vector<int32_t> first;  // per group of `all`
     if ((int)all.size() > kGroupsAtOnce) {
@@ -339,13 +343,13 @@ void build_records(skg_pattern *p, const std::vector<int32_t> &ip, cudaStream_t 
         };
         offsets(hc_small, p->hc_small_off);
         offsets(hc_large, p->hc_large_off);
-        upload(hc_small, p->hc_small);
-        upload(hc_large, p->hc_large);
+        upload(std::move(hc_small), p->hc_small);
+        upload(std::move(hc_large), p->hc_large);
     }
     p->n_groups_small = (int32_t)small.size();
     p->n_groups_large = (int32_t)large.size();
-    upload(small, p->groups_small);
-    upload(large, p->groups_large);
+    upload(std::move(small), p->groups_small);
+    upload(std::move(large), p->groups_large);
     p->max_row_len = longest;
 }
 
@@ -373,6 +377,7 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
                 "pattern too large");
         cudaStream_t s = as_stream(stream);
         auto *p = new skg_pattern();
+        std::vector<std::vector<int2>> keep;
         try {
             p->n_elements = n_elements; p->row_local = row_local; p->col_local = col_local;
             p->n_rows = n_rows; p->n_cols = n_cols;
@@ -436,10 +441,11 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
                                                                  row_local, col_local, n_rows, 1, nullptr, p->indptr.get(),
                                                                  p->indices.get());
             SKG_LAUNCH_CHECK("row_columns_write");
-            build_records(p, ip, s);
+            build_records(p, ip, keep, s);
             build_pair_plan(p, d_row_dofs == d_col_dofs && row_local == col_local && n_rows == n_cols, s);
             SKG_CUDA(cudaStreamSynchronize(s));  // the handle may be used on any stream
         } catch (...) {
+            cudaStreamSynchronize(s);  // copies of host arrays may be queued
             delete p;
             throw;
         }
