@@ -350,14 +350,17 @@ std::vector<double> form_table(int nodes, int nq, const double *X, const double 
     return T;
 }
 
-// True when the rule's table of gradient products is that of exact integration.
+// True when the rule's table of gradient products is that of exact integration,
+// to the rounding of its sums (at most 5e-16 for the rules of up to 343 points that
+// are exact; the entries are at least 1/30).  A rule further off keeps its own
+// table: the results follow the caller's rule.
 bool p2_form_is_exact(const std::vector<double> &T) {
     for (int a = 0; a < 10; ++a)
         for (int b = a; b < 10; ++b)
             for (int u = 0; u < 4; ++u) {
                 if ((u & 2 && a < 4) || (u & 1 && b < 4)) continue;
                 const int k = u & 2 ? hi_of(a) : lo_of(a), l = u & 1 ? hi_of(b) : lo_of(b);
-                if (!(std::fabs(T[tri_index(10, a, b) * 4 + u] + exact_term(a, k, b, l) / 30.0) <= 1e-13)) return false;
+                if (!(std::fabs(T[tri_index(10, a, b) * 4 + u] + exact_term(a, k, b, l) / 30.0) <= 1e-15)) return false;
             }
     return true;
 }
