@@ -406,7 +406,7 @@ void expand_blocks(int64_t ne, int n, const double *K, double *full, cudaStream_
 }
 
 // Plans of a pattern: the pair plan when its row and column DOFs are the same
-// array (`square`) and its shape is one that is assembled symmetric; the whole
+// (`square`) and its shape is one that is assembled symmetric; the whole
 // sums for the shapes that no row group serves.  None when the positions exceed
 // 32 bits (the assemblies then walk the rows).
 void build_pair_plan(skg_pattern *p, bool square, cudaStream_t s) {

@@ -86,6 +86,12 @@ __global__ void k_check_range(const int32_t *v, int64_t n, int64_t hi, int32_t *
     }
 }
 
+__global__ void k_differ(const int32_t *a, const int32_t *b, int64_t n, int32_t *differ) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * blockDim.x)
+        if (a[i] != b[i]) *differ = 1;
+}
+
 __global__ void k_count_rows(const int32_t *row_dofs, int64_t total, int32_t *cnt) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (int64_t)gridDim.x * blockDim.x)
@@ -386,15 +392,26 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
             if (tr) SKG_CUDA(cudaMemcpyAsync(p->row_dofs.get(), d_row_dofs, tr * 4, cudaMemcpyDeviceToDevice, s));
             if (tc) SKG_CUDA(cudaMemcpyAsync(p->col_dofs.get(), d_col_dofs, tc * 4, cudaMemcpyDeviceToDevice, s));
             // range checks (the reference raises "element DOF index is out of bounds")
-            DevBuf<int32_t> err(2, s);
-            SKG_CUDA(cudaMemsetAsync(err.get(), 0, 8, s));
+            DevBuf<int32_t> err(3, s);
+            SKG_CUDA(cudaMemsetAsync(err.get(), 0, 12, s));
             if (tr) k_check_range<<<grid_for(tr, 256), 256, 0, s>>>(p->row_dofs.get(), tr, n_rows, err.get());
             if (tc) k_check_range<<<grid_for(tc, 256), 256, 0, s>>>(p->col_dofs.get(), tc, n_cols, err.get() + 1);
             SKG_LAUNCH_CHECK("check_range");
-            int32_t herr[2];
+            // the rows' and the columns' DOFs are the same: one array, or two of the same
+            // content.  Two arrays of an element matrix that the row groups do not take (30 x
+            // 30) are two bases: their forms need the sums of every entry.
+            bool square = row_local == col_local && n_rows == n_cols;
+            const bool two = square && d_row_dofs != d_col_dofs;
+            if (two) square = row_local <= 12;
+            if (two && square && tr) {
+                k_differ<<<grid_for(tr, 256), 256, 0, s>>>(p->row_dofs.get(), p->col_dofs.get(), tr, err.get() + 2);
+                SKG_LAUNCH_CHECK("differ");
+            }
+            int32_t herr[3];
             SKG_CUDA(cudaMemcpyAsync(herr, err.get(), sizeof(herr), cudaMemcpyDeviceToHost, s));
             SKG_CUDA(cudaStreamSynchronize(s));
             require(!herr[0] && !herr[1], "element DOF index is out of bounds", SKG_ERANGE);
+            if (herr[2]) square = false;
 
             DevBuf<int32_t> cnt(n_rows + 1, s), cursor(n_rows + 1, s);
             SKG_CUDA(cudaMemsetAsync(cnt.get(), 0, (n_rows + 1) * 4, s));
@@ -442,7 +459,7 @@ extern "C" int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_co
                                                                  p->indices.get());
             SKG_LAUNCH_CHECK("row_columns_write");
             build_records(p, ip, keep, s);
-            build_pair_plan(p, d_row_dofs == d_col_dofs && row_local == col_local && n_rows == n_cols, s);
+            build_pair_plan(p, square, s);
             SKG_CUDA(cudaStreamSynchronize(s));  // the handle may be used on any stream
         } catch (...) {
             cudaStreamSynchronize(s);  // copies of host arrays may be queued
