@@ -58,6 +58,7 @@ __host__ __device__ constexpr int end0(int b) {
 __host__ __device__ constexpr int end1(int b) { return b < 4 ? b : (b == 4 ? 1 : b == 5 ? 2 : b == 6 ? 0 : 3); }
 
 constexpr int kLoadBlock = 64;
+constexpr size_t kSharedBytes = 227 * 1024;  // of one block
 
 // Thread per element: its vector (E, NN CC) of f.v + G:grad v, the sums of all
 // entries in registers, one pass over the points.  tab: per point the weight,
@@ -198,9 +199,14 @@ extern "C" int skg_linear_assemble_affine(const skg_pattern *pat, const double *
         const LoadStrides vs{ve, vq, vc, 0}, gs{ge, gq, gc, gd};
         if (ne) {
             const size_t smem = T.size() * sizeof(double);
+            // The limit belongs to the kernel, not to the launch: it is always set to the
+            // same value, or a thread with a smaller rule would lower it between another's
+            // two calls.
+            const size_t limit = kSharedBytes - kLoadBlock * nodes * comp * sizeof(double);
+            require(smem <= limit, "quadrature tables exceed shared memory");
             const auto launch = [&](auto kernel) {
                 if (smem > 16 * 1024)
-                    SKG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                    SKG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
                 kernel<<<grid_for(ne, kLoadBlock), kLoadBlock, smem, s>>>(ne, d_p, npts, d_t, nq, tab, (int)T.size(), d_value, vs,
                                                                d_gradient, gs, le.get());
                 SKG_LAUNCH_CHECK("linear_affine");
