@@ -236,5 +236,6 @@ class Basis:
                 p, t = self.mesh._dev("p"), self.mesh._dev("t").long()
                 i, j = (list(e) for e in zip(*quad.TET_EDGES))
                 off = (p[:, t[4:]] - 0.5 * (p[:, t[i]] + p[:, t[j]])).abs().max()
-                self._affine = not bool(off > 1e-14 * p.abs().max().clamp(min=1.0))
+                scale = p.abs().max()  # not a number when a point that no element uses is not
+                self._affine = not bool(off > 1e-14 * scale.where(scale > 1.0, 1.0))
         return self._affine
