@@ -94,7 +94,12 @@ def per_element(c, E, Q, name):
         b = np.broadcast_to(c, (E, Q))
     except ValueError as error:
         raise ValueError(f"{name} coefficient must broadcast to {(E, Q)}") from error
-    if Q == 1 or b.strides[1] == 0 or np.array_equal(b, b[:, :1] * np.ones((1, Q))):
+    if Q == 1 or b.strides[1] == 0:
+        return np.ascontiguousarray(b[:, 0])
+    # some elements across the mesh first: coefficients that vary over the points
+    # rarely do so in a few elements only
+    if all(np.array_equal(part[:, 1:], np.broadcast_to(part[:, :1], (len(part), Q - 1)))
+           for part in (b[:: max(1, E // 64)], b)):
         return np.ascontiguousarray(b[:, 0])
     return None
 
@@ -339,7 +344,14 @@ class NativeBilinearForm:
         forms = self._affine_forms(value, gradient, symmetric_gradient, divergence)
         if forms is not None:
             self._affine_forms_launch(forms, dev.ptr(self.target.d_values), None)
-            return self.target.d_values
+        else:
+            self._tabulated(value, gradient, symmetric_gradient, divergence)
+        return self.target.d_values
+
+    def _tabulated(self, value, gradient, symmetric_gradient, divergence):
+        """Assembly from the device tabulation with coefficients per point."""
+        b = self.basis
+        E, Q = b._coefficient_shape
         tab = b._device_tabulation()
         coefs = [self._point_coefficient(c, E, Q, n)
                  for c, n in ((value, "value"), (gradient, "gradient"),
@@ -347,7 +359,6 @@ class NativeBilinearForm:
         call("skg_h1_assemble_tabulated", self.pattern.h, dev.ptr(b._dev_dofs()), E, b._nodes, b._comp, Q,
              dev.ptr(tab["shape"]), dev.ptr(tab["grad"]), dev.ptr(tab["dx"]), *(dev.ptr(c) for c in coefs),
              dev.ptr(self.target.d_values), None, dev.stream_ptr())
-        return self.target.d_values
 
     def _affine_forms(self, value, gradient, symmetric_gradient, divergence):
         """The four coefficients as (E,) arrays, 0-d scalars or None when the
@@ -356,6 +367,8 @@ class NativeBilinearForm:
         b = self.basis
         if b._comp not in (1, 3) or not b.is_affine:
             return None
+        if b._comp == 1 and value is None and symmetric_gradient is None and divergence is None:
+            return None  # the diffusion path would have taken it
         E, Q = b._coefficient_shape
         out = []
         for c, name in ((value, "value"), (gradient, "gradient"),
@@ -430,12 +443,13 @@ class NativeBilinearForm:
         if fast is not None:
             self._affine(fast, _precision(precision), self.target.pinned_ptr(), host=True)
             return self.target.finish_direct()
+        if _precision(precision) != SKG_FP64:
+            raise UnsupportedNativeForm("split precision is available on the affine scalar gradient path")
         forms = self._affine_forms(value, gradient, symmetric_gradient, divergence)
-        if forms is not None and _precision(precision) == SKG_FP64:
+        if forms is not None:
             self._affine_forms_launch(forms, dev.ptr(self.target.d_values), self.target.pinned_ptr())
             return self.target.finish_direct()
-        self.assemble_device(value=value, gradient=gradient, symmetric_gradient=symmetric_gradient,
-                             divergence=divergence, precision=precision)
+        self._tabulated(value, gradient, symmetric_gradient, divergence)
         return self.target.download()
 
 
