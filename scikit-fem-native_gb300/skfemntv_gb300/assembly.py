@@ -17,6 +17,7 @@ matrices, fixed-order sums).
 from __future__ import annotations
 
 import ctypes
+import math
 import time
 from dataclasses import dataclass
 
@@ -611,7 +612,8 @@ class NativeCrossBilinearForm:
     def _affine_kind(self, kind, scalar):
         """Assembles ``kind`` straight from coordinates into the host matrix when
         its components fit, the bases share mesh and rule, the mesh is affine and the coefficient (broadcast
-        to (cell, point)) is constant on each element; else False."""
+        to (cell, point)) is finite and constant on each element; else False (a coefficient that is not finite
+        meets the zeros of the kind's tensor and the points' signs in the general path)."""
         tb, cb = self.test_basis, self.trial_basis
         Ct, Cc, d = self.test_components, self.trial_components, self.dimension
         code = {"value": 0, "gradient": 1, "row_divergence": 2, "column_divergence": 3}.get(kind)
@@ -625,10 +627,13 @@ class NativeCrossBilinearForm:
         d_coef, constant = None, 0.0
         if E == 0 or scalar.strides == (0, 0):
             constant = float(scalar[0, 0]) if E else 0.0
+            if not math.isfinite(constant):
+                return False
         else:
             pe = per_element(scalar, E, Q, kind)
-            if pe is None:
-                return False
+            with np.errstate(all="ignore"):
+                if pe is None or not math.isfinite(pe.sum()):
+                    return False
             d_coef = dev.to_device(pe, np.float64)
         mesh = tb.mesh
         call("skg_cross_assemble_affine", self.pattern.h, dev.ptr(mesh._dev("p")), mesh.p.shape[1],
