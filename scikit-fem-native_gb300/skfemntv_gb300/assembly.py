@@ -444,9 +444,9 @@ class NativeBilinearForm:
         if fast is not None:
             self._affine(fast, _precision(precision), self.target.pinned_ptr(), host=True)
             return self.target.finish_direct()
+        forms = self._affine_forms(value, gradient, symmetric_gradient, divergence)
         if _precision(precision) != SKG_FP64:
             raise UnsupportedNativeForm("split precision is available on the affine scalar gradient path")
-        forms = self._affine_forms(value, gradient, symmetric_gradient, divergence)
         if forms is not None:
             self._affine_forms_launch(forms, dev.ptr(self.target.d_values), self.target.pinned_ptr())
             return self.target.finish_direct()
