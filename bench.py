@@ -14,7 +14,7 @@ A = Q diag(exp(N(0, 0.5^2))) Q^T, 4-point quadrature (seeded synthetic data).
          read from host memory (by the element kernel over NVLink-C2C on
          Grace-Blackwell) and the CSR values land in the page-locked buffer
          behind the returned scipy matrix, copied in row chunks while the
-         row pass runs.
+         sums run.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 

@@ -84,7 +84,9 @@ typedef struct skg_pattern skg_pattern;
  * element-major (the reference's `dofs (E, nodes, components)`).  n_rows /
  * n_cols: matrix shape (rows must exceed every row dof).  With d_col_dofs
  * NULL only the row incidence lists are built (nnz = 0): the handle then
- * serves vector (linear-form) assembly.  Synchronous. */
+ * serves vector (linear-form) assembly.  Rows and columns with the same DOFs, in
+ * one array or two (two up to 12 per element), get the plan of the symmetric
+ * sums, which the assemblies of symmetric forms use.  Synchronous. */
 int skg_pattern_create(const int32_t *d_row_dofs, const int32_t *d_col_dofs,
                        int64_t n_elements, int32_t row_local, int32_t col_local,
                        int64_t n_rows, int64_t n_cols, void *stream,

@@ -30,13 +30,13 @@
 //
 // Precision modes.
 //  SKG_FP64           FP64 end to end (FP64 pipe).
-//  SKG_FP64_EMULATED  element pass and row pass in double-float (FP32 pairs,
-//                     error-free transformations; ~48-bit significands) and
-//                     slot sums in double-float, converted to FP64 exactly:
+//  SKG_FP64_EMULATED  element pass in double-float (FP32 pairs, error-free
+//                     transformations; ~48-bit significands) and sums in
+//                     double-float, converted to FP64 exactly:
 //                     FP64-accurate (1e-12 class) on the FP32 pipe.
 //  SKG_SPLIT_FP32     double-float element pass (FP64-class G), element
 //                     contraction in FP32 with split hi/lo products and FP32
-//                     accumulation, double-float slot sums.
+//                     accumulation, double-float sums.
 // The FP32-pair modes work in units scaled by 2^-s (s from the largest
 // vertex coordinate) so FP32 range holds; a mesh or coefficient outside that
 // range is detected in the element pass and re-run in FP64.
@@ -694,8 +694,8 @@ __global__ void __launch_bounds__(kRowWarps * 32) k_rows_group(
 // ------------------------------------------- element matrices, double-float
 // The double-float mode of P2 with an exact rule: the element pass evaluates
 // K_ab = sum t30 G/30 (integer factors, double-float G) once per entry (upper
-// triangle for a symmetric coefficient) and stores the 10 x 10 matrix as FP32
-// (hi, lo) pairs; the row pass adds rows into double-float slots.
+// triangle for a symmetric coefficient) and stores the packed triangle as FP32
+// (hi, lo) pairs; the pair sums add them in double-float.
 
 template <int I, int N, class F>
 __device__ __forceinline__ void static_for(F &&f) {
@@ -883,7 +883,7 @@ __device__ __forceinline__ bool tile_symmetric(bool sym, int64_t tile, const Pac
 // from the integer table with compile-time factors and shared sums
 // (shared_entry), else from the rule's table in shared memory.  Each entry is
 // stored as it is computed, so no entry array is held in registers or staged.
-// Bound by the FP64 pipe: 169 instructions per element, about 110 of them for
+// Bound by the FP64 pipe: 166 instructions per element, about 110 of them for
 // G: 469 us at 64^3, 90 % of the pipe's rate (with DADD / DMUL instead of
 // skg_fp64.cuh 507 us; with the 64 registers of an unbounded launch, which
 // recomputes, 534 us; four blocks per SM leave it 128).
@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(kTile, 4) k_elem_packed(int64_t ne, int64_t e_
 // in double-float, the entries from the integer table (exact_entry_sym for a
 // symmetric coefficient) summed error-free in double-float (MODE_DF64, stored
 // as (hi, lo) pairs) or in FP32 with split products (MODE_SPLIT, rounded to
-// FP32), each stored to the stage as it is computed.
+// FP32), each stored as it is computed.
 template <int MODE>
 __global__ void __launch_bounds__(kTile) k_elem_packed_df(
     int64_t ne, int64_t e_begin, int64_t e_end, const double *__restrict__ p, int64_t npts, const int32_t *__restrict__ t, int coef_kind,
@@ -1240,7 +1240,7 @@ void affine_assemble_pairs(const skg_pattern *pat, const double *d_p, int64_t np
 
 // Shared by the C ABI entry points below.
 // h_values (optional, page-locked host): the values also go there, copied in
-// row chunks overlapping the row pass (run_row_pass).
+// row chunks overlapping the passes (run_pair_passes, run_row_pass).
 void affine_assemble(const skg_pattern *pat, const double *d_p, int64_t npts, const int32_t *d_t, int32_t nodes,
                      int64_t ne, int32_t nq, const double *h_X, const double *h_W, int32_t coef_kind,
                      const double *d_coef, int32_t precision, double *d_values, cudaStream_t s, cudaEvent_t *ev,
@@ -1391,9 +1391,10 @@ extern "C" int skg_h1_assemble_affine_profiled(const skg_pattern *pat, const dou
 // all device memory to their own pool allocator at start-up and forbid other
 // allocations, and time-stepping solvers that re-assemble inside a loop where
 // a cudaMalloc / cudaFree (which may synchronise the device) is not allowed.
-// This entry point computes exactly what skg_h1_assemble_affine computes, with
-// the same kernels, but its scratch (per-element G, the quadrature table, the
-// scale exponent and the range flag) lives in one file-scope device array of
+// This entry point computes what skg_h1_assemble_affine computes, to rounding:
+// per-element G and rows evaluated from it (the kernels of the patterns without a
+// pair plan), so that its scratch (per-element G, the quadrature table, the
+// scale exponent and the range flag) fits one file-scope device array of
 // fixed size instead of stream-ordered allocations.  The array is part of the
 // library's device image, so every GPU on which the library is loaded holds it
 // (kNoAllocBytes) until the process exits.

@@ -197,10 +197,10 @@ struct PairStep {
     int64_t ready = 0;
 };
 
-// A host-output chunk: rows [row0, row1), CSR positions [slot0, slot1), complete
+// A host-output chunk of rows: CSR positions [slot0, slot1), complete
 // once the slices below `slice` are summed.
 struct PairCopy {
-    int32_t row0 = 0, row1 = 0, slot0 = 0, slot1 = 0, slice = 0;
+    int32_t slot0 = 0, slot1 = 0, slice = 0;
 };
 
 // Contributions of the node pairs of a symmetric pattern (skg_pairs.cuh).

@@ -367,8 +367,6 @@ PairPlan build(const skg_pattern *p, cudaStream_t s) {
         download(h, chunk.get(), 3 * (kHostChunks + 1), s);
         for (int k = 0; k < n_chunks; ++k) {
             PairCopy c;
-            c.row0 = C * h[k];
-            c.row1 = k + 1 < n_chunks ? C * h[k + 1] : (int32_t)p->n_rows;
             c.slot0 = h[kHostChunks + 1 + k];
             c.slot1 = k + 1 < n_chunks ? h[kHostChunks + 2 + k] : (int32_t)p->nnz;
             c.slice = h[2 * (kHostChunks + 1) + k] * (kPairWindow / 32);

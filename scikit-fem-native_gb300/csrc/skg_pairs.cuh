@@ -11,12 +11,12 @@
 // additions: bitwise reproducible.
 //
 // Why pairs: an FP64 instruction costs the pipe the same for 1 lane as for 32
-// (9.3 ns per DADD and SM, measured for 1 to 32 active lanes), and walking the
+// (9.3 to 9.7 ns per DADD, warp and SM, for 1 to 32 active lanes), and walking the
 // rows' incidences issues additions for warps whose rows end at different
 // times, with a load and a store of shared memory for each.  A pair needs one
 // addition less than it has contributions, in nearly full warps, and half of
-// the entries are neither stored, loaded nor added: 35 FP64 additions per P2
-// element at 64^3 instead of 95, 440 bytes per element matrix instead of 800.
+// the entries are neither stored, loaded nor added: 42 FP64 additions per P2
+// element (32^3, counted) instead of 95, 440 bytes per element matrix instead of 800.
 //
 // Slices: the pairs are taken in row order in windows of kPairWindow; inside a
 // window they are sorted by their number of contributions, so that the 32
@@ -236,7 +236,6 @@ inline void pair_sum(const PairPlan &plan, int s0, int s1, const E *K, const Pai
 // 32 elements are one contiguous, 16-byte aligned range.  A block of threads
 // per slice, nine threads per pair.
 constexpr int kPairBlock3 = 288;
-constexpr int kPairStage = 32;  // contributions per pair whose codes are staged together
 
 __global__ void __launch_bounds__(kPairBlock3) k_pair_sum3(int s0, PairArrays p, const double *__restrict__ K,
                                                            double *__restrict__ values);

@@ -53,8 +53,8 @@ class Pattern:
         self.n_rows, self.n_cols = n_rows, n_cols
         mrl = ctypes.c_int32(0)
         call("skg_pattern_row_groups", h, ctypes.byref(mrl))
-        # the fixed-order row-group passes (and their chunked host outputs) serve
-        # this pattern; otherwise assemblies gather per row from global memory
+        # the fixed-order row-group passes (and their chunked host outputs) can serve
+        # this pattern, beside the pair sums
         self.row_groups = mrl.value > 0
 
     def device_csr(self):
@@ -303,7 +303,7 @@ class NativeBilinearForm:
             if coef is None:
                 keep = dev.to_device(fast, np.float64)
                 coef = dev.ptr(keep)
-        if host:  # values to the host matrix: copies overlap the row pass
+        if host:  # values to the host matrix: copies overlap the sums
             call("skg_h1_assemble_affine_host", self.pattern.h, dev.ptr(b.mesh._dev("p")), b.mesh.p.shape[1],
                  dev.ptr(b.mesh._dev("t")), b._nodes, E, Q, dev.hptr(b.X),
                  dev.hptr(b.W), 0, coef, prec, dev.ptr(self.target.d_values), out, dev.stream_ptr())
@@ -497,7 +497,7 @@ class NativeTensorForm:
                     keep = self._staging.upload(arr)
                     coef = dev.ptr(keep)
         if coef is not None:
-            if out is not None:  # values to the host matrix: copies overlap the row pass
+            if out is not None:  # values to the host matrix: copies overlap the sums
                 call("skg_h1_assemble_affine_host", self.pattern.h, dev.ptr(b.mesh._dev("p")), b.mesh.p.shape[1],
                      dev.ptr(b.mesh._dev("t")), b._nodes, E, Q, dev.hptr(b.X),
                      dev.hptr(b.W), kind, coef, prec, dev.ptr(self.target.d_values), out, dev.stream_ptr())
