@@ -278,7 +278,7 @@ FP64_PROFILE = {
     "dram_bytes_64": {"k_elem_packed": 693509233.8, "k_pair_sum": 1790956278.5},
 }
 # The plain neo-Hookean call: element blocks k_nh_packed, pair sums k_pair_sum3, residual gather.
-NH_FP64_OPS_PER_ELEMENT = 352.0 + 81.3 + 12.0
+NH_FP64_OPS_PER_ELEMENT = 426.0 + 81.3 + 12.0
 
 
 def fp64_roof(call, passes, elements):
