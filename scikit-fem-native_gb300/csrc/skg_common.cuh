@@ -205,8 +205,8 @@ struct PairCopy {
 
 // Contributions of the node pairs of a symmetric pattern (skg_pairs.cuh).
 struct PairPlan {
-    int32_t block = 0;  // components per node: 1 or 3; 0: no plan
-    int32_t nodes = 0;  // local nodes n
+    int32_t block = 0;  // components per pair: 1 or 3; 0: no plan
+    int32_t nodes = 0;  // local nodes n; 12 with block 1: the DOFs of four nodes' 3 x 3 blocks
     int32_t np = 0;     // n (n + 1) / 2 packed node blocks per element
     int32_t n_slices = 0;
     DevBuf<unsigned char> store;  // the arrays below

@@ -409,10 +409,9 @@ void affine_forms_assemble(const skg_pattern *pat, const double *d_p, int64_t np
             k_form_scalar<10><<<grid_for(e1 - e0, kTile), kTile, 0, s>>>(ne, e0, e1, stride, d_p, npts, d_t, fc, tab, Ke.get());
         SKG_LAUNCH_CHECK("form");
     };
-    if (pat->pairs.block == comp && pat->pairs.nodes == nodes) {
+    if (comp == 3 ? has_block_plan(pat, nodes) : pat->pairs.block == 1 && pat->pairs.nodes == nodes) {
         run_pair_passes(pat, ne, d_values, h_values, s, elem, [&](int s0, int s1, cudaStream_t st) {
-            if (comp == 3) pair_sum3(pat->pairs, s0, s1, Ke.get(), d_values, st);
-            else pair_sum<double>(pat->pairs, s0, s1, Ke.get(), PairLower<double>{}, PairIdentity{}, nullptr, d_values, st);
+            block_sums(pat->pairs, s0, s1, Ke.get(), d_values, st);
         });
         return;
     }

@@ -600,9 +600,12 @@ __device__ __forceinline__ bool surrogate_finish(const SurState &st, const float
                 const float f = w1 * Fg[b][i], h = w2 * hg[b][i];
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
+                    if (a == b && k < i) continue;  // diagonal block: symmetric
                     float v = X[i] * Fg[b][k] + Y[i] * Dg[b][k] + Z[i] * hg[b][k];
                     v -= f * Fg[a][k] + h * hg[a][k] + q * FFt[i * 3 + k];
-                    block(a, b, i, k, i == k ? v + diag : v);
+                    if (i == k) v += diag;
+                    block(a, b, i, k, v);
+                    if (a == b && k > i) block(a, b, k, i, v);
                 }
             }
         }
@@ -663,11 +666,17 @@ __device__ __forceinline__ void surrogate_fallback_packed(int64_t e, int64_t str
             for (int i = 0; i < 3; ++i)
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
+                    if (a == b && k < i) continue;  // diagonal block: symmetric
                     const double v =
                         g.V * ((i == k ? mu * gg : 0.0) + c2 * h[b][i] * h[a][k] + lmbda * h[a][i] * h[b][k]);
-                    const float hi = (float)v;
+                    const float hi = (float)v, lo = (float)(v - (double)hi);
+                    const int64_t at = tri_index(4, a, b) * stride + e;
                     out[tri_index(4, a, b) * kFinishStage + i * 3 + k] = hi;
-                    blk.K_low[(tri_index(4, a, b) * stride + e) * 9 + i * 3 + k] = (float)(v - (double)hi);
+                    blk.K_low[at * 9 + i * 3 + k] = lo;
+                    if (a == b && k > i) {
+                        out[tri_index(4, a, b) * kFinishStage + k * 3 + i] = hi;
+                        blk.K_low[at * 9 + k * 3 + i] = lo;
+                    }
                 }
         }
 }
@@ -1375,7 +1384,7 @@ void nh_assemble_surrogate(const skg_pattern *pat, const double *d_p, int64_t np
     d_u = device_resident(d_u, pat->n_rows, u_stage, s);
     DevBuf<unsigned long long> fb(2, s);  // [0] fallback elements, [1] tensor-core waits given up
     SKG_CUDA(cudaMemsetAsync(fb.get(), 0, 16, s));
-    if (d_values && pat->pairs.block == 3) {  // network on the tensor cores, pair sums
+    if (d_values && has_block_plan(pat, 4)) {  // network on the tensor cores, pair sums
         const int64_t stride = block_stride(ne);
         DevBuf<float> K((size_t)stride * 90, s), K_low((size_t)stride * 90, s), re((size_t)ne * 24, s);
         DevBuf<float> net((size_t)ne * kNetOut, s), geo((size_t)ne * kGeoRec, s);

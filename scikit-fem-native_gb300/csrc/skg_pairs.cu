@@ -82,11 +82,14 @@ __global__ void k_expand_blocks(int64_t ne, int64_t stride, int n, const double 
     full[i] = K[(t * stride + e) * 9 + (a <= b ? x * 3 + y : y * 3 + x)];
 }
 
-// Node-level view of a pattern with C components per node (C = 1: its DOFs);
-// C = 0: the DOFs of a pattern whose element matrices are summed whole.
+// Node-level view of a pattern, by kind of plan.  1: DOFs of a symmetric
+// pattern; 3: nodes of three components; 2: the DOFs of four nodes of three
+// components that are not numbered node by node, whose pairs are entries of
+// the nodes' packed blocks; 0: DOFs of a pattern whose element matrices are summed
+// whole.
 template <int K>
 struct NodeView {
-    static constexpr int C = K == 0 ? 1 : K;
+    static constexpr int C = K == 3 ? 3 : 1;
     const int32_t *cols, *indptr, *indices, *inc_ptr, *inc;
     int32_t L, Lc, n;  // local rows, local columns, local column nodes
     __device__ int32_t node(int64_t e, int b) const { return cols[e * Lc + C * b] / C; }
@@ -263,6 +266,14 @@ __global__ void __launch_bounds__(kPairWindow) k_pair_fill(NodeView<K> v, const 
     if (j >= 0) {
         const int32_t r = pair_row[j], c = pair_column(v, r, j, pair_ptr);
         each_contribution(v, r, c, [&](int32_t e, int a, int b) {
+            if (K == 2) {  // entry (x, y) of block (na, nb), or (y, x) of block (nb, na)
+                const int na = a / 3, nb = b / 3, x = a - 3 * na, y = b - 3 * nb;
+                const uint32_t t = (uint32_t)tri_index(4, min(na, nb), max(na, nb));
+                codes[(int64_t)k * 32 + lane] =
+                    (t * (uint32_t)stride + (uint32_t)e) * 9u + (uint32_t)(na <= nb ? 3 * x + y : 3 * y + x);
+                ++k;
+                return;
+            }
             const uint32_t t = (uint32_t)(K == 0 ? a * v.n + b : tri_index(v.n, min(a, b), max(a, b)));
             codes[(int64_t)k * 32 + lane] =
                 K == 0 ? (uint32_t)e * (uint32_t)np + t
@@ -404,8 +415,9 @@ void expand_blocks(int64_t ne, int n, const double *K, double *full, cudaStream_
 }
 
 // Plans of a pattern: the pair plan when its row and column DOFs are the same
-// (`square`) and its shape is one that is assembled symmetric; the whole
-// sums for the shapes that no row group serves.  None when the positions exceed
+// (`square`) and its shape is one that is assembled symmetric (four nodes of
+// three components in any numbering, by entries where it is not node by node);
+// the whole sums for the shapes that no row group serves.  None when the positions exceed
 // 32 bits (the assemblies then walk the rows).
 void build_pair_plan(skg_pattern *p, bool square, cudaStream_t s) {
     if (p->n_rows == 0 || p->n_elements == 0) return;
@@ -427,6 +439,7 @@ void build_pair_plan(skg_pattern *p, bool square, cudaStream_t s) {
             p->pairs = build<3>(p, s);
             return;
         }
+        if (L == 12 && block_stride(p->n_elements) * 90 < (int64_t)kPairNone) p->pairs = build<2>(p, s);
     }
     const bool grouped = p->max_row_len > 0 && L == p->col_local && (L == 4 || L == 6 || L == 10 || L == 12);
     if (!grouped && p->n_elements * L * (int64_t)p->col_local < (int64_t)kPairNone) p->whole = build<0>(p, s);

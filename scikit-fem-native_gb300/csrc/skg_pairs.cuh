@@ -250,6 +250,18 @@ inline void pair_sum3(const PairPlan &plan, int s0, int s1, const double *K, dou
     SKG_LAUNCH_CHECK("pair_sum3");
 }
 
+// A plan of the packed 3 x 3 blocks of `nodes` nodes: by pairs of nodes, or (four
+// nodes) by pairs of DOFs that are not numbered node by node.
+inline bool has_block_plan(const skg_pattern *pat, int nodes) {
+    return (pat->pairs.block == 3 && pat->pairs.nodes == nodes) ||
+           (nodes == 4 && pat->pairs.block == 1 && pat->pairs.nodes == 12);
+}
+
+inline void block_sums(const PairPlan &plan, int s0, int s1, const double *K, double *values, cudaStream_t s) {
+    if (plan.block == 3) pair_sum3(plan, s0, s1, K, values, s);
+    else pair_sum<double>(plan, s0, s1, K, PairLower<double>{}, PairIdentity{}, nullptr, values, s);
+}
+
 // ----------------------------------------------------------------- passes
 
 // Element pass and pair sums; elem(e0, e1) launches the element pass over
